@@ -21,13 +21,24 @@ template <int MODE>
 __device__ __forceinline__ void route_token(const float* __restrict__ row, int64_t stride_s, int splits,
                                             const float* __restrict__ bias, int num_experts, float scale, int lane,
                                             float (&w)[4], int (&sel_id)[4]) {
-  float score[4], choice[4];
+  float score[4], choice[4], sum4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  for (int s0 = 0; s0 < splits; s0 += 4) {  // 16 independent loads in flight, added in split order
+    float v[4][4];
+#pragma unroll
+    for (int s = 0; s < 4; ++s)
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (s0 + s < splits && lane + 32 * j < num_experts) v[s][j] = __ldcg(row + (s0 + s) * stride_s + lane + 32 * j);
+#pragma unroll
+    for (int s = 0; s < 4; ++s)
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (s0 + s < splits && lane + 32 * j < num_experts) sum4[j] = sum4[j] + v[s][j];
+  }
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     const int e = lane + 32 * j;
-    float acc = 0.0f;
-    if (e < num_experts)
-      for (int s = 0; s < splits; ++s) acc = acc + row[s * stride_s + e];
+    const float acc = sum4[j];
     if (MODE == B200MOE_ROUTE_SIGMOID_BIAS) {
       score[j] = 1.0f / (1.0f + expf(-acc));
       choice[j] = score[j] + (bias && e < num_experts ? bias[e] : 0.0f);
