@@ -27,6 +27,19 @@ class Weights(Structure):
                 ("gate_split", c_void_p)]
 
 
+class SharedWeights(Structure):
+    """struct b200moe_shared_weights"""
+    _fields_ = [("w13t", c_void_p), ("w2t", c_void_p)]
+
+
+class Prepared(Structure):
+    """struct b200moe_prepared"""
+    _fields_ = [("codes4", c_void_p), ("scales4", c_void_p), ("topk_weights", c_void_p), ("topk_ids", c_void_p),
+                ("codes8", c_void_p), ("scales8", c_void_p), ("mask4", c_void_p)]
+
+
+LAYER_ROUTER, LAYER_SHARED, LAYER_OWN_SLOTS, LAYER_OWN_SHARED_OUT, LAYER_COMPACT = 1, 2, 4, 8, 16
+
 _P = c_void_p
 SIGNATURES = {
     "b200moe_version": (c_int, []),
@@ -84,6 +97,11 @@ SIGNATURES = {
     "b200moe_router_gemm_quant": (c_int, [_P, _P, c_int64, c_int, c_int, _P, _P, _P, _P, _P, _P]),
     "b200moe_workspace_bytes": (c_size_t, [c_int64, c_int]),
     "b200moe_workspace_bytes_x": (c_size_t, [c_int64, c_int]),
+    "b200moe_layer_workspace_bytes": (c_size_t, [c_int64, c_int, c_int]),
+    "b200moe_layer": (c_int, [POINTER(Weights), POINTER(SharedWeights), _P, _P, c_int64, _P, c_size_t, _P, _P, _P, _P, _P]),
+    "b200moe_layer_prepared": (c_int, [POINTER(Weights), POINTER(SharedWeights), POINTER(Prepared), c_int64, _P, c_size_t, _P,
+                                       _P, _P, _P, _P]),
+    "b200moe_prepare": (c_int, [POINTER(Weights), _P, c_int64, _P, _P, _P, _P, _P, _P, _P, _P, _P]),
     "b200moe_forward_x": (c_int, [POINTER(Weights), _P, c_int64, _P, c_size_t, _P, _P, _P, _P]),
     "b200moe_set_wait_limit_ns": (c_int, [c_uint64]),
     "b200moe_route_sort_partials": (c_int, [_P, c_int64, c_int64, c_int, _P, c_int64, c_int, c_int, c_float, c_int, _P, _P,

@@ -1,5 +1,6 @@
 // Library identity, workspace carving and the whole-layer entry points.
 #include "common.cuh"
+#include "shared_role.cuh"
 
 namespace b200moe {
 
@@ -17,32 +18,54 @@ struct Workspace {
   uint8_t* sfx;           // [R/bm][48][512]
   uint8_t* hq;            // [R][384]
   uint8_t* sfh;           // [R/bm][6][512]
-  int32_t* done;          // [R/bm] GEMM1 tiles finished per row block (one-launch GEMM1+GEMM2)
-  // only with the router inside the call (b200moe_forward_x):
+  int32_t* done;          // [R/bm] GEMM1 tiles finished per row block, then [8]: the shared expert's per block of tokens
+  // only with the router inside the call:
   float* partials;        // [S][T][E] split-K logit partials
-  uint8_t* q4;            // [T][3072] row-major MXFP4 codes of x
+  uint8_t* q4;            // [T][3072] row-major MXFP4 codes of x (also rebuilt from a compact prepared input)
   uint8_t* s4;            // [T][192] their scales
+  // only with the shared expert:
+  SharedWorkspace sh;
+  // results the caller does not take:
+  __nv_bfloat16* shared_out;  // [T][6144]
+  __nv_bfloat16* slots;       // [T][4][6144]
   size_t bytes;
   int bm;
   int64_t rows;
 };
+constexpr int kSharedDone = 8;  // blocks of shared-expert tokens a decode launch may count (512 tokens in blocks of 128: 4)
 
 int dispatch_rows_done(const uint8_t* codes, const uint8_t* scales, const int32_t* sorted_ids, const int32_t* num_valid,
                        int64_t tokens, int bm, int by_pair, int64_t max_rows, uint8_t* xq_sorted, uint8_t* sfx,
-                       int32_t* done, void* stream);
+                       int32_t* done, int n_done, void* stream);
+int quant_dispatch_done(const void* x_bf16, const int32_t* sorted_ids, const int32_t* num_valid, int64_t tokens, int bm,
+                        int64_t max_rows, uint8_t* xq_sorted, uint8_t* sfx, int32_t* done, int n_done, void* stream);
 int prep_small(const float* partials, int64_t stride_t, int64_t stride_s, int splits, const float* bias, int64_t tokens,
                int num_experts, int mode, float scale, int bm, float* out_w, int32_t* out_ids, int32_t* sorted_ids,
                float* sorted_w, int32_t* block_expert, int32_t* num_valid, const void* x_bf16, const uint8_t* q4,
                const uint8_t* s4, int64_t max_rows, uint8_t* xq_sorted, uint8_t* sfx, int32_t* done, int n_done,
                void* stream);
 int quant_rows(const void* x_bf16, int64_t tokens, uint8_t* codes, uint8_t* scales, void* stream);
+int quant_rows_both(const void* x_bf16, int64_t tokens, uint8_t* codes, uint8_t* scales, uint8_t* codes8, uint8_t* scales8,
+                    uint8_t* atoms8, int bm8, void* stream);
+int router_gemm_quant(const void* x_bf16, const float* gate, int64_t tokens, int num_experts, int splits, float* partials,
+                      uint8_t* codes4, uint8_t* scales4, uint8_t* codes8, uint8_t* scales8, uint8_t* atoms8, int bm8,
+                      void* stream);
+int gemm12_beside(const uint8_t* w13t, const uint8_t* w2t, int num_experts, const uint8_t* xq_sorted, const uint8_t* sfx,
+                  const int32_t* block_expert, const int32_t* num_valid, const int32_t* sorted_ids, const float* sorted_w,
+                  int64_t max_rows, int bm, int64_t tokens, uint8_t* hq, uint8_t* sfh, int32_t* done, void* slots_bf16,
+                  int32_t* status, const SharedPlan* sp, void* stream);
+int gemm1_beside(const uint8_t* w13t, int num_experts, const uint8_t* xq_sorted, const uint8_t* sfx,
+                 const int32_t* block_expert, const int32_t* num_valid, int64_t max_rows, int bm, uint8_t* hq, uint8_t* sfh,
+                 const uint8_t* prefetch_w2t, int32_t* status, const SharedPlan* sp, void* stream);
+int shared_gemms(const uint8_t* w13t, const uint8_t* w2t, const uint8_t* codes8, int64_t code_rows, const SharedWorkspace& ws,
+                 void* out_bf16, int64_t tokens, int32_t* status, void* stream);
 int set_wait_limit_routed(unsigned long long ns);
 int set_wait_limit_shared(unsigned long long ns);
 int set_wait_limit_pair(unsigned long long ns);
 int set_wait_limit_router(unsigned long long ns);
 int set_wait_limit_ep_sync(unsigned long long ns);
 
-static Workspace carve(uint8_t* base, int64_t tokens, int num_experts, bool with_router = false) {
+static Workspace carve(uint8_t* base, int64_t tokens, int num_experts, int flags) {
   Workspace ws{};
   ws.bm = b200moe_block_rows(tokens);
   ws.rows = b200moe_max_sorted_rows(tokens, ws.bm, num_experts);
@@ -60,17 +83,26 @@ static Workspace carve(uint8_t* base, int64_t tokens, int num_experts, bool with
   ws.block_expert = reinterpret_cast<int32_t*>(take(blocks * 4));
   ws.num_valid = reinterpret_cast<int32_t*>(take(16));
   ws.scratch = reinterpret_cast<int32_t*>(take(b200moe_permute_scratch_bytes(tokens, num_experts) + 16));
-  ws.xq_sorted = take(ws.rows * (kH / 2));
-  ws.sfx = take(blocks * (kH / 128) * kAtomBytes);
+  if (ws.bm < 128) {  // at block height 128 GEMM1 gathers its rows itself
+    ws.xq_sorted = take(ws.rows * (kH / 2));
+    ws.sfx = take(blocks * (kH / 128) * kAtomBytes);
+  }
   ws.hq = take(ws.rows * (kI / 2));
   ws.sfh = take(blocks * (kI / 128) * kAtomBytes);
-  ws.done = reinterpret_cast<int32_t*>(take(blocks * 4));
-  if (with_router)
+  ws.done = reinterpret_cast<int32_t*>(take((blocks + kSharedDone) * 4));
+  if (flags & B200MOE_LAYER_ROUTER)
     ws.partials = reinterpret_cast<float*>(take(static_cast<size_t>(b200moe_router_splits(tokens)) * tokens * num_experts * 4));
-  if (with_router || ws.bm == 128) {  // row-major quantised tokens: the router path always, the logits path at prefill sizes
+  if ((flags & (B200MOE_LAYER_ROUTER | B200MOE_LAYER_COMPACT)) || ws.bm == 128) {
     ws.q4 = take(tokens * (kH / 2));
     ws.s4 = take(tokens * (kH / 32));
   }
+  if (flags & B200MOE_LAYER_SHARED) {
+    ws.sh = carve_shared(nullptr, tokens);
+    uint8_t* p = take(ws.sh.bytes);
+    if (p) ws.sh = carve_shared(p, tokens);
+    if (flags & B200MOE_LAYER_OWN_SHARED_OUT) ws.shared_out = reinterpret_cast<__nv_bfloat16*>(take(tokens * kH * 2));
+  }
+  if (flags & B200MOE_LAYER_OWN_SLOTS) ws.slots = reinterpret_cast<__nv_bfloat16*>(take(tokens * kTopK * kH * 2));
   ws.bytes = off;
   return ws;
 }
@@ -80,14 +112,17 @@ static Workspace carve(uint8_t* base, int64_t tokens, int num_experts, bool with
 extern "C" int b200moe_version(void) { return 1; }
 extern "C" const char* b200moe_arch(void) { return "sm_100a"; }
 
-extern "C" size_t b200moe_workspace_bytes(int64_t tokens, int num_experts) {
+extern "C" size_t b200moe_layer_workspace_bytes(int64_t tokens, int num_experts, int flags) {
   if (tokens < 1 || tokens > B200MOE_MAX_TOKENS || num_experts < 1 || num_experts > b200moe::kMaxE) return 0;
-  return b200moe::carve(nullptr, tokens, num_experts).bytes;
+  return b200moe::carve(nullptr, tokens, num_experts, flags).bytes;
+}
+
+extern "C" size_t b200moe_workspace_bytes(int64_t tokens, int num_experts) {
+  return b200moe_layer_workspace_bytes(tokens, num_experts, 0);
 }
 
 extern "C" size_t b200moe_workspace_bytes_x(int64_t tokens, int num_experts) {
-  if (tokens < 1 || tokens > B200MOE_MAX_TOKENS || num_experts < 1 || num_experts > b200moe::kMaxE) return 0;
-  return b200moe::carve(nullptr, tokens, num_experts, true).bytes;
+  return b200moe_layer_workspace_bytes(tokens, num_experts, B200MOE_LAYER_ROUTER);
 }
 
 extern "C" int b200moe_set_wait_limit_ns(uint64_t ns) {
@@ -101,113 +136,190 @@ extern "C" int b200moe_set_wait_limit_ns(uint64_t ns) {
 }
 
 namespace b200moe {
-constexpr int64_t kSmallTokens = 32;  // up to here a layer call is three launches: preparation, both GEMMs, reduce
-// sorted, gathered, quantised rows are in the workspace: the grouped GEMMs and the reduce
-static int experts_and_reduce(const b200moe_weights* w, const Workspace& ws, int64_t tokens, void* slots_bf16,
-                              void* out_bf16, int32_t* status, void* stream) {
+constexpr int64_t kSmallTokens = 32;  // up to here a layer call is three launches (and the router): preparation, GEMMs, reduce
+
+// One call of the layer, in any of its forms.
+struct LayerCall {
+  const b200moe_weights* w;
+  const b200moe_shared_weights* shared;  // null: routed experts only
+  const void* x;                         // bf16 rows, or (null) a prepared input:
+  const b200moe_prepared* prep;
+  const float* logits;                   // with x: plain logits, null: the router runs inside the call
+  int64_t tokens;
+  void* workspace;
+  size_t workspace_bytes;
+  void *slots, *shared_out, *out;
+  int32_t* status;
+  void* stream;
+};
+
+static int run_layer(const LayerCall& c) {
+  const b200moe_weights* w = c.w;
+  if (!w || !c.workspace || !c.status || (!c.x == !c.prep) || (!c.slots && !c.out)) return B200MOE_E_ARG;
+  if (c.tokens < 1 || c.tokens > B200MOE_MAX_TOKENS) return B200MOE_E_ARG;
+  const bool shared = c.shared != nullptr, router = c.x && !c.logits, compact = c.prep && c.prep->mask4;
+  if (router && !w->gate) return B200MOE_E_ARG;
+  if (shared && (!c.shared->w13t || !c.shared->w2t || (!c.shared_out && !c.out))) return B200MOE_E_ARG;
+  if (c.prep && (!c.prep->scales4 || !c.prep->topk_weights || !c.prep->topk_ids || (!c.prep->codes4 && !compact) ||
+                 ((shared || compact) && (!c.prep->codes8 || !c.prep->scales8))))
+    return B200MOE_E_ARG;
+  if (reinterpret_cast<uintptr_t>(c.workspace) & 255) return B200MOE_E_ALIGN;
+  if (shared && ((reinterpret_cast<uintptr_t>(c.shared->w13t) | reinterpret_cast<uintptr_t>(c.shared->w2t) |
+                  reinterpret_cast<uintptr_t>(c.shared_out)) & 15))
+    return B200MOE_E_ALIGN;
+  if (c.prep && ((reinterpret_cast<uintptr_t>(c.prep->codes4) | reinterpret_cast<uintptr_t>(c.prep->codes8)) & 15))
+    return B200MOE_E_ALIGN;
   const int ne = w->num_experts;
-  int r;
-  if (tokens <= kSmallTokens) {  // small batches: both grouped GEMMs in one persistent launch (measured faster there only)
-    if ((r = b200moe_gemm12(w->w13t, w->w2t, ne, ws.xq_sorted, ws.sfx, ws.block_expert, ws.num_valid, ws.sorted_ids,
-                            ws.sorted_w, ws.rows, ws.bm, tokens, ws.hq, ws.sfh, ws.done, slots_bf16, status, stream)))
-      return r;
+  const int64_t tokens = c.tokens;
+  void* st = c.stream;
+  int flags = 0;
+  if (router) flags |= B200MOE_LAYER_ROUTER;
+  if (compact) flags |= B200MOE_LAYER_COMPACT;
+  if (shared) flags |= B200MOE_LAYER_SHARED;
+  if (shared && !c.shared_out) flags |= B200MOE_LAYER_OWN_SHARED_OUT;
+  if (!c.slots) flags |= B200MOE_LAYER_OWN_SLOTS;
+  const Workspace ws = carve(static_cast<uint8_t*>(c.workspace), tokens, ne, flags);
+  if (c.workspace_bytes < ws.bytes) return B200MOE_E_ARG;
+  void* slots = c.slots ? c.slots : ws.slots;
+  void* shared_out = c.shared_out ? c.shared_out : ws.shared_out;
+  const int blocks = static_cast<int>(ws.rows / ws.bm), n_done = blocks + (shared ? kSharedDone : 0);
+  const int splits = router ? b200moe_router_splits(tokens) : 1;
+  const float* partials = router ? ws.partials : c.logits;
+  const int64_t stride_s = router ? tokens * ne : 0;
+  const uint8_t *q4 = c.prep ? c.prep->codes4 : ws.q4, *s4 = c.prep ? c.prep->scales4 : ws.s4;
+  const uint8_t* codes8 = c.prep ? c.prep->codes8 : ws.sh.x8;
+  bool have_q4 = true;
+  int r = 0;
+
+  // the operands: quantised rows and, with the router inside, the logits' split-K partials
+  if (c.prep) {
+    if (compact) {
+      if ((r = b200moe_sidecar_unpack(c.prep->mask4, s4, codes8, c.prep->scales8, tokens, ws.q4, st))) return r;
+      q4 = ws.q4;
+    }
+    if (shared && (r = b200moe_scales_to_atoms(c.prep->scales8, tokens, kH / 32, ws.sh.bm, ws.sh.sfx8, st))) return r;
+  } else if (router && (tokens < 128 || !w->gate_split)) {  // one pass over x
+    r = router_gemm_quant(c.x, w->gate, tokens, ne, splits, ws.partials, ws.q4, ws.s4, shared ? ws.sh.x8 : nullptr, nullptr,
+                          shared ? ws.sh.sfx8 : nullptr, ws.sh.bm, st);
+    if (r) return r;
   } else {
-    if ((r = b200moe_gemm1_swiglu_quant(w->w13t, ne, ws.xq_sorted, ws.sfx, ws.block_expert, ws.num_valid, ws.rows, ws.bm,
-                                        ws.hq, ws.sfh, w->w2t, status, stream)))
+    if (router && (r = b200moe_router_gemm_tc(c.x, w->gate_split, tokens, ne, splits, ws.partials, c.status, st))) return r;
+    if (router || ws.bm == 128) {
+      r = shared ? quant_rows_both(c.x, tokens, ws.q4, ws.s4, ws.sh.x8, nullptr, ws.sh.sfx8, ws.sh.bm, st)
+                 : quant_rows(c.x, tokens, ws.q4, ws.s4, st);
+    } else {  // decode sizes with logits: the routed rows are quantised by the gather
+      have_q4 = false;
+      if (shared) r = b200moe_shared_quant(c.x, tokens, ws.sh.bm, ws.sh.x8, ws.sh.sfx8, st);
+    }
+    if (r) return r;
+  }
+  SharedPlan plan{};
+  const SharedPlan* sp = nullptr;
+  if (shared) {
+    if (ws.bm < 128) {  // decode sizes: a role of the launch that streams the routed experts' W13
+      if ((r = shared_plan(&plan, c.shared->w13t, c.shared->w2t, codes8, tokens, ws.sh, shared_out, tokens, ws.done + blocks)))
+        return r;
+      sp = &plan;
+    } else if ((r = shared_gemms(c.shared->w13t, c.shared->w2t, codes8, tokens, ws.sh, shared_out, tokens, c.status, st))) {
       return r;
+    }
+  }
+
+  // routing, sort, and at decode sizes the gather into sorted order
+  if (!c.prep && tokens <= kSmallTokens && ne >= 4) {  // one launch
+    r = prep_small(partials, ne, stride_s, splits, w->bias, tokens, ne, w->route_mode, w->route_scale, ws.bm, ws.w, ws.ids,
+                   ws.sorted_ids, ws.sorted_w, ws.block_expert, ws.num_valid, have_q4 ? nullptr : c.x,
+                   have_q4 ? q4 : nullptr, have_q4 ? s4 : nullptr, ws.rows, ws.xq_sorted, ws.sfx, ws.done, n_done, st);
+    if (r) return r;
+  } else {
+    if (c.prep)
+      r = b200moe_permute(c.prep->topk_ids, c.prep->topk_weights, tokens, ne, ws.bm, ws.sorted_ids, ws.sorted_w,
+                          ws.block_expert, ws.num_valid, ws.scratch, st);
+    else
+      r = b200moe_route_sort_partials(partials, ne, stride_s, splits, w->bias, tokens, ne, w->route_mode, w->route_scale, ws.bm,
+                                      ws.w, ws.ids, ws.sorted_ids, ws.sorted_w, ws.block_expert, ws.num_valid, ws.scratch, st);
+    if (r) return r;
+    if (ws.bm < 128) {
+      r = have_q4 ? dispatch_rows_done(q4, s4, ws.sorted_ids, ws.num_valid, tokens, ws.bm, 0, ws.rows, ws.xq_sorted, ws.sfx,
+                                       ws.done, n_done, st)
+                  : quant_dispatch_done(c.x, ws.sorted_ids, ws.num_valid, tokens, ws.bm, ws.rows, ws.xq_sorted, ws.sfx, ws.done,
+                                        n_done, st);
+      if (r) return r;
+    }
+  }
+
+  // the routed experts
+  if (tokens <= kSmallTokens) {  // both grouped GEMMs in one persistent launch (measured faster there only)
+    r = gemm12_beside(w->w13t, w->w2t, ne, ws.xq_sorted, ws.sfx, ws.block_expert, ws.num_valid, ws.sorted_ids, ws.sorted_w,
+                      ws.rows, ws.bm, tokens, ws.hq, ws.sfh, ws.done, slots, c.status, sp, st);
+    if (r) return r;
+  } else {
+    if (ws.bm < 128)
+      r = gemm1_beside(w->w13t, ne, ws.xq_sorted, ws.sfx, ws.block_expert, ws.num_valid, ws.rows, ws.bm, ws.hq, ws.sfh, w->w2t,
+                       c.status, sp, st);
+    else  // GEMM1 gathers its token rows from the row-major quantised tokens by the sorted list
+      r = b200moe_gemm1_swiglu_quant_gather(w->w13t, ne, q4, s4, tokens, 0, ws.sorted_ids, ws.block_expert, ws.num_valid,
+                                            ws.rows, ws.hq, ws.sfh, c.status, st);
+    if (r) return r;
     if ((r = b200moe_gemm2_weighted(w->w2t, ne, ws.hq, ws.sfh, ws.block_expert, ws.num_valid, ws.sorted_ids, ws.sorted_w,
-                                    ws.rows, ws.bm, tokens, slots_bf16, status, stream)))
+                                    ws.rows, ws.bm, tokens, slots, c.status, st)))
       return r;
   }
-  if (out_bf16 && (r = b200moe_reduce_slots(slots_bf16, nullptr, tokens, out_bf16, stream))) return r;
-  return 0;
-}
-
-// Block height 128: GEMM1 gathers its token rows from the row-major quantised tokens (ws.q4, ws.s4) by the sorted list, so
-// no sorted copy of the activations is written (measured against gather + GEMM1: 20 to 30 us less from 1024 to 16384 tokens).
-static int experts_gathering_and_reduce(const b200moe_weights* w, const Workspace& ws, int64_t tokens, void* slots_bf16,
-                                        void* out_bf16, int32_t* status, void* stream) {
-  const int ne = w->num_experts;
-  int r;
-  if ((r = b200moe_gemm1_swiglu_quant_gather(w->w13t, ne, ws.q4, ws.s4, tokens, 0, ws.sorted_ids, ws.block_expert, ws.num_valid,
-                                             ws.rows, ws.hq, ws.sfh, status, stream)))
-    return r;
-  if ((r = b200moe_gemm2_weighted(w->w2t, ne, ws.hq, ws.sfh, ws.block_expert, ws.num_valid, ws.sorted_ids, ws.sorted_w,
-                                  ws.rows, ws.bm, tokens, slots_bf16, status, stream)))
-    return r;
-  if (out_bf16 && (r = b200moe_reduce_slots(slots_bf16, nullptr, tokens, out_bf16, stream))) return r;
+  if (c.out && (r = b200moe_reduce_slots(slots, shared ? shared_out : nullptr, tokens, c.out, st))) return r;
   return 0;
 }
 }  // namespace b200moe
 
+extern "C" int b200moe_layer(const b200moe_weights* w, const b200moe_shared_weights* shared, const void* x_bf16,
+                             const float* logits, int64_t tokens, void* workspace, size_t workspace_bytes, void* slots_bf16,
+                             void* shared_out_bf16, void* out_bf16, int32_t* status, void* stream) {
+  return b200moe::run_layer({w, shared, x_bf16, nullptr, logits, tokens, workspace, workspace_bytes, slots_bf16,
+                             shared_out_bf16, out_bf16, status, stream});
+}
+
+extern "C" int b200moe_layer_prepared(const b200moe_weights* w, const b200moe_shared_weights* shared,
+                                      const b200moe_prepared* input, int64_t tokens, void* workspace, size_t workspace_bytes,
+                                      void* slots_bf16, void* shared_out_bf16, void* out_bf16, int32_t* status,
+                                      void* stream) {
+  return b200moe::run_layer({w, shared, nullptr, input, nullptr, tokens, workspace, workspace_bytes, slots_bf16,
+                             shared_out_bf16, out_bf16, status, stream});
+}
+
+extern "C" int b200moe_prepare(const b200moe_weights* w, const void* x_bf16, int64_t tokens, float* partials, uint8_t* codes4,
+                               uint8_t* scales4, float* topk_weights, int32_t* topk_ids, uint8_t* codes8, uint8_t* scales8,
+                               int32_t* status, void* stream) {
+  using namespace b200moe;
+  if (!w || !w->gate || !x_bf16 || !partials || !codes4 || !scales4 || !topk_weights || !topk_ids || !status)
+    return B200MOE_E_ARG;
+  if (tokens < 1 || tokens > B200MOE_MAX_TOKENS || (codes8 != nullptr) != (scales8 != nullptr)) return B200MOE_E_ARG;
+  const int ne = w->num_experts, splits = b200moe_router_splits(tokens);
+  int r;
+  if (tokens < 128 || !w->gate_split) {
+    r = router_gemm_quant(x_bf16, w->gate, tokens, ne, splits, partials, codes4, scales4, codes8, scales8, nullptr, 16, stream);
+  } else {
+    if ((r = b200moe_router_gemm_tc(x_bf16, w->gate_split, tokens, ne, splits, partials, status, stream))) return r;
+    r = codes8 ? quant_rows_both(x_bf16, tokens, codes4, scales4, codes8, scales8, nullptr, 16, stream)
+               : quant_rows(x_bf16, tokens, codes4, scales4, stream);
+  }
+  if (r) return r;
+  return b200moe_route_topk(partials, ne, tokens * ne, splits, w->bias, tokens, ne, w->route_mode, w->route_scale, topk_weights,
+                            topk_ids, stream);
+}
+
 extern "C" int b200moe_forward_x(const b200moe_weights* w, const void* x_bf16, int64_t tokens, void* workspace,
                                  size_t workspace_bytes, void* slots_bf16, void* out_bf16, int32_t* status,
                                  void* stream) {
-  using namespace b200moe;
-  if (!w || !x_bf16 || !workspace || !slots_bf16 || !status || !w->gate) return B200MOE_E_ARG;
-  if (tokens < 1 || tokens > B200MOE_MAX_TOKENS) return B200MOE_E_ARG;
-  if (reinterpret_cast<uintptr_t>(workspace) & 255) return B200MOE_E_ALIGN;
-  const int ne = w->num_experts;
-  Workspace ws = carve(static_cast<uint8_t*>(workspace), tokens, ne, true);
-  if (workspace_bytes < ws.bytes) return B200MOE_E_ARG;
-  const int splits = b200moe_router_splits(tokens);
-  int r;
-  if (tokens >= 128 && w->gate_split != nullptr) {
-    // prefill sizes: the router GEMM on the tensor cores (three bf16 terms of the gate), the quantiser beside it
-    if ((r = b200moe_router_gemm_tc(x_bf16, w->gate_split, tokens, ne, splits, ws.partials, status, stream))) return r;
-    if ((r = quant_rows(x_bf16, tokens, ws.q4, ws.s4, stream))) return r;
-  } else if ((r = b200moe_router_gemm_quant(x_bf16, w->gate, tokens, ne, splits, ws.partials, ws.q4, ws.s4, nullptr, nullptr,
-                                            stream))) {  // one pass over x: logit partials and the MXFP4 operands, row-major
-    return r;
-  }
-  if (tokens <= kSmallTokens && ne >= 4) {  // routing on the partials, sort and gather of the quantised rows in one launch
-    if ((r = prep_small(ws.partials, ne, tokens * ne, splits, w->bias, tokens, ne, w->route_mode, w->route_scale, ws.bm, ws.w,
-                        ws.ids, ws.sorted_ids, ws.sorted_w, ws.block_expert, ws.num_valid, nullptr, ws.q4, ws.s4, ws.rows,
-                        ws.xq_sorted, ws.sfx, ws.done, static_cast<int>(ws.rows / ws.bm), stream)))
-      return r;
-    return experts_and_reduce(w, ws, tokens, slots_bf16, out_bf16, status, stream);
-  }
-  if ((r = b200moe_route_sort_partials(ws.partials, ne, tokens * ne, splits, w->bias, tokens, ne, w->route_mode,
-                                       w->route_scale, ws.bm, ws.w, ws.ids, ws.sorted_ids, ws.sorted_w, ws.block_expert,
-                                       ws.num_valid, ws.scratch, stream)))
-    return r;
-  if (ws.bm == 128) return experts_gathering_and_reduce(w, ws, tokens, slots_bf16, out_bf16, status, stream);
-  if ((r = dispatch_rows_done(ws.q4, ws.s4, ws.sorted_ids, ws.num_valid, tokens, ws.bm, 0, ws.rows, ws.xq_sorted, ws.sfx,
-                              ws.done, stream)))
-    return r;
-  return experts_and_reduce(w, ws, tokens, slots_bf16, out_bf16, status, stream);
+  if (!slots_bf16) return B200MOE_E_ARG;
+  return b200moe_layer(w, nullptr, x_bf16, nullptr, tokens, workspace, workspace_bytes, slots_bf16, nullptr, out_bf16, status,
+                       stream);
 }
 
 extern "C" int b200moe_forward(const b200moe_weights* w, const void* x_bf16, const float* logits, int64_t tokens,
                                void* workspace, size_t workspace_bytes, void* slots_bf16, void* out_bf16,
                                int32_t* status, void* stream) {
-  using namespace b200moe;
-  if (!w || !x_bf16 || !logits || !workspace || !slots_bf16 || !status) return B200MOE_E_ARG;
-  if (tokens < 1 || tokens > B200MOE_MAX_TOKENS) return B200MOE_E_ARG;
-  if (reinterpret_cast<uintptr_t>(workspace) & 255) return B200MOE_E_ALIGN;
-  const int ne = w->num_experts;
-  Workspace ws = carve(static_cast<uint8_t*>(workspace), tokens, ne);
-  if (workspace_bytes < ws.bytes) return B200MOE_E_ARG;
-  int r;
-  if (tokens <= kSmallTokens && ne >= 4) {  // routing, sort, quantisation and gather in one launch
-    if ((r = prep_small(logits, ne, 0, 1, w->bias, tokens, ne, w->route_mode, w->route_scale, ws.bm, ws.w, ws.ids,
-                        ws.sorted_ids, ws.sorted_w, ws.block_expert, ws.num_valid, x_bf16, nullptr, nullptr, ws.rows,
-                        ws.xq_sorted, ws.sfx, ws.done, static_cast<int>(ws.rows / ws.bm), stream)))
-      return r;
-    return experts_and_reduce(w, ws, tokens, slots_bf16, out_bf16, status, stream);
-  }
-  if ((r = b200moe_route_sort(logits, w->bias, tokens, ne, w->route_mode, w->route_scale, ws.bm, ws.w, ws.ids,
-                              ws.sorted_ids, ws.sorted_w, ws.block_expert, ws.num_valid, ws.scratch, stream)))
-    return r;
-  if (ws.bm == 128) {
-    // prefill sizes: quantise every token once (row-major); GEMM1 gathers the rows itself
-    if ((r = quant_rows(x_bf16, tokens, ws.q4, ws.s4, stream))) return r;
-    return experts_gathering_and_reduce(w, ws, tokens, slots_bf16, out_bf16, status, stream);
-  } else if ((r = b200moe_quant_dispatch(x_bf16, ws.sorted_ids, ws.num_valid, tokens, ws.bm, ws.rows, ws.xq_sorted, ws.sfx,
-                                         ws.done, stream))) {
-    return r;
-  }
-  return experts_and_reduce(w, ws, tokens, slots_bf16, out_bf16, status, stream);
+  if (!slots_bf16 || !logits) return B200MOE_E_ARG;
+  return b200moe_layer(w, nullptr, x_bf16, logits, tokens, workspace, workspace_bytes, slots_bf16, nullptr, out_bf16, status,
+                       stream);
 }
 
 extern "C" int b200moe_forward_host(const b200moe_weights* w, const void* host_x_bf16, const float* host_logits,

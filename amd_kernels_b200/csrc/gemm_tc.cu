@@ -19,6 +19,7 @@
 //
 // Every mbarrier wait is bounded: after about two seconds it records B200MOE_DEV_TIMEOUT in the status word, raises a
 // CTA-wide abort flag, the roles drain and the CTA frees its TMEM and returns.
+#include "shared_role.cuh"
 #include "tc_host.cuh"
 #include "tc_ptx.cuh"
 
@@ -142,13 +143,16 @@ __device__ __forceinline__ RowPlacer make_placer(const EpilogueArgs& ep, __nv_bf
   return p;
 }
 
-template <int MODE, int BM>
+// SHARED: the last `sh.ctas` CTAs of the launch run the shared expert instead (shared_role.cuh)
+template <int MODE, int BM, bool SHARED>
 __global__ void __launch_bounds__((Cfg<MODE, BM>::kThreads), 1)
     grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const uint8_t* __restrict__ w_tiles,
                         const uint8_t* __restrict__ sf_x, const int32_t* __restrict__ block_expert,
                         const int32_t* __restrict__ num_valid, EpilogueArgs ep, int32_t* status, int num_experts,
-                        int max_blocks) {
+                        int max_blocks, const __grid_constant__ CUtensorMap map_sx,
+                        const __grid_constant__ CUtensorMap map_sh, const SharedArgs sh) {
   using C = Cfg<MODE, BM>;
+  constexpr uint32_t kTmemCols = SHARED ? 512 : C::kTmemCols;
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t bar_full[C::kStages];
   __shared__ __align__(8) uint64_t bar_empty[C::kStages];
@@ -184,7 +188,7 @@ __global__ void __launch_bounds__((Cfg<MODE, BM>::kThreads), 1)
   }
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_slot)),
-                 "r"(static_cast<uint32_t>(C::kTmemCols))
+                 "r"(kTmemCols)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -218,8 +222,12 @@ __global__ void __launch_bounds__((Cfg<MODE, BM>::kThreads), 1)
     n_blocks = max(b_lo, min(__ldcg(range + 1), n_blocks)) - b_lo;
   }
   const int total_units = n_blocks * C::kTilesM;
+  const int n_ctas = static_cast<int>(gridDim.x) - (SHARED ? sh.ctas : 0);  // CTAs of the routed experts
 
-  if (warp == 0) {
+  if (SHARED && static_cast<int>(blockIdx.x) >= n_ctas) {
+    shared_role(sh, &map_sx, &map_sh, smem_raw + (tiles - smem_u32(smem_raw)), tiles, tmem_base, bar_full, bar_empty, bar_sf,
+                bar_tfull, bar_tempty, bar_drain, abort_v, status);
+  } else if (warp == 0) {
     // ---------------------------------------------------------------- producer
     if (lane == 0) {
       bool ok = true;
@@ -229,10 +237,10 @@ __global__ void __launch_bounds__((Cfg<MODE, BM>::kThreads), 1)
       // the expert id of a unit is fetched one unit ahead: a GEMM2 unit is only three stages long, and an L2 round trip
       // in front of each would leave the copy queue short
       int e_ahead = static_cast<int>(blockIdx.x) < total_units ? __ldcg(block_expert + b_lo + blockIdx.x / C::kTilesM) : 0;
-      for (int u = blockIdx.x; u < total_units && ok; u += gridDim.x) {
+      for (int u = blockIdx.x; u < total_units && ok; u += n_ctas) {
         const int b = b_lo + u / C::kTilesM, mt = u % C::kTilesM;
         int e = e_ahead;
-        const int un = u + static_cast<int>(gridDim.x);
+        const int un = u + n_ctas;
         if (un < total_units) e_ahead = __ldcg(block_expert + b_lo + un / C::kTilesM);
         if (e < 0 || e >= num_experts) {  // never form an address from an expert id outside the weights
           atomicExch(status, B200MOE_DEV_BAD_INDEX);
@@ -260,7 +268,7 @@ __global__ void __launch_bounds__((Cfg<MODE, BM>::kThreads), 1)
         // This CTA's weight stream has ended: ask L2 for the W2 tiles that the following GEMM2 reads first (its unit u2 =
         // row block u2 / 48, tile u2 % 48; four rounds of one unit per SM), while the slower CTAs finish.
         const int lim = total_units / C::kTilesM * kW2Tiles < 592 ? total_units / C::kTilesM * kW2Tiles : 592;
-        for (int u2 = blockIdx.x; u2 < lim; u2 += gridDim.x) {
+        for (int u2 = blockIdx.x; u2 < lim; u2 += n_ctas) {
           const int e = __ldcg(block_expert + u2 / kW2Tiles);
           if (e >= 0 && e < num_experts)
             l2_prefetch_bulk(ep.next_tiles + static_cast<int64_t>(e * kW2Tiles + u2 % kW2Tiles) * kK2Tiles * kTileRecordBytes,
@@ -284,7 +292,7 @@ __global__ void __launch_bounds__((Cfg<MODE, BM>::kThreads), 1)
       uint32_t slot = 0, ph = 0, sfset = 0, ui = 0;
       uint32_t lo = tiles >> 4, full = sf0, empty = empty0;
       bool ok = true;
-      for (int u = blockIdx.x; u < total_units && ok; u += gridDim.x, ++ui) {
+      for (int u = blockIdx.x; u < total_units && ok; u += n_ctas, ++ui) {
         const uint32_t acc = ui & 1u, aph = (ui >> 1) & 1u;
         if (!mbar_wait(smem_u32(&bar_tempty[acc]), aph ^ 1u, abort_v, status)) break;
         tc_fence_after();
@@ -326,7 +334,7 @@ __global__ void __launch_bounds__((Cfg<MODE, BM>::kThreads), 1)
       uint32_t slot = 0, ph = 0, sfset = 0;
       uint32_t lo = tiles >> 4, full = full0, sf = sf0;
       bool ok = true;
-      for (int u = blockIdx.x; u < total_units && ok; u += gridDim.x) {
+      for (int u = blockIdx.x; u < total_units && ok; u += n_ctas) {
         for (int kt = 0; kt < C::kTilesK; ++kt) {
           // full: the stage's bytes have landed, and (through the producer's wait) the MMAs that last read this slot and
           // this scale set, kStages <= kSfSets stages ago, have completed
@@ -359,7 +367,7 @@ __global__ void __launch_bounds__((Cfg<MODE, BM>::kThreads), 1)
     bool have_ahead = false;
     int ahead_sid = 0;
     float ahead_wt = 0.0f;
-    for (int u = blockIdx.x; u < total_units; u += gridDim.x, ++ui) {
+    for (int u = blockIdx.x; u < total_units; u += n_ctas, ++ui) {
       if (C::kEpiGroups == 2 && static_cast<int>(ui & 1u) != group) continue;  // group g owns accumulator buffer g
       const int b = b_lo + u / C::kTilesM, mt = u % C::kTilesM;
       const uint32_t acc = ui & 1u, aph = (ui >> 1) & 1u;
@@ -382,7 +390,7 @@ __global__ void __launch_bounds__((Cfg<MODE, BM>::kThreads), 1)
       if (!epilogue_all(mbar_wait(smem_u32(&bar_tfull[acc]), aph, abort_v, status), 1u + group)) break;
       tc_fence_after();
       if (MODE == 2 && !C::kTokensAreM) {  // look ahead: the rows of this CTA's next unit
-        const int un = u + static_cast<int>(gridDim.x);
+        const int un = u + n_ctas;
         have_ahead = un < total_units;
         if (have_ahead && et < BM) {
           const int64_t r1 = static_cast<int64_t>(b_lo + un / C::kTilesM) * BM + et;
@@ -564,7 +572,7 @@ __global__ void __launch_bounds__((Cfg<MODE, BM>::kThreads), 1)
   if (warp == 1) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base),
-                 "r"(static_cast<uint32_t>(C::kTmemCols))
+                 "r"(kTmemCols)
                  : "memory");
   }
 }
@@ -586,33 +594,18 @@ struct Cfg12 {
   static constexpr int kSmemBytes = kStages * kStageBytes + kEpiBytes + 1024;
 };
 
-__device__ __forceinline__ bool wait_count(const int32_t* counter, int target, volatile int* abort_flag, int32_t* status) {
-  const uint64_t t0 = global_timer();
-  uint32_t spins = 0;
-  while (true) {
-    int v;
-    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(counter) : "memory");
-    if (v >= target) return true;
-    if ((++spins & 63u) == 0u) {
-      if (*abort_flag) return false;
-      if (global_timer() - t0 > wait_limit_ns()) {
-        *abort_flag = 1;
-        atomicExch(status, B200MOE_DEV_TIMEOUT);
-        return false;
-      }
-    }
-  }
-}
-
-template <int BM>
+template <int BM, bool SHARED>
 __global__ void __launch_bounds__(256, 1)
     gemm12_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_h,
                   const uint8_t* __restrict__ w13t, const uint8_t* __restrict__ w2t, const uint8_t* __restrict__ sf_x,
                   const int32_t* __restrict__ block_expert, const int32_t* __restrict__ num_valid, EpilogueArgs ep,
-                  int32_t* done, int32_t* status, int num_experts, int max_blocks) {
+                  int32_t* done, int32_t* status, int num_experts, int max_blocks,
+                  const __grid_constant__ CUtensorMap map_sx, const __grid_constant__ CUtensorMap map_sh,
+                  const SharedArgs sh) {
   using C = Cfg<1, BM>;  // stage layout, TMEM columns and epilogue geometry are those of the swap orientation
   using C2 = Cfg<2, BM>;
   using CC = Cfg12<BM>;
+  constexpr uint32_t kTmemCols = SHARED ? 512 : C::kTmemCols;
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t bar_full[CC::kStages];
   __shared__ __align__(8) uint64_t bar_empty[CC::kStages];
@@ -647,7 +640,7 @@ __global__ void __launch_bounds__(256, 1)
   }
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_slot)),
-                 "r"(static_cast<uint32_t>(C::kTmemCols))
+                 "r"(kTmemCols)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -675,8 +668,12 @@ __global__ void __launch_bounds__(256, 1)
   }
   const int units1 = n_blocks * kW13Tiles;
   const int total_units = units1 + n_blocks * kW2Tiles;
+  const int n_ctas = static_cast<int>(gridDim.x) - (SHARED ? sh.ctas : 0);  // CTAs of the routed experts
 
-  if (warp == 0) {
+  if (SHARED && static_cast<int>(blockIdx.x) >= n_ctas) {
+    shared_role(sh, &map_sx, &map_sh, smem_raw + (tiles - smem_u32(smem_raw)), tiles, tmem_base, bar_full, bar_empty, bar_sf,
+                bar_tfull, bar_tempty, bar_drain, abort_v, status);
+  } else if (warp == 0) {
     // ---------------------------------------------------------------- weight producer: arms each stage, streams tile records
     if (lane == 0) {
       uint32_t it = 0;
@@ -684,13 +681,13 @@ __global__ void __launch_bounds__(256, 1)
       auto block_of = [&](int u) { return u >= units1 ? (u - units1) / kW2Tiles : u / kW13Tiles; };
       // the expert id of a unit is fetched one unit ahead (a GEMM2 unit is only three stages long)
       int e_ahead = static_cast<int>(blockIdx.x) < total_units ? __ldcg(block_expert + block_of(blockIdx.x)) : 0;
-      for (int u = blockIdx.x; u < total_units && ok; u += gridDim.x) {
+      for (int u = blockIdx.x; u < total_units && ok; u += n_ctas) {
         const bool second = u >= units1;
         const int v = second ? u - units1 : u;
         const int tiles_m = second ? kW2Tiles : kW13Tiles, tiles_k = second ? kK2Tiles : kK1Tiles;
         const int mt = v % tiles_m;
         int e = e_ahead;
-        const int un = u + static_cast<int>(gridDim.x);
+        const int un = u + n_ctas;
         if (un < total_units) e_ahead = __ldcg(block_expert + block_of(un));
         if (e < 0 || e >= num_experts) {
           atomicExch(status, B200MOE_DEV_BAD_INDEX);
@@ -717,7 +714,7 @@ __global__ void __launch_bounds__(256, 1)
       uint32_t it = 0;
       bool ok = true, have_next = false;
       int next_count = 0;
-      for (int u = blockIdx.x; u < total_units && ok; u += gridDim.x) {
+      for (int u = blockIdx.x; u < total_units && ok; u += n_ctas) {
         const bool second = u >= units1;
         const int v = second ? u - units1 : u;
         const int tiles_m = second ? kW2Tiles : kW13Tiles, tiles_k = second ? kK2Tiles : kK1Tiles;
@@ -743,7 +740,7 @@ __global__ void __launch_bounds__(256, 1)
           tma_load_2d(base + C::kBOffset, second ? &map_h : &map_x, kt * 128, b * BM, full);
           bulk_load(base + C::kSfbOffset, sfb_src + kt * C::kSfBytes, C::kSfBytes, full);
         }
-        const int un = u + static_cast<int>(gridDim.x);  // look ahead: the next unit's completion count
+        const int un = u + n_ctas;  // look ahead: the next unit's completion count
         have_next = un < total_units && un >= units1;
         if (have_next)
           asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(next_count) : "l"(done + (un - units1) / kW2Tiles) : "memory");
@@ -759,7 +756,7 @@ __global__ void __launch_bounds__(256, 1)
       uint32_t slot = 0, ph = 0, sfset = 0, ui = 0;
       uint32_t lo = tiles >> 4, sf = sf0, empty = empty0;
       bool ok = true;
-      for (int u = blockIdx.x; u < total_units && ok; u += gridDim.x, ++ui) {
+      for (int u = blockIdx.x; u < total_units && ok; u += n_ctas, ++ui) {
         const int tiles_k = u >= units1 ? kK2Tiles : kK1Tiles;
         const uint32_t acc = ui & 1u, aph = (ui >> 1) & 1u;
         if (!mbar_wait(smem_u32(&bar_tempty[acc]), aph ^ 1u, abort_v, status)) break;
@@ -793,7 +790,7 @@ __global__ void __launch_bounds__(256, 1)
       uint32_t slot = 0, ph = 0, sfset = 0;
       uint32_t lo = tiles >> 4, full = full0, sf = sf0;
       bool ok = true;
-      for (int u = blockIdx.x; u < total_units && ok; u += gridDim.x) {
+      for (int u = blockIdx.x; u < total_units && ok; u += n_ctas) {
         const int tiles_k = u >= units1 ? kK2Tiles : kK1Tiles;
         for (int kt = 0; kt < tiles_k; ++kt) {
           if (!mbar_wait(full, ph, abort_v, status)) { ok = false; break; }
@@ -823,7 +820,7 @@ __global__ void __launch_bounds__(256, 1)
     bool have_ahead = false;
     int ahead_sid = 0;
     float ahead_wt = 0.0f;
-    for (int u = blockIdx.x; u < total_units; u += gridDim.x, ++ui) {
+    for (int u = blockIdx.x; u < total_units; u += n_ctas, ++ui) {
       const bool second = u >= units1;
       const int v = second ? u - units1 : u;
       const int tiles_m = second ? kW2Tiles : kW13Tiles;
@@ -841,7 +838,7 @@ __global__ void __launch_bounds__(256, 1)
       if (!epilogue_all(mbar_wait(smem_u32(&bar_tfull[acc]), aph, abort_v, status), 1u)) break;
       tc_fence_after();
       {  // look ahead: the rows of this CTA's next unit, when that is a GEMM2 unit
-        const int un = u + static_cast<int>(gridDim.x);
+        const int un = u + n_ctas;
         have_ahead = un < total_units && un >= units1;
         if (have_ahead && et < BM) {
           const int64_t r1 = static_cast<int64_t>((un - units1) / kW2Tiles) * BM + et;
@@ -947,63 +944,86 @@ __global__ void __launch_bounds__(256, 1)
   if (warp == 1) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base),
-                 "r"(static_cast<uint32_t>(C::kTmemCols))
+                 "r"(kTmemCols)
                  : "memory");
   }
 }
 
 // ------------------------------------------------------------------------------------------------ host side
 constexpr int64_t kWideFromRows = 20000;  // sorted rows (about 3000 tokens) from which GEMM1 uses 256 weight rows per MMA
-template <int MODE, int BM>
+// grid and dynamic shared memory of a launch with `units` units of routed work, with or without the shared-expert role
+struct LaunchShape {
+  int grid, smem;
+};
+static LaunchShape launch_shape(int64_t units, int max_ctas, int smem, const SharedPlan* sp) {
+  const int extra = sp ? sp->args.ctas : 0;
+  int64_t ctas = sm_count() - extra;
+  if (units < ctas) ctas = units;
+  if (max_ctas > 0 && ctas > max_ctas) ctas = max_ctas;
+  const int need = sp ? shared_smem_bytes(sp->args.bm) : 0;
+  return {static_cast<int>(ctas) + extra, need > smem ? need : smem};
+}
+
+template <int MODE, int BM, bool SHARED>
 static int launch(const CUtensorMap& mx, const uint8_t* w_tiles, const uint8_t* sf_x,
                   const int32_t* block_expert, const int32_t* num_valid, const EpilogueArgs& ep, int64_t max_rows,
-                  int num_experts, int32_t* status, cudaStream_t stream) {
+                  int num_experts, int32_t* status, const SharedPlan* sp, cudaStream_t stream) {
   using C = Cfg<MODE, BM>;
   static PerDeviceOnce once;
   const int rc = once.run([] {
-    return static_cast<int>(cudaFuncSetAttribute(grouped_gemm_kernel<MODE, BM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 C::kSmemBytes));
+    return static_cast<int>(cudaFuncSetAttribute(grouped_gemm_kernel<MODE, BM, SHARED>,
+                                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 SHARED ? kSharedMaxSmem : C::kSmemBytes));
   });
   if (rc) return rc;
-  const int64_t max_units = max_rows / BM * C::kTilesM;
-  const int64_t ctas = sm_count();
-  int grid = static_cast<int>(max_units < ctas ? max_units : ctas);
-  if (ep.max_ctas > 0 && grid > ep.max_ctas) grid = ep.max_ctas;
-  if (grid <= 0) return 0;
-  B200MOE_LAUNCH((grouped_gemm_kernel<MODE, BM>), grid, C::kThreads, C::kSmemBytes, stream, mx, w_tiles, sf_x, block_expert, num_valid, ep, status, num_experts, static_cast<int>(max_rows / BM));
+  const LaunchShape ls = launch_shape(max_rows / BM * C::kTilesM, ep.max_ctas, C::kSmemBytes, sp);
+  if (ls.grid <= 0) return 0;
+  static const SharedPlan none{};
+  if (!sp) sp = &none;
+  B200MOE_LAUNCH((grouped_gemm_kernel<MODE, BM, SHARED>), ls.grid, C::kThreads, ls.smem, stream, mx, w_tiles, sf_x, block_expert,
+                 num_valid, ep, status, num_experts, static_cast<int>(max_rows / BM), sp->map_x, sp->map_h, sp->args);
   return 0;
 }
 
 template <int MODE>
 static int launch_bm(int bm, const CUtensorMap& mx, const uint8_t* w_tiles, const uint8_t* sf_x,
                      const int32_t* block_expert, const int32_t* num_valid, const EpilogueArgs& ep, int64_t max_rows,
-                     int num_experts, int32_t* status, cudaStream_t stream) {
-  switch (bm) {
-    case 16: return launch<MODE, 16>(mx, w_tiles, sf_x, block_expert, num_valid, ep, max_rows, num_experts, status, stream);
-    case 32: return launch<MODE, 32>(mx, w_tiles, sf_x, block_expert, num_valid, ep, max_rows, num_experts, status, stream);
-    case 64: return launch<MODE, 64>(mx, w_tiles, sf_x, block_expert, num_valid, ep, max_rows, num_experts, status, stream);
-    case 128:
-      return launch<MODE, 128>(mx, w_tiles, sf_x, block_expert, num_valid, ep, max_rows, num_experts, status, stream);
+                     int num_experts, int32_t* status, const SharedPlan* sp, cudaStream_t stream) {
+#define B200MOE_GG(BM, SH) \
+  launch<MODE, BM, SH>(mx, w_tiles, sf_x, block_expert, num_valid, ep, max_rows, num_experts, status, sp, stream)
+  if (sp) {  // the decode block heights only
+    if (MODE == 1 && bm == 16) return B200MOE_GG(16, MODE == 1);
+    if (MODE == 1 && bm == 32) return B200MOE_GG(32, MODE == 1);
+    return B200MOE_E_ARG;
   }
+  switch (bm) {
+    case 16: return B200MOE_GG(16, false);
+    case 32: return B200MOE_GG(32, false);
+    case 64: return B200MOE_GG(64, false);
+    case 128: return B200MOE_GG(128, false);
+  }
+#undef B200MOE_GG
   return B200MOE_E_ARG;
 }
 
-
-template <int BM>
+template <int BM, bool SHARED>
 static int launch12(const CUtensorMap& mx, const CUtensorMap& mh, const uint8_t* w13t, const uint8_t* w2t,
                     const uint8_t* sfx, const int32_t* block_expert, const int32_t* num_valid, const EpilogueArgs& ep,
-                    int32_t* done, int64_t max_rows, int num_experts, int32_t* status, cudaStream_t stream) {
+                    int32_t* done, int64_t max_rows, int num_experts, int32_t* status, const SharedPlan* sp,
+                    cudaStream_t stream) {
   using CC = Cfg12<BM>;
   static PerDeviceOnce once;
   const int rc = once.run([] {
-    return static_cast<int>(cudaFuncSetAttribute(gemm12_kernel<BM>, cudaFuncAttributeMaxDynamicSharedMemorySize, CC::kSmemBytes));
+    return static_cast<int>(cudaFuncSetAttribute(gemm12_kernel<BM, SHARED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 SHARED ? kSharedMaxSmem : CC::kSmemBytes));
   });
   if (rc) return rc;
-  const int64_t max_units = max_rows / BM * (kW13Tiles + kW2Tiles);
-  const int grid = static_cast<int>(max_units < sm_count() ? max_units : sm_count());
-  if (grid <= 0) return 0;
-  B200MOE_LAUNCH((gemm12_kernel<BM>), grid, 256, CC::kSmemBytes, stream, mx, mh, w13t, w2t, sfx, block_expert, num_valid, ep,
-                 done, status, num_experts, static_cast<int>(max_rows / BM));
+  const LaunchShape ls = launch_shape(max_rows / BM * (kW13Tiles + kW2Tiles), 0, CC::kSmemBytes, sp);
+  if (ls.grid <= 0) return 0;
+  static const SharedPlan none{};
+  if (!sp) sp = &none;
+  B200MOE_LAUNCH((gemm12_kernel<BM, SHARED>), ls.grid, 256, ls.smem, stream, mx, mh, w13t, w2t, sfx, block_expert, num_valid, ep,
+                 done, status, num_experts, static_cast<int>(max_rows / BM), sp->map_x, sp->map_h, sp->args);
   return 0;
 }
 
@@ -1011,11 +1031,12 @@ int set_wait_limit_routed(unsigned long long ns) { return set_wait_limit_here(ns
 
 }  // namespace b200moe
 
-extern "C" int b200moe_gemm12(const uint8_t* w13t, const uint8_t* w2t, int num_experts, const uint8_t* xq_sorted,
-                              const uint8_t* sfx, const int32_t* block_expert, const int32_t* num_valid,
-                              const int32_t* sorted_ids, const float* sorted_w, int64_t max_rows, int bm, int64_t tokens,
-                              uint8_t* hq, uint8_t* sfh, int32_t* done, void* slots_bf16, int32_t* status, void* stream) {
-  using namespace b200moe;
+namespace b200moe {
+// b200moe_gemm12 / b200moe_gemm1_swiglu_quant, with the shared expert beside the routed experts when `sp` is given
+int gemm12_beside(const uint8_t* w13t, const uint8_t* w2t, int num_experts, const uint8_t* xq_sorted, const uint8_t* sfx,
+                  const int32_t* block_expert, const int32_t* num_valid, const int32_t* sorted_ids, const float* sorted_w,
+                  int64_t max_rows, int bm, int64_t tokens, uint8_t* hq, uint8_t* sfh, int32_t* done, void* slots_bf16,
+                  int32_t* status, const SharedPlan* sp, void* stream) {
   if (!w13t || !w2t || !xq_sorted || !sfx || !block_expert || !num_valid || !sorted_ids || !sorted_w || !hq || !sfh ||
       !done || !slots_bf16 || !status)
     return B200MOE_E_ARG;
@@ -1039,19 +1060,21 @@ extern "C" int b200moe_gemm12(const uint8_t* w13t, const uint8_t* w2t, int num_e
   ep.slots = static_cast<__nv_bfloat16*>(slots_bf16);
   ep.tokens = tokens;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+#define B200MOE_G12(BM, SH) \
+  launch12<BM, SH>(mx, mh, w13t, w2t, sfx, block_expert, num_valid, ep, done, max_rows, num_experts, status, sp, st)
+  if (sp) return bm == 16 ? B200MOE_G12(16, true) : B200MOE_E_ARG;
   switch (bm) {
-    case 16: return launch12<16>(mx, mh, w13t, w2t, sfx, block_expert, num_valid, ep, done, max_rows, num_experts, status, st);
-    case 32: return launch12<32>(mx, mh, w13t, w2t, sfx, block_expert, num_valid, ep, done, max_rows, num_experts, status, st);
-    case 64: return launch12<64>(mx, mh, w13t, w2t, sfx, block_expert, num_valid, ep, done, max_rows, num_experts, status, st);
+    case 16: return B200MOE_G12(16, false);
+    case 32: return B200MOE_G12(32, false);
+    case 64: return B200MOE_G12(64, false);
   }
+#undef B200MOE_G12
   return B200MOE_E_ARG;
 }
 
-extern "C" int b200moe_gemm1_swiglu_quant(const uint8_t* w13t, int num_experts, const uint8_t* xq_sorted,
-                                          const uint8_t* sfx, const int32_t* block_expert, const int32_t* num_valid,
-                                          int64_t max_rows, int bm, uint8_t* hq, uint8_t* sfh,
-                                          const uint8_t* prefetch_w2t, int32_t* status, void* stream) {
-  using namespace b200moe;
+int gemm1_beside(const uint8_t* w13t, int num_experts, const uint8_t* xq_sorted, const uint8_t* sfx,
+                 const int32_t* block_expert, const int32_t* num_valid, int64_t max_rows, int bm, uint8_t* hq, uint8_t* sfh,
+                 const uint8_t* prefetch_w2t, int32_t* status, const SharedPlan* sp, void* stream) {
   if (!w13t || !xq_sorted || !sfx || !block_expert || !num_valid || !hq || !sfh || !status) return B200MOE_E_ARG;
   if (num_experts < 1 || num_experts > kMaxE || max_rows < 0 || (bm != 16 && bm != 32 && bm != 64 && bm != 128) ||
       max_rows % bm)
@@ -1062,7 +1085,7 @@ extern "C" int b200moe_gemm1_swiglu_quant(const uint8_t* w13t, int num_experts, 
   if (max_rows == 0) return 0;
   // Prefill sizes: 256 weight rows per MMA on one CTA (twice the math per issued instruction). Measured, GEMM1 alone, us:
   // 4096 tokens 127 (128-column kernel 129), 8192 tokens 183 (197; CTA pairs 199), 16384 tokens 312 (320; pairs 320).
-  if (bm == 128 && max_rows >= kWideFromRows)
+  if (bm == 128 && max_rows >= kWideFromRows && !sp)
     return b200moe_gemm1_swiglu_quant_wide(w13t, num_experts, xq_sorted, sfx, block_expert, num_valid, max_rows, hq, sfh,
                                            status, stream);
   CUtensorMap mx;
@@ -1072,8 +1095,25 @@ extern "C" int b200moe_gemm1_swiglu_quant(const uint8_t* w13t, int num_experts, 
   ep.hq = hq;
   ep.sfh = sfh;
   ep.next_tiles = misaligned(prefetch_w2t, 16) ? nullptr : prefetch_w2t;
-  return launch_bm<1>(bm, mx, w13t, sfx, block_expert, num_valid, ep, max_rows, num_experts, status,
+  return launch_bm<1>(bm, mx, w13t, sfx, block_expert, num_valid, ep, max_rows, num_experts, status, sp,
                       static_cast<cudaStream_t>(stream));
+}
+}  // namespace b200moe
+
+extern "C" int b200moe_gemm12(const uint8_t* w13t, const uint8_t* w2t, int num_experts, const uint8_t* xq_sorted,
+                              const uint8_t* sfx, const int32_t* block_expert, const int32_t* num_valid,
+                              const int32_t* sorted_ids, const float* sorted_w, int64_t max_rows, int bm, int64_t tokens,
+                              uint8_t* hq, uint8_t* sfh, int32_t* done, void* slots_bf16, int32_t* status, void* stream) {
+  return b200moe::gemm12_beside(w13t, w2t, num_experts, xq_sorted, sfx, block_expert, num_valid, sorted_ids, sorted_w, max_rows,
+                                bm, tokens, hq, sfh, done, slots_bf16, status, nullptr, stream);
+}
+
+extern "C" int b200moe_gemm1_swiglu_quant(const uint8_t* w13t, int num_experts, const uint8_t* xq_sorted,
+                                          const uint8_t* sfx, const int32_t* block_expert, const int32_t* num_valid,
+                                          int64_t max_rows, int bm, uint8_t* hq, uint8_t* sfh,
+                                          const uint8_t* prefetch_w2t, int32_t* status, void* stream) {
+  return b200moe::gemm1_beside(w13t, num_experts, xq_sorted, sfx, block_expert, num_valid, max_rows, bm, hq, sfh, prefetch_w2t,
+                               status, nullptr, stream);
 }
 
 static int gemm2_common(const uint8_t* w2t, int num_experts, const uint8_t* hq, const uint8_t* sfh,
@@ -1093,7 +1133,7 @@ static int gemm2_common(const uint8_t* w2t, int num_experts, const uint8_t* hq, 
   ep.sorted_ids = sorted_ids;
   ep.sorted_w = sorted_w;
   ep.tokens = tokens;
-  return launch_bm<2>(bm, mx, w2t, sfh, block_expert, num_valid, ep, max_rows, num_experts, status,
+  return launch_bm<2>(bm, mx, w2t, sfh, block_expert, num_valid, ep, max_rows, num_experts, status, nullptr,
                       static_cast<cudaStream_t>(stream));
 }
 

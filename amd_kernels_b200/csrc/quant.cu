@@ -33,11 +33,21 @@ __global__ void __launch_bounds__(256) quant_mxfp4_kernel(const uint4* __restric
   (void)k;
 }
 
+// What the row quantiser also writes when the layer has a shared expert: its MXFP8 operands of the same row, the scales
+// row-major or as the scale atoms of 2^atom_shift-row blocks.
+struct QuantRow8 {
+  uint8_t* codes;   // [T][6144]
+  uint8_t* scales;  // [T][192], or null:
+  uint8_t* atoms;   // [ceil(T / 2^atom_shift)][48][512]
+  int atom_shift;
+};
+
 // Row-major quantisation at prefill sizes: one 256-thread CTA per token row, its three 16-byte loads per thread in flight
 // at once; codes [T][3072] and scales [T][192], the bits of quant_mxfp4_kernel. Used ahead of the gather so that a token is
-// read and quantised once, not once per routed slot.
+// read and quantised once, not once per routed slot -- and (Q8) read once for both quantisers.
+template <bool Q8>
 __global__ void __launch_bounds__(256) quant_rows_kernel(const uint4* __restrict__ x, uint8_t* __restrict__ codes,
-                                                         uint8_t* __restrict__ scales) {
+                                                         uint8_t* __restrict__ scales, QuantRow8 q8) {
   pdl_enter(x);
   constexpr int kIters = kH / 8 / 256;  // 3
   const int lane = threadIdx.x & 31;
@@ -74,6 +84,23 @@ __global__ void __launch_bounds__(256) quant_rows_kernel(const uint4* __restrict
     sc |= __shfl_down_sync(0xffffffffu, sc, 4) << 8;
     sc |= __shfl_down_sync(0xffffffffu, sc, 8) << 16;
     if ((lane & 15) == 0) *reinterpret_cast<uint32_t*>(sdst + (idx >> 4) * 4) = sc;
+    if (Q8) {
+      const int e8 = mxfp8_scale(amax);
+      const float inv8 = __uint_as_float(static_cast<uint32_t>(254 - e8) << 23);  // e8 <= 247
+      reinterpret_cast<uint2*>(q8.codes + row * kH)[idx] =
+          make_uint2(cvt_e4m3x2(v[0] * inv8, v[1] * inv8) | (cvt_e4m3x2(v[2] * inv8, v[3] * inv8) << 16),
+                     cvt_e4m3x2(v[4] * inv8, v[5] * inv8) | (cvt_e4m3x2(v[6] * inv8, v[7] * inv8) << 16));
+      uint32_t s8 = static_cast<uint32_t>(e8);
+      s8 |= __shfl_down_sync(0xffffffffu, s8, 4) << 8;
+      s8 |= __shfl_down_sync(0xffffffffu, s8, 8) << 16;
+      if ((lane & 15) == 0) {
+        uint8_t* d8 = q8.scales != nullptr
+                          ? q8.scales + row * (kH / 32) + (idx >> 4) * 4
+                          : q8.atoms + ((row >> q8.atom_shift) * (kH / 128) + (idx >> 4)) * kAtomBytes +
+                                atom_offset(static_cast<int>(row & ((1 << q8.atom_shift) - 1)), 0);
+        *reinterpret_cast<uint32_t*>(d8) = s8;
+      }
+    }
   }
 }
 
@@ -285,14 +312,29 @@ int quant_rows(const void* x_bf16, int64_t tokens, uint8_t* codes, uint8_t* scal
       (reinterpret_cast<uintptr_t>(scales) & 3))
     return B200MOE_E_ALIGN;
   if (tokens == 0) return 0;
-  B200MOE_LAUNCH(quant_rows_kernel, static_cast<unsigned>(tokens), 256, 0, static_cast<cudaStream_t>(stream),
-                 static_cast<const uint4*>(x_bf16), codes, scales);
+  B200MOE_LAUNCH(quant_rows_kernel<false>, static_cast<unsigned>(tokens), 256, 0, static_cast<cudaStream_t>(stream),
+                 static_cast<const uint4*>(x_bf16), codes, scales, QuantRow8{});
+  return 0;
+}
+
+// Both quantisers in one pass over x; the MXFP8 scales as rows (scales8) or as the atoms of bm8-row blocks (atoms8).
+int quant_rows_both(const void* x_bf16, int64_t tokens, uint8_t* codes, uint8_t* scales, uint8_t* codes8, uint8_t* scales8,
+                    uint8_t* atoms8, int bm8, void* stream) {
+  if (!x_bf16 || !codes || !scales || !codes8 || (!scales8 && !atoms8) || tokens < 0) return B200MOE_E_ARG;
+  if (((reinterpret_cast<uintptr_t>(x_bf16) | reinterpret_cast<uintptr_t>(atoms8)) & 15) ||
+      (reinterpret_cast<uintptr_t>(codes8) & 7) ||
+      ((reinterpret_cast<uintptr_t>(codes) | reinterpret_cast<uintptr_t>(scales) | reinterpret_cast<uintptr_t>(scales8)) & 3))
+    return B200MOE_E_ALIGN;
+  if (tokens == 0) return 0;
+  const int shift = bm8 == 16 ? 4 : bm8 == 32 ? 5 : bm8 == 64 ? 6 : 7;
+  B200MOE_LAUNCH(quant_rows_kernel<true>, static_cast<unsigned>(tokens), 256, 0, static_cast<cudaStream_t>(stream),
+                 static_cast<const uint4*>(x_bf16), codes, scales, QuantRow8{codes8, scales8, atoms8, shift});
   return 0;
 }
 
 int dispatch_rows_done(const uint8_t* codes, const uint8_t* scales, const int32_t* sorted_ids, const int32_t* num_valid,
                        int64_t tokens, int bm, int by_pair, int64_t max_rows, uint8_t* xq_sorted, uint8_t* sfx,
-                       int32_t* done, void* stream) {
+                       int32_t* done, int n_done, void* stream) {
   if (!codes || !scales || !sorted_ids || !num_valid || !xq_sorted || !sfx || tokens < 0 || max_rows < 0)
     return B200MOE_E_ARG;
   if (bm != 16 && bm != 32 && bm != 64 && bm != 128) return B200MOE_E_ARG;
@@ -302,7 +344,7 @@ int dispatch_rows_done(const uint8_t* codes, const uint8_t* scales, const int32_
   if (max_rows == 0) return 0;
   const unsigned grid = static_cast<unsigned>((max_rows + 7) / 8);
   B200MOE_LAUNCH(dispatch_rows_kernel, grid, 256, 0, static_cast<cudaStream_t>(stream), codes, scales, sorted_ids,
-                 num_valid, tokens, bm, by_pair, xq_sorted, sfx, done, static_cast<int>(max_rows / bm));
+                 num_valid, tokens, bm, by_pair, xq_sorted, sfx, done, n_done);
   return 0;
 }
 }  // namespace b200moe
@@ -311,13 +353,13 @@ extern "C" int b200moe_dispatch_rows(const uint8_t* codes, const uint8_t* scales
                                      const int32_t* num_valid, int64_t tokens, int bm, int by_pair, int64_t max_rows,
                                      uint8_t* xq_sorted, uint8_t* sfx, void* stream) {
   return b200moe::dispatch_rows_done(codes, scales, sorted_ids, num_valid, tokens, bm, by_pair, max_rows, xq_sorted, sfx,
-                                     nullptr, stream);
+                                     nullptr, 0, stream);
 }
 
-extern "C" int b200moe_quant_dispatch(const void* x_bf16, const int32_t* sorted_ids, const int32_t* num_valid,
-                                      int64_t tokens, int bm, int64_t max_rows, uint8_t* xq_sorted, uint8_t* sfx,
-                                      int32_t* done, void* stream) {
-  using namespace b200moe;
+namespace b200moe {
+// b200moe_quant_dispatch zeroing `n_done` counts (the grid has 256 threads per sorted row, more than counts)
+int quant_dispatch_done(const void* x_bf16, const int32_t* sorted_ids, const int32_t* num_valid, int64_t tokens, int bm,
+                        int64_t max_rows, uint8_t* xq_sorted, uint8_t* sfx, int32_t* done, int n_done, void* stream) {
   if (!x_bf16 || !sorted_ids || !num_valid || !xq_sorted || !sfx || tokens < 0 || max_rows < 0) return B200MOE_E_ARG;
   const int shift = bm == 16 ? 4 : bm == 32 ? 5 : bm == 64 ? 6 : bm == 128 ? 7 : -1;
   if (shift < 0) return B200MOE_E_ARG;
@@ -325,7 +367,15 @@ extern "C" int b200moe_quant_dispatch(const void* x_bf16, const int32_t* sorted_
       (reinterpret_cast<uintptr_t>(sfx) & 15))
     return B200MOE_E_ALIGN;
   if (max_rows == 0) return 0;
-  const unsigned grid = static_cast<unsigned>(max_rows);
-  B200MOE_LAUNCH(quant_dispatch_kernel, grid, 256, 0, static_cast<cudaStream_t>(stream), static_cast<const uint4*>(x_bf16), sorted_ids, num_valid, tokens, shift, xq_sorted, sfx, done, static_cast<int>(max_rows / bm));
+  B200MOE_LAUNCH(quant_dispatch_kernel, static_cast<unsigned>(max_rows), 256, 0, static_cast<cudaStream_t>(stream),
+                 static_cast<const uint4*>(x_bf16), sorted_ids, num_valid, tokens, shift, xq_sorted, sfx, done, n_done);
   return 0;
+}
+}  // namespace b200moe
+
+extern "C" int b200moe_quant_dispatch(const void* x_bf16, const int32_t* sorted_ids, const int32_t* num_valid,
+                                      int64_t tokens, int bm, int64_t max_rows, uint8_t* xq_sorted, uint8_t* sfx,
+                                      int32_t* done, void* stream) {
+  return b200moe::quant_dispatch_done(x_bf16, sorted_ids, num_valid, tokens, bm, max_rows, xq_sorted, sfx, done,
+                                      bm > 0 ? static_cast<int>(max_rows / bm) : 0, stream);
 }

@@ -25,7 +25,9 @@ struct QuantOut {
   uint8_t* codes4;   // [T][3072]
   uint8_t* scales4;  // [T][192]
   uint8_t* codes8;   // [T][6144], may be null
-  uint8_t* scales8;  // [T][192]
+  uint8_t* scales8;  // [T][192], or null:
+  uint8_t* atoms8;   // the same bytes as the scale atoms of 2^atom_shift-row blocks
+  int atom_shift;
 };
 
 // One step of the transposing sum over the lanes: before it, N values per lane; after it N / 2, the lanes with BIT clear
@@ -137,7 +139,13 @@ __global__ void __launch_bounds__(256) router_gemm_kernel(const __nv_bfloat16* _
           store_bytes(q.codes8 + t * kH + k,
               make_uint2(cvt_e4m3x2(v[0] * inv8, v[1] * inv8) | (cvt_e4m3x2(v[2] * inv8, v[3] * inv8) << 16),
                          cvt_e4m3x2(v[4] * inv8, v[5] * inv8) | (cvt_e4m3x2(v[6] * inv8, v[7] * inv8) << 16)), vec);
-          if ((v8 & 3) == 0) q.scales8[t * (kH / 32) + (k >> 5)] = static_cast<uint8_t>(e8);
+          if ((v8 & 3) == 0) {
+            uint8_t* dst = q.scales8 != nullptr
+                               ? q.scales8 + t * (kH / 32) + (k >> 5)
+                               : q.atoms8 + ((t >> q.atom_shift) * (kH / 128) + (k >> 7)) * kAtomBytes +
+                                     atom_offset(static_cast<int>(t & ((1 << q.atom_shift) - 1)), (k >> 5) & 3);
+            *dst = static_cast<uint8_t>(e8);
+          }
         }
       }
     }
@@ -196,21 +204,31 @@ extern "C" int b200moe_router_gemm(const void* x_bf16, const float* gate, int64_
   return 0;
 }
 
-extern "C" int b200moe_router_gemm_quant(const void* x_bf16, const float* gate, int64_t tokens, int num_experts, int splits,
-                                         float* partials, uint8_t* codes4, uint8_t* scales4, uint8_t* codes8,
-                                         uint8_t* scales8, void* stream) {
-  using namespace b200moe;
+namespace b200moe {
+// b200moe_router_gemm_quant; the shared expert's scales as rows (scales8) or as the atoms of bm8-row blocks (atoms8)
+int router_gemm_quant(const void* x_bf16, const float* gate, int64_t tokens, int num_experts, int splits, float* partials,
+                      uint8_t* codes4, uint8_t* scales4, uint8_t* codes8, uint8_t* scales8, uint8_t* atoms8, int bm8,
+                      void* stream) {
   if (!x_bf16 || !gate || !partials || !codes4 || !scales4 || tokens < 0 || num_experts < 1 || num_experts > kMaxE)
     return B200MOE_E_ARG;
-  if ((codes8 != nullptr) != (scales8 != nullptr)) return B200MOE_E_ARG;
+  if ((codes8 != nullptr) != (scales8 != nullptr || atoms8 != nullptr)) return B200MOE_E_ARG;
   if (splits < 1 || kH % splits || (kH / splits) % 32) return B200MOE_E_ARG;
   if (reinterpret_cast<uintptr_t>(codes8) & 1) return B200MOE_E_ALIGN;
   if (tokens == 0) return 0;
+  const int shift = bm8 == 16 ? 4 : bm8 == 32 ? 5 : bm8 == 64 ? 6 : 7;
   const dim3 grid(static_cast<unsigned>((num_experts + kRgExperts - 1) / kRgExperts), static_cast<unsigned>(splits),
                   static_cast<unsigned>((tokens + kRgTokens - 1) / kRgTokens));
-  const QuantOut q{codes4, scales4, codes8, scales8};
+  const QuantOut q{codes4, scales4, codes8, scales8, atoms8, shift};
   B200MOE_LAUNCH(router_gemm_kernel<true>, grid, 256, 0, static_cast<cudaStream_t>(stream),
                  static_cast<const __nv_bfloat16*>(x_bf16), gate, tokens, num_experts, kH / splits, partials, q,
                  aligned16(x_bf16, gate, codes4, codes8));
   return 0;
+}
+}  // namespace b200moe
+
+extern "C" int b200moe_router_gemm_quant(const void* x_bf16, const float* gate, int64_t tokens, int num_experts, int splits,
+                                         float* partials, uint8_t* codes4, uint8_t* scales4, uint8_t* codes8,
+                                         uint8_t* scales8, void* stream) {
+  return b200moe::router_gemm_quant(x_bf16, gate, tokens, num_experts, splits, partials, codes4, scales4, codes8, scales8,
+                                    nullptr, 16, stream);
 }

@@ -5,13 +5,11 @@
 //
 // Weight records: one tile of 128 rows x 128 K-elements = 16384 bytes of E4M3 codes in the 128-byte-swizzled image,
 // then one scale atom (4 scales per row), padded to 17408 bytes so the token tile behind it stays 1024-byte aligned.
+#include "shared_role.cuh"
 #include "tc_host.cuh"
 #include "tc_ptx.cuh"
 
 namespace b200moe {
-
-constexpr int kS1TilesK = kH / 128;  // 48 K-tiles of 128 elements in the first GEMM
-constexpr int kS2TilesK = kI / 128;  // 6 in the second
 
 // ------------------------------------------------------------------------------------------------ weight preshuffle
 template <int K_BYTES, int TILES_M, bool IS_W13>
@@ -373,14 +371,7 @@ static int launch_shared_bm(int bm, const CUtensorMap& mx, const uint8_t* w_tile
 
 static size_t up1k(size_t v) { return (v + 1023) / 1024 * 1024; }
 
-struct SharedWorkspace {
-  uint8_t *x8, *sfx8, *h8, *sfh8;
-  size_t bytes;
-  int bm;
-  int64_t rows;
-};
-
-static SharedWorkspace carve_shared(uint8_t* base, int64_t tokens) {
+SharedWorkspace carve_shared(uint8_t* base, int64_t tokens) {
   SharedWorkspace ws{};
   ws.bm = b200moe_shared_block_rows(tokens);
   ws.rows = (tokens + ws.bm - 1) / ws.bm * ws.bm;
@@ -397,6 +388,29 @@ static SharedWorkspace carve_shared(uint8_t* base, int64_t tokens) {
   ws.sfh8 = take(blocks * kS2TilesK * kAtomBytes);
   ws.bytes = off;
   return ws;
+}
+
+// The role's part of a launch (shared_role.cuh): codes8 [code_rows][6144] and ws.sfx8 hold the quantised tokens, `done` is one
+// zeroed count per block. CTAs: one per tile of the first GEMM, and four more that start on the second one's share.
+int shared_plan(SharedPlan* plan, const uint8_t* w13t, const uint8_t* w2t, const uint8_t* codes8, int64_t code_rows,
+                const SharedWorkspace& ws, void* out_bf16, int64_t tokens, int32_t* done) {
+  int r;
+  if ((r = make_map(&plan->map_x, codes8, kH, static_cast<uint64_t>(code_rows), static_cast<uint32_t>(ws.bm)))) return r;
+  if ((r = make_map(&plan->map_h, ws.h8, kI, static_cast<uint64_t>(ws.rows), static_cast<uint32_t>(ws.bm)))) return r;
+  SharedArgs& a = plan->args;
+  a.w13t = w13t;
+  a.w2t = w2t;
+  a.sfx8 = ws.sfx8;
+  a.h8 = ws.h8;
+  a.sfh8 = ws.sfh8;
+  a.out = static_cast<__nv_bfloat16*>(out_bf16);
+  a.done = done;
+  a.tokens = tokens;
+  a.n_blocks = static_cast<int>(ws.rows / ws.bm);
+  a.bm = ws.bm;
+  a.stages = shared_stages(ws.bm);
+  a.ctas = kW13Tiles + 4;
+  return 0;
 }
 
 int set_wait_limit_shared(unsigned long long ns) { return set_wait_limit_here(ns); }
@@ -449,9 +463,9 @@ extern "C" int b200moe_shared_quant_rows(const void* x_bf16, int64_t tokens, uin
   return 0;
 }
 
-static int shared_gemms(const uint8_t* w13t, const uint8_t* w2t, const uint8_t* codes8, int64_t code_rows,
-                        const b200moe::SharedWorkspace& ws, void* out_bf16, int64_t tokens, int32_t* status, void* stream) {
-  using namespace b200moe;
+namespace b200moe {
+int shared_gemms(const uint8_t* w13t, const uint8_t* w2t, const uint8_t* codes8, int64_t code_rows, const SharedWorkspace& ws,
+                 void* out_bf16, int64_t tokens, int32_t* status, void* stream) {
   const int n_blocks = static_cast<int>(ws.rows / ws.bm);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   CUtensorMap mx, mh;
@@ -467,6 +481,7 @@ static int shared_gemms(const uint8_t* w13t, const uint8_t* w2t, const uint8_t* 
   if ((r = launch_shared_bm<1>(ws.bm, mx, w13t, ws.sfx8, n_blocks, ep, status, st))) return r;
   return launch_shared_bm<2>(ws.bm, mh, w2t, ws.sfh8, n_blocks, ep, status, st);
 }
+}  // namespace b200moe
 
 extern "C" int b200moe_shared_expert(const uint8_t* w13t, const uint8_t* w2t, const void* x_bf16, int64_t tokens,
                                      void* workspace, size_t workspace_bytes, void* out_bf16, int32_t* status,
@@ -482,8 +497,6 @@ extern "C" int b200moe_shared_expert(const uint8_t* w13t, const uint8_t* w2t, co
   if (r) return r;
   return shared_gemms(w13t, w2t, ws.x8, ws.rows, ws, out_bf16, tokens, status, stream);
 }
-
-extern "C" int b200moe_scales_to_atoms(const uint8_t* rows, int64_t tokens, int cols, int bm, uint8_t* atoms, void* stream);
 
 extern "C" int b200moe_shared_expert_quantized(const uint8_t* w13t, const uint8_t* w2t, const uint8_t* codes8,
                                                const uint8_t* scales, int64_t tokens, void* workspace,

@@ -21,7 +21,13 @@ def _ptr(t):
 
 
 def _stream(device):
-    return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+    return ctypes.c_void_p(_raw_stream(device))
+
+
+def _raw_stream(device) -> int:
+    """The current stream's handle on ``device`` (what ``torch.cuda.current_stream(device).cuda_stream`` gives, without making
+    a stream object: a tenth of the host time)."""
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if device.index is None else device.index)
 
 
 _status: dict = {}
@@ -29,11 +35,14 @@ _status: dict = {}
 
 def status_word(device) -> torch.Tensor:
     """The per-device int32 word kernels write device-side conditions to (0 = none, 1 = a bounded wait ran out)."""
-    key = torch.device(device).index if torch.device(device).index is not None else torch.cuda.current_device()
-    if key not in _status:
+    if not isinstance(device, torch.device):
+        device = torch.device(device)
+    key = device.index if device.index is not None else torch.cuda.current_device()
+    word = _status.get(key)
+    if word is None:
         with torch.inference_mode(False):  # a normal tensor even when first used under inference_mode
-            _status[key] = torch.zeros(1, dtype=torch.int32, device=f"cuda:{key}")
-    return _status[key]
+            word = _status[key] = torch.zeros(1, dtype=torch.int32, device=f"cuda:{key}")
+    return word
 
 
 def last_status(device=None) -> int:
@@ -531,12 +540,43 @@ def route(x, w, router_logits=None):
 def mxfp4_moe_experts(x_quant, topk_weights, topk_ids, w):
     """The routed experts on the MXFP4 input ``x_quant`` = (codes, scales), already routed (``topk_weights`` include
     the routed scale) -> the BF16 [M, 4, H] slots (reference chain.py:113-124). Served at every M here."""
-    n = x_quant[0].shape[0]
-    bm = variant_for(n)
-    sort = moe_sort(topk_ids, topk_weights, bm, w.num_experts)
-    xq, sfx = dispatch_rows(x_quant, sort)
-    hq, sfh = grouped_gemm1(xq, sfx, sort, w)
-    return grouped_gemm2(hq, sfh, sort, w)
+    codes, scales = x_quant
+    n = codes.shape[0]
+    variant_for(n)
+    if topk_ids.dtype != torch.int32 or topk_weights.dtype != torch.float32 or topk_ids.shape != topk_weights.shape \
+            or tuple(topk_ids.shape) != (n, TOPK):
+        raise ValueError("expected int32 ids and fp32 weights of shape [M, 4]")
+    dev = codes.device
+    codes, scales, topk_weights, topk_ids = (t.contiguous() for t in (codes, scales, topk_weights, topk_ids))
+    slots = torch.empty((n, TOPK, H), dtype=torch.bfloat16, device=dev)
+    prep = _lib.Prepared(codes.data_ptr(), scales.data_ptr(), topk_weights.data_ptr(), topk_ids.data_ptr(), None, None, None)
+    layer_prepared(prep, n, w, None, slots, None, None, dev)
+    return slots
+
+
+def layer_prepared(prep, n, w, sw, slots, shared, out, dev):
+    """One ``b200moe_layer_prepared`` on the current stream. ``prep``: the C struct; ``slots`` / ``shared`` None: not wanted."""
+    lib = w.lib()
+    flags = (_lib.LAYER_COMPACT if prep.mask4 else 0) | _result_flags(sw, slots, shared)
+    ws_bytes = lib.b200moe_layer_workspace_bytes(n, w.num_experts, flags)
+    workspace = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
+    _lib.check(lib.b200moe_layer_prepared(
+        ctypes.byref(w.abi()), None if sw is None else ctypes.byref(sw.abi()), ctypes.byref(prep), n, workspace.data_ptr(),
+        ws_bytes, None if slots is None else slots.data_ptr(), None if shared is None else shared.data_ptr(),
+        None if out is None else out.data_ptr(), status_word(dev).data_ptr(), _raw_stream(dev)), "layer_prepared")
+
+
+def _result_flags(sw, slots, shared):
+    flags = 0 if slots is not None else _lib.LAYER_OWN_SLOTS
+    if sw is not None:
+        flags |= _lib.LAYER_SHARED if shared is not None else _lib.LAYER_SHARED | _lib.LAYER_OWN_SHARED_OUT
+    return flags
+
+
+# Token count from which the shared expert runs on the side stream: below, it is a role of a routed launch (48 against 161 us
+# for the layer at 1 token, 112 against 244 at 32, most of it host time); above, in front of the routed kernels on one stream
+# it made the layer 2 to 3 % slower (240 -> 245 us at 777 tokens).
+SIDE_STREAM_FROM = 512
 
 
 def mxfp4_moe(x, w, *, return_partials=False, router_logits=None):
@@ -544,56 +584,58 @@ def mxfp4_moe(x, w, *, return_partials=False, router_logits=None):
 
     Reduced mode returns BF16 [M, 6144] = slots 0..3, then the shared expert's output, summed in fp32; partials mode
     returns (slots BF16 [M, 4, H], shared BF16 [M, H]); without ``w.shared_weights`` the shared term is absent (None).
-    ``router_logits`` fp32 [M, E] skips the router GEMM. The routed part is one ``b200moe_forward`` on the current
-    stream; the shared expert runs on the device's side stream beside it and the current stream joins it before the
-    reduce. Without ``router_logits`` the router runs inside the same call (``b200moe_forward_x``). Scratch and outputs come
-    from ``torch.empty``."""
+    ``router_logits`` fp32 [M, E] skips the router GEMM. The whole layer is one C-ABI call (``b200moe_layer``) on the current
+    stream: up to 512 tokens the shared expert runs on SMs of its own inside the routed experts' launches; above, it runs on
+    the device's side stream, which the current stream joins before the reduce. Scratch and outputs come from ``torch.empty``."""
     if not isinstance(x, torch.Tensor):
         from .prepared_input import MoeInput, MoeInputCompact, mxfp4_moe_prepared
         if not isinstance(x, (MoeInput, MoeInputCompact)):
             raise ValueError("expected BF16 [M,6144] rows, a MoeInput or a MoeInputCompact")
         return mxfp4_moe_prepared(x, w, return_partials=return_partials)
-    variant_for(x.shape[0])
+    n = x.shape[0]
+    if not 0 < n <= MAX_TOKENS:
+        raise ValueError(f"unsupported token count {n}")
     if x.ndim != 2 or x.shape[1] != H or x.dtype != torch.bfloat16 or not x.is_contiguous():
         raise ValueError("expected contiguous BF16 [M,6144]")
-    n, dev = x.shape[0], x.device
-    sw = w.shared_weights
-    shared = None
-    if sw is not None:
-        from .shared_expert import shared_expert_parallel
-        current = torch.cuda.current_stream(dev)
-        shared = shared_expert_parallel(x, sw, current)
-    slots = torch.empty((n, TOPK, H), dtype=torch.bfloat16, device=dev)
-    out = None if (return_partials or sw is not None) else torch.empty((n, H), dtype=torch.bfloat16, device=dev)
-    _routed_layer(x, w, router_logits, slots, out)
-    if sw is None:
-        return (slots, None) if return_partials else out
-    current = torch.cuda.current_stream(dev)
-    current.wait_stream(sw.stream)
-    shared.record_stream(current)
-    return (slots, shared) if return_partials else reduce_slots(slots, shared)
-
-
-def _routed_layer(x, w, router_logits, slots, out):
-    """One C-ABI call for the routed layer on the current stream: ``b200moe_forward`` when the caller hands fp32 logits,
-    ``b200moe_forward_x`` (router GEMM fused with the input quantiser inside the call) when it hands only ``x``."""
-    lib = w.lib()
-    n, dev = x.shape[0], x.device
+    dev, sw, lib = x.device, w.shared_weights, w.lib()
+    n_exp = w.num_experts
     if router_logits is not None:
-        if router_logits.shape != (n, w.num_experts) or router_logits.dtype != torch.float32:
-            raise ValueError(f"router_logits: expected fp32 [{n}, {w.num_experts}]")
+        if router_logits.shape != (n, n_exp) or router_logits.dtype != torch.float32:
+            raise ValueError(f"router_logits: expected fp32 [{n}, {n_exp}]")
         logits = router_logits.contiguous()
-        ws_bytes = int(lib.b200moe_workspace_bytes(n, w.num_experts))
-        workspace = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
-        _lib.check(lib.b200moe_forward(ctypes.byref(w.abi()), _ptr(x), _ptr(logits), n, _ptr(workspace), ws_bytes,
-                                       _ptr(slots), _ptr(out), _ptr(status_word(dev)), _stream(dev)), "forward")
-        return
-    if w.router_weight is None:
-        raise ValueError("needs router_logits= or MoeWeights with router_weight")
-    ws_bytes = int(lib.b200moe_workspace_bytes_x(n, w.num_experts))
+        flags = 0
+    else:
+        if w.router_weight is None:
+            raise ValueError("needs router_logits= or MoeWeights with router_weight")
+        logits, flags = None, _lib.LAYER_ROUTER
+    slots = shared = out = None
+    if return_partials:
+        slots = torch.empty((n, TOPK, H), dtype=torch.bfloat16, device=dev)
+        if sw is not None:
+            shared = torch.empty((n, H), dtype=torch.bfloat16, device=dev)
+    else:
+        out = torch.empty((n, H), dtype=torch.bfloat16, device=dev)
+    side = sw is not None and n > SIDE_STREAM_FROM
+    if side:
+        from .shared_expert import shared_expert_parallel
+        shared, sw, side_stream = shared_expert_parallel(x, sw, torch.cuda.current_stream(dev)), None, sw.stream
+        if slots is None:
+            slots = torch.empty((n, TOPK, H), dtype=torch.bfloat16, device=dev)
+            out = None
+    flags |= _result_flags(sw, slots, shared)
+    ws_bytes = lib.b200moe_layer_workspace_bytes(n, n_exp, flags)
     workspace = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
-    _lib.check(lib.b200moe_forward_x(ctypes.byref(w.abi()), _ptr(x), n, _ptr(workspace), ws_bytes, _ptr(slots), _ptr(out),
-                                     _ptr(status_word(dev)), _stream(dev)), "forward_x")
+    _lib.check(lib.b200moe_layer(
+        ctypes.byref(w.abi()), None if sw is None else ctypes.byref(sw.abi()), x.data_ptr(),
+        None if logits is None else logits.data_ptr(), n, workspace.data_ptr(), ws_bytes,
+        None if slots is None else slots.data_ptr(), None if shared is None or side else shared.data_ptr(),
+        None if out is None else out.data_ptr(), status_word(dev).data_ptr(), _raw_stream(dev)), "layer")
+    if side:
+        current = torch.cuda.current_stream(dev)
+        current.wait_stream(side_stream)
+        shared.record_stream(current)
+        out = None if return_partials else reduce_slots(slots, shared)
+    return (slots, shared) if return_partials else out
 
 
 def set_wait_limit_ns(ns: int) -> None:

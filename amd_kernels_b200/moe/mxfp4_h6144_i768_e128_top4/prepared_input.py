@@ -134,39 +134,55 @@ def prepare_mxfp4_moe(x, w) -> MoeInput:
     a shared expert, its MXFP8 operands, every scale row-major: below 128 tokens from ONE pass over x (the router GEMM fused
     with both quantisers), from 128 tokens on with the router on the tensor cores. The payload carries exactly the routing
     and codes ``mxfp4_moe(x, w)`` computes. Returns only tensor payloads; the caller owns the gather."""
-    from .chain import router_gemm_quant, topk_route, variant_for
+    from .chain import _raw_stream, status_word, variant_for
     if (not isinstance(x, torch.Tensor) or x.ndim != 2 or x.shape[1] != H or x.dtype != torch.bfloat16
             or not x.is_contiguous()):
         raise ValueError("expected contiguous BF16 [M,6144]")
-    variant_for(x.shape[0])
+    n, dev = x.shape[0], x.device
+    variant_for(n)
     if w.router_weight is None:
         raise ValueError("needs MoeWeights with router_weight: MoeWeights.from_row_major(router_weight, ...)")
-    w.abi()  # makes the gate's bf16 terms on first use
-    parts, (q, s), (q8, s8) = router_gemm_quant(x, w.router_weight, shared=w.shared_weights is not None,
-                                                split=w.router_split)
-    wt, ids = topk_route(parts, w.correction_bias, w.routed_scaling_factor, w.routing_mode)
-    return MoeInput(q, s, wt, ids, q8, s8)
+    lib, abi = _lib.load(), w.abi()
+    shared = w.shared_weights is not None
+    parts = torch.empty((lib.b200moe_router_splits(n), n, w.num_experts), dtype=torch.float32, device=dev)
+    q4 = torch.empty((n, H // 2), dtype=torch.uint8, device=dev)
+    s4 = torch.empty((n, H // 32), dtype=torch.uint8, device=dev)
+    wt = torch.empty((n, TOPK), dtype=torch.float32, device=dev)
+    ids = torch.empty((n, TOPK), dtype=torch.int32, device=dev)
+    q8 = torch.empty((n, H), dtype=torch.uint8, device=dev) if shared else None
+    s8 = torch.empty((n, H // 32), dtype=torch.uint8, device=dev) if shared else None
+    _lib.check(lib.b200moe_prepare(ctypes.byref(abi), x.data_ptr(), n, parts.data_ptr(), q4.data_ptr(), s4.data_ptr(),
+                                   wt.data_ptr(), ids.data_ptr(), q8.data_ptr() if shared else None,
+                                   s8.data_ptr() if shared else None, status_word(dev).data_ptr(), _raw_stream(dev)), "prepare")
+    return MoeInput(q4, s4, wt, ids, q8, s8)
 
 
 def mxfp4_moe_prepared(x, w, *, return_partials):
-    """``mxfp4_moe`` on a prepared input (reference prepared_input.py:159-187): the routed experts on the MXFP4 operands,
-    the shared expert on the MXFP8 ones on the side stream, summed in slot order then shared."""
-    from .chain import mxfp4_moe_experts, reduce_slots
-    from .shared_expert import shared_expert_parallel
+    """``mxfp4_moe`` on a prepared input (reference prepared_input.py:159-187): the routed experts on the MXFP4 operands (of a
+    compact input: rebuilt inside the call), the shared expert on the MXFP8 ones, summed in slot order then shared."""
+    from .chain import layer_prepared
+    sw, dev = w.shared_weights, w.w13.device
     if isinstance(x, MoeInputCompact):
-        x = x.expand()
-    x.validate(w)
-    dev = x.routed_codes.device
-    sw = w.shared_weights
-    shared = None
-    current = torch.cuda.current_stream(dev)
-    if sw is not None:
-        shared = shared_expert_parallel(None, sw, current, x_quant=(x.shared_codes, x.shared_scales))
-    parts = mxfp4_moe_experts((x.routed_codes, x.routed_scales), x.topk_weights, x.topk_ids, w)
-    if sw is not None:
-        current.wait_stream(sw.stream)
-        shared.record_stream(current)
-    return (parts, shared) if return_partials else reduce_slots(parts, shared)
+        if x.shared_codes.device.type != "cuda":
+            raise ValueError("compact input requires CUDA operands")
+        n = _rows_of(x, "shared_codes")
+        _require(x, ("routed_scales", "topk_weights", "topk_ids", "shared_codes", "shared_scales", "correction_mask"), n, dev)
+        codes4, mask4 = None, x.correction_mask.data_ptr()
+    else:
+        x.validate(w)
+        n = x.routed_codes.shape[0]
+        codes4, mask4 = x.routed_codes.data_ptr(), None
+    use8 = mask4 is not None or sw is not None
+    prep = _lib.Prepared(codes4, x.routed_scales.data_ptr(), x.topk_weights.data_ptr(), x.topk_ids.data_ptr(),
+                         x.shared_codes.data_ptr() if use8 else None, x.shared_scales.data_ptr() if use8 else None, mask4)
+    slots = shared = out = None
+    if return_partials:
+        slots = torch.empty((n, TOPK, H), dtype=torch.bfloat16, device=dev)
+        shared = None if sw is None else torch.empty((n, H), dtype=torch.bfloat16, device=dev)
+    else:
+        out = torch.empty((n, H), dtype=torch.bfloat16, device=dev)
+    layer_prepared(prep, n, w, sw, slots, shared, out, dev)
+    return (slots, shared) if return_partials else out
 
 
 def gather_mxfp4_moe(local: MoeInput, comm) -> MoeInputCompact:

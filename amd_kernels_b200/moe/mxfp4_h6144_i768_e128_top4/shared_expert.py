@@ -64,6 +64,10 @@ class SharedWeights:
     def intermediate(self) -> int:
         return self.w13.shape[0] * 64
 
+    def abi(self) -> _lib.SharedWeights:
+        """``struct b200moe_shared_weights`` over this object's tensors."""
+        return _lib.SharedWeights(self.w13.data_ptr(), self.w2.data_ptr())
+
     @classmethod
     def from_row_major(cls, w13, s13, w2, s2):
         """From row-major e4m3 [N, K] weights and e8m0 [N, K / 32] scales (gate rows, then up rows in ``w13``)."""

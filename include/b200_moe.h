@@ -405,6 +405,50 @@ size_t b200moe_workspace_bytes_x(int64_t tokens, int num_experts);
 int b200moe_forward_x(const b200moe_weights* w, const void* x_bf16, int64_t tokens, void* workspace,
                       size_t workspace_bytes, void* slots_bf16, void* out_bf16, int32_t* status, void* stream);
 
+/* The whole layer in one call, with or without the shared expert (MOE/chain.py:127-197 mxfp4_moe; the shared expert runs
+ * beside the routed experts inside the same launches at decode sizes, before them at prefill sizes, so no second stream is
+ * involved). logits fp32 [T][num_experts], or null: the router runs inside the call (w->gate). shared may be null.
+ * slots [T][4][6144], shared_out [T][6144] and out [T][6144] are bf16; a null slots (shared_out) means that the caller does
+ * not want it: it then lives in the workspace, and out must be given. Same bits as the separate calls.
+ * workspace: b200moe_layer_workspace_bytes(T, num_experts, flags) bytes, 256-byte aligned; flags: the sum of those below that
+ * hold for the call. */
+typedef struct b200moe_shared_weights {
+  const uint8_t* w13t; /* b200moe_preshuffle_shared */
+  const uint8_t* w2t;
+} b200moe_shared_weights;
+#define B200MOE_LAYER_ROUTER 1         /* no logits are given */
+#define B200MOE_LAYER_SHARED 2         /* shared is given */
+#define B200MOE_LAYER_OWN_SLOTS 4      /* slots is null */
+#define B200MOE_LAYER_OWN_SHARED_OUT 8 /* shared is given and shared_out is null */
+#define B200MOE_LAYER_COMPACT 16       /* a prepared input with a correction mask instead of FP4 codes */
+size_t b200moe_layer_workspace_bytes(int64_t tokens, int num_experts, int flags);
+int b200moe_layer(const b200moe_weights* w, const b200moe_shared_weights* shared, const void* x_bf16, const float* logits,
+                  int64_t tokens, void* workspace, size_t workspace_bytes, void* slots_bf16, void* shared_out_bf16,
+                  void* out_bf16, int32_t* status, void* stream);
+
+/* The same layer on a prepared input (MOE/prepared_input.py:159-187 mxfp4_moe on MoeInput / MoeInputCompact): row-major
+ * operands and routing as b200moe_prepare makes them. Either codes4 or (compact form) mask4, from which the codes are rebuilt;
+ * codes8 / scales8 are needed by the shared expert and by the compact form. */
+typedef struct b200moe_prepared {
+  const uint8_t* codes4;     /* [T][3072] or null */
+  const uint8_t* scales4;    /* [T][192] */
+  const float* topk_weights; /* [T][4] */
+  const int32_t* topk_ids;   /* [T][4] */
+  const uint8_t* codes8;     /* [T][6144] */
+  const uint8_t* scales8;    /* [T][192] */
+  const uint8_t* mask4;      /* [T][768] or null */
+} b200moe_prepared;
+int b200moe_layer_prepared(const b200moe_weights* w, const b200moe_shared_weights* shared, const b200moe_prepared* input,
+                           int64_t tokens, void* workspace, size_t workspace_bytes, void* slots_bf16, void* shared_out_bf16,
+                           void* out_bf16, int32_t* status, void* stream);
+
+/* Quantise and route a shard (MOE/prepared_input.py:117-136 prepare_mxfp4_moe): the payload carries exactly the routing and
+ * codes b200moe_layer computes from the same rows. partials: scratch, fp32 [b200moe_router_splits(T)][T][num_experts];
+ * codes8 / scales8 may both be null. */
+int b200moe_prepare(const b200moe_weights* w, const void* x_bf16, int64_t tokens, float* partials, uint8_t* codes4,
+                    uint8_t* scales4, float* topk_weights, int32_t* topk_ids, uint8_t* codes8, uint8_t* scales8,
+                    int32_t* status, void* stream);
+
 /* Host-buffer form of the same call, the one the end-to-end benchmark times: copies x and logits from (pinned) host
  * memory to `dev_x`/`dev_logits`, runs b200moe_forward, copies out to `host_out`, all on `stream`, no synchronise. */
 int b200moe_forward_host(const b200moe_weights* w, const void* host_x_bf16, const float* host_logits, int64_t tokens,

@@ -148,3 +148,34 @@ def test_argument_errors(S, shared_layer):
     bad = C.unsupported_reason(z(128, 2 * I, H // 2), z(128, 2 * I, H // 32), z(128, H, I // 2), z(128, H, I // 32),
                                z(2 * I, H), z(2 * I, H // 32), z(H, I, dt=e4), z(H, I // 32))
     assert bad is not None and "shared w13" in bad
+
+
+@pytest.mark.parametrize("m,router", [(1, True), (16, False), (17, True), (32, False), (33, True), (127, True), (128, True),
+                                      (481, False), (512, True)])
+def test_shared_expert_inside_the_routed_launches(S, shared_layer, config0, m, router):
+    """Up to 512 tokens the entry runs the shared expert on CTAs of the routed launches (one launch for both GEMMs up to 32
+    tokens, GEMM1's launch above; token blocks of 16 / 32 / 64 / 128, one to four of them): slots, shared rows and the reduced
+    sum bit for bit those of the separate calls, from bf16 rows and from the prepared forms."""
+    from amd_kernels_b200.moe.mxfp4_h6144_i768_e128_top4 import chain as C, prepared_input as P
+    _, sw = shared_layer
+    raw, _, _ = config0
+    gen = torch.Generator().manual_seed(300 + m)
+    gate = (torch.randn((128, H), generator=gen) / H ** 0.5).cuda()
+    on_gpu = [dev(a) for a in raw]
+    w0 = C.MoeWeights.from_row_major(gate, None, *on_gpu)
+    w1 = C.MoeWeights.from_row_major(gate, None, *on_gpu, shared=sw)
+    x = random_rows(m, 900 + m).cuda()
+    lg = None if router else torch.randn((m, 128), generator=gen).cuda()
+    slots0, _ = C.mxfp4_moe(x, w0, return_partials=True, router_logits=lg)
+    want = S.shared_expert(x, sw)
+    slots, shared = C.mxfp4_moe(x, w1, return_partials=True, router_logits=lg)
+    out = C.mxfp4_moe(x, w1, router_logits=lg)
+    assert torch.equal(slots, slots0) and torch.equal(shared, want)
+    assert torch.equal(out, C.reduce_slots(slots0, want))
+    if router:
+        inp = P.prepare_mxfp4_moe(x, w1)
+        for form in (inp, inp.compact()):
+            p_slots, p_shared = C.mxfp4_moe(form, w1, return_partials=True)
+            assert torch.equal(p_slots, slots0) and torch.equal(p_shared, want)
+    torch.cuda.synchronize()
+    assert C.last_status() == 0
