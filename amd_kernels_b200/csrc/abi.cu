@@ -61,6 +61,7 @@ int shared_gemms(const uint8_t* w13t, const uint8_t* w2t, const uint8_t* codes8,
                  void* out_bf16, int64_t tokens, int32_t* status, void* stream);
 int set_wait_limit_routed(unsigned long long ns);
 int set_wait_limit_shared(unsigned long long ns);
+int set_wait_limit_shared_pair(unsigned long long ns);
 int set_wait_limit_pair(unsigned long long ns);
 int set_wait_limit_router(unsigned long long ns);
 int set_wait_limit_ep_sync(unsigned long long ns);
@@ -129,6 +130,7 @@ extern "C" int b200moe_set_wait_limit_ns(uint64_t ns) {
   if (ns == 0) return B200MOE_E_ARG;
   int r = b200moe::set_wait_limit_routed(ns);
   if (!r) r = b200moe::set_wait_limit_shared(ns);
+  if (!r) r = b200moe::set_wait_limit_shared_pair(ns);
   if (!r) r = b200moe::set_wait_limit_pair(ns);
   if (!r) r = b200moe::set_wait_limit_router(ns);
   if (!r) r = b200moe::set_wait_limit_ep_sync(ns);

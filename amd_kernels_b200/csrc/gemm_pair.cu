@@ -21,10 +21,7 @@
 //
 // No load is a multicast load; stage release and accumulator hand-over use one plain tcgen05.commit per CTA. Every wait
 // is bounded as in the other kernels (status word B200MOE_DEV_TIMEOUT, drain, free, return).
-#include <cuda.h>
-
-#include "tc_host.cuh"
-#include "tc_ptx.cuh"
+#include "tc_pair.cuh"
 
 namespace b200moe {
 
@@ -50,40 +47,6 @@ struct PairCfg {
 static_assert(PairCfg::kSfCol + 24 * PairCfg::kSfSets <= PairCfg::kTmemCols, "tensor memory columns");
 static_assert(kW13Tiles % 2 == 0, "W13 tiles come in pairs");
 
-// ------------------------------------------------------------------------------------------------ PTX, pair forms
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-// the shared::cluster address of `addr` (a shared::cta address of this CTA) in CTA `rank` of the cluster
-__device__ __forceinline__ uint32_t map_to_cta(uint32_t addr, uint32_t rank) {
-  uint32_t out;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(out) : "r"(addr), "r"(rank));
-  return out;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
-// 2-D tile load whose bytes are counted on a barrier that may sit in the partner CTA (`bar` is a shared::cluster address)
-__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::
-          "r"(dst),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(x), "r"(y)
-      : "memory");
-}
-__device__ __forceinline__ void tc_commit_pair(uint32_t cluster_addr) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(cluster_addr) : "memory");
-}
-__device__ __forceinline__ void tc_cp_scales_pair(uint32_t taddr, uint32_t desc_lo) {
-  asm volatile("{\n.reg .b64 d;\nmov.b64 d, {%1, %2};\ntcgen05.cp.cta_group::2.32x128b.warpx4 [%0], d;\n}\n" ::"r"(taddr),
-               "r"(desc_lo), "n"(kScaleDescHi)
-               : "memory");
-}
 __device__ __forceinline__ void tc_mma_mxf4_pair(uint32_t d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t sfa,
                                                  uint32_t sfb, uint32_t accumulate) {
   asm volatile(
@@ -92,12 +55,6 @@ __device__ __forceinline__ void tc_mma_mxf4_pair(uint32_t d, uint32_t a_lo, uint
       "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(sfa), "r"(sfb), "r"(accumulate), "n"(kOperandDescHi)
       : "memory");
 }
-__device__ __forceinline__ void drain_tcgen05_pair(uint32_t bar) {
-  tc_commit_pair(bar);
-  const uint64_t t0 = global_timer(), limit = wait_limit_ns();
-  while (!mbar_try_wait(bar, 0) && global_timer() - t0 < limit) {}
-}
-
 // One (token row, 32-column group of the intermediate): SwiGLU-OAI of the 32 gate / up accumulators, the block maximum, the
 // E8M0 byte and the 32 E2M1 codes -> one 16-byte store of codes and one scale byte; everything thread-local.
 __device__ __forceinline__ void swiglu_quant_store(const uint32_t (&gv)[32], const uint32_t (&uv)[32], uint8_t* hq,
@@ -657,7 +614,6 @@ __global__ void __launch_bounds__(WideCfg::kThreads, 1)
           if (!mbar_wait(smem_u32(&bar_sf[j]), sph, abort_v, status)) { ok = false; break; }   // long since complete
           if (!mbar_wait(smem_u32(&bar_full[s]), ph, abort_v, status)) { ok = false; break; }  // the wait that matters
           tc_fence_after();
-          if (GATHER) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // rows written by plain copies
           const uint32_t lo = (tiles + s * C::kStageBytes) >> 4;
           const uint32_t x_lo = lo + (C::kTokOff >> 4), w_lo = lo + (C::kWOff >> 4);
           const uint32_t t_sft = tmem_base + C::kSfCol + 24u * j, t_sfw = t_sft + 8u;
@@ -742,50 +698,12 @@ __global__ void __launch_bounds__(WideCfg::kThreads, 1)
 }
 
 // ------------------------------------------------------------------------------------------------ host side
-// byte matrix [rows][128], boxes of 128 bytes x box_rows, no swizzle (the bytes are stored as shared memory wants them)
-static int make_flat_map(CUtensorMap* map, const void* base, uint64_t rows, uint32_t box_rows) {
-  EncodeTiledFn fn = encode_fn();
-  if (!fn) return B200MOE_E_DRIVER;
-  const cuuint64_t dims[2] = {128, rows};
-  const cuuint64_t strides[1] = {128};
-  const cuuint32_t box[2] = {128, box_rows};
-  const cuuint32_t estr[2] = {1, 1};
-  const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, estr,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? 0 : B200MOE_E_DRIVER;
-}
-
 // CTA pairs that can be resident at once on the current device (0: cluster launch unavailable)
 static int resident_pairs() {
   static std::mutex mu;
   static int pairs[kMaxDevices] = {};
   static bool known[kMaxDevices] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 0;
-  std::lock_guard<std::mutex> lock(mu);
-  if (!known[dev]) {
-    int n = 0;
-    if (cudaFuncSetAttribute(gemm1_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PairCfg::kSmemBytes) ==
-        cudaSuccess) {
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3(2 * sm_count());
-      cfg.blockDim = dim3(PairCfg::kThreads);
-      cfg.dynamicSmemBytes = PairCfg::kSmemBytes;
-      cudaLaunchAttribute attr[1];
-      attr[0].id = cudaLaunchAttributeClusterDimension;
-      attr[0].val.clusterDim.x = 2;
-      attr[0].val.clusterDim.y = 1;
-      attr[0].val.clusterDim.z = 1;
-      cfg.attrs = attr;
-      cfg.numAttrs = 1;
-      if (cudaOccupancyMaxActiveClusters(&n, gemm1_pair_kernel, &cfg) != cudaSuccess) n = 0;
-    }
-    (void)cudaGetLastError();
-    pairs[dev] = n;
-    known[dev] = true;
-  }
-  return pairs[dev];
+  return resident_pairs_of(gemm1_pair_kernel, PairCfg::kThreads, PairCfg::kSmemBytes, mu, known, pairs);
 }
 
 int set_wait_limit_pair(unsigned long long ns) { return set_wait_limit_here(ns); }
@@ -889,21 +807,6 @@ extern "C" int b200moe_gemm1_swiglu_quant_pair(const uint8_t* w13t, int num_expe
   if ((r = make_flat_map(&mws, w13t, w_rows, 8))) return r;
   const int64_t max_units = max_rows / 128 * PairCfg::kTilePairs;
   const int clusters = static_cast<int>(max_units < pairs ? max_units : pairs);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(2 * clusters);
-  cfg.blockDim = dim3(PairCfg::kThreads);
-  cfg.dynamicSmemBytes = PairCfg::kSmemBytes;
-  cfg.stream = static_cast<cudaStream_t>(stream);
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 2;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm1_pair_kernel, mx, msf, mwc, mws, block_expert, num_valid, hq, sfh,
-                                           status, num_experts, static_cast<int>(max_rows / 128));
-  return e == cudaSuccess ? 0 : static_cast<int>(e);
+  return launch_pairs(gemm1_pair_kernel, clusters, PairCfg::kThreads, PairCfg::kSmemBytes, static_cast<cudaStream_t>(stream), mx,
+                      msf, mwc, mws, block_expert, num_valid, hq, sfh, status, num_experts, static_cast<int>(max_rows / 128));
 }

@@ -413,6 +413,11 @@ int shared_plan(SharedPlan* plan, const uint8_t* w13t, const uint8_t* w2t, const
   return 0;
 }
 
+// shared_pair.cu
+bool shared_pair_supported();
+int shared_gemms_pair(const CUtensorMap& map_x, const CUtensorMap& map_h, const uint8_t* w13t, const uint8_t* w2t,
+                      const SharedWorkspace& ws, void* out_bf16, int64_t tokens, int32_t* status, cudaStream_t stream);
+
 int set_wait_limit_shared(unsigned long long ns) { return set_wait_limit_here(ns); }
 
 }  // namespace b200moe
@@ -464,6 +469,12 @@ extern "C" int b200moe_shared_quant_rows(const void* x_bf16, int64_t tokens, uin
 }
 
 namespace b200moe {
+// From this many blocks of 128 tokens on both GEMMs run on CTA pairs (shared_pair.cu). Measured, both GEMMs and the scale layout,
+// one-CTA kernel / pairs, us: 38 / 42 at 777 tokens, 40 / 42 at 1024, 44 / 44 at 1400, 60 / 46 at 1800, 93 / 75 at 4096, 167 / 114
+// at 8191, 303 / 202 at 16384. Below, a GEMM1 unit per pair leaves most SMs idle (24 pairs busy at 1024 tokens) and one unit's
+// chain of 48 K-tiles is the time; the one-CTA kernel has four times the units.
+constexpr int kSharedPairBlocks = 12;
+
 int shared_gemms(const uint8_t* w13t, const uint8_t* w2t, const uint8_t* codes8, int64_t code_rows, const SharedWorkspace& ws,
                  void* out_bf16, int64_t tokens, int32_t* status, void* stream) {
   const int n_blocks = static_cast<int>(ws.rows / ws.bm);
@@ -473,6 +484,8 @@ int shared_gemms(const uint8_t* w13t, const uint8_t* w2t, const uint8_t* codes8,
   // code_rows may be the unpadded token count: boxes that reach beyond it read zeros
   if ((r = make_map(&mx, codes8, kH, static_cast<uint64_t>(code_rows), static_cast<uint32_t>(ws.bm)))) return r;
   if ((r = make_map(&mh, ws.h8, kI, static_cast<uint64_t>(ws.rows), static_cast<uint32_t>(ws.bm)))) return r;
+  if (ws.bm == 128 && n_blocks >= kSharedPairBlocks && shared_pair_supported())
+    return shared_gemms_pair(mx, mh, w13t, w2t, ws, out_bf16, tokens, status, st);
   SharedEpilogue ep{};
   ep.h8 = ws.h8;
   ep.sfh8 = ws.sfh8;

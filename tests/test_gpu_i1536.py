@@ -123,3 +123,17 @@ def test_shared_expert_of_the_sibling_shape(P, C, tokens):
     got = out.float().cpu().numpy()
     cos = (got * ref).sum(1) / np.linalg.norm(got, axis=1) / np.linalg.norm(ref, axis=1)
     assert cos.min() >= 0.9999 and np.linalg.norm(got - ref) / np.linalg.norm(ref) < 4e-3
+
+
+@pytest.mark.parametrize("tokens", [1409, 1665])
+def test_shared_expert_on_cta_pairs(P, C, tokens):
+    """The pair kernels (12 blocks of 128 tokens and more) at this intermediate: 12 tile pairs and 12 K-tiles in the second GEMM,
+    an even and an odd number of blocks; the bits of batches of 256."""
+    from amd_kernels_b200.moe.mxfp4_h6144_i768_e128_top4 import shared_expert as S
+    sw = P.SharedWeights.from_row_major(*(dev(a) for a in orc.make_shared_weights(seed=611, inter=I2)))
+    x = (torch.randn((tokens, H), generator=torch.Generator().manual_seed(tokens)) * 0.5).bfloat16().cuda()
+    out = S.shared_expert(x, sw)
+    for a in range(0, tokens, 256):
+        assert torch.equal(S.shared_expert(x[a:a + 256].contiguous(), sw), out[a:a + 256])
+    torch.cuda.synchronize()
+    assert C.last_status() == 0

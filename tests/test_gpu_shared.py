@@ -88,6 +88,18 @@ def test_output_matches_oracle_and_is_batch_invariant(S, shared_layer, m):
     assert torch.equal(alone, out[pick])
 
 
+@pytest.mark.parametrize("m", [1408, 1409, 1536, 1537, 1665, 2048, 3001])
+def test_pair_kernels_give_the_small_batch_bits(S, shared_layer, m):
+    """From 12 blocks of 128 tokens on both GEMMs run on CTA pairs: at the edge of that rule, with an even and an odd number of
+    blocks (an idle partner) and with one row in the last block, every row has the bits that it gets in a batch of 256."""
+    _, sw = shared_layer
+    x = random_rows(m, 700 + m).cuda()
+    out = S.shared_expert(x, sw)
+    for a in range(0, m, 256):
+        assert torch.equal(S.shared_expert(x[a:a + 256].contiguous(), sw), out[a:a + 256])
+    assert torch.equal(S.shared_expert(x, sw, x_quant=S.shared_quant_rows(x)), out)
+
+
 def test_graph_replay_and_side_stream(S, shared_layer):
     _, sw = shared_layer
     x = random_rows(48, 5).cuda()
