@@ -604,16 +604,20 @@ __global__ void __launch_bounds__(WideCfg::kThreads, 1)
                                   (static_cast<uint32_t>(128 >> 4) << 24);
       constexpr uint32_t kId0 = kIdesc, kId1 = kIdesc | (2u << 29) | (2u << 4);
       uint32_t it = 0, ui = 0;
-      bool ok = true;
+      bool ok = true, sf_ready = false, full_ready = false;
       for (int u = first; u < total && ok; u += stride, ++ui) {
         if (!mbar_wait(smem_u32(&bar_tempty), (ui & 1u) ^ 1u, abort_v, status)) break;
         tc_fence_after();
-        for (int kt = 0; kt < kK1Tiles; ++kt, ++it) {
+        for (int kt = 0; kt < kK1Tiles; ++kt) {
           const uint32_t s = it % C::kStages, ph = (it / C::kStages) & 1u;
           const uint32_t j = it % C::kSfStages, sph = (it / C::kSfStages) & 1u;
-          if (!mbar_wait(smem_u32(&bar_sf[j]), sph, abort_v, status)) { ok = false; break; }   // long since complete
-          if (!mbar_wait(smem_u32(&bar_full[s]), ph, abort_v, status)) { ok = false; break; }  // the wait that matters
+          if (!sf_ready && !mbar_wait(smem_u32(&bar_sf[j]), sph, abort_v, status)) { ok = false; break; }
+          if (!full_ready && !mbar_wait(smem_u32(&bar_full[s]), ph, abort_v, status)) { ok = false; break; }
           tc_fence_after();
+          ++it;  // look at the next K-tile's barriers while this one's MMAs are issued (320 -> 308 us at 16384 tokens)
+          sf_ready = mbar_test(smem_u32(&bar_sf[it % C::kSfStages]), (it / C::kSfStages) & 1u);
+          full_ready = mbar_test(smem_u32(&bar_full[it % C::kStages]), (it / C::kStages) & 1u);
+          if (GATHER) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // rows written by plain copies
           const uint32_t lo = (tiles + s * C::kStageBytes) >> 4;
           const uint32_t x_lo = lo + (C::kTokOff >> 4), w_lo = lo + (C::kWOff >> 4);
           const uint32_t t_sft = tmem_base + C::kSfCol + 24u * j, t_sfw = t_sft + 8u;
@@ -632,15 +636,18 @@ __global__ void __launch_bounds__(WideCfg::kThreads, 1)
     if (lane == 0) {
       const bool head = warp == 2;
       uint32_t it = 0;
-      bool ok = true;
+      bool ok = true, landed = false, free_set = false;
       for (int u = first; u < total && ok; u += stride) {
-        for (int kt = 0; kt < kK1Tiles; ++kt, ++it) {
+        for (int kt = 0; kt < kK1Tiles; ++kt) {
           const uint32_t s = it % C::kStages, ph = (it / C::kStages) & 1u;
           const uint32_t j = it % C::kSfStages, sph = (it / C::kSfStages) & 1u;
-          if (!mbar_wait(smem_u32(&bar_sfull[j]), sph, abort_v, status)) { ok = false; break; }
+          if (!landed && !mbar_wait(smem_u32(&bar_sfull[j]), sph, abort_v, status)) { ok = false; break; }
           // scale set j was last read by the MMAs of K-tile it - 8: complete once those of K-tile it - 4 are
-          if (!mbar_wait(smem_u32(&bar_empty[s]), ph ^ 1u, abort_v, status)) { ok = false; break; }
+          if (!free_set && !mbar_wait(smem_u32(&bar_empty[s]), ph ^ 1u, abort_v, status)) { ok = false; break; }
           tc_fence_after();
+          ++it;
+          landed = mbar_test(smem_u32(&bar_sfull[it % C::kSfStages]), (it / C::kSfStages) & 1u);
+          free_set = mbar_test(smem_u32(&bar_empty[it % C::kStages]), ((it / C::kStages) & 1u) ^ 1u);
           if (GATHER) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
           const uint32_t lo = (sf_ring + j * C::kSfSlotBytes) >> 4;
           const uint32_t t_sft = tmem_base + C::kSfCol + 24u * j, t_sfw = t_sft + 8u;
