@@ -109,6 +109,51 @@ def test_route_matches_oracle(C, m, mode):
     assert torch.equal(ids, ids2) and torch.equal(wt, wt2)
 
 
+def _pick4(row):
+    """The selection rule, one value at a time: the larger value wins, equal values go to the lower id, a NaN never wins, a
+    picked value counts as -inf from then on, and where nothing comparable is left the round number is the pick."""
+    v, ids = row.copy(), []
+    for r in range(4):
+        best = -1
+        for e in range(len(v)):
+            if not np.isnan(v[e]) and (best < 0 or v[e] > v[best]):
+                best = e
+        ids.append(best if best >= 0 else r)
+        if ids[-1] < len(v):
+            v[ids[-1]] = -np.inf
+    return ids
+
+
+@pytest.mark.parametrize("experts", [4, 8, 33, 127, 128])
+@pytest.mark.parametrize("splits,offset", [(1, 0), (1, 1), (3, 0), (8, 0), (9, 2), (16, 0), (17, 0)])
+def test_route_special_values_and_row_layouts(C, experts, splits, offset):
+    """NaNs, infinities, signed zeros, subnormals and the type's lowest value, on rows that start on and off a 16-byte boundary
+    and for split counts around the batches that are loaded at a time: ids by the selection rule, weights those of the oracle's
+    formula on finite rows."""
+    rng = np.random.default_rng(100 * experts + splits)
+    lg = rng.standard_normal((12, experts)).astype(np.float32)
+    lg[0] = np.nan
+    lg[1] = -np.inf
+    lg[2] = np.finfo(np.float32).min
+    lg[3] = np.where(np.arange(experts) % 2, 0.0, -0.0)
+    lg[4, ::2] = np.nan
+    lg[5, :] = -np.inf
+    lg[5, -1] = 1.0
+    lg[6, 0] = np.inf
+    lg[7, 1:] = np.nan
+    lg[8] = rng.integers(-3, 4, experts) * np.float32(1e-45)
+    # split 0 carries the value, the others zeros (x + 0.0 is x, and -0.0 + 0.0 is 0.0, which ties with it)
+    flat = torch.zeros(splits * 12 * experts + 8, device="cuda")
+    parts = flat[offset:offset + splits * 12 * experts].view(splits, 12, experts)
+    parts[0] = dev(lg)
+    wt, ids = C.topk_route(parts.permute(1, 0, 2), None, 1.0, "softmax")
+    want = np.array([_pick4(r) for r in lg])
+    assert np.array_equal(ids.cpu().numpy(), want)
+    sel = np.take_along_axis(lg[9:], want[9:], 1).astype(np.float64)
+    p = np.exp(sel - sel[:, :1])
+    np.testing.assert_allclose(wt.cpu().numpy()[9:], p / p.sum(1, keepdims=True), rtol=orc.WEIGHT_RTOL)
+
+
 @pytest.mark.parametrize("m", [1, 5, 16, 17, 64, 255, 256, 257, 1000, 4097])
 @pytest.mark.parametrize("kind", ["uniform", "hot", "four", "one", "dup"])
 def test_permute_bit_exact(C, m, kind):
