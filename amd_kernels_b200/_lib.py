@@ -98,9 +98,9 @@ SIGNATURES = {
     "b200moe_workspace_bytes": (c_size_t, [c_int64, c_int]),
     "b200moe_workspace_bytes_x": (c_size_t, [c_int64, c_int]),
     "b200moe_layer_workspace_bytes": (c_size_t, [c_int64, c_int, c_int]),
-    "b200moe_layer": (c_int, [POINTER(Weights), POINTER(SharedWeights), _P, _P, c_int64, _P, c_size_t, _P, _P, _P, _P, _P]),
+    "b200moe_layer": (c_int, [POINTER(Weights), POINTER(SharedWeights), _P, _P, c_int64, _P, c_size_t, _P, _P, _P, _P, _P, _P]),
     "b200moe_layer_prepared": (c_int, [POINTER(Weights), POINTER(SharedWeights), POINTER(Prepared), c_int64, _P, c_size_t, _P,
-                                       _P, _P, _P, _P]),
+                                       _P, _P, _P, _P, _P]),
     "b200moe_prepare": (c_int, [POINTER(Weights), _P, c_int64, _P, _P, _P, _P, _P, _P, _P, _P, _P]),
     "b200moe_forward_x": (c_int, [POINTER(Weights), _P, c_int64, _P, c_size_t, _P, _P, _P, _P]),
     "b200moe_set_wait_limit_ns": (c_int, [c_uint64]),

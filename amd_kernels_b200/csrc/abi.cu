@@ -153,6 +153,40 @@ struct LayerCall {
   void *slots, *shared_out, *out;
   int32_t* status;
   void* stream;
+  void* side;  // may be null: another stream of the device, for the shared expert's two GEMMs above 512 tokens
+};
+
+// The side stream's part of a call: starts behind what the main stream holds at fork() and is joined by join(), at the latest when
+// the call returns, error returns included (a capture must not end with an unjoined stream, and the caller frees the workspace in
+// main-stream order). Both events live for the call only, so calls from several threads and streams share nothing.
+class SideStream {
+ public:
+  SideStream(void* main, void* side) : main_(static_cast<cudaStream_t>(main)), side_(static_cast<cudaStream_t>(side)) {}
+  ~SideStream() {
+    (void)join();
+    if (begin_) cudaEventDestroy(begin_);
+    if (end_) cudaEventDestroy(end_);
+  }
+  int fork() {
+    cudaError_t e = cudaEventCreateWithFlags(&begin_, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&end_, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventRecord(begin_, main_);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(side_, begin_, 0);
+    forked_ = e == cudaSuccess;
+    return static_cast<int>(e);
+  }
+  int join() {
+    if (!forked_) return 0;
+    forked_ = false;
+    cudaError_t e = cudaEventRecord(end_, side_);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(main_, end_, 0);
+    return static_cast<int>(e);
+  }
+
+ private:
+  cudaStream_t main_, side_;
+  cudaEvent_t begin_ = nullptr, end_ = nullptr;
+  bool forked_ = false;
 };
 
 static int run_layer(const LayerCall& c) {
@@ -192,7 +226,7 @@ static int run_layer(const LayerCall& c) {
   const uint8_t* codes8 = c.prep ? c.prep->codes8 : ws.sh.x8;
   bool have_q4 = true;
   int r = 0;
-
+  SideStream side(c.stream, c.side);
   // the operands: quantised rows and, with the router inside, the logits' split-K partials
   if (c.prep) {
     if (compact) {
@@ -222,8 +256,10 @@ static int run_layer(const LayerCall& c) {
       if ((r = shared_plan(&plan, c.shared->w13t, c.shared->w2t, codes8, tokens, ws.sh, shared_out, tokens, ws.done + blocks)))
         return r;
       sp = &plan;
-    } else if ((r = shared_gemms(c.shared->w13t, c.shared->w2t, codes8, tokens, ws.sh, shared_out, tokens, c.status, st))) {
-      return r;
+    } else {  // beside the routing and the sort, whose few short launches leave the SMs to it
+      if (c.side && (r = side.fork())) return r;
+      r = shared_gemms(c.shared->w13t, c.shared->w2t, codes8, tokens, ws.sh, shared_out, tokens, c.status, c.side ? c.side : st);
+      if (r) return r;
     }
   }
 
@@ -267,6 +303,7 @@ static int run_layer(const LayerCall& c) {
                                     ws.rows, ws.bm, tokens, slots, c.status, st)))
       return r;
   }
+  if ((r = side.join())) return r;
   if (c.out && (r = b200moe_reduce_slots(slots, shared ? shared_out : nullptr, tokens, c.out, st))) return r;
   return 0;
 }
@@ -274,17 +311,18 @@ static int run_layer(const LayerCall& c) {
 
 extern "C" int b200moe_layer(const b200moe_weights* w, const b200moe_shared_weights* shared, const void* x_bf16,
                              const float* logits, int64_t tokens, void* workspace, size_t workspace_bytes, void* slots_bf16,
-                             void* shared_out_bf16, void* out_bf16, int32_t* status, void* stream) {
+                             void* shared_out_bf16, void* out_bf16, int32_t* status, void* stream,
+                             void* side_stream) {
   return b200moe::run_layer({w, shared, x_bf16, nullptr, logits, tokens, workspace, workspace_bytes, slots_bf16,
-                             shared_out_bf16, out_bf16, status, stream});
+                             shared_out_bf16, out_bf16, status, stream, side_stream});
 }
 
 extern "C" int b200moe_layer_prepared(const b200moe_weights* w, const b200moe_shared_weights* shared,
                                       const b200moe_prepared* input, int64_t tokens, void* workspace, size_t workspace_bytes,
                                       void* slots_bf16, void* shared_out_bf16, void* out_bf16, int32_t* status,
-                                      void* stream) {
+                                      void* stream, void* side_stream) {
   return b200moe::run_layer({w, shared, nullptr, input, nullptr, tokens, workspace, workspace_bytes, slots_bf16,
-                             shared_out_bf16, out_bf16, status, stream});
+                             shared_out_bf16, out_bf16, status, stream, side_stream});
 }
 
 extern "C" int b200moe_prepare(const b200moe_weights* w, const void* x_bf16, int64_t tokens, float* partials, uint8_t* codes4,
@@ -313,7 +351,7 @@ extern "C" int b200moe_forward_x(const b200moe_weights* w, const void* x_bf16, i
                                  void* stream) {
   if (!slots_bf16) return B200MOE_E_ARG;
   return b200moe_layer(w, nullptr, x_bf16, nullptr, tokens, workspace, workspace_bytes, slots_bf16, nullptr, out_bf16, status,
-                       stream);
+                       stream, nullptr);
 }
 
 extern "C" int b200moe_forward(const b200moe_weights* w, const void* x_bf16, const float* logits, int64_t tokens,
@@ -321,7 +359,7 @@ extern "C" int b200moe_forward(const b200moe_weights* w, const void* x_bf16, con
                                int32_t* status, void* stream) {
   if (!slots_bf16 || !logits) return B200MOE_E_ARG;
   return b200moe_layer(w, nullptr, x_bf16, logits, tokens, workspace, workspace_bytes, slots_bf16, nullptr, out_bf16, status,
-                       stream);
+                       stream, nullptr);
 }
 
 extern "C" int b200moe_forward_host(const b200moe_weights* w, const void* host_x_bf16, const float* host_logits,

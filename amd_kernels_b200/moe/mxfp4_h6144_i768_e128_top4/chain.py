@@ -563,7 +563,8 @@ def layer_prepared(prep, n, w, sw, slots, shared, out, dev):
     _lib.check(lib.b200moe_layer_prepared(
         ctypes.byref(w.abi()), None if sw is None else ctypes.byref(sw.abi()), ctypes.byref(prep), n, workspace.data_ptr(),
         ws_bytes, None if slots is None else slots.data_ptr(), None if shared is None else shared.data_ptr(),
-        None if out is None else out.data_ptr(), status_word(dev).data_ptr(), _raw_stream(dev)), "layer_prepared")
+        None if out is None else out.data_ptr(), status_word(dev).data_ptr(), _raw_stream(dev), _side_stream(sw, n)),
+        "layer_prepared")
 
 
 def _result_flags(sw, slots, shared):
@@ -573,10 +574,18 @@ def _result_flags(sw, slots, shared):
     return flags
 
 
-# Token count from which the shared expert runs on the side stream: below, it is a role of a routed launch (48 against 161 us
-# for the layer at 1 token, 112 against 244 at 32, most of it host time); above, in front of the routed kernels on one stream
-# it made the layer 2 to 3 % slower (240 -> 245 us at 777 tokens).
+# Token count above which the shared expert's GEMMs are launches of their own, on the side stream: below, it is a role of a routed
+# launch (48 against 161 us for the layer at 1 token, 112 against 244 at 32, most of it host time). The side stream's work starts
+# behind the quantisation of x, which serves both experts in one pass, and is joined inside the C call.
 SIDE_STREAM_FROM = 512
+
+
+def _side_stream(sw, n):
+    """The raw handle of the device's side stream for a call of ``n`` tokens, None: not needed, or a DBO microbatch."""
+    if sw is None or n <= SIDE_STREAM_FROM:
+        return None
+    from .shared_expert import in_dbo
+    return None if in_dbo() else sw.stream.cuda_stream
 
 
 def mxfp4_moe(x, w, *, return_partials=False, router_logits=None):
@@ -585,8 +594,8 @@ def mxfp4_moe(x, w, *, return_partials=False, router_logits=None):
     Reduced mode returns BF16 [M, 6144] = slots 0..3, then the shared expert's output, summed in fp32; partials mode
     returns (slots BF16 [M, 4, H], shared BF16 [M, H]); without ``w.shared_weights`` the shared term is absent (None).
     ``router_logits`` fp32 [M, E] skips the router GEMM. The whole layer is one C-ABI call (``b200moe_layer``) on the current
-    stream: up to 512 tokens the shared expert runs on SMs of its own inside the routed experts' launches; above, it runs on
-    the device's side stream, which the current stream joins before the reduce. Scratch and outputs come from ``torch.empty``."""
+    stream: up to 512 tokens the shared expert runs on SMs of its own inside the routed experts' launches; above, its GEMMs run
+    on the device's side stream, which the current stream joins before the reduce. Scratch and outputs come from ``torch.empty``."""
     if not isinstance(x, torch.Tensor):
         from .prepared_input import MoeInput, MoeInputCompact, mxfp4_moe_prepared
         if not isinstance(x, (MoeInput, MoeInputCompact)):
@@ -615,26 +624,14 @@ def mxfp4_moe(x, w, *, return_partials=False, router_logits=None):
             shared = torch.empty((n, H), dtype=torch.bfloat16, device=dev)
     else:
         out = torch.empty((n, H), dtype=torch.bfloat16, device=dev)
-    side = sw is not None and n > SIDE_STREAM_FROM
-    if side:
-        from .shared_expert import shared_expert_parallel
-        shared, sw, side_stream = shared_expert_parallel(x, sw, torch.cuda.current_stream(dev)), None, sw.stream
-        if slots is None:
-            slots = torch.empty((n, TOPK, H), dtype=torch.bfloat16, device=dev)
-            out = None
     flags |= _result_flags(sw, slots, shared)
     ws_bytes = lib.b200moe_layer_workspace_bytes(n, n_exp, flags)
     workspace = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
     _lib.check(lib.b200moe_layer(
         ctypes.byref(w.abi()), None if sw is None else ctypes.byref(sw.abi()), x.data_ptr(),
         None if logits is None else logits.data_ptr(), n, workspace.data_ptr(), ws_bytes,
-        None if slots is None else slots.data_ptr(), None if shared is None or side else shared.data_ptr(),
-        None if out is None else out.data_ptr(), status_word(dev).data_ptr(), _raw_stream(dev)), "layer")
-    if side:
-        current = torch.cuda.current_stream(dev)
-        current.wait_stream(side_stream)
-        shared.record_stream(current)
-        out = None if return_partials else reduce_slots(slots, shared)
+        None if slots is None else slots.data_ptr(), None if shared is None else shared.data_ptr(),
+        None if out is None else out.data_ptr(), status_word(dev).data_ptr(), _raw_stream(dev), _side_stream(sw, n)), "layer")
     return (slots, shared) if return_partials else out
 
 

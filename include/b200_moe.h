@@ -406,8 +406,10 @@ int b200moe_forward_x(const b200moe_weights* w, const void* x_bf16, int64_t toke
                       size_t workspace_bytes, void* slots_bf16, void* out_bf16, int32_t* status, void* stream);
 
 /* The whole layer in one call, with or without the shared expert (MOE/chain.py:127-197 mxfp4_moe; the shared expert runs
- * beside the routed experts inside the same launches at decode sizes, before them at prefill sizes, so no second stream is
- * involved). logits fp32 [T][num_experts], or null: the router runs inside the call (w->gate). shared may be null.
+ * beside the routed experts inside the same launches up to 512 tokens; above, its two GEMMs are launches of their own, on
+ * side_stream when one is given: they start behind the input's quantisation and are joined before the reduce, or before the call
+ * returns. side_stream, another stream of the same device, may be null). logits fp32 [T][num_experts], or null: the router
+ * runs inside the call (w->gate). shared may be null.
  * slots [T][4][6144], shared_out [T][6144] and out [T][6144] are bf16; a null slots (shared_out) means that the caller does
  * not want it: it then lives in the workspace, and out must be given. Same bits as the separate calls.
  * workspace: b200moe_layer_workspace_bytes(T, num_experts, flags) bytes, 256-byte aligned; flags: the sum of those below that
@@ -424,7 +426,7 @@ typedef struct b200moe_shared_weights {
 size_t b200moe_layer_workspace_bytes(int64_t tokens, int num_experts, int flags);
 int b200moe_layer(const b200moe_weights* w, const b200moe_shared_weights* shared, const void* x_bf16, const float* logits,
                   int64_t tokens, void* workspace, size_t workspace_bytes, void* slots_bf16, void* shared_out_bf16,
-                  void* out_bf16, int32_t* status, void* stream);
+                  void* out_bf16, int32_t* status, void* stream, void* side_stream);
 
 /* The same layer on a prepared input (MOE/prepared_input.py:159-187 mxfp4_moe on MoeInput / MoeInputCompact): row-major
  * operands and routing as b200moe_prepare makes them. Either codes4 or (compact form) mask4, from which the codes are rebuilt;
@@ -440,7 +442,7 @@ typedef struct b200moe_prepared {
 } b200moe_prepared;
 int b200moe_layer_prepared(const b200moe_weights* w, const b200moe_shared_weights* shared, const b200moe_prepared* input,
                            int64_t tokens, void* workspace, size_t workspace_bytes, void* slots_bf16, void* shared_out_bf16,
-                           void* out_bf16, int32_t* status, void* stream);
+                           void* out_bf16, int32_t* status, void* stream, void* side_stream);
 
 /* Quantise and route a shard (MOE/prepared_input.py:117-136 prepare_mxfp4_moe): the payload carries exactly the routing and
  * codes b200moe_layer computes from the same rows. partials: scratch, fp32 [b200moe_router_splits(T)][T][num_experts];
