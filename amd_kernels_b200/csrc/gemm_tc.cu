@@ -584,6 +584,33 @@ __global__ void __launch_bounds__((Cfg<MODE, BM>::kThreads), 1)
 // add on done[b]) and the GEMM2 producer waits -- bounded like every other wait -- until done[b] == 12 before it loads h.
 // GEMM1 units never wait, so progress does not depend on scheduling order. What this buys over two launches: no ramp
 // between the kernels, and the short GEMM2 units (52 KB of weights) fill the uneven last round of GEMM1 (418 KB units).
+//
+// Dealing. GEMM1 units are 8 (I = 1536: 4) times as long as GEMM2 units, so an unfinished last round of them is made up in the
+// second list: with units1 = q n + r units on n CTAs, CTAs r .. n - 1 have one GEMM1 unit less and are dealt as many GEMM2 units
+// as one takes before the rest goes round to everybody. With plain round-robin 7 tokens (25 experts, 306 units on 148 CTAs) ran as
+// long as the ten CTAs with three GEMM1 units and their full share of GEMM2: layer 46.1 us, now 43.7.
+struct Deal12 {
+  int units1, total;  // GEMM1 units; all units
+  int n, c;           // CTAs, this one
+  int r, m, early;    // CTAs with a GEMM1 unit more, the others, GEMM2 units dealt to those first
+  __device__ __forceinline__ Deal12(int blocks, int n_ctas, int cta) : units1(blocks * kW13Tiles), n(n_ctas), c(cta) {
+    const int units2 = blocks * kW2Tiles;
+    total = units1 + units2;
+    r = units1 % n;
+    m = n - r;
+    // (with a single round of GEMM1 there is nothing to start on before it ends)
+    early = r == 0 || units1 <= n ? 0 : min(units2, m * (kK1Tiles / kK2Tiles));
+  }
+  __device__ __forceinline__ int second() const { return units1 + (c >= r && c - r < early ? c - r : early + c); }
+  __device__ __forceinline__ int first() const { return c < units1 ? c : second(); }
+  __device__ __forceinline__ int next(int u) const {
+    if (u < units1) return u + n < units1 ? u + n : second();
+    const int v = u - units1;
+    if (v >= early) return u + n;
+    return units1 + (v + m < early ? v + m : early + c);
+  }
+};
+
 template <int BM>
 struct Cfg12 {
   using C1 = Cfg<1, BM>;
@@ -666,9 +693,9 @@ __global__ void __launch_bounds__(256, 1)
     if (threadIdx.x == 0) atomicExch(status, B200MOE_DEV_BAD_INDEX);
     n_blocks = 0;
   }
-  const int units1 = n_blocks * kW13Tiles;
-  const int total_units = units1 + n_blocks * kW2Tiles;
   const int n_ctas = static_cast<int>(gridDim.x) - (SHARED ? sh.ctas : 0);  // CTAs of the routed experts
+  const Deal12 deal(n_blocks, n_ctas, blockIdx.x);
+  const int units1 = deal.units1, total_units = deal.total;
 
   if (SHARED && static_cast<int>(blockIdx.x) >= n_ctas) {
     shared_role(sh, &map_sx, &map_sh, smem_raw + (tiles - smem_u32(smem_raw)), tiles, tmem_base, bar_full, bar_empty, bar_sf,
@@ -680,14 +707,14 @@ __global__ void __launch_bounds__(256, 1)
       bool ok = true;
       auto block_of = [&](int u) { return u >= units1 ? (u - units1) / kW2Tiles : u / kW13Tiles; };
       // the expert id of a unit is fetched one unit ahead (a GEMM2 unit is only three stages long)
-      int e_ahead = static_cast<int>(blockIdx.x) < total_units ? __ldcg(block_expert + block_of(blockIdx.x)) : 0;
-      for (int u = blockIdx.x; u < total_units && ok; u += n_ctas) {
+      int e_ahead = deal.first() < total_units ? __ldcg(block_expert + block_of(deal.first())) : 0;
+      for (int u = deal.first(); u < total_units && ok; u = deal.next(u)) {
         const bool second = u >= units1;
         const int v = second ? u - units1 : u;
         const int tiles_m = second ? kW2Tiles : kW13Tiles, tiles_k = second ? kK2Tiles : kK1Tiles;
         const int mt = v % tiles_m;
         int e = e_ahead;
-        const int un = u + n_ctas;
+        const int un = deal.next(u);
         if (un < total_units) e_ahead = __ldcg(block_expert + block_of(un));
         if (e < 0 || e >= num_experts) {
           atomicExch(status, B200MOE_DEV_BAD_INDEX);
@@ -714,7 +741,7 @@ __global__ void __launch_bounds__(256, 1)
       uint32_t it = 0;
       bool ok = true, have_next = false;
       int next_count = 0;
-      for (int u = blockIdx.x; u < total_units && ok; u += n_ctas) {
+      for (int u = deal.first(); u < total_units && ok; u = deal.next(u)) {
         const bool second = u >= units1;
         const int v = second ? u - units1 : u;
         const int tiles_m = second ? kW2Tiles : kW13Tiles, tiles_k = second ? kK2Tiles : kK1Tiles;
@@ -740,7 +767,7 @@ __global__ void __launch_bounds__(256, 1)
           tma_load_2d(base + C::kBOffset, second ? &map_h : &map_x, kt * 128, b * BM, full);
           bulk_load(base + C::kSfbOffset, sfb_src + kt * C::kSfBytes, C::kSfBytes, full);
         }
-        const int un = u + n_ctas;  // look ahead: the next unit's completion count
+        const int un = deal.next(u);  // look ahead: the next unit's completion count
         have_next = un < total_units && un >= units1;
         if (have_next)
           asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(next_count) : "l"(done + (un - units1) / kW2Tiles) : "memory");
@@ -756,7 +783,7 @@ __global__ void __launch_bounds__(256, 1)
       uint32_t slot = 0, ph = 0, sfset = 0, ui = 0;
       uint32_t lo = tiles >> 4, sf = sf0, empty = empty0;
       bool ok = true;
-      for (int u = blockIdx.x; u < total_units && ok; u += n_ctas, ++ui) {
+      for (int u = deal.first(); u < total_units && ok; u = deal.next(u), ++ui) {
         const int tiles_k = u >= units1 ? kK2Tiles : kK1Tiles;
         const uint32_t acc = ui & 1u, aph = (ui >> 1) & 1u;
         if (!mbar_wait(smem_u32(&bar_tempty[acc]), aph ^ 1u, abort_v, status)) break;
@@ -790,7 +817,7 @@ __global__ void __launch_bounds__(256, 1)
       uint32_t slot = 0, ph = 0, sfset = 0;
       uint32_t lo = tiles >> 4, full = full0, sf = sf0;
       bool ok = true;
-      for (int u = blockIdx.x; u < total_units && ok; u += n_ctas) {
+      for (int u = deal.first(); u < total_units && ok; u = deal.next(u)) {
         const int tiles_k = u >= units1 ? kK2Tiles : kK1Tiles;
         for (int kt = 0; kt < tiles_k; ++kt) {
           if (!mbar_wait(full, ph, abort_v, status)) { ok = false; break; }
@@ -820,7 +847,7 @@ __global__ void __launch_bounds__(256, 1)
     bool have_ahead = false;
     int ahead_sid = 0;
     float ahead_wt = 0.0f;
-    for (int u = blockIdx.x; u < total_units; u += n_ctas, ++ui) {
+    for (int u = deal.first(); u < total_units; u = deal.next(u), ++ui) {
       const bool second = u >= units1;
       const int v = second ? u - units1 : u;
       const int tiles_m = second ? kW2Tiles : kW13Tiles;
@@ -838,7 +865,7 @@ __global__ void __launch_bounds__(256, 1)
       if (!epilogue_all(mbar_wait(smem_u32(&bar_tfull[acc]), aph, abort_v, status), 1u)) break;
       tc_fence_after();
       {  // look ahead: the rows of this CTA's next unit, when that is a GEMM2 unit
-        const int un = u + n_ctas;
+        const int un = deal.next(u);
         have_ahead = un < total_units && un >= units1;
         if (have_ahead && et < BM) {
           const int64_t r1 = static_cast<int64_t>((un - units1) / kW2Tiles) * BM + et;
