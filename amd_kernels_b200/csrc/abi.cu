@@ -138,7 +138,12 @@ extern "C" int b200moe_set_wait_limit_ns(uint64_t ns) {
 }
 
 namespace b200moe {
-constexpr int64_t kSmallTokens = 32;  // up to here a layer call is three launches (and the router): preparation, GEMMs, reduce
+constexpr int64_t kSmallTokens = 32;  // up to here routing, sort and gather are one launch
+// Both grouped GEMMs in one persistent launch: up to 32 tokens, and with I = 1536 wherever the row blocks have 16 rows (up to 480).
+// Measured, whole layer, two launches / one, us: I = 1536 287 / 255 at 64 tokens, 330 / 294 at 128, 355 / 318 at 400 (router and
+// shared expert inside: 318 / 298, 342 / 321, 385 / 367): 24 W13 tiles of an expert leave more of an unfinished last round, and
+// GEMM2 fills it. I = 768: 114 / 111 at 33, 141 / 139 at 64, 171 / 171 at 128, 179 / 184 at 400 (181 / 187 at 128 with both inside).
+static bool one_launch(int64_t tokens, int bm) { return tokens <= kSmallTokens || (kI == 1536 && bm == 16); }
 
 // One call of the layer, in any of its forms.
 struct LayerCall {
@@ -253,7 +258,8 @@ static int run_layer(const LayerCall& c) {
   const SharedPlan* sp = nullptr;
   if (shared) {
     if (ws.bm < 128) {  // decode sizes: a role of the launch that streams the routed experts' W13
-      if ((r = shared_plan(&plan, c.shared->w13t, c.shared->w2t, codes8, tokens, ws.sh, shared_out, tokens, ws.done + blocks)))
+      if ((r = shared_plan(&plan, c.shared->w13t, c.shared->w2t, codes8, tokens, ws.sh, shared_out, tokens, ws.done + blocks,
+                           one_launch(tokens, ws.bm))))
         return r;
       sp = &plan;
     } else {  // beside the routing and the sort, whose few short launches leave the SMs to it
@@ -287,7 +293,7 @@ static int run_layer(const LayerCall& c) {
   }
 
   // the routed experts
-  if (tokens <= kSmallTokens) {  // both grouped GEMMs in one persistent launch (measured faster there only)
+  if (one_launch(tokens, ws.bm)) {
     r = gemm12_beside(w->w13t, w->w2t, ne, ws.xq_sorted, ws.sfx, ws.block_expert, ws.num_valid, ws.sorted_ids, ws.sorted_w,
                       ws.rows, ws.bm, tokens, ws.hq, ws.sfh, ws.done, slots, c.status, sp, st);
     if (r) return r;

@@ -4,7 +4,7 @@
 // Why inside another launch. At decode sizes the shared expert is 14.6 MB of weights against 7.5 MB for every routed expert
 // that is hit, and a chain of its own (quantise, GEMM1 on 12 CTAs, GEMM2 on 48) is 30 us of latency: 17 + 15 us measured at 1
 // token, with most SMs idle, in front of or behind kernels that fill the chip with one 170 KB CTA per SM. A side stream does
-// not overlap them (whichever starts first holds the SMs) and costs four event calls on the host. As a role of 16 CTAs it
+// not overlap them (whichever starts first holds the SMs) and costs four event calls on the host. As a role of 16 to 48 CTAs it
 // runs beside the routed experts' weight stream, which is bound by HBM and does not miss those SMs.
 //
 // What bounds it: the thread that issues the MMAs (about 60 cycles per tcgen05 instruction, 48 K-tiles of 128 elements per
@@ -51,7 +51,7 @@ struct SharedWorkspace {
 };
 SharedWorkspace carve_shared(uint8_t* base, int64_t tokens);
 int shared_plan(SharedPlan* plan, const uint8_t* w13t, const uint8_t* w2t, const uint8_t* codes8, int64_t code_rows,
-                const SharedWorkspace& ws, void* out_bf16, int64_t tokens, int32_t* done);
+                const SharedWorkspace& ws, void* out_bf16, int64_t tokens, int32_t* done, bool both);
 
 constexpr int kSharedMaxStages = 8;
 constexpr int kSharedMaxSmem = 225 * 1024;  // opt-in limit of the kernels that carry the role

@@ -391,9 +391,20 @@ SharedWorkspace carve_shared(uint8_t* base, int64_t tokens) {
 }
 
 // The role's part of a launch (shared_role.cuh): codes8 [code_rows][6144] and ws.sfx8 hold the quantised tokens, `done` is one
-// zeroed count per block. CTAs: one per tile of the first GEMM, and four more that start on the second one's share.
+// zeroed count per block. `both`: the launch does both routed GEMMs, so the role has their whole time.
+// CTAs of the role, measured (whole layer with the router inside, us; I = 768 / I = 1536): the routed experts' weight stream misses
+// 16 SMs least, 24 or 48 cost it 1 to 15 % (32 tokens 127 / 130 / 148; 128 tokens, I = 1536, 317 / 325 / 384), so
+//   16 while the role ends before they do;
+//   24 from 257 tokens on where it has GEMM1's launch only (three and four blocks of 128: 400 tokens 214 -> 201, 512 237 -> 207);
+//   24 at 4 and 5 tokens (47.1 -> 45.6 / 69 -> 60 at 4; 48.9 -> 49.2 at 6);
+//   48, a CTA per tile of its second GEMM, up to 3 tokens, where the role is what the launch waits for (40.0 -> 35.5 / 62 -> 39 at 1
+//   token, 45.4 -> 41.0 at 3).
+static int role_ctas(int64_t tokens, int n_blocks, bool both) {
+  const int ctas = tokens <= 3 ? 48 : tokens <= 5 || (n_blocks >= 3 && !both) ? 24 : 16;
+  return ctas < sm_count() / 2 ? ctas : sm_count() / 2;
+}
 int shared_plan(SharedPlan* plan, const uint8_t* w13t, const uint8_t* w2t, const uint8_t* codes8, int64_t code_rows,
-                const SharedWorkspace& ws, void* out_bf16, int64_t tokens, int32_t* done) {
+                const SharedWorkspace& ws, void* out_bf16, int64_t tokens, int32_t* done, bool both) {
   int r;
   if ((r = make_map(&plan->map_x, codes8, kH, static_cast<uint64_t>(code_rows), static_cast<uint32_t>(ws.bm)))) return r;
   if ((r = make_map(&plan->map_h, ws.h8, kI, static_cast<uint64_t>(ws.rows), static_cast<uint32_t>(ws.bm)))) return r;
@@ -409,7 +420,7 @@ int shared_plan(SharedPlan* plan, const uint8_t* w13t, const uint8_t* w2t, const
   a.n_blocks = static_cast<int>(ws.rows / ws.bm);
   a.bm = ws.bm;
   a.stages = shared_stages(ws.bm);
-  a.ctas = kW13Tiles + 4;
+  a.ctas = role_ctas(tokens, a.n_blocks, both);
   return 0;
 }
 

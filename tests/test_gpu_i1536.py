@@ -137,3 +137,20 @@ def test_shared_expert_on_cta_pairs(P, C, tokens):
         assert torch.equal(S.shared_expert(x[a:a + 256].contiguous(), sw), out[a:a + 256])
     torch.cuda.synchronize()
     assert C.last_status() == 0
+
+
+@pytest.mark.parametrize("tokens", [33, 64, 480, 481])
+def test_decode_gemms_in_one_launch_equal_two(P, C, sibling, tokens):
+    """Up to 480 tokens (row blocks of 16) the entry runs both GEMMs in one launch at this intermediate: the slots of the two staged
+    kernels, bit for bit, on both sides of the rule."""
+    _, w, _ = sibling
+    gen = torch.Generator().manual_seed(tokens)
+    xb, lg = orc.make_inputs(gen, tokens, experts=EXPERTS)
+    x, logits = bf16_dev(xb), dev(lg)
+    slots, _ = P.mxfp4_moe(x, w, router_logits=logits, return_partials=True)
+    wt, ids, _ = C.route_sort(logits, w)
+    sort = C.moe_sort(ids, wt, 16 if tokens <= 480 else 32, w.num_experts)
+    hq, sfh = C.grouped_gemm1(*C.quant_dispatch(x, sort), sort, w)
+    assert torch.equal(slots, C.grouped_gemm2(hq, sfh, sort, w))
+    torch.cuda.synchronize()
+    assert C.last_status() == 0

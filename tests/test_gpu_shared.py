@@ -191,3 +191,18 @@ def test_shared_expert_inside_the_routed_launches(S, shared_layer, config0, m, r
             assert torch.equal(p_slots, slots0) and torch.equal(p_shared, want)
     torch.cuda.synchronize()
     assert C.last_status() == 0
+
+
+@pytest.mark.parametrize("m", [2, 3, 4, 5, 6, 256, 257, 385])
+def test_role_sizes_give_the_same_bits(S, shared_layer, config0, m):
+    """The number of CTAs that run the shared expert inside the routed launches changes at 3 / 4, 5 / 6 and 256 / 257 tokens."""
+    from amd_kernels_b200.moe.mxfp4_h6144_i768_e128_top4 import chain as C
+    _, sw = shared_layer
+    raw, _, _ = config0
+    w = C.MoeWeights.from_row_major(None, None, *[dev(a) for a in raw], shared=sw, routing_mode="softmax", routed_scaling_factor=1.0)
+    x = random_rows(m, 60 + m).cuda()
+    lg = torch.randn((m, 128), generator=torch.Generator().manual_seed(m)).cuda()
+    _, shared = C.mxfp4_moe(x, w, return_partials=True, router_logits=lg)
+    assert torch.equal(shared, S.shared_expert(x, sw))
+    torch.cuda.synchronize()
+    assert C.last_status() == 0
