@@ -3,21 +3,24 @@
 // bits) and each partial is short fp32 FMA chains joined by a tree, so the error per partial stays far below
 // 2^-18 * sum|x||w| (the bound the reference states for its three-term bf16 split).
 //
+// A partial is ONE chain of FMAs over the K elements of its split, in rising K from 0.0: the sum does not depend on the
+// token count or on how the work is dealt, and a change of tiling here never moves a logit's last bit.
+//
 // Used below 128 tokens, where the product is latency: 3.1 MB of gate, 12 KB of x per token. A CTA owns 16 experts x one K
-// split x 16 tokens, so one token alone already spreads the gate over 128 CTAs (with 16 splits) of 24 KB each; every lane's
-// gate values go to registers in one batch of independent 16-byte loads, issued before the wait for the predecessor's x.
-// Bound by that one round trip up to about 16 tokens, by FMA issue above. Measured with both quantisers, us back to back:
-// 2.5 / 3.7 / 4.5 / 8.6 / 13.7 at 1 / 16 / 32 / 64 / 100 tokens. The form before this one gave a CTA all 128 experts of one
-// K split (16 CTAs, gate and x through 32-element shared-memory tiles, a barrier pair and a memory round trip per tile) and
-// took 87 us at 1 token and 111 at 100.
+// split x 16 tokens, so one token alone already spreads the gate over 128 CTAs (with 16 splits) of 24 KB each, fetched in one
+// batch of asynchronous copies. Measured with both quantisers, us back to back: 4.0 / 9.9 / 10.4 / 10.6 / 18.8 at 1 / 16 / 32 /
+// 64 / 100 tokens. K dealt over the lanes of a warp and joined by a tree takes 3.9 / 3.9 / 4.5 / 8.7 / 13.8, but its sums
+// have other last bits, which reach the weights and through them the layer's result.
 #include "common.cuh"
 
 namespace b200moe {
 
-constexpr int kRgTokens = 16;             // tokens per CTA, 8 per warp
-constexpr int kRgExperts = 16;            // experts per CTA, 4 per warp
-constexpr int kRgChunk = 384;             // K elements in registers at a time: 3 x 4 per lane
-constexpr int kRgRow = kRgChunk / 8;      // 16-byte vectors of a token's chunk in shared memory
+constexpr int kRgTokens = 16;             // tokens per CTA
+constexpr int kRgExperts = 16;            // experts per CTA
+constexpr int kRgChunk = 384;             // K elements in shared memory at a time
+constexpr int kRgVecs = kRgChunk / 4;     // 16-byte vectors of a row of them
+constexpr int kRgPerThread = 2;           // tokens (chains) per thread
+constexpr int kRgThreads = kRgTokens * kRgExperts / kRgPerThread;
 
 // What the fused form also writes, row-major: the routed experts' MXFP4 operands and (optionally) the shared expert's
 // MXFP8 operands of the same rows.
@@ -30,22 +33,7 @@ struct QuantOut {
   int atom_shift;
 };
 
-// One step of the transposing sum over the lanes: before it, N values per lane; after it N / 2, the lanes with BIT clear
-// holding the sums of the lower half and the others those of the upper half.
-template <int N, int BIT>
-__device__ __forceinline__ void fold_lanes(float* v, int lane) {
-  const bool up = (lane & BIT) != 0;
-#pragma unroll
-  for (int i = 0; i < N / 2; ++i) {
-    const float keep = up ? v[i + N / 2] : v[i], give = up ? v[i] : v[i + N / 2];
-    v[i] = keep + __shfl_xor_sync(0xffffffffu, give, BIT);
-  }
-}
-
 // 16 bytes from an address that need not be aligned (`vec`: it is)
-__device__ __forceinline__ float4 load_f32x4(const float* p, bool vec) {
-  return vec ? __ldg(reinterpret_cast<const float4*>(p)) : make_float4(p[0], p[1], p[2], p[3]);
-}
 __device__ __forceinline__ uint4 load_bf16x8(const __nv_bfloat16* p, bool vec) {
   if (vec) return __ldcg(reinterpret_cast<const uint4*>(p));
   const unsigned short* h = reinterpret_cast<const unsigned short*>(p);
@@ -63,64 +51,75 @@ __device__ __forceinline__ void store_bytes(uint8_t* p, T v, bool vec) {
   }
 }
 
-// grid (ceil(E / 16), S, ceil(T / 16)); warp w: experts 4 (w % 4) .. + 3, tokens 8 (w / 4) .. + 7 of the CTA's; the 32
-// lanes share K, lane L holding elements 128 c + 4 L .. + 3 of every chunk.
+// vector c of row r in shared memory: the eight lanes of a load phase read one c of eight rows, so the vectors of a row are
+// permuted by the row to spread those over the banks
+__device__ __forceinline__ int rg_at(int r, int c) { return r * kRgVecs + (c ^ (r & 7)); }
+
+// grid (ceil(E / 16), S, ceil(T / 16)); thread: one expert (tid % 16), the tokens tid / 16 and tid / 16 + 8 of the CTA's
 template <bool QUANT>
-__global__ void __launch_bounds__(256) router_gemm_kernel(const __nv_bfloat16* __restrict__ x,
-                                                          const float* __restrict__ gate, int64_t tokens,
-                                                          int num_experts, int k_per_split,
-                                                          float* __restrict__ partials, QuantOut q, bool vec) {
-  __shared__ uint4 xs[kRgTokens][kRgRow];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int e0 = blockIdx.x * kRgExperts + 4 * (warp & 3), th = 8 * (warp >> 2);
+__global__ void __launch_bounds__(kRgThreads) router_gemm_kernel(const __nv_bfloat16* __restrict__ x,
+                                                                 const float* __restrict__ gate, int64_t tokens,
+                                                                 int num_experts, int k_per_split,
+                                                                 float* __restrict__ partials, QuantOut q, bool vec) {
+  __shared__ float4 ws[kRgExperts * kRgVecs];
+  __shared__ float4 xs[kRgTokens * kRgVecs];
+  const int tid = threadIdx.x;
+  const int e0 = blockIdx.x * kRgExperts, e = tid % kRgExperts, tg = tid / kRgExperts;
+  constexpr int kGroups = kRgThreads / kRgExperts;
   const int64_t t0 = static_cast<int64_t>(blockIdx.z) * kRgTokens;
   const int nt = static_cast<int>(min(static_cast<int64_t>(kRgTokens), tokens - t0));
   const int k0 = blockIdx.y * k_per_split;
-  float4 g[3][4];
   auto load_gate = [&](int kk) {
-#pragma unroll
-    for (int c = 0; c < 3; ++c)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int k = kk + 128 * c + 4 * lane;
-        g[c][j] = k < k_per_split && e0 + j < num_experts
-                      ? load_f32x4(gate + static_cast<int64_t>(e0 + j) * kH + k0 + k, vec)
-                      : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-      }
+    const int vecs = min(kRgChunk, k_per_split - kk) / 4;
+    for (int i = tid; i < kRgExperts * kRgVecs; i += kRgThreads) {
+      const int r = i / kRgVecs, c = i % kRgVecs;
+      if (c >= vecs || e0 + r >= num_experts) continue;  // never read
+      const float* src = gate + static_cast<int64_t>(e0 + r) * kH + k0 + kk + 4 * c;
+      float4* dst = ws + rg_at(r, c);
+      if (vec)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
+                     "l"(src)
+                     : "memory");
+      else
+        *dst = make_float4(__ldcg(src), __ldcg(src + 1), __ldcg(src + 2), __ldcg(src + 3));
+    }
   };
   load_gate(0);  // weights: no kernel of this library that lets its successor start early writes them
   pdl_enter(x);
-  float acc[32];  // [token 0..7][expert 0..3]
+  float acc[kRgPerThread];
+  int row[kRgPerThread];  // (rows beyond the last token: the last one again, not stored)
 #pragma unroll
-  for (int i = 0; i < 32; ++i) acc[i] = 0.0f;
+  for (int j = 0; j < kRgPerThread; ++j) {
+    acc[j] = 0.0f;
+    row[j] = min(tg + j * kGroups, nt - 1);
+  }
   for (int kk = 0; kk < k_per_split; kk += kRgChunk) {
-    const int vecs = min(kRgChunk, k_per_split - kk) / 8;  // 16-byte vectors of a row in this chunk
+    const int chunk = min(kRgChunk, k_per_split - kk), v8s = chunk / 8;  // 16-byte vectors of a bf16 row in this chunk
     if (kk) {
-      load_gate(kk);
       __syncthreads();
+      load_gate(kk);
     }
-    for (int i = tid; i < nt * kRgRow; i += 256) {
-      const int r = i / kRgRow, c = i % kRgRow;
-      xs[r][c] = c < vecs ? load_bf16x8(x + (t0 + r) * kH + k0 + kk + 8 * c, vec) : make_uint4(0, 0, 0, 0);
+    for (int i = tid; i < nt * v8s; i += kRgThreads) {
+      const int r = i / v8s, c = i % v8s;
+      const uint4 raw = load_bf16x8(x + (t0 + r) * kH + k0 + kk + 8 * c, vec);
+      xs[rg_at(r, 2 * c)] = make_float4(__uint_as_float(raw.x << 16), __uint_as_float(raw.x & 0xffff0000u),
+                                        __uint_as_float(raw.y << 16), __uint_as_float(raw.y & 0xffff0000u));
+      xs[rg_at(r, 2 * c + 1)] = make_float4(__uint_as_float(raw.z << 16), __uint_as_float(raw.z & 0xffff0000u),
+                                            __uint_as_float(raw.w << 16), __uint_as_float(raw.w & 0xffff0000u));
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
     if (QUANT) {
       // one pass over x: the CTAs of the expert groups share the chunk's blocks of 32 values; 4 threads x 8 values per block
       const int groups = gridDim.x, mine = (nt - static_cast<int>(blockIdx.x) + groups - 1) / groups;  // tokens of this CTA
-      const int blocks = vecs / 4;
-      for (int i = tid; i < ((mine * blocks * 4 + 31) & ~31); i += 256) {  // whole warps stay together for the shuffles
-        const bool live = i < mine * blocks * 4;
-        const int r = live ? (i / (blocks * 4)) * groups + static_cast<int>(blockIdx.x) : 0, v8 = live ? i % (blocks * 4) : 0;
-        const uint4 raw = xs[r][v8];
-        const uint32_t rr[4] = {raw.x, raw.y, raw.z, raw.w};
-        float v[8];
+      for (int i = tid; i < ((mine * v8s + 31) & ~31); i += kRgThreads) {  // whole warps stay together for the shuffles
+        const bool live = i < mine * v8s;
+        const int r = live ? (i / v8s) * groups + static_cast<int>(blockIdx.x) : 0, v8 = live ? i % v8s : 0;
+        const float4 lo = xs[rg_at(r, 2 * v8)], hi = xs[rg_at(r, 2 * v8 + 1)];
+        const float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
         float amax = 0.0f;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          v[2 * j] = __uint_as_float(rr[j] << 16);
-          v[2 * j + 1] = __uint_as_float(rr[j] & 0xffff0000u);
-          amax = fmaxf(amax, fmaxf(fabsf(v[2 * j]), fabsf(v[2 * j + 1])));
-        }
+        for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(v[j]));
         amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
         amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
         if (!live) continue;
@@ -149,36 +148,26 @@ __global__ void __launch_bounds__(256) router_gemm_kernel(const __nv_bfloat16* _
         }
       }
     }
+    if (tg < nt) {
+#pragma unroll 8
+      for (int c = 0; c < chunk / 4; ++c) {
+        const float4 w = ws[rg_at(e, c)];
 #pragma unroll
-    for (int t = 0; t < 8; ++t) {
-      if (th + t < nt) {  // the same for the whole warp
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          const uint2 b = reinterpret_cast<const uint2*>(&xs[th + t][0])[32 * c + lane];
-          const float x0 = __uint_as_float(b.x << 16), x1 = __uint_as_float(b.x & 0xffff0000u);
-          const float x2 = __uint_as_float(b.y << 16), x3 = __uint_as_float(b.y & 0xffff0000u);
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            float a = acc[4 * t + j];
-            a = fmaf(x0, g[c][j].x, a);
-            a = fmaf(x1, g[c][j].y, a);
-            a = fmaf(x2, g[c][j].z, a);
-            acc[4 * t + j] = fmaf(x3, g[c][j].w, a);
-          }
+        for (int j = 0; j < kRgPerThread; ++j) {
+          const float4 v = xs[rg_at(row[j], c)];
+          acc[j] = fmaf(v.x, w.x, acc[j]);
+          acc[j] = fmaf(v.y, w.y, acc[j]);
+          acc[j] = fmaf(v.z, w.z, acc[j]);
+          acc[j] = fmaf(v.w, w.w, acc[j]);
         }
       }
     }
   }
-  if (th >= nt) return;
-  // 32 sums over the 32 lanes in 31 shuffles: lane L ends with entry L = token L / 4, expert L % 4
-  fold_lanes<32, 16>(acc, lane);
-  fold_lanes<16, 8>(acc, lane);
-  fold_lanes<8, 4>(acc, lane);
-  fold_lanes<4, 2>(acc, lane);
-  fold_lanes<2, 1>(acc, lane);
-  const int64_t t = t0 + th + (lane >> 2);
-  const int e = e0 + (lane & 3);
-  if (t < tokens && e < num_experts) partials[(static_cast<int64_t>(blockIdx.y) * tokens + t) * num_experts + e] = acc[0];
+  if (e0 + e >= num_experts) return;
+#pragma unroll
+  for (int j = 0; j < kRgPerThread; ++j)
+    if (tg + j * kGroups < nt)
+      partials[(static_cast<int64_t>(blockIdx.y) * tokens + t0 + tg + j * kGroups) * num_experts + e0 + e] = acc[j];
 }
 
 static bool aligned16(const void* a, const void* b, const void* c, const void* d) {
@@ -198,7 +187,7 @@ extern "C" int b200moe_router_gemm(const void* x_bf16, const float* gate, int64_
   if (tokens == 0) return 0;
   const dim3 grid(static_cast<unsigned>((num_experts + kRgExperts - 1) / kRgExperts), static_cast<unsigned>(splits),
                   static_cast<unsigned>((tokens + kRgTokens - 1) / kRgTokens));
-  B200MOE_LAUNCH(router_gemm_kernel<false>, grid, 256, 0, static_cast<cudaStream_t>(stream),
+  B200MOE_LAUNCH(router_gemm_kernel<false>, grid, kRgThreads, 0, static_cast<cudaStream_t>(stream),
                  static_cast<const __nv_bfloat16*>(x_bf16), gate, tokens, num_experts, kH / splits, partials, QuantOut{},
                  aligned16(x_bf16, gate, nullptr, nullptr));
   return 0;
@@ -219,7 +208,7 @@ int router_gemm_quant(const void* x_bf16, const float* gate, int64_t tokens, int
   const dim3 grid(static_cast<unsigned>((num_experts + kRgExperts - 1) / kRgExperts), static_cast<unsigned>(splits),
                   static_cast<unsigned>((tokens + kRgTokens - 1) / kRgTokens));
   const QuantOut q{codes4, scales4, codes8, scales8, atoms8, shift};
-  B200MOE_LAUNCH(router_gemm_kernel<true>, grid, 256, 0, static_cast<cudaStream_t>(stream),
+  B200MOE_LAUNCH(router_gemm_kernel<true>, grid, kRgThreads, 0, static_cast<cudaStream_t>(stream),
                  static_cast<const __nv_bfloat16*>(x_bf16), gate, tokens, num_experts, kH / splits, partials, q,
                  aligned16(x_bf16, gate, codes4, codes8));
   return 0;

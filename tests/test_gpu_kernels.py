@@ -248,6 +248,40 @@ def test_quant_dispatch_equals_quant_then_gather(C, m, bm):
     assert np.array_equal(sa[live], sr[live]) and np.all(sa[~live] == 1)
 
 
+def _fma32(a, b, c):
+    """fma(a, b, c) in fp32, exactly, for finite values in fp32's normal range: a bf16 or shorter ``a`` makes a * b exact in
+    fp64; the sum is rounded to odd there (two-sum), from which one rounding to fp32 is the rounding of the exact sum."""
+    p, c = a.astype(np.float64) * b.astype(np.float64), c.astype(np.float64)
+    s = p + c
+    t = s - p
+    err = (p - (s - t)) + (c - t)
+    bits = s.view(np.int64)
+    even = (bits & 1) == 0
+    toward = np.where((err > 0) == (s > 0), 1, -1)  # the neighbour of s on the side of the exact sum
+    return np.where((err != 0) & even, bits + toward, bits).view(np.float64).astype(np.float32)
+
+
+@pytest.mark.parametrize("m,experts,offset", [(1, 128, 0), (7, 128, 0), (16, 33, 0), (17, 128, 1), (100, 128, 0), (127, 4, 0),
+                                              (2049, 128, 0)])
+def test_router_partials_are_one_fma_chain_per_split(C, m, experts, offset):
+    """The CUDA-core router's partial is the FMA chain over its split's K elements in rising K from 0.0, bit for bit, whatever
+    the token count, the expert count and the alignment of the operands, alone and fused with the quantisers."""
+    gen = torch.Generator().manual_seed(7 * m + experts)
+    xs = torch.randn(m * 6144 + 1, generator=gen).bfloat16()
+    gs = torch.randn(experts * 6144 + 1, generator=gen) / 6144 ** 0.5
+    x, gate = xs.cuda()[offset:offset + m * 6144].view(m, 6144), gs.cuda()[offset:offset + experts * 6144].view(experts, 6144)
+    parts = C.router_gemm_partials(x, gate)
+    assert torch.equal(parts, C.router_gemm_quant(x, gate)[0])
+    splits = parts.shape[1]
+    rows = sorted({0, m // 2, m - 1})
+    xk = x[rows].float().cpu().numpy().reshape(len(rows), splits, 1, -1)
+    gk = np.ascontiguousarray(gate.cpu().numpy().reshape(experts, splits, -1).transpose(1, 0, 2))[None]
+    acc = np.zeros((len(rows), splits, experts), np.float32)
+    for k in range(6144 // splits):
+        acc = _fma32(xk[..., k], gk[..., k], acc)
+    assert np.array_equal(parts[rows].cpu().numpy(), acc)
+
+
 @pytest.mark.parametrize("m,tensor_cores", [(1, False), (17, False), (256, False), (2049, False), (128, True), (300, True),
                                             (2049, True), (8192, True)])
 def test_router_gemm_partials_within_the_reference_bound(C, m, tensor_cores):
