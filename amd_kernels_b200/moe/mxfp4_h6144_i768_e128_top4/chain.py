@@ -26,7 +26,10 @@ def _stream(device):
 
 def _raw_stream(device) -> int:
     """The current stream's handle on ``device`` (what ``torch.cuda.current_stream(device).cuda_stream`` gives, without making
-    a stream object: a tenth of the host time)."""
+    a stream object: a tenth of the host time). As there, a device that is no CUDA device is a ValueError: every launch asks
+    for its stream here, so no kernel is handed a host tensor's address."""
+    if device.type != "cuda":
+        raise ValueError(f"expected tensors on a CUDA device, got {device}")
     return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if device.index is None else device.index)
 
 
@@ -543,6 +546,8 @@ def mxfp4_moe_experts(x_quant, topk_weights, topk_ids, w):
     codes, scales = x_quant
     n = codes.shape[0]
     variant_for(n)
+    if any(t.device != w.w13.device for t in (codes, scales, topk_weights, topk_ids)):
+        raise ValueError(f"expected every operand on the weights' device, {w.w13.device}")
     if topk_ids.dtype != torch.int32 or topk_weights.dtype != torch.float32 or topk_ids.shape != topk_weights.shape \
             or tuple(topk_ids.shape) != (n, TOPK):
         raise ValueError("expected int32 ids and fp32 weights of shape [M, 4]")
@@ -608,9 +613,13 @@ def mxfp4_moe(x, w, *, return_partials=False, router_logits=None):
         raise ValueError("expected contiguous BF16 [M,6144]")
     dev, sw, lib = x.device, w.shared_weights, w.lib()
     n_exp = w.num_experts
+    if dev != w.w13.device:
+        raise ValueError(f"x is on {dev}, the weights on {w.w13.device}")
     if router_logits is not None:
         if router_logits.shape != (n, n_exp) or router_logits.dtype != torch.float32:
             raise ValueError(f"router_logits: expected fp32 [{n}, {n_exp}]")
+        if router_logits.device != dev and not router_logits.is_pinned():  # (pinned host memory has a device address)
+            raise ValueError(f"router_logits are on {router_logits.device}, x on {dev}")
         logits = router_logits.contiguous()
         flags = 0
     else:

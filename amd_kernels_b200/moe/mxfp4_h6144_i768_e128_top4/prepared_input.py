@@ -140,6 +140,8 @@ def prepare_mxfp4_moe(x, w) -> MoeInput:
         raise ValueError("expected contiguous BF16 [M,6144]")
     n, dev = x.shape[0], x.device
     variant_for(n)
+    if dev != w.w13.device:
+        raise ValueError(f"x is on {dev}, the weights on {w.w13.device}")
     if w.router_weight is None:
         raise ValueError("needs MoeWeights with router_weight: MoeWeights.from_row_major(router_weight, ...)")
     lib, abi = _lib.load(), w.abi()

@@ -113,3 +113,82 @@ def test_c_abi_rejects_null_and_bad_sizes():
         _lib.check(_lib.E_ARG, "x")
     with pytest.raises(RuntimeError):
         _lib.check(700, "x")
+
+
+class _NoLaunch:
+    """Stands in for the library handle: the functions that only compute sizes answer as the library does, every other one is
+    a launch and fails the test."""
+    HOST = ("b200moe_block_rows", "b200moe_max_sorted_rows", "b200moe_permute_scratch_bytes", "b200moe_router_splits",
+            "b200moe_layer_workspace_bytes", "b200moe_shared_block_rows", "b200moe_shared_workspace_bytes")
+
+    def __init__(self, real):
+        self.real = real
+
+    def __getattr__(self, name):
+        if name in self.HOST:
+            return getattr(self.real, name)
+
+        def launch(*_):
+            raise AssertionError(f"{name} was called with host pointers")
+        return launch
+
+
+def _host_layer(monkeypatch):
+    """A layer and its operands on the CPU, with the library replaced and the CUDA queries answered as on a machine with one
+    GPU, so that only the entry's own checks stand between the host tensors and a launch."""
+    real = _lib.load()
+    monkeypatch.setattr(_lib, "load", lambda *a: _NoLaunch(real))
+    monkeypatch.setattr(chain, "status_word", lambda device: torch.zeros(1, dtype=torch.int32))
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 0)
+    monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream", lambda index: 0, raising=False)
+    u8 = lambda *shape: torch.zeros(shape, dtype=torch.uint8)  # noqa: E731
+    w = chain.MoeWeights(torch.zeros((8, 6144)), None, u8(8, 12, 1), None, u8(8, 1), None, 1.0, "softmax",
+                         router_split=torch.zeros((3, 128, 6144), dtype=torch.bfloat16))
+    x = torch.zeros((5, 6144), dtype=torch.bfloat16)
+    sort = chain.SortBuffers(torch.zeros(160, dtype=torch.int32), torch.zeros(160), torch.zeros(10, dtype=torch.int32),
+                             torch.zeros(2, dtype=torch.int32), 16, 5)
+    return w, x, sort, u8
+
+
+HOST_CALLS = {
+    "mxfp4_moe": lambda w, x, sort, u8: P.mxfp4_moe(x, w),
+    "mxfp4_moe_logits": lambda w, x, sort, u8: P.mxfp4_moe(x, w, router_logits=torch.zeros((5, 8))),
+    "prepare_mxfp4_moe": lambda w, x, sort, u8: P.prepare_mxfp4_moe(x, w),
+    "mxfp4_moe_experts": lambda w, x, sort, u8: chain.mxfp4_moe_experts(
+        (u8(5, 3072), u8(5, 192)), torch.zeros((5, 4)), torch.zeros((5, 4), dtype=torch.int32), w),
+    "mxfp4_quant": lambda w, x, sort, u8: chain.mxfp4_quant(x),
+    "topk_route": lambda w, x, sort, u8: chain.topk_route(torch.zeros((5, 8)), None, 1.0, "softmax"),
+    "route": lambda w, x, sort, u8: chain.route(x, w),
+    "moe_sort": lambda w, x, sort, u8: chain.moe_sort(torch.zeros((5, 4), dtype=torch.int32), torch.zeros((5, 4)), 16, 8),
+    "route_sort": lambda w, x, sort, u8: chain.route_sort(torch.zeros((5, 8)), w),
+    "dispatch_rows": lambda w, x, sort, u8: chain.dispatch_rows((u8(5, 3072), u8(5, 192)), sort),
+    "quant_dispatch": lambda w, x, sort, u8: chain.quant_dispatch(x, sort),
+    "grouped_gemm1": lambda w, x, sort, u8: chain.grouped_gemm1(u8(160, 3072), u8(10, 48, 512), sort, w),
+    "grouped_gemm2": lambda w, x, sort, u8: chain.grouped_gemm2(u8(160, 384), u8(10, 6, 512), sort, w),
+    "grouped_gemm12": lambda w, x, sort, u8: chain.grouped_gemm12(u8(160, 3072), u8(10, 48, 512), sort, w),
+    "router_gemm_partials": lambda w, x, sort, u8: chain.router_gemm_partials(x, w.router_weight),
+    "router_gemm_quant": lambda w, x, sort, u8: chain.router_gemm_quant(x, w.router_weight, shared=True),
+    "split_gate": lambda w, x, sort, u8: chain.split_gate(w.router_weight),
+    "reduce_slots": lambda w, x, sort, u8: chain.reduce_slots(torch.zeros((5, 4, 6144), dtype=torch.bfloat16)),
+    "reduce_rows": lambda w, x, sort, u8: chain.reduce_rows(torch.zeros((20, 6144), dtype=torch.bfloat16),
+                                                            torch.zeros((5, 4), dtype=torch.int32), 5),
+}
+
+
+@pytest.mark.parametrize("call", sorted(HOST_CALLS))
+def test_host_tensors_are_refused_before_any_launch(monkeypatch, call):
+    layer = _host_layer(monkeypatch)
+    with pytest.raises(ValueError):
+        HOST_CALLS[call](*layer)
+
+
+def test_operands_on_another_device_than_the_weights_are_refused(monkeypatch):
+    """(The meta device stands in for the other one.)"""
+    w, x, sort, u8 = _host_layer(monkeypatch)
+    w.w13 = w.w13.to("meta")
+    for call in ("mxfp4_moe", "mxfp4_moe_logits", "prepare_mxfp4_moe", "mxfp4_moe_experts"):
+        with pytest.raises(ValueError, match="weights"):
+            HOST_CALLS[call](w, x, sort, u8)
+    w.w13, x = w.w13.to("meta"), x.to("meta")
+    with pytest.raises(ValueError, match="router_logits are on cpu"):
+        P.mxfp4_moe(x, w, router_logits=torch.zeros((5, 8)))
