@@ -29,7 +29,7 @@ class Weights(Structure):
 
 class SharedWeights(Structure):
     """struct b200moe_shared_weights"""
-    _fields_ = [("w13t", c_void_p), ("w2t", c_void_p)]
+    _fields_ = [("w13t", c_void_p), ("w2t", c_void_p), ("intermediate", c_int)]
 
 
 class Prepared(Structure):

@@ -201,6 +201,7 @@ static int run_layer(const LayerCall& c) {
   const bool shared = c.shared != nullptr, router = c.x && !c.logits, compact = c.prep && c.prep->mask4;
   if (router && !w->gate) return B200MOE_E_ARG;
   if (shared && (!c.shared->w13t || !c.shared->w2t || (!c.shared_out && !c.out))) return B200MOE_E_ARG;
+  if (shared && c.shared->intermediate != 0 && c.shared->intermediate != kI) return B200MOE_E_ARG;
   if (c.prep && (!c.prep->scales4 || !c.prep->topk_weights || !c.prep->topk_ids || (!c.prep->codes4 && !compact) ||
                  ((shared || compact) && (!c.prep->codes8 || !c.prep->scales8))))
     return B200MOE_E_ARG;

@@ -593,6 +593,24 @@ def _side_stream(sw, n):
     return None if in_dbo() else sw.stream.cuda_stream
 
 
+def routed_beside_shared(x, w, *, return_partials, x_quant=None, router_logits=None):
+    """The layer where the shared expert has another intermediate size than the routed experts, so that one library serves
+    neither: the shared expert through its own library, on the side stream, and the routed experts alone, joined before the
+    reduce. ``x``: bf16 rows, or (``x_quant`` the shared expert's operands) a ``MoeInput``."""
+    from dataclasses import replace
+    from .shared_expert import shared_expert_parallel
+    sw = w.shared_weights
+    dev = w.w13.device
+    current = torch.cuda.current_stream(dev)
+    if x_quant is None:
+        w.abi()  # what is made on first use stays with ``w``, not with the copy below
+    shared = shared_expert_parallel(x if x_quant is None else None, sw, current, x_quant=x_quant)
+    slots, _ = mxfp4_moe(x, replace(w, shared_weights=None), return_partials=True, router_logits=router_logits)
+    current.wait_stream(sw.stream)
+    shared.record_stream(current)
+    return (slots, shared) if return_partials else reduce_slots(slots, shared)
+
+
 def mxfp4_moe(x, w, *, return_partials=False, router_logits=None):
     """Normed BF16 [M, 6144] -> the routed experts' output (reference chain.py:127-197).
 
@@ -615,6 +633,8 @@ def mxfp4_moe(x, w, *, return_partials=False, router_logits=None):
     n_exp = w.num_experts
     if dev != w.w13.device:
         raise ValueError(f"x is on {dev}, the weights on {w.w13.device}")
+    if sw is not None and sw.intermediate != w.intermediate:
+        return routed_beside_shared(x, w, return_partials=return_partials, router_logits=router_logits)
     if router_logits is not None:
         if router_logits.shape != (n, n_exp) or router_logits.dtype != torch.float32:
             raise ValueError(f"router_logits: expected fp32 [{n}, {n_exp}]")

@@ -162,8 +162,12 @@ def prepare_mxfp4_moe(x, w) -> MoeInput:
 def mxfp4_moe_prepared(x, w, *, return_partials):
     """``mxfp4_moe`` on a prepared input (reference prepared_input.py:159-187): the routed experts on the MXFP4 operands (of a
     compact input: rebuilt inside the call), the shared expert on the MXFP8 ones, summed in slot order then shared."""
-    from .chain import layer_prepared
+    from .chain import layer_prepared, routed_beside_shared
     sw, dev = w.shared_weights, w.w13.device
+    if sw is not None and sw.intermediate != w.intermediate:
+        x = x.expand() if isinstance(x, MoeInputCompact) else x
+        x.validate(w)
+        return routed_beside_shared(x, w, return_partials=return_partials, x_quant=(x.shared_codes, x.shared_scales))
     if isinstance(x, MoeInputCompact):
         if x.shared_codes.device.type != "cuda":
             raise ValueError("compact input requires CUDA operands")

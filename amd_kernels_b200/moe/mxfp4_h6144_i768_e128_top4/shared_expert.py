@@ -66,7 +66,7 @@ class SharedWeights:
 
     def abi(self) -> _lib.SharedWeights:
         """``struct b200moe_shared_weights`` over this object's tensors."""
-        return _lib.SharedWeights(self.w13.data_ptr(), self.w2.data_ptr())
+        return _lib.SharedWeights(self.w13.data_ptr(), self.w2.data_ptr(), self.intermediate)
 
     @classmethod
     def from_row_major(cls, w13, s13, w2, s2):

@@ -417,6 +417,8 @@ int b200moe_forward_x(const b200moe_weights* w, const void* x_bf16, int64_t toke
 typedef struct b200moe_shared_weights {
   const uint8_t* w13t; /* b200moe_preshuffle_shared */
   const uint8_t* w2t;
+  int intermediate; /* of these weights; 0: the library's. B200MOE_E_ARG where it is not the library's: the shared expert of
+                       another size is b200moe_shared_expert of the library that was built for it, then b200moe_reduce_slots */
 } b200moe_shared_weights;
 #define B200MOE_LAYER_ROUTER 1         /* no logits are given */
 #define B200MOE_LAYER_SHARED 2         /* shared is given */

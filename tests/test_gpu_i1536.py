@@ -154,3 +154,35 @@ def test_decode_gemms_in_one_launch_equal_two(P, C, sibling, tokens):
     assert torch.equal(slots, C.grouped_gemm2(hq, sfh, sort, w))
     torch.cuda.synchronize()
     assert C.last_status() == 0
+
+
+@pytest.mark.parametrize("tokens", [1, 48, 700])
+@pytest.mark.parametrize("routed", [768, 1536])
+def test_a_shared_expert_of_the_other_intermediate_size(P, C, tokens, routed):
+    """Routed experts and shared expert of different intermediate sizes: each through the library built for it, from bf16 rows
+    and from both prepared forms."""
+    from amd_kernels_b200.moe import mxfp4_h6144_i768_e128_top4 as P768
+    from amd_kernels_b200.moe.mxfp4_h6144_i768_e128_top4 import shared_expert as S
+    routed_pkg, shared_pkg = (P768, P) if routed == 768 else (P, P768)
+    sw = shared_pkg.SharedWeights.from_row_major(*(dev(a) for a in orc.make_shared_weights(seed=31, inter=2304 - routed)))
+    raw, gen = orc.make_weights(seed=32, experts=8, inter=routed)
+    gate = torch.randn((8, H), generator=gen).cuda() / H ** 0.5
+    on_gpu = [dev(a) for a in raw]
+    w = routed_pkg.MoeWeights.from_row_major(gate, None, *on_gpu, shared=sw)
+    alone = routed_pkg.MoeWeights.from_row_major(gate, None, *on_gpu)
+    x = torch.randn((tokens, H), generator=gen).bfloat16().cuda()
+    lg = torch.randn((tokens, 8), generator=gen).cuda()
+    want = S.shared_expert(x, sw)
+    for logits in (None, lg):
+        slots0, _ = P.mxfp4_moe(x, alone, return_partials=True, router_logits=logits)
+        slots, shared = P.mxfp4_moe(x, w, return_partials=True, router_logits=logits)
+        assert torch.equal(slots, slots0) and torch.equal(shared, want)
+        assert torch.equal(P.mxfp4_moe(x, w, router_logits=logits), C.reduce_slots(slots0, want))
+    inp = P.prepare_mxfp4_moe(x, w)
+    slots0, _ = P.mxfp4_moe(x, alone, return_partials=True)
+    for form in (inp, inp.compact()):
+        slots, shared = P.mxfp4_moe(form, w, return_partials=True)
+        assert torch.equal(slots, slots0) and torch.equal(shared, want)
+        assert torch.equal(P.mxfp4_moe(form, w), C.reduce_slots(slots0, want))
+    torch.cuda.synchronize()
+    assert C.last_status() == 0

@@ -192,3 +192,19 @@ def test_operands_on_another_device_than_the_weights_are_refused(monkeypatch):
     w.w13, x = w.w13.to("meta"), x.to("meta")
     with pytest.raises(ValueError, match="router_logits are on cpu"):
         P.mxfp4_moe(x, w, router_logits=torch.zeros((5, 8)))
+
+
+@pytest.mark.parametrize("inter", [768, 1536])
+def test_c_abi_refuses_shared_weights_of_another_intermediate_size(inter):
+    """The kernels take the tile counts from the size the library was built for, so the struct says which size its weights
+    have. (The misaligned workspace ends the accepted calls before anything is launched.)"""
+    lib = _lib.load(inter)
+    one = ctypes.c_void_p(256)
+    w = _lib.Weights(256, 256, None, 128, _lib.ROUTE_SOFTMAX, 1.0, None, None)
+    prep = _lib.Prepared(256, 256, 256, 256, 256, 256, None)
+    for size, want in ((inter, _lib.E_ALIGN), (0, _lib.E_ALIGN), (2304 - inter, _lib.E_ARG)):
+        sw = _lib.SharedWeights(256, 256, size)
+        bad = ctypes.c_void_p(8)
+        assert lib.b200moe_layer(ctypes.byref(w), ctypes.byref(sw), one, one, 4, bad, 1 << 40, one, one, one, one, None, None) == want
+        assert lib.b200moe_layer_prepared(ctypes.byref(w), ctypes.byref(sw), ctypes.byref(prep), 4, bad, 1 << 40, one, one, one,
+                                          one, None, None) == want
