@@ -138,18 +138,23 @@ class MoeWeights:
     def abi(self) -> _lib.Weights:
         """``struct b200moe_weights`` over this object's tensors."""
         if self._abi is None:
-            gate = self.router_weight
-            if gate is not None and (gate.dtype != torch.float32 or not gate.is_contiguous() or gate.device != self.w13.device
-                                     or tuple(gate.shape) != (self.num_experts, H)):
-                raise ValueError(f"router_weight: expected contiguous fp32 [{self.num_experts}, {H}] on {self.w13.device}")
-            if gate is not None and self.router_split is None:
-                self.router_split = split_gate(gate)
-            self._abi = _lib.Weights(self.w13.data_ptr(), self.w2.data_ptr(),
-                                     None if self.correction_bias is None else self.correction_bias.data_ptr(),
-                                     self.num_experts, ROUTING_MODES[self.routing_mode],
-                                     self.routed_scaling_factor, None if gate is None else gate.data_ptr(),
-                                     None if gate is None else self.router_split.data_ptr())
+            self._abi = self.abi_now()
         return self._abi
+
+    def abi_now(self, router: bool = True) -> _lib.Weights:
+        """The same from the fields as they are now. ``router`` False: for a call whose tokens are routed already, which must
+        not make the gate's bf16 terms (the call may be under capture, and they would be the captured graph's)."""
+        gate = self.router_weight if router else None
+        if gate is not None and (gate.dtype != torch.float32 or not gate.is_contiguous() or gate.device != self.w13.device
+                                 or tuple(gate.shape) != (self.num_experts, H)):
+            raise ValueError(f"router_weight: expected contiguous fp32 [{self.num_experts}, {H}] on {self.w13.device}")
+        if gate is not None and self.router_split is None:
+            self.router_split = split_gate(gate)
+        return _lib.Weights(self.w13.data_ptr(), self.w2.data_ptr(),
+                            None if self.correction_bias is None else self.correction_bias.data_ptr(),
+                            self.num_experts, ROUTING_MODES[self.routing_mode],
+                            self.routed_scaling_factor, None if gate is None else gate.data_ptr(),
+                            None if gate is None else self.router_split.data_ptr())
 
 
 def unsupported_reason(w13, w13_scale, w2, w2_scale, shared_w13, shared_s13, shared_w2, shared_s2,
@@ -566,7 +571,8 @@ def layer_prepared(prep, n, w, sw, slots, shared, out, dev):
     ws_bytes = lib.b200moe_layer_workspace_bytes(n, w.num_experts, flags)
     workspace = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
     _lib.check(lib.b200moe_layer_prepared(
-        ctypes.byref(w.abi()), None if sw is None else ctypes.byref(sw.abi()), ctypes.byref(prep), n, workspace.data_ptr(),
+        ctypes.byref(w.abi_now(router=False)), None if sw is None else ctypes.byref(sw.abi()), ctypes.byref(prep), n,
+        workspace.data_ptr(),
         ws_bytes, None if slots is None else slots.data_ptr(), None if shared is None else shared.data_ptr(),
         None if out is None else out.data_ptr(), status_word(dev).data_ptr(), _raw_stream(dev), _side_stream(sw, n)),
         "layer_prepared")

@@ -144,7 +144,7 @@ def prepare_mxfp4_moe(x, w) -> MoeInput:
         raise ValueError(f"x is on {dev}, the weights on {w.w13.device}")
     if w.router_weight is None:
         raise ValueError("needs MoeWeights with router_weight: MoeWeights.from_row_major(router_weight, ...)")
-    lib, abi = _lib.load(), w.abi()
+    lib, abi = _lib.load(), w.abi_now()
     shared = w.shared_weights is not None
     parts = torch.empty((lib.b200moe_router_splits(n), n, w.num_experts), dtype=torch.float32, device=dev)
     q4 = torch.empty((n, H // 2), dtype=torch.uint8, device=dev)

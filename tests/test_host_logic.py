@@ -208,3 +208,40 @@ def test_c_abi_refuses_shared_weights_of_another_intermediate_size(inter):
         assert lib.b200moe_layer(ctypes.byref(w), ctypes.byref(sw), one, one, 4, bad, 1 << 40, one, one, one, one, None, None) == want
         assert lib.b200moe_layer_prepared(ctypes.byref(w), ctypes.byref(sw), ctypes.byref(prep), 4, bad, 1 << 40, one, one, one,
                                           one, None, None) == want
+
+
+class _Recorder(_NoLaunch):
+    """The library handle's stand-in that accepts the whole-layer calls and keeps the weights struct they were given."""
+    def __init__(self, real):
+        super().__init__(real)
+        self.weights = []
+
+    def __getattr__(self, name):
+        if name in ("b200moe_prepare", "b200moe_layer_prepared"):
+            def call(w, *_):
+                s = w._obj
+                self.weights.append((s.w13t, s.bias, s.route_mode, s.route_scale, s.gate, s.gate_split))
+                return 0
+            return call
+        return super().__getattr__(name)
+
+
+def test_prepared_calls_take_the_weights_as_they_are(monkeypatch):
+    """prepare_mxfp4_moe reads the bias, the scale, the mode and the gate that the weights hold at the call, and the calls on
+    routed tokens neither need nor make the gate's bf16 terms."""
+    w, x, sort, u8 = _host_layer(monkeypatch)
+    rec = _Recorder(_lib.load().real)
+    monkeypatch.setattr(_lib, "load", lambda *a: rec)
+    monkeypatch.setattr(chain, "_raw_stream", lambda device: 0)
+    monkeypatch.setattr(chain, "split_gate", lambda gate: pytest.fail("the gate's terms were made"))
+    w.abi()
+    w.correction_bias, w.routed_scaling_factor, w.routing_mode = torch.ones(8), 2.5, "sigmoid_bias"
+    w.router_weight = torch.ones((8, 6144))
+    P.prepare_mxfp4_moe(x, w)
+    got = rec.weights.pop()
+    assert got[1:5] == (w.correction_bias.data_ptr(), _lib.ROUTE_SIGMOID_BIAS, 2.5, w.router_weight.data_ptr())
+    w.router_split = w._abi = None
+    w.w13 = w.w13.clone()
+    HOST_CALLS["mxfp4_moe_experts"](w, x, sort, u8)
+    got = rec.weights.pop()
+    assert got[0] == w.w13.data_ptr() and got[4] is None and got[5] is None and w.router_split is None
