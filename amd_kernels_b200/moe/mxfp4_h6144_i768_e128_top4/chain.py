@@ -547,10 +547,13 @@ def route(x, w, router_logits=None):
 
 def mxfp4_moe_experts(x_quant, topk_weights, topk_ids, w):
     """The routed experts on the MXFP4 input ``x_quant`` = (codes, scales), already routed (``topk_weights`` include
-    the routed scale) -> the BF16 [M, 4, H] slots (reference chain.py:113-124). Served at every M here."""
+    the routed scale) -> the BF16 [M, 4, H] slots (reference chain.py:113-124). Served at every M here; M is the number of
+    routed rows, and ``x_quant`` may be a padded buffer with more."""
     codes, scales = x_quant
-    n = codes.shape[0]
-    variant_for(n)
+    variant_for(codes.shape[0])
+    n = topk_ids.shape[0]
+    if not 0 < n <= codes.shape[0] or scales.shape[0] < n:
+        raise ValueError(f"{n} routed rows for {codes.shape[0]} quantised ones")
     if any(t.device != w.w13.device for t in (codes, scales, topk_weights, topk_ids)):
         raise ValueError(f"expected every operand on the weights' device, {w.w13.device}")
     if topk_ids.dtype != torch.int32 or topk_weights.dtype != torch.float32 or topk_ids.shape != topk_weights.shape \

@@ -245,3 +245,15 @@ def test_prepared_calls_take_the_weights_as_they_are(monkeypatch):
     HOST_CALLS["mxfp4_moe_experts"](w, x, sort, u8)
     got = rec.weights.pop()
     assert got[0] == w.w13.data_ptr() and got[4] is None and got[5] is None and w.router_split is None
+
+
+def test_routed_experts_on_a_padded_input(monkeypatch):
+    """The routing says how many rows there are; the quantised input may have more rows, never fewer."""
+    w, _, _, u8 = _host_layer(monkeypatch)
+    monkeypatch.setattr(chain, "layer_prepared", lambda prep, n, *_: None)
+    routing = torch.zeros((5, 4)), torch.zeros((5, 4), dtype=torch.int32)
+    for rows in (5, 8, 300):
+        assert chain.mxfp4_moe_experts((u8(rows, 3072), u8(rows, 192)), *routing, w).shape == (5, 4, 6144)
+    for rows in (0, 4):
+        with pytest.raises(ValueError):
+            chain.mxfp4_moe_experts((u8(rows, 3072), u8(rows, 192)), *routing, w)
