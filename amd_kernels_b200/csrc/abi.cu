@@ -209,7 +209,8 @@ static int run_layer(const LayerCall& c) {
   if (shared && ((reinterpret_cast<uintptr_t>(c.shared->w13t) | reinterpret_cast<uintptr_t>(c.shared->w2t) |
                   reinterpret_cast<uintptr_t>(c.shared_out)) & 15))
     return B200MOE_E_ALIGN;
-  if (c.prep && ((reinterpret_cast<uintptr_t>(c.prep->codes4) | reinterpret_cast<uintptr_t>(c.prep->codes8)) & 15))
+  // (the rebuild of a compact input checks its own operands: 8 bytes for the FP8 codes)
+  if (c.prep && ((reinterpret_cast<uintptr_t>(c.prep->codes4) | (shared ? reinterpret_cast<uintptr_t>(c.prep->codes8) : 0)) & 15))
     return B200MOE_E_ALIGN;
   const int ne = w->num_experts;
   const int64_t tokens = c.tokens;

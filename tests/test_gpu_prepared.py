@@ -123,3 +123,24 @@ def test_router_gemm_fused_with_the_quantisers(full_layer, m):
     assert torch.equal(q8, want8[0]) and torch.equal(s8, want8[1])
     _, _, (n8, ns8) = C.router_gemm_quant(x, w.router_weight)
     assert n8 is None and ns8 is None
+
+
+def test_compact_input_with_codes_on_an_8_byte_boundary(P, full_layer):
+    """A layer without a shared expert needs the FP8 codes for the rebuild of the FP4 codes alone, which reads them 8 bytes at a
+    time (with a shared expert they are a TMA operand and need 16)."""
+    from dataclasses import replace
+    C, _, w = full_layer
+    gen = torch.Generator().manual_seed(8)
+    x = torch.randn((37, 6144), generator=gen).bfloat16().cuda()
+    form = P.prepare_mxfp4_moe(x, w).compact()
+    room = torch.empty(37 * 6144 + 8, dtype=torch.uint8, device="cuda")
+    codes = room[8:].view(37, 6144)
+    codes.copy_(form.shared_codes)
+    assert codes.data_ptr() % 16 == 8
+    odd = P.MoeInputCompact(form.routed_scales, form.topk_weights, form.topk_ids, codes, form.shared_scales, form.correction_mask)
+    alone = replace(w, shared_weights=None)
+    assert torch.equal(C.mxfp4_moe(odd, alone), C.mxfp4_moe(x, alone))
+    with pytest.raises(ValueError):
+        C.mxfp4_moe(odd, w)
+    torch.cuda.synchronize()
+    assert C.last_status() == 0
