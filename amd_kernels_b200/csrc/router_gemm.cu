@@ -69,6 +69,10 @@ __global__ void __launch_bounds__(kRgThreads) router_gemm_kernel(const __nv_bflo
   const int64_t t0 = static_cast<int64_t>(blockIdx.z) * kRgTokens;
   const int nt = static_cast<int>(min(static_cast<int64_t>(kRgTokens), tokens - t0));
   const int k0 = blockIdx.y * k_per_split;
+  // this CTA's slice of the gate: into L2 before the wait, read behind it (the work in front may have written it)
+  if (vec && tid < kRgExperts && e0 + tid < num_experts)
+    l2_prefetch_bulk(gate + static_cast<int64_t>(e0 + tid) * kH + k0, static_cast<uint32_t>(k_per_split * 4));
+  pdl_enter(x, gate);
   auto load_gate = [&](int kk) {
     const int vecs = min(kRgChunk, k_per_split - kk) / 4;
     for (int i = tid; i < kRgExperts * kRgVecs; i += kRgThreads) {
@@ -84,8 +88,7 @@ __global__ void __launch_bounds__(kRgThreads) router_gemm_kernel(const __nv_bflo
         *dst = make_float4(__ldcg(src), __ldcg(src + 1), __ldcg(src + 2), __ldcg(src + 3));
     }
   };
-  load_gate(0);  // weights: no kernel of this library that lets its successor start early writes them
-  pdl_enter(x);
+  load_gate(0);
   float acc[kRgPerThread];
   int row[kRgPerThread];  // (rows beyond the last token: the last one again, not stored)
 #pragma unroll

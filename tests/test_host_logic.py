@@ -257,3 +257,28 @@ def test_routed_experts_on_a_padded_input(monkeypatch):
     for rows in (0, 4):
         with pytest.raises(ValueError):
             chain.mxfp4_moe_experts((u8(rows, 3072), u8(rows, 192)), *routing, w)
+
+
+def _kernels():
+    """(file, name, body) of every __global__ function of the sources, comments removed."""
+    csrc = os.path.join(ROOT, "amd_kernels_b200", "csrc")
+    for f in sorted(os.listdir(csrc)):
+        text = re.sub(r"//[^\n]*", "", open(os.path.join(csrc, f)).read())
+        for m in re.finditer(r"__global__", text):
+            body = text[m.start():]
+            end = body.find("\n}\n")
+            yield f, re.search(r"(\w+)\s*\(const|(\w+_kernel)\s*\(", body).group(0), body[:end]
+
+
+def test_no_kernel_reads_global_memory_before_its_wait():
+    """A kernel that is launched early may ask L2 for data before griddepcontrol.wait, never load it: what the launch before
+    it wrote (weights among them) is only certain to be seen behind the wait, and only through L2."""
+    seen = 0
+    for f, name, body in _kernels():
+        at = re.search(r"\bpdl_(enter|wait)\s*\(", body)
+        if at is None:
+            continue  # ordinary stream order
+        seen += 1
+        early = re.findall(r"__ldg\(|__ldcg\(|\bld\.|cp\.async\.c[ag]\b|\bload_\w+\(|\*\s*reinterpret_cast<const", body[:at.start()])
+        assert not early, (f, name, early)
+    assert seen >= 15
