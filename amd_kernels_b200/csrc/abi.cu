@@ -18,7 +18,7 @@ struct Workspace {
   uint8_t* sfx;           // [R/bm][48][512]
   uint8_t* hq;            // [R][384]
   uint8_t* sfh;           // [R/bm][6][512]
-  int32_t* done;          // [R/bm] GEMM1 tiles finished per row block, then [8]: the shared expert's per block of tokens
+  int32_t* done;          // [R/bm] GEMM1 tiles finished per row block, then [kSharedDone]: the shared expert's
   // only with the router inside the call:
   float* partials;        // [S][T][E] split-K logit partials
   uint8_t* q4;            // [T][3072] row-major MXFP4 codes of x (also rebuilt from a compact prepared input)
@@ -32,7 +32,6 @@ struct Workspace {
   int bm;
   int64_t rows;
 };
-constexpr int kSharedDone = 8;  // blocks of shared-expert tokens a decode launch may count (512 tokens in blocks of 128: 4)
 
 int dispatch_rows_done(const uint8_t* codes, const uint8_t* scales, const int32_t* sorted_ids, const int32_t* num_valid,
                        int64_t tokens, int bm, int by_pair, int64_t max_rows, uint8_t* xq_sorted, uint8_t* sfx,

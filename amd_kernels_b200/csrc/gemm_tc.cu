@@ -155,6 +155,8 @@ __global__ void __launch_bounds__((Cfg<MODE, BM>::kThreads), 1)
   constexpr uint32_t kTmemCols = SHARED ? 512 : C::kTmemCols;
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t bar_full[C::kStages];
+  __shared__ __align__(8) uint64_t bar_unit[SHARED ? kUnitRing : 1];  // the shared expert's units
+  __shared__ int s_unit[SHARED ? kUnitRing : 1];
   __shared__ __align__(8) uint64_t bar_empty[C::kStages];
   __shared__ __align__(8) uint64_t bar_sf[C::kStages];  // the stage's scales are in tensor memory
   __shared__ __align__(8) uint64_t bar_tfull[2];
@@ -173,6 +175,8 @@ __global__ void __launch_bounds__((Cfg<MODE, BM>::kThreads), 1)
 
   if (threadIdx.x == 0) {
     abort_flag = 0;
+    if (SHARED)
+      for (int i = 0; i < kUnitRing; ++i) mbar_init(smem_u32(&bar_unit[i]), 1);
     for (int s = 0; s < C::kStages; ++s) {
       mbar_init(smem_u32(&bar_full[s]), 1);
       mbar_init(smem_u32(&bar_empty[s]), 1);
@@ -226,7 +230,7 @@ __global__ void __launch_bounds__((Cfg<MODE, BM>::kThreads), 1)
 
   if (SHARED && static_cast<int>(blockIdx.x) >= n_ctas) {
     shared_role(sh, &map_sx, &map_sh, smem_raw + (tiles - smem_u32(smem_raw)), tiles, tmem_base, bar_full, bar_empty, bar_sf,
-                bar_tfull, bar_tempty, bar_drain, abort_v, status);
+                bar_tfull, bar_tempty, bar_drain, UnitRing{bar_unit, s_unit}, abort_v, status);
   } else if (warp == 0) {
     // ---------------------------------------------------------------- producer
     if (lane == 0) {
@@ -579,37 +583,27 @@ __global__ void __launch_bounds__((Cfg<MODE, BM>::kThreads), 1)
 
 // ------------------------------------------------------------------------------------------------ GEMM1 + GEMM2 in one launch
 // Decode sizes (bm < 128): both grouped GEMMs as ONE persistent kernel. The unit list is all GEMM1 units followed by all
-// GEMM2 units, dealt round-robin to the CTAs, so every CTA finishes its GEMM1 units before its first GEMM2 unit. A GEMM2
-// unit of row block b needs the 12 GEMM1 tiles of b: each GEMM1 epilogue publishes its stores (fence, then one atomic
-// add on done[b]) and the GEMM2 producer waits -- bounded like every other wait -- until done[b] == 12 before it loads h.
-// GEMM1 units never wait, so progress does not depend on scheduling order. What this buys over two launches: no ramp
-// between the kernels, and the short GEMM2 units (52 KB of weights) fill the uneven last round of GEMM1 (418 KB units).
+// GEMM2 units; the CTAs claim them in that order from a ticket. A GEMM2 unit of row block b needs the GEMM1 tiles of b: each
+// GEMM1 epilogue publishes its stores (fence, then one atomic add on done[b]) and the GEMM2 producer waits -- bounded like
+// every other wait -- until done[b] shows them all before it loads h. What this buys over two launches: no ramp between the
+// kernels, and the short GEMM2 units (52 KB of weights) fill the uneven last round of GEMM1 (418 KB units).
 //
-// Dealing. GEMM1 units are 8 (I = 1536: 4) times as long as GEMM2 units, so an unfinished last round of them is made up in the
-// second list: with units1 = q n + r units on n CTAs, CTAs r .. n - 1 have one GEMM1 unit less and are dealt as many GEMM2 units
-// as one takes before the rest goes round to everybody. With plain round-robin 7 tokens (25 experts, 306 units on 148 CTAs) ran as
-// long as the ten CTAs with three GEMM1 units and their full share of GEMM2: layer 46.1 us, now 43.7.
-struct Deal12 {
-  int units1, total;  // GEMM1 units; all units
-  int n, c;           // CTAs, this one
-  int r, m, early;    // CTAs with a GEMM1 unit more, the others, GEMM2 units dealt to those first
-  __device__ __forceinline__ Deal12(int blocks, int n_ctas, int cta) : units1(blocks * kW13Tiles), n(n_ctas), c(cta) {
-    const int units2 = blocks * kW2Tiles;
-    total = units1 + units2;
-    r = units1 % n;
-    m = n - r;
-    // (with a single round of GEMM1 there is nothing to start on before it ends)
-    early = r == 0 || units1 <= n ? 0 : min(units2, m * (kK1Tiles / kK2Tiles));
-  }
-  __device__ __forceinline__ int second() const { return units1 + (c >= r && c - r < early ? c - r : early + c); }
-  __device__ __forceinline__ int first() const { return c < units1 ? c : second(); }
-  __device__ __forceinline__ int next(int u) const {
-    if (u < units1) return u + n < units1 ? u + n : second();
-    const int v = u - units1;
-    if (v >= early) return u + n;
-    return units1 + (v + m < early ? v + m : early + c);
-  }
-};
+// Why a ticket and not a fixed deal: a waiting CTA keeps its SM, so it may only wait for CTAs that run. GEMM1 units never
+// wait, and one that has been claimed belongs to a CTA that is resident; with a fixed deal it could belong to a CTA that
+// another launch (a second stream, another long kernel) keeps off the device while both launches hold SMs in such waits.
+//
+// A unit is claimed late in the one before it (GEMM1: 8 K-tiles before its last stage is issued, GEMM2: 2, behind the wait for
+// a free slot), so CTAs that are ahead take more: GEMM2 units make up a GEMM1 round that does not come out even. Measured, whole
+// layer, dealt by block index with the uneven round made up by rule / claimed, us: 45.1 / 42.1 at 7 tokens, 37.5 / 37.4 at 1 and
+// 108.6 / 108.7 at 32 (router and shared expert inside), 242.6 / 242.5 at 64 with I = 1536.
+//
+// done[b]: the low byte counts the finished GEMM1 tiles of row block b (signed); done[0] hands out the units above it.
+__device__ __forceinline__ int claim_unit12(int32_t* done, int32_t* status) {
+  const int u = (atomicAdd(done, 256) + 128) >> 8;
+  if (u >= 0) return u;
+  atomicExch(status, B200MOE_DEV_BAD_INDEX);  // the counts were not zero: no unit, no address
+  return kNoUnit;
+}
 
 template <int BM>
 struct Cfg12 {
@@ -640,6 +634,8 @@ __global__ void __launch_bounds__(256, 1)
   __shared__ __align__(8) uint64_t bar_tfull[2];
   __shared__ __align__(8) uint64_t bar_tempty[2];
   __shared__ __align__(8) uint64_t bar_drain[2];  // used after an abort only
+  __shared__ __align__(8) uint64_t bar_unit[kUnitRing];
+  __shared__ int s_unit[kUnitRing];
   __shared__ uint32_t tmem_base_slot;
   __shared__ int abort_flag;
   __shared__ __nv_bfloat16* s_dst[BM];
@@ -649,9 +645,11 @@ __global__ void __launch_bounds__(256, 1)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t tiles = (smem_u32(smem_raw) + 1023u) & ~1023u;
   volatile int* abort_v = &abort_flag;
+  const UnitRing ring{bar_unit, s_unit};
   pdl_launch_dependents();
   if (threadIdx.x == 0) {
     abort_flag = 0;
+    for (int i = 0; i < kUnitRing; ++i) mbar_init(smem_u32(&bar_unit[i]), 1);
     for (int s = 0; s < CC::kStages; ++s) {
       mbar_init(smem_u32(&bar_full[s]), 1);
       mbar_init(smem_u32(&bar_empty[s]), 1);
@@ -694,28 +692,26 @@ __global__ void __launch_bounds__(256, 1)
     n_blocks = 0;
   }
   const int n_ctas = static_cast<int>(gridDim.x) - (SHARED ? sh.ctas : 0);  // CTAs of the routed experts
-  const Deal12 deal(n_blocks, n_ctas, blockIdx.x);
-  const int units1 = deal.units1, total_units = deal.total;
+  const int units1 = n_blocks * kW13Tiles, total_units = units1 + n_blocks * kW2Tiles;
 
   if (SHARED && static_cast<int>(blockIdx.x) >= n_ctas) {
     shared_role(sh, &map_sx, &map_sh, smem_raw + (tiles - smem_u32(smem_raw)), tiles, tmem_base, bar_full, bar_empty, bar_sf,
-                bar_tfull, bar_tempty, bar_drain, abort_v, status);
+                bar_tfull, bar_tempty, bar_drain, ring, abort_v, status);
   } else if (warp == 0) {
     // ---------------------------------------------------------------- weight producer: arms each stage, streams tile records
     if (lane == 0) {
       uint32_t it = 0;
       bool ok = true;
       auto block_of = [&](int u) { return u >= units1 ? (u - units1) / kW2Tiles : u / kW13Tiles; };
-      // the expert id of a unit is fetched one unit ahead (a GEMM2 unit is only three stages long)
-      int e_ahead = deal.first() < total_units ? __ldcg(block_expert + block_of(deal.first())) : 0;
-      for (int u = deal.first(); u < total_units && ok; u = deal.next(u)) {
+      int u = claim_unit12(done, status);
+      ring.put(0, u);
+      int e = u < total_units ? __ldcg(block_expert + block_of(u)) : 0;
+      for (uint32_t ui = 0; u < total_units; ++ui) {
         const bool second = u >= units1;
         const int v = second ? u - units1 : u;
         const int tiles_m = second ? kW2Tiles : kW13Tiles, tiles_k = second ? kK2Tiles : kK1Tiles;
-        const int mt = v % tiles_m;
-        int e = e_ahead;
-        const int un = deal.next(u);
-        if (un < total_units) e_ahead = __ldcg(block_expert + block_of(un));
+        const int mt = v % tiles_m, claim_at = tiles_k - (second ? 2 : 8);
+        int un = kNoUnit, e_next = 0;
         if (e < 0 || e >= num_experts) {
           atomicExch(status, B200MOE_DEV_BAD_INDEX);
           e = 0;
@@ -724,10 +720,17 @@ __global__ void __launch_bounds__(256, 1)
         for (int kt = 0; kt < tiles_k; ++kt, ++it) {
           const uint32_t s = it % CC::kStages, ph = (it / CC::kStages) & 1u;
           if (!mbar_wait(smem_u32(&bar_empty[s]), ph ^ 1u, abort_v, status)) { ok = false; break; }
+          // the next unit and its expert: two memory round trips, both beside copies in flight
+          if (kt == claim_at) un = claim_unit12(done, status);
+          if (kt == tiles_k - 1 && un < total_units) e_next = __ldcg(block_expert + block_of(un));
           const uint32_t full = smem_u32(&bar_full[s]);
           mbar_arrive_expect_tx(full, C::kStageBytes);  // the whole stage: the activation producer's bytes included
           bulk_load(tiles + s * C::kStageBytes, w_src + static_cast<int64_t>(kt) * kTileRecordBytes, kTileRecordBytes, full);
         }
+        if (!ok) break;
+        ring.put(ui + 1, un);
+        u = un;
+        e = e_next;
       }
       if (!ok) {
         drain_copies(bar_full, it, CC::kStages);
@@ -739,9 +742,10 @@ __global__ void __launch_bounds__(256, 1)
     // thread that keeps the weight stream full.
     if (lane == 0) {
       uint32_t it = 0;
-      bool ok = true, have_next = false;
-      int next_count = 0;
-      for (int u = deal.first(); u < total_units && ok; u = deal.next(u)) {
+      bool ok = true;
+      for (uint32_t ui = 0; ok; ++ui) {
+        const int u = ring.get(ui, abort_v, status);
+        if (u >= total_units) break;
         const bool second = u >= units1;
         const int v = second ? u - units1 : u;
         const int tiles_m = second ? kW2Tiles : kW13Tiles, tiles_k = second ? kK2Tiles : kK1Tiles;
@@ -749,12 +753,12 @@ __global__ void __launch_bounds__(256, 1)
         const uint8_t* sfb_src = second ? ep.sfh + static_cast<int64_t>(b) * C2::kActAtomsPerBlock * kAtomBytes
                                         : sf_x + static_cast<int64_t>(b) * C::kActAtomsPerBlock * kAtomBytes;
         if (second) {
-          // h of this row block must be complete and visible to the copy engine before it is read. The count was
-          // fetched while the previous unit's copies were issued, so the usual case costs no memory round trip.
-          // Usual case: the look-ahead (an acquire load: a load, not a fence, so it does not wait for this thread's
-          // copies in flight) has already seen 12. The writers ordered their stores for the copy engine before they
-          // counted (see the GEMM1 epilogue), so no fence is needed here.
-          if (!(have_next && next_count >= kW13Tiles)) {
+          // h of this row block must be complete and visible to the copy engine before it is read. Usual case: an acquire
+          // load (a load, not a fence, so it does not wait for this thread's copies in flight) sees all tiles. The writers
+          // ordered their stores for the copy engine before they counted (see the GEMM1 epilogue), so no fence is needed.
+          int seen;
+          asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(seen) : "l"(done + b) : "memory");
+          if (tiles_done(seen) < kW13Tiles) {
             if (!wait_count(done + b, kW13Tiles, abort_v, status)) { ok = false; break; }
             asm volatile("fence.proxy.async;" ::: "memory");
           }
@@ -767,10 +771,6 @@ __global__ void __launch_bounds__(256, 1)
           tma_load_2d(base + C::kBOffset, second ? &map_h : &map_x, kt * 128, b * BM, full);
           bulk_load(base + C::kSfbOffset, sfb_src + kt * C::kSfBytes, C::kSfBytes, full);
         }
-        const int un = deal.next(u);  // look ahead: the next unit's completion count
-        have_next = un < total_units && un >= units1;
-        if (have_next)
-          asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(next_count) : "l"(done + (un - units1) / kW2Tiles) : "memory");
       }
     }
   } else if (warp == 1) {
@@ -780,10 +780,12 @@ __global__ void __launch_bounds__(256, 1)
       constexpr uint32_t kId0 = kIdesc, kId1 = kIdesc | (2u << 29) | (2u << 4);
       // as in grouped_gemm_kernel: warp 7 copies the scales, this thread waits for that and issues the MMAs
       const uint32_t sf0 = smem_u32(&bar_sf[0]), empty0 = smem_u32(&bar_empty[0]);
-      uint32_t slot = 0, ph = 0, sfset = 0, ui = 0;
+      uint32_t slot = 0, ph = 0, sfset = 0;
       uint32_t lo = tiles >> 4, sf = sf0, empty = empty0;
       bool ok = true;
-      for (int u = deal.first(); u < total_units && ok; u = deal.next(u), ++ui) {
+      for (uint32_t ui = 0; ok; ++ui) {
+        const int u = ring.get(ui, abort_v, status);
+        if (u >= total_units) break;
         const int tiles_k = u >= units1 ? kK2Tiles : kK1Tiles;
         const uint32_t acc = ui & 1u, aph = (ui >> 1) & 1u;
         if (!mbar_wait(smem_u32(&bar_tempty[acc]), aph ^ 1u, abort_v, status)) break;
@@ -817,7 +819,9 @@ __global__ void __launch_bounds__(256, 1)
       uint32_t slot = 0, ph = 0, sfset = 0;
       uint32_t lo = tiles >> 4, full = full0, sf = sf0;
       bool ok = true;
-      for (int u = deal.first(); u < total_units && ok; u = deal.next(u)) {
+      for (uint32_t ui = 0; ok; ++ui) {
+        const int u = ring.get(ui, abort_v, status);
+        if (u >= total_units) break;
         const int tiles_k = u >= units1 ? kK2Tiles : kK1Tiles;
         for (int kt = 0; kt < tiles_k; ++kt) {
           if (!mbar_wait(full, ph, abort_v, status)) { ok = false; break; }
@@ -847,8 +851,8 @@ __global__ void __launch_bounds__(256, 1)
     bool have_ahead = false;
     int ahead_sid = 0;
     float ahead_wt = 0.0f;
-    for (int u = deal.first(); u < total_units; u = deal.next(u), ++ui) {
-      const bool second = u >= units1;
+    for (int u = ring.get(0, abort_v, status), un;; u = un, ++ui) {
+      const bool live = u < total_units, second = live && u >= units1;
       const int v = second ? u - units1 : u;
       const int tiles_m = second ? kW2Tiles : kW13Tiles;
       const int b = v / tiles_m, mt = v % tiles_m;
@@ -862,10 +866,10 @@ __global__ void __launch_bounds__(256, 1)
         s_dst[et] = placer.row(ahead_sid);
         s_wt[et] = ahead_wt;
       }
-      if (!epilogue_all(mbar_wait(smem_u32(&bar_tfull[acc]), aph, abort_v, status), 1u)) break;
+      if (!epilogue_all(live && mbar_wait(smem_u32(&bar_tfull[acc]), aph, abort_v, status), 1u)) break;
       tc_fence_after();
       {  // look ahead: the rows of this CTA's next unit, when that is a GEMM2 unit
-        const int un = deal.next(u);
+        un = ring.get(ui + 1, abort_v, status);
         have_ahead = un < total_units && un >= units1;
         if (have_ahead && et < BM) {
           const int64_t r1 = static_cast<int64_t>((un - units1) / kW2Tiles) * BM + et;

@@ -9,8 +9,9 @@
 //
 // What bounds it: the thread that issues the MMAs (about 60 cycles per tcgen05 instruction, 48 K-tiles of 128 elements per
 // unit), not the bytes. Unit = (block of bm tokens, weight tile of 128 rows); first all GEMM1 units, then all GEMM2 units,
-// dealt round-robin. A GEMM2 unit waits -- bounded -- until the W13 tiles of its block are counted done; GEMM1 units never
-// wait and every CTA has its GEMM1 units first, so progress does not depend on the order in which CTAs are scheduled.
+// claimed in that order from a ticket. A GEMM2 unit waits -- bounded -- until the W13 tiles of its block are counted done;
+// GEMM1 units never wait, and whoever claimed one is running, so the wait ends whichever CTAs of the launch are resident and
+// whatever else runs on the device.
 //
 //   warp 0    producer (weights, tokens, token scales)     warp 1    MMA issue
 //   warp 6    scale copies to tensor memory                warps 2-5 epilogue
@@ -31,6 +32,7 @@ struct SharedArgs {
   uint8_t* sfh8;        // GEMM1 out: scale atoms [blocks][I/128][512]
   __nv_bfloat16* out;   // bf16 [tokens][6144]
   int32_t* done;        // [blocks] finished GEMM1 tiles, zero at entry
+  int32_t* ticket;      // units claimed so far, zero at entry
   int64_t tokens;
   int n_blocks, bm;     // dense blocks of bm = 16 / 32 / 64 / 128 tokens
   int stages;
@@ -53,6 +55,9 @@ SharedWorkspace carve_shared(uint8_t* base, int64_t tokens);
 int shared_plan(SharedPlan* plan, const uint8_t* w13t, const uint8_t* w2t, const uint8_t* codes8, int64_t code_rows,
                 const SharedWorkspace& ws, void* out_bf16, int64_t tokens, int32_t* done, bool both);
 
+// int32 words of a decode launch that belong to the role, zero at entry: finished GEMM1 tiles per block of tokens (at most 512
+// tokens in blocks of 128), the last one its ticket
+constexpr int kSharedDone = 8;
 constexpr int kSharedMaxStages = 8;
 constexpr int kSharedMaxSmem = 225 * 1024;  // opt-in limit of the kernels that carry the role
 // shared memory: [stages x (record | tokens | scales)][epilogue staging]
@@ -61,14 +66,17 @@ __host__ __device__ inline int shared_epi_bytes(int bm) { return (bm < 64 ? bm :
 static inline int shared_stages(int bm) { return bm == 128 ? 5 : bm == 64 ? 6 : 8; }
 static inline int shared_smem_bytes(int bm) { return shared_stages(bm) * shared_stage_bytes(bm) + shared_epi_bytes(bm) + 1024; }
 
-// Bounded wait for a completion count in global memory (an acquire load).
+// A word that counts finished tiles: the low byte, signed (gemm12_kernel hands out its units above that).
+__device__ __forceinline__ int tiles_done(int word) { return static_cast<int8_t>(word & 255); }
+
+// Bounded wait for such a count in global memory (an acquire load).
 __device__ __forceinline__ bool wait_count(const int32_t* counter, int target, volatile int* abort_flag, int32_t* status) {
   const uint64_t t0 = global_timer();
   uint32_t spins = 0;
   while (true) {
     int v;
     asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(counter) : "memory");
-    if (v >= target) return true;
+    if (tiles_done(v) >= target) return true;
     if ((++spins & 63u) == 0u) {
       if (*abort_flag) return false;
       if (global_timer() - t0 > wait_limit_ns()) {
@@ -80,13 +88,34 @@ __device__ __forceinline__ bool wait_count(const int32_t* counter, int target, v
   }
 }
 
+// The units of a CTA whose work is handed out while it runs. One thread (the weight producer) claims a unit and puts it into a
+// ring in shared memory; the other roles take the units from there in the same order. The barriers have count 1. An entry is
+// written again kUnitRing units later: the producer is at most ceil(8 / 3) units ahead of the MMA thread (8 stages, units of at
+// least 3), that one at most two ahead of the epilogue (two accumulators), and one unit is claimed ahead.
+constexpr int kUnitRing = 16;
+constexpr int kNoUnit = 0x7fffffff;  // beyond every list: the CTA is aborting
+struct UnitRing {
+  uint64_t* bar;
+  volatile int* unit;
+  __device__ __forceinline__ void put(uint32_t i, int u) const {
+    unit[i % kUnitRing] = u;
+    mbar_arrive(smem_u32(bar + i % kUnitRing));
+  }
+  __device__ __forceinline__ int get(uint32_t i, volatile int* abort_flag, int32_t* status) const {
+    if (!mbar_wait(smem_u32(bar + i % kUnitRing), (i / kUnitRing) & 1u, abort_flag, status)) return kNoUnit;
+    return unit[i % kUnitRing];
+  }
+};
+
 // The barriers (bar_full, bar_empty, bar_sf: count 1 and at least a.stages long; bar_tfull[2] count 1; bar_tempty[2] count 128;
-// bar_drain[2] count 1) are initialised by the caller, tensor memory has at least 2 * bm + 64 columns, and the caller has
-// passed its wait for the predecessor. `smem` is the 1024-byte aligned dynamic shared memory, `tiles` its 32-bit address.
+// bar_drain[2] count 1; those of `ring`) are initialised by the caller, tensor memory has at least 2 * bm + 64 columns, and the
+// caller has passed its wait for the predecessor. `smem` is the 1024-byte aligned dynamic shared memory, `tiles` its 32-bit
+// address.
 __device__ __forceinline__ void shared_role(const SharedArgs& a, const CUtensorMap* map_x, const CUtensorMap* map_h,
                                             uint8_t* smem, uint32_t tiles, uint32_t tmem_base, uint64_t* bar_full,
                                             uint64_t* bar_empty, uint64_t* bar_sf, uint64_t* bar_tfull, uint64_t* bar_tempty,
-                                            uint64_t* bar_drain, volatile int* abort_v, int32_t* status) {
+                                            uint64_t* bar_drain, const UnitRing ring, volatile int* abort_v,
+                                            int32_t* status) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int bm = a.bm, ctas = a.ctas;
   const uint32_t stages = a.stages;
@@ -100,12 +129,12 @@ __device__ __forceinline__ void shared_role(const SharedArgs& a, const CUtensorM
       const uint32_t full0 = smem_u32(bar_full), empty0 = smem_u32(bar_empty);
       uint32_t it = 0, slot = 0, ph = 1u, base = tiles, full = full0, empty = empty0;
       bool ok = true;
-      for (int u = first; u < total; u += ctas) {  // the GEMM2 weights this CTA reads later
-        if (u >= units1)
-          l2_prefetch_bulk(a.w2t + static_cast<int64_t>((u - units1) % kW2Tiles) * kS2TilesK * kTileRecordBytes,
-                           kS2TilesK * kTileRecordBytes);
-      }
-      for (int u = first; u < total && ok; u += ctas) {
+      int u = atomicAdd(a.ticket, 1);
+      ring.put(0, u);
+      for (int mt = first; mt < kW2Tiles; mt += ctas)  // the CTAs share the GEMM2 weights' way into L2
+        l2_prefetch_bulk(a.w2t + static_cast<int64_t>(mt) * kS2TilesK * kTileRecordBytes, kS2TilesK * kTileRecordBytes);
+      for (uint32_t ui = 0; u < total && ok; ++ui) {
+        int next = kNoUnit;
         const bool second = u >= units1;
         const int v = second ? u - units1 : u, tiles_m = second ? kW2Tiles : kW13Tiles;
         const int tiles_k = second ? kS2TilesK : kS1TilesK;
@@ -118,6 +147,8 @@ __device__ __forceinline__ void shared_role(const SharedArgs& a, const CUtensorM
         }
         for (int kt = 0; kt < tiles_k; ++kt, ++it) {
           if (!mbar_wait(empty, ph, abort_v, status)) { ok = false; break; }
+          // late in the unit, so that a CTA which is ahead gets more of them, and early enough to hide the atomic's way
+          if (kt == tiles_k - 4) next = atomicAdd(a.ticket, 1);
           mbar_arrive_expect_tx(full, 128 * 128 + kAtomBytes + bm * 128 + kAtomBytes);
           bulk_load(base, w_src, 128 * 128 + kAtomBytes, full);
           tma_load_2d(base + b_off, second ? map_h : map_x, kt * 128, b * bm, full);
@@ -130,6 +161,9 @@ __device__ __forceinline__ void shared_role(const SharedArgs& a, const CUtensorM
             base += stage_bytes; full += 8; empty += 8;
           }
         }
+        if (!ok) break;
+        ring.put(ui + 1, next);
+        u = next;
       }
       if (!ok) drain_copies(bar_full, it, stages);
     }
@@ -138,10 +172,12 @@ __device__ __forceinline__ void shared_role(const SharedArgs& a, const CUtensorM
       // E4M3 x E4M3 (format 0), UE8M0 scales, M = 128 weight rows, N = bm tokens; scale byte k of a row's cell for MMA k
       const uint32_t idesc = (static_cast<uint32_t>(bm >> 3) << 17) | (1u << 23) | (8u << 24);
       const uint32_t sf0 = smem_u32(bar_sf), empty0 = smem_u32(bar_empty);
-      uint32_t slot = 0, ph = 0, sfset = 0, ui = 0;
+      uint32_t slot = 0, ph = 0, sfset = 0;
       uint32_t lo = tiles >> 4, sf = sf0, empty = empty0;
       bool ok = true;
-      for (int u = first; u < total && ok; u += ctas, ++ui) {
+      for (uint32_t ui = 0; ok; ++ui) {
+        const int u = ring.get(ui, abort_v, status);
+        if (u >= total) break;
         const int tiles_k = u >= units1 ? kS2TilesK : kS1TilesK;
         const uint32_t acc = ui & 1u, aph = (ui >> 1) & 1u;
         if (!mbar_wait(smem_u32(bar_tempty + acc), aph ^ 1u, abort_v, status)) break;
@@ -174,7 +210,9 @@ __device__ __forceinline__ void shared_role(const SharedArgs& a, const CUtensorM
       uint32_t slot = 0, ph = 0, sfset = 0;
       uint32_t lo = tiles >> 4, full = full0, sf = sf0;
       bool ok = true;
-      for (int u = first; u < total && ok; u += ctas) {
+      for (uint32_t ui = 0; ok; ++ui) {
+        const int u = ring.get(ui, abort_v, status);
+        if (u >= total) break;
         const int tiles_k = u >= units1 ? kS2TilesK : kS1TilesK;
         for (int kt = 0; kt < tiles_k; ++kt) {
           if (!mbar_wait(full, ph, abort_v, status)) { ok = false; break; }
@@ -198,14 +236,14 @@ __device__ __forceinline__ void shared_role(const SharedArgs& a, const CUtensorM
     const int q = warp & 3;
     const int et = threadIdx.x - 64;
     float* stage_f = reinterpret_cast<float*>(smem + stages * stage_bytes);
-    uint32_t ui = 0;
-    for (int u = first; u < total; u += ctas, ++ui) {
+    for (uint32_t ui = 0;; ++ui) {
+      const int u = ring.get(ui, abort_v, status);
       const bool second = u >= units1;
       const int v = second ? u - units1 : u, tiles_m = second ? kW2Tiles : kW13Tiles;
       const int b = v / tiles_m, mt = v % tiles_m;
       const uint32_t acc = ui & 1u, aph = (ui >> 1) & 1u;
       const int64_t row0 = static_cast<int64_t>(b) * bm;
-      if (!epilogue_all(mbar_wait(smem_u32(bar_tfull + acc), aph, abort_v, status), 1u)) break;
+      if (!epilogue_all(u < total && mbar_wait(smem_u32(bar_tfull + acc), aph, abort_v, status), 1u)) break;
       tc_fence_after();
       const uint32_t t_acc = tmem_base + acc * bm + (static_cast<uint32_t>(q * 32) << 16);
       const int row_floats = second ? 132 : 136, cols = min(bm, second ? 32 : 64);

@@ -390,8 +390,8 @@ SharedWorkspace carve_shared(uint8_t* base, int64_t tokens) {
   return ws;
 }
 
-// The role's part of a launch (shared_role.cuh): codes8 [code_rows][6144] and ws.sfx8 hold the quantised tokens, `done` is one
-// zeroed count per block. `both`: the launch does both routed GEMMs, so the role has their whole time.
+// The role's part of a launch (shared_role.cuh): codes8 [code_rows][6144] and ws.sfx8 hold the quantised tokens, `done` the
+// kSharedDone zeroed words. `both`: the launch does both routed GEMMs, so the role has their whole time.
 // CTAs of the role, measured (whole layer with the router inside, us; I = 768 / I = 1536): the routed experts' weight stream misses
 // 16 SMs least, 24 or 48 cost it 1 to 15 % (32 tokens 127 / 130 / 148; 128 tokens, I = 1536, 317 / 325 / 384), so
 //   16 while the role ends before they do;
@@ -416,6 +416,7 @@ int shared_plan(SharedPlan* plan, const uint8_t* w13t, const uint8_t* w2t, const
   a.sfh8 = ws.sfh8;
   a.out = static_cast<__nv_bfloat16*>(out_bf16);
   a.done = done;
+  a.ticket = done + kSharedDone - 1;
   a.tokens = tokens;
   a.n_blocks = static_cast<int>(ws.rows / ws.bm);
   a.bm = ws.bm;

@@ -374,8 +374,8 @@ def grouped_gemm1_gather(codes, scales, sort: SortBuffers, w: MoeWeights, by_pai
 
 def grouped_gemm12(xq_sorted, sfx, sort: SortBuffers, w: MoeWeights, slots=None, done=None):
     """Both grouped GEMMs in one persistent launch (block heights 16 / 32 / 64): -> (slots, h codes, h scale atoms), the
-    same bits as ``grouped_gemm1`` followed by ``grouped_gemm2`` (reference gemm12_a4w4.py:24). ``done``: the per-block
-    completion counts, int32 [rows / bm], zero on entry (allocated when not given)."""
+    same bits as ``grouped_gemm1`` followed by ``grouped_gemm2`` (reference gemm12_a4w4.py:24). ``done``: the launch's
+    per-block completion counts, int32 [rows / bm], zero on entry (allocated when not given)."""
     dev = xq_sorted.device
     hq = torch.empty((sort.max_rows, w.intermediate // 2), dtype=torch.uint8, device=dev)
     sfh = torch.empty((sort.max_rows // sort.bm, w.intermediate // 128, 512), dtype=torch.uint8, device=dev)

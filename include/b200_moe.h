@@ -261,10 +261,11 @@ int b200moe_gemm2_weighted(const uint8_t* w2t, int num_experts, const uint8_t* h
 
 /* Both grouped GEMMs in ONE persistent launch, for bm = 16 / 32 / 64 (MOE/gemm12_a4w4.py:24 gemm12_a4w4: GEMM1 and GEMM2
  * work in one launch ordered by ready counters). Same inputs, outputs and bits as b200moe_gemm1_swiglu_quant followed by
- * b200moe_gemm2_weighted. `done` int32 [max_rows/bm] must be zero on entry (b200moe_quant_dispatch zeroes it); it counts
- * the finished GEMM1 tiles of every row block, and a GEMM2 unit starts when its block shows 12. Unlike the reference's
- * wait, the wait here is bounded (about two seconds, then status = B200MOE_DEV_TIMEOUT and the kernel winds down), and
- * GEMM1 work never waits, so completion does not depend on the order in which CTAs are scheduled. */
+ * b200moe_gemm2_weighted. `done` int32 [max_rows/bm] must be zero on entry (b200moe_quant_dispatch zeroes it). It is the
+ * launch's scratch: the low byte of a word counts the finished GEMM1 tiles of its row block, and a GEMM2 unit starts when its
+ * block shows all of them; the first word also hands out the units, GEMM1 first, to the CTAs that run. GEMM1 work never waits,
+ * so a wait ends whichever CTAs are resident and whatever other launches hold SMs; unlike the reference's it is also bounded
+ * (about two seconds, then status = B200MOE_DEV_TIMEOUT and the kernel winds down). */
 int b200moe_gemm12(const uint8_t* w13t, const uint8_t* w2t, int num_experts, const uint8_t* xq_sorted, const uint8_t* sfx,
                    const int32_t* block_expert, const int32_t* num_valid, const int32_t* sorted_ids, const float* sorted_w,
                    int64_t max_rows, int bm, int64_t tokens, uint8_t* hq, uint8_t* sfh, int32_t* done, void* slots_bf16,

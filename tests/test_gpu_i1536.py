@@ -186,3 +186,26 @@ def test_a_shared_expert_of_the_other_intermediate_size(P, C, tokens, routed):
         assert torch.equal(P.mxfp4_moe(form, w), C.reduce_slots(slots0, want))
     torch.cuda.synchronize()
     assert C.last_status() == 0
+
+
+@pytest.mark.parametrize("tokens", [1, 64, 200])
+def test_two_calls_at_once(P, C, tokens):
+    """Two streams of different priority, each with calls whose CTAs wait for one another (both GEMMs and the shared expert in
+    one launch): every result has the bits of the call alone, and no wait runs out."""
+    raw, gen = orc.make_weights(seed=77, experts=EXPERTS, inter=I2)
+    sw = P.SharedWeights.from_row_major(*(dev(a) for a in orc.make_shared_weights(seed=78, inter=I2)))
+    w = P.MoeWeights.from_row_major(None, None, *(dev(a) for a in raw), shared=sw, routing_mode="softmax", routed_scaling_factor=1.0)
+    xs = [torch.randn((tokens, H), generator=gen).bfloat16().cuda() for _ in range(2)]
+    lgs = [torch.randn((tokens, EXPERTS), generator=gen).cuda() for _ in range(2)]
+    alone = [P.mxfp4_moe(x, w, router_logits=lg) for x, lg in zip(xs, lgs)]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream(priority=p) for p in (0, -1)]
+    outs = [[], []]
+    for _ in range(40):
+        for i, st in enumerate(streams):
+            with torch.cuda.stream(st):
+                outs[i].append(P.mxfp4_moe(xs[i], w, router_logits=lgs[i]))
+    torch.cuda.synchronize()
+    assert C.last_status() == 0
+    for got, want in zip(outs, alone):
+        assert all(torch.equal(o, want) for o in got)

@@ -282,3 +282,25 @@ def test_no_kernel_reads_global_memory_before_its_wait():
         early = re.findall(r"__ldg\(|__ldcg\(|\bld\.|cp\.async\.c[ag]\b|\bload_\w+\(|\*\s*reinterpret_cast<const", body[:at.start()])
         assert not early, (f, name, early)
     assert seen >= 15
+
+
+def _function(file, start):
+    """The source of the function that begins at ``start``, comments removed."""
+    text = re.sub(r"//[^\n]*", "", open(os.path.join(ROOT, "amd_kernels_b200", "csrc", file)).read())
+    body = text[text.index(start):]
+    return body[:body.index("\n}\n")]
+
+
+@pytest.mark.parametrize("file,start,claim", [("gemm_tc.cu", "gemm12_kernel(const", "claim_unit12(done"),
+                                              ("shared_role.cuh", "void shared_role(", "atomicAdd(a.ticket, 1)")])
+def test_units_that_others_wait_for_belong_to_running_ctas(file, start, claim):
+    """Where work of one CTA waits for work of another, a unit is claimed by a CTA that runs. A fixed deal by block index gives
+    GEMM1 units to CTAs that may not be resident while waiting ones hold the SMs (two launches on two streams), and then the
+    waits run out. So the block index chooses a role here, never a unit."""
+    body = _function(file, start)
+    assert body.count(claim) == 2  # the first unit, and the next one
+    assert "wait_count(" in body and "ring.put(0, u)" in body and body.count("ring.get(") >= 3
+    for line in body.splitlines():
+        if "blockIdx" in line:
+            assert re.search(r"blockIdx\.x\) (>= n_ctas|- \(static_cast<int>\(gridDim\.x\) - ctas\))", line), line
+    assert not re.search(r"u \+= (n_ctas|ctas|gridDim)", body)
