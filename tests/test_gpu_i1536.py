@@ -8,7 +8,7 @@ import torch
 
 from oracle import moe_oracle as orc
 from tests.test_gpu_moe import check_against_oracle
-from tests.util import H, atoms_to_rowmajor, bf16_dev, bits_of, dev, make_routing, oracle_slots
+from tests.util import H, atoms_to_rowmajor, bf16_dev, bits_of, dev, make_routing, oracle_slots, staged_slots
 
 pytestmark = pytest.mark.gpu
 I2, EXPERTS = 1536, 8  # noqa: E741
@@ -102,6 +102,7 @@ def test_entry_against_the_oracle(P, C, sibling, tokens):
     x_only, _ = P.mxfp4_moe(x, w, return_partials=True)
     wt, ids = P.route(x, w)
     assert torch.equal(x_only, P.mxfp4_moe_experts(C.mxfp4_quant(x), wt, ids, w))
+    assert torch.equal(x_only, staged_slots(C, C.mxfp4_quant(x), wt, ids, w))
     got = oracle_slots(ref["xq"], ref["xs"], raw, ids.cpu().numpy()[pick], wt.cpu().numpy()[pick])
     check_against_oracle(x_only.float().cpu().numpy()[pick].sum(1), got.sum(1))
     torch.cuda.synchronize()

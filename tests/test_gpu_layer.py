@@ -1,0 +1,109 @@
+"""The whole-layer call with the shared expert, at both intermediate sizes and on both sides of every rule that chooses its
+route, against kernels that share nothing with it above the grouped GEMMs: the routed experts by the staged kernels (sort,
+gather, GEMM1, GEMM2, a launch each) and the shared expert alone. All comparisons are bit for bit."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import moe_oracle as orc
+from tests.util import H, bits_of, dev, staged_slots
+
+pytestmark = pytest.mark.gpu
+EXPERTS = 8
+
+
+@pytest.fixture(scope="module")
+def C():
+    from amd_kernels_b200.moe.mxfp4_h6144_i768_e128_top4 import chain
+    return chain
+
+
+@pytest.fixture(scope="module")
+def S():
+    from amd_kernels_b200.moe.mxfp4_h6144_i768_e128_top4 import shared_expert
+    return shared_expert
+
+
+def build_layer(inter):
+    from amd_kernels_b200.moe import mxfp4_h6144_i768_e128_top4 as p768, mxfp4_h6144_i1536_e128_top4 as p1536
+    pkg = p768 if inter == 768 else p1536
+    raw, gen = orc.make_weights(seed=inter, experts=EXPERTS, inter=inter)
+    sw = pkg.SharedWeights.from_row_major(*(dev(a) for a in orc.make_shared_weights(seed=inter + 1, inter=inter)))
+    gate = torch.randn((EXPERTS, H), generator=gen) / H ** 0.5
+    return pkg.MoeWeights.from_row_major(gate.cuda(), None, *(dev(a) for a in raw), shared=sw, routing_mode="softmax",
+                                         routed_scaling_factor=1.0)
+
+
+@pytest.fixture(scope="module", params=[768, 1536])
+def layer(request):
+    return build_layer(request.param)
+
+
+def inputs(m, seed=0):
+    gen = torch.Generator().manual_seed(10 * m + seed)
+    return (torch.randn((m, H), generator=gen) * 0.7).bfloat16().cuda(), torch.randn((m, EXPERTS), generator=gen).cuda()
+
+
+def separate_calls(C, S, x, w, logits):
+    """(slots, shared rows, their sum) of the same layer by separate launches."""
+    wt, ids = C.route(x, w, logits)
+    slots = staged_slots(C, C.mxfp4_quant(x), wt, ids, w)
+    # the shared expert in batches of 64: below the sizes of the CTA-pair kernels, on a stream of its own launches
+    shared = torch.cat([S.shared_expert(x[a:a + 64].contiguous(), w.shared_weights) for a in range(0, len(x), 64)])
+    return slots, shared, torch.from_numpy(orc.reduce_slots_bf16(bits_of(slots), bits_of(shared)).view(np.int16)).cuda().view(torch.bfloat16)
+
+
+@pytest.mark.parametrize("router", [True, False])
+@pytest.mark.parametrize("m", [1, 32, 33, 127, 128, 480, 481, 512, 513, 777, 1409, 4096])
+def test_layer_equals_the_separate_calls(C, S, layer, m, router):
+    """One launch for both GEMMs / two, the role at 16-, 32-, 64- and 128-token blocks, above 512 tokens both quantisers in one
+    pass and the shared GEMMs forked to the side stream, from 1409 on CTA pairs."""
+    x, lg = inputs(m)
+    lg = None if router else lg
+    slots0, shared0, sum0 = separate_calls(C, S, x, layer, lg)
+    slots, shared = C.mxfp4_moe(x, layer, return_partials=True, router_logits=lg)
+    assert torch.equal(slots, slots0) and torch.equal(shared, shared0)
+    assert torch.equal(C.mxfp4_moe(x, layer, router_logits=lg), sum0)
+    torch.cuda.synchronize()
+    assert C.last_status() == 0
+
+
+@pytest.mark.parametrize("m", [1, 40, 512, 700, 1600])
+def test_layer_in_a_graph(C, S, layer, m):
+    """Capture and replay, the role and (above 512 tokens) the fork to the side stream and its join included: replayed into a
+    poisoned result, and again with other tokens in the same buffers."""
+    x, lg = inputs(m)
+    C.mxfp4_moe(x, layer, router_logits=lg)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = C.mxfp4_moe(x, layer, router_logits=lg)
+    for seed in (0, 1, 2):
+        x2, lg2 = inputs(m, seed)
+        want = separate_calls(C, S, x2, layer, lg2)[2]
+        x.copy_(x2)
+        lg.copy_(lg2)
+        out.fill_(float("nan"))
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, want)
+    assert C.last_status() == 0
+
+
+@pytest.mark.parametrize("m", [40, 700])
+def test_layer_inside_a_dual_batch_microbatch(C, S, layer, m):
+    """Inside a microbatch no side stream is used, from bf16 rows and from a prepared input, with the same bits."""
+    from amd_kernels_b200.moe.mxfp4_h6144_i768_e128_top4 import prepared_input as P
+    x, lg = inputs(m)
+    want = separate_calls(C, S, x, layer, lg)[2]
+    routed = separate_calls(C, S, x, layer, None)[2]
+    assert (C._side_stream(layer.shared_weights, m) is not None) == (m > 512)
+    S.set_dbo_query(lambda: True)
+    try:
+        assert C._side_stream(layer.shared_weights, m) is None
+        assert torch.equal(C.mxfp4_moe(x, layer, router_logits=lg), want)
+        assert torch.equal(C.mxfp4_moe(P.prepare_mxfp4_moe(x, layer), layer), routed)
+    finally:
+        S.set_dbo_query(None)
+    torch.cuda.synchronize()
+    assert C.last_status() == 0

@@ -11,7 +11,7 @@ import torch
 
 from oracle import moe_oracle as orc
 from tests.conftest import golden
-from tests.util import (H, atoms_to_rowmajor, bf16_dev, bits_of, cosine, dev, make_routing, oracle_slots, rel_l2)
+from tests.util import (H, atoms_to_rowmajor, bf16_dev, bits_of, cosine, dev, make_routing, oracle_slots, rel_l2, staged_slots)
 
 pytestmark = pytest.mark.gpu
 COS_MIN, REL_L2_MAX, MAX_ABS_FRACTION = 0.9999, 4e-3, 0.02
@@ -239,7 +239,8 @@ def test_entry_with_the_router_inside(C, layer, tokens, mode):
     assert np.array_equal(ids.cpu().numpy()[dec], ir[dec])
     np.testing.assert_allclose(wt.cpu().numpy()[dec.all(1)], wr[dec.all(1)], atol=1e-3, rtol=0)
     staged = C.mxfp4_moe_experts(C.mxfp4_quant(xd), wt, ids, w)
-    assert torch.equal(slots, staged), "the one-call entry and the staged kernels disagree"
+    assert torch.equal(slots, staged), "the one-call entry and the call on routed tokens disagree"
+    assert torch.equal(slots, staged_slots(C, C.mxfp4_quant(xd), wt, ids, w)), "the entry and the staged kernels disagree"
     assert np.array_equal(bits_of(out), orc.reduce_slots_bf16(bits_of(slots)))
     pick = np.unique(np.linspace(0, tokens - 1, 6).astype(int))
     xq, xs = orc.quant_mxfp4(x.float().numpy())

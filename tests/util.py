@@ -66,3 +66,10 @@ def cosine(a, b):
 
 def rel_l2(a, b):
     return float(np.linalg.norm(a.astype(np.float64) - b) / np.linalg.norm(b))
+
+
+def staged_slots(C, x_quant, wt, ids, w):
+    """The routed experts by the single kernels, a launch each (sort, gather, GEMM1, GEMM2) on quantised, routed rows: the bf16
+    slots [M, 4, H] that the one-call forms must reproduce bit for bit."""
+    sort = C.moe_sort(ids, wt, C.variant_for(len(ids)), w.num_experts)
+    return C.grouped_gemm2(*C.grouped_gemm1(*C.dispatch_rows(x_quant, sort), sort, w), sort, w)
