@@ -991,6 +991,7 @@ static LaunchShape launch_shape(int64_t units, int max_ctas, int smem, const Sha
   int64_t ctas = sm_count() - extra;
   if (units < ctas) ctas = units;
   if (max_ctas > 0 && ctas > max_ctas) ctas = max_ctas;
+  if (ctas < 1 && units > 0) ctas = 1;  // (fewer SMs than the role takes: both parts run, one after the other)
   const int need = sp ? shared_smem_bytes(sp->args.bm) : 0;
   return {static_cast<int>(ctas) + extra, need > smem ? need : smem};
 }

@@ -121,109 +121,109 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SharedPairCfg<MODE>:
 
   // The issuing warpgroup and the two epilogue warpgroups do not meet again before the kernel's last lines.
   if (warp < 4) {
-  asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
-  if (warp == 0) {
-    // ---------------------------------------------------------------- code producer (both CTAs)
-    if (lane == 0) {
-      const uint32_t full0 = map_to_cta(smem_u32(&bar_full[0]), 0);  // the leader's barriers, as seen from this CTA
-      uint32_t it = 0, s = 0, ph = 1u;
-      bool ok = true;
-      for (int u = cluster; u < total && ok; u += n_clusters) {
-        const int b = u / C::kTilePairs * 2 + static_cast<int>(rank), tp = u % C::kTilePairs;
-        // the weights seen as rows of 128 bytes: a record is 128 rows of codes, 4 of scales, 4 of padding
-        const int rec = (2 * tp + static_cast<int>(rank)) * C::kTilesK * 136;
-        for (int kt = 0; kt < C::kTilesK; ++kt, ++it) {
-          if (!mbar_wait(smem_u32(&bar_empty[s]), ph, abort_v, status)) { ok = false; break; }
-          const uint32_t full = full0 + 8u * s, base = tiles + s * C::kStageBytes;
-          if (leader) mbar_arrive_expect_tx(smem_u32(&bar_full[s]), 2 * C::kStageBytes);
-          // token rows beyond the last (an odd block count, the ragged end) are read as zeros and count all the same
-          tma_load_2d_pair(base + C::kTokOff, &map_x, kt * 128, b * 128, full);
-          tma_load_2d_pair(base + C::kWOff, &map_wc, 0, rec + kt * 136, full);
-          if (++s == C::kStages) { s = 0; ph ^= 1u; }
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
+    if (warp == 0) {
+      // ---------------------------------------------------------------- code producer (both CTAs)
+      if (lane == 0) {
+        const uint32_t full0 = map_to_cta(smem_u32(&bar_full[0]), 0);  // the leader's barriers, as seen from this CTA
+        uint32_t it = 0, s = 0, ph = 1u;
+        bool ok = true;
+        for (int u = cluster; u < total && ok; u += n_clusters) {
+          const int b = u / C::kTilePairs * 2 + static_cast<int>(rank), tp = u % C::kTilePairs;
+          // the weights seen as rows of 128 bytes: a record is 128 rows of codes, 4 of scales, 4 of padding
+          const int rec = (2 * tp + static_cast<int>(rank)) * C::kTilesK * 136;
+          for (int kt = 0; kt < C::kTilesK; ++kt, ++it) {
+            if (!mbar_wait(smem_u32(&bar_empty[s]), ph, abort_v, status)) { ok = false; break; }
+            const uint32_t full = full0 + 8u * s, base = tiles + s * C::kStageBytes;
+            if (leader) mbar_arrive_expect_tx(smem_u32(&bar_full[s]), 2 * C::kStageBytes);
+            // token rows beyond the last (an odd block count, the ragged end) are read as zeros and count all the same
+            tma_load_2d_pair(base + C::kTokOff, &map_x, kt * 128, b * 128, full);
+            tma_load_2d_pair(base + C::kWOff, &map_wc, 0, rec + kt * 136, full);
+            if (++s == C::kStages) { s = 0; ph ^= 1u; }
+          }
         }
+        if (!ok && leader) drain_copies(bar_full, it, C::kStages);
       }
-      if (!ok && leader) drain_copies(bar_full, it, C::kStages);
-    }
-  } else if (warp == 3) {
-    // ---------------------------------------------------------------- scale producer (both CTAs)
-    if (lane == 0) {
-      const uint32_t sfull0 = map_to_cta(smem_u32(&bar_sfull[0]), 0);
-      uint32_t it = 0;
-      bool ok = true;
-      for (int u = cluster; u < total && ok; u += n_clusters) {
-        const int b = u / C::kTilePairs * 2 + static_cast<int>(rank), tp = u % C::kTilePairs;
-        const int rec_lo = 2 * tp * C::kTilesK * 136 + 128, rec_hi = rec_lo + C::kTilesK * 136;
-        for (int kt = 0; kt < C::kTilesK; ++kt, ++it) {
-          const uint32_t j = it % C::kSfStages, ph = (it / C::kSfStages) & 1u;
-          // free once its previous contents are in tensor memory
-          if (!mbar_wait(smem_u32(&bar_sf[j]), ph ^ 1u, abort_v, status)) { ok = false; break; }
-          const uint32_t sfull = sfull0 + 8u * j, slot = sf_ring + j * C::kSfSlotBytes;
-          if (leader) mbar_arrive_expect_tx(smem_u32(&bar_sfull[j]), 2 * C::kSfSlotBytes);
-          tma_load_2d_pair(slot + C::kSfTokOff, &map_sfx, 0, (b * C::kTilesK + kt) * 4, sfull);
-          tma_load_2d_pair(slot + C::kSfWLoOff, &map_ws, 0, rec_lo + kt * 136, sfull);
-          tma_load_2d_pair(slot + C::kSfWHiOff, &map_ws, 0, rec_hi + kt * 136, sfull);
+    } else if (warp == 3) {
+      // ---------------------------------------------------------------- scale producer (both CTAs)
+      if (lane == 0) {
+        const uint32_t sfull0 = map_to_cta(smem_u32(&bar_sfull[0]), 0);
+        uint32_t it = 0;
+        bool ok = true;
+        for (int u = cluster; u < total && ok; u += n_clusters) {
+          const int b = u / C::kTilePairs * 2 + static_cast<int>(rank), tp = u % C::kTilePairs;
+          const int rec_lo = 2 * tp * C::kTilesK * 136 + 128, rec_hi = rec_lo + C::kTilesK * 136;
+          for (int kt = 0; kt < C::kTilesK; ++kt, ++it) {
+            const uint32_t j = it % C::kSfStages, ph = (it / C::kSfStages) & 1u;
+            // free once its previous contents are in tensor memory
+            if (!mbar_wait(smem_u32(&bar_sf[j]), ph ^ 1u, abort_v, status)) { ok = false; break; }
+            const uint32_t sfull = sfull0 + 8u * j, slot = sf_ring + j * C::kSfSlotBytes;
+            if (leader) mbar_arrive_expect_tx(smem_u32(&bar_sfull[j]), 2 * C::kSfSlotBytes);
+            tma_load_2d_pair(slot + C::kSfTokOff, &map_sfx, 0, (b * C::kTilesK + kt) * 4, sfull);
+            tma_load_2d_pair(slot + C::kSfWLoOff, &map_ws, 0, rec_lo + kt * 136, sfull);
+            tma_load_2d_pair(slot + C::kSfWHiOff, &map_ws, 0, rec_hi + kt * 136, sfull);
+          }
         }
+        if (!ok && leader) drain_copies(bar_sfull, it, C::kSfStages);
       }
-      if (!ok && leader) drain_copies(bar_sfull, it, C::kSfStages);
-    }
-  } else if (warp == 1) {
-    // ---------------------------------------------------------------- MMA issue (leader only)
-    if (lane == 0 && leader) {
-      // E4M3 x E4M3, UE8M0 scales, M = 256, N = 256; scale byte k of a row's cell for MMA k
-      constexpr uint32_t kIdesc = (static_cast<uint32_t>(256 >> 3) << 17) | (1u << 23) | (static_cast<uint32_t>(256 >> 4) << 24);
-      uint32_t ui = 0, s = 0, ph = 0, j = 0, sph = 0;
-      bool ok = true, sf_ready = false, full_ready = false;
-      for (int u = cluster; u < total && ok; u += n_clusters, ++ui) {
-        if (!mbar_wait(smem_u32(&bar_tempty), (ui & 1u) ^ 1u, abort_v, status)) break;
-        tc_fence_after();
-        for (int kt = 0; kt < C::kTilesK; ++kt) {
-          if (!sf_ready && !mbar_wait(smem_u32(&bar_sf[j]), sph, abort_v, status)) { ok = false; break; }
-          if (!full_ready && !mbar_wait(smem_u32(&bar_full[s]), ph, abort_v, status)) { ok = false; break; }
+    } else if (warp == 1) {
+      // ---------------------------------------------------------------- MMA issue (leader only)
+      if (lane == 0 && leader) {
+        // E4M3 x E4M3, UE8M0 scales, M = 256, N = 256; scale byte k of a row's cell for MMA k
+        constexpr uint32_t kIdesc = (static_cast<uint32_t>(256 >> 3) << 17) | (1u << 23) | (static_cast<uint32_t>(256 >> 4) << 24);
+        uint32_t ui = 0, s = 0, ph = 0, j = 0, sph = 0;
+        bool ok = true, sf_ready = false, full_ready = false;
+        for (int u = cluster; u < total && ok; u += n_clusters, ++ui) {
+          if (!mbar_wait(smem_u32(&bar_tempty), (ui & 1u) ^ 1u, abort_v, status)) break;
           tc_fence_after();
-          const uint32_t s_now = s, j_now = j;
-          if (++s == C::kStages) { s = 0; ph ^= 1u; }
-          if (++j == C::kSfStages) { j = 0; sph ^= 1u; }
-          sf_ready = mbar_test(smem_u32(&bar_sf[j]), sph);
-          full_ready = mbar_test(smem_u32(&bar_full[s]), ph);
-          const uint32_t lo = (tiles + s_now * C::kStageBytes) >> 4;
-          const uint32_t x_lo = lo + (C::kTokOff >> 4), w_lo = lo + (C::kWOff >> 4);
-          const uint32_t t_sft = tmem_base + C::kSfCol + 16u * j_now, t_sfw = t_sft + 8u;
-          tc_mma_mxf8_pair(tmem_base, x_lo, w_lo, kIdesc, t_sft, t_sfw, static_cast<uint32_t>(kt != 0));
-          tc_mma_mxf8_pair(tmem_base, x_lo + 2, w_lo + 2, kIdesc | (1u << 29) | (1u << 4), t_sft, t_sfw, 1u);
-          tc_mma_mxf8_pair(tmem_base, x_lo + 4, w_lo + 4, kIdesc | (2u << 29) | (2u << 4), t_sft, t_sfw, 1u);
-          tc_mma_mxf8_pair(tmem_base, x_lo + 6, w_lo + 6, kIdesc | (3u << 29) | (3u << 4), t_sft, t_sfw, 1u);
-          tc_commit_both(smem_u32(&bar_empty[s_now]));  // the stage is free again, in both CTAs
+          for (int kt = 0; kt < C::kTilesK; ++kt) {
+            if (!sf_ready && !mbar_wait(smem_u32(&bar_sf[j]), sph, abort_v, status)) { ok = false; break; }
+            if (!full_ready && !mbar_wait(smem_u32(&bar_full[s]), ph, abort_v, status)) { ok = false; break; }
+            tc_fence_after();
+            const uint32_t s_now = s, j_now = j;
+            if (++s == C::kStages) { s = 0; ph ^= 1u; }
+            if (++j == C::kSfStages) { j = 0; sph ^= 1u; }
+            sf_ready = mbar_test(smem_u32(&bar_sf[j]), sph);
+            full_ready = mbar_test(smem_u32(&bar_full[s]), ph);
+            const uint32_t lo = (tiles + s_now * C::kStageBytes) >> 4;
+            const uint32_t x_lo = lo + (C::kTokOff >> 4), w_lo = lo + (C::kWOff >> 4);
+            const uint32_t t_sft = tmem_base + C::kSfCol + 16u * j_now, t_sfw = t_sft + 8u;
+            tc_mma_mxf8_pair(tmem_base, x_lo, w_lo, kIdesc, t_sft, t_sfw, static_cast<uint32_t>(kt != 0));
+            tc_mma_mxf8_pair(tmem_base, x_lo + 2, w_lo + 2, kIdesc | (1u << 29) | (1u << 4), t_sft, t_sfw, 1u);
+            tc_mma_mxf8_pair(tmem_base, x_lo + 4, w_lo + 4, kIdesc | (2u << 29) | (2u << 4), t_sft, t_sfw, 1u);
+            tc_mma_mxf8_pair(tmem_base, x_lo + 6, w_lo + 6, kIdesc | (3u << 29) | (3u << 4), t_sft, t_sfw, 1u);
+            tc_commit_both(smem_u32(&bar_empty[s_now]));  // the stage is free again, in both CTAs
+          }
+          if (ok) tc_commit_both(smem_u32(&bar_tfull));
         }
-        if (ok) tc_commit_both(smem_u32(&bar_tfull));
+        if (*abort_v) drain_tcgen05_pair(smem_u32(&bar_drain[0]));
       }
-      if (*abort_v) drain_tcgen05_pair(smem_u32(&bar_drain[0]));
-    }
-  } else {
-    // ---------------------------------------------------------------- scale copies into both CTAs' tensor memory (leader)
-    if (lane == 0 && leader) {
-      uint32_t s = 0, ph = 1u, j = 0, sph = 0;
-      bool ok = true, landed = false, free_set = false;
-      for (int u = cluster; u < total && ok; u += n_clusters) {
-        for (int kt = 0; kt < C::kTilesK; ++kt) {
-          if (!landed && !mbar_wait(smem_u32(&bar_sfull[j]), sph, abort_v, status)) { ok = false; break; }
-          // set j was last read by the MMAs 8 K-tiles back: complete once those 6 K-tiles back are
-          if (!free_set && !mbar_wait(smem_u32(&bar_empty[s]), ph, abort_v, status)) { ok = false; break; }
-          tc_fence_after();
-          const uint32_t lo = (sf_ring + j * C::kSfSlotBytes) >> 4, sf_bar = smem_u32(&bar_sf[j]);
-          const uint32_t t_sft = tmem_base + C::kSfCol + 16u * j, t_sfw = t_sft + 8u;
-          if (++s == C::kStages) { s = 0; ph ^= 1u; }
-          if (++j == C::kSfStages) { j = 0; sph ^= 1u; }
-          landed = mbar_test(smem_u32(&bar_sfull[j]), sph);
-          free_set = mbar_test(smem_u32(&bar_empty[s]), ph);
-          tc_cp_scales_pair(t_sft, lo + (C::kSfTokOff >> 4));      // each CTA its own token rows
-          tc_cp_scales_pair(t_sfw, lo + (C::kSfWLoOff >> 4));      // weight rows 0..127 of N
-          tc_cp_scales_pair(t_sfw + 4, lo + (C::kSfWHiOff >> 4));  // 128..255
-          tc_commit_both(sf_bar);
+    } else {
+      // ---------------------------------------------------------------- scale copies into both CTAs' tensor memory (leader)
+      if (lane == 0 && leader) {
+        uint32_t s = 0, ph = 1u, j = 0, sph = 0;
+        bool ok = true, landed = false, free_set = false;
+        for (int u = cluster; u < total && ok; u += n_clusters) {
+          for (int kt = 0; kt < C::kTilesK; ++kt) {
+            if (!landed && !mbar_wait(smem_u32(&bar_sfull[j]), sph, abort_v, status)) { ok = false; break; }
+            // set j was last read by the MMAs 8 K-tiles back: complete once those 6 K-tiles back are
+            if (!free_set && !mbar_wait(smem_u32(&bar_empty[s]), ph, abort_v, status)) { ok = false; break; }
+            tc_fence_after();
+            const uint32_t lo = (sf_ring + j * C::kSfSlotBytes) >> 4, sf_bar = smem_u32(&bar_sf[j]);
+            const uint32_t t_sft = tmem_base + C::kSfCol + 16u * j, t_sfw = t_sft + 8u;
+            if (++s == C::kStages) { s = 0; ph ^= 1u; }
+            if (++j == C::kSfStages) { j = 0; sph ^= 1u; }
+            landed = mbar_test(smem_u32(&bar_sfull[j]), sph);
+            free_set = mbar_test(smem_u32(&bar_empty[s]), ph);
+            tc_cp_scales_pair(t_sft, lo + (C::kSfTokOff >> 4));      // each CTA its own token rows
+            tc_cp_scales_pair(t_sfw, lo + (C::kSfWLoOff >> 4));      // weight rows 0..127 of N
+            tc_cp_scales_pair(t_sfw + 4, lo + (C::kSfWHiOff >> 4));  // 128..255
+            tc_commit_both(sf_bar);
+          }
         }
+        if (*abort_v) drain_tcgen05_pair(smem_u32(&bar_drain[1]));
       }
-      if (*abort_v) drain_tcgen05_pair(smem_u32(&bar_drain[1]));
     }
-  }
   } else {
     // ---------------------------------------------------------------- epilogue (both CTAs, warps 4..11)
     asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");

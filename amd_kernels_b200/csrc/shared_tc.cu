@@ -401,7 +401,8 @@ SharedWorkspace carve_shared(uint8_t* base, int64_t tokens) {
 //   token, 45.4 -> 41.0 at 3).
 static int role_ctas(int64_t tokens, int n_blocks, bool both) {
   const int ctas = tokens <= 3 ? 48 : tokens <= 5 || (n_blocks >= 3 && !both) ? 24 : 16;
-  return ctas < sm_count() / 2 ? ctas : sm_count() / 2;
+  const int most = sm_count() / 2 > 1 ? sm_count() / 2 : 1;
+  return ctas < most ? ctas : most;
 }
 int shared_plan(SharedPlan* plan, const uint8_t* w13t, const uint8_t* w2t, const uint8_t* codes8, int64_t code_rows,
                 const SharedWorkspace& ws, void* out_bf16, int64_t tokens, int32_t* done, bool both) {

@@ -99,8 +99,8 @@ extern "C" int b200moe_sidecar_pack(const uint8_t* q4, const uint8_t* s4, const 
   if (r || tokens == 0) return r;
   const int64_t n = tokens * (kH / 8);
   B200MOE_LAUNCH(sidecar_pack_kernel, static_cast<unsigned>((n + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream),
-                       reinterpret_cast<const uint32_t*>(q4), s4, reinterpret_cast<const uint2*>(q8), s8,
-                 static_cast<uint32_t>(n), mask);
+                 reinterpret_cast<const uint32_t*>(q4), s4, reinterpret_cast<const uint2*>(q8), s8, static_cast<uint32_t>(n),
+                 mask);
   return 0;
 }
 
@@ -110,9 +110,8 @@ extern "C" int b200moe_sidecar_unpack(const uint8_t* mask, const uint8_t* s4, co
   const int r = sidecar_args(q4, s4, q8, s8, mask, tokens);
   if (r || tokens == 0) return r;
   const int64_t n = tokens * (kH / 8);
-  B200MOE_LAUNCH(sidecar_unpack_kernel, static_cast<unsigned>((n + 255) / 256), 256, 0,
-                       static_cast<cudaStream_t>(stream), mask, s4, reinterpret_cast<const uint2*>(q8), s8, static_cast<uint32_t>(n),
-                       reinterpret_cast<uint32_t*>(q4));
+  B200MOE_LAUNCH(sidecar_unpack_kernel, static_cast<unsigned>((n + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream), mask,
+                 s4, reinterpret_cast<const uint2*>(q8), s8, static_cast<uint32_t>(n), reinterpret_cast<uint32_t*>(q4));
   return 0;
 }
 
@@ -124,7 +123,7 @@ extern "C" int b200moe_scales_to_atoms(const uint8_t* rows, int64_t tokens, int 
   if ((reinterpret_cast<uintptr_t>(rows) & 3) || (reinterpret_cast<uintptr_t>(atoms) & 15)) return B200MOE_E_ALIGN;
   const int64_t padded = (tokens + bm - 1) / bm * bm;
   const int64_t n = padded * (cols >> 2);
-  B200MOE_LAUNCH(scales_to_atoms_kernel, static_cast<unsigned>((n + 255) / 256), 256, 0,
-                       static_cast<cudaStream_t>(stream), rows, tokens, cols, shift, padded, atoms);
+  B200MOE_LAUNCH(scales_to_atoms_kernel, static_cast<unsigned>((n + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream), rows,
+                 tokens, cols, shift, padded, atoms);
   return 0;
 }

@@ -50,7 +50,8 @@ def separate_calls(C, S, x, w, logits):
     slots = staged_slots(C, C.mxfp4_quant(x), wt, ids, w)
     # the shared expert in batches of 64: below the sizes of the CTA-pair kernels, on a stream of its own launches
     shared = torch.cat([S.shared_expert(x[a:a + 64].contiguous(), w.shared_weights) for a in range(0, len(x), 64)])
-    return slots, shared, torch.from_numpy(orc.reduce_slots_bf16(bits_of(slots), bits_of(shared)).view(np.int16)).cuda().view(torch.bfloat16)
+    total = orc.reduce_slots_bf16(bits_of(slots), bits_of(shared))
+    return slots, shared, torch.from_numpy(total.view(np.int16)).cuda().view(torch.bfloat16)
 
 
 @pytest.mark.parametrize("router", [True, False])
