@@ -1,26 +1,34 @@
 // Router GEMM on the CUDA cores: bf16 activations x fp32 gate -> fp32 split-K partial logits [S][T][E], consumed by the
 // top-4 kernel, which adds the partials from 0.0 in split order. Products are exact in fp32 (a bf16 factor has 8 significant
-// bits) and each partial is short fp32 FMA chains joined by a tree, so the error per partial stays far below
-// 2^-18 * sum|x||w| (the bound the reference states for its three-term bf16 split).
+// bits) and each partial is a short fp32 FMA chain, so the error per partial stays far below 2^-18 * sum|x||w| (the bound the
+// reference states for its three-term bf16 split).
 //
 // A partial is ONE chain of FMAs over the K elements of its split, in rising K from 0.0: the sum does not depend on the
 // token count or on how the work is dealt, and a change of tiling here never moves a logit's last bit.
 //
 // Used below 128 tokens, where the product is latency: 3.1 MB of gate, 12 KB of x per token. A CTA owns 16 experts x one K
-// split x 16 tokens, so one token alone already spreads the gate over 128 CTAs (with 16 splits) of 24 KB each, fetched in one
-// batch of asynchronous copies. Measured with both quantisers, us back to back: 4.0 / 9.9 / 10.4 / 10.6 / 18.8 at 1 / 16 / 32 /
-// 64 / 100 tokens. K dealt over the lanes of a warp and joined by a tree takes 3.9 / 3.9 / 4.5 / 8.7 / 13.8, but its sums
-// have other last bits, which reach the weights and through them the layer's result.
+// split x 16 (32) tokens, so one token alone already spreads the gate over 128 CTAs (with 16 splits) of 24 KB each, fetched in
+// one batch of asynchronous copies. What bounds it is how fast a warp issues -- one instruction in three to five cycles with
+// one warp per scheduler -- so eight warps with few instructions each: a thread runs one chain (two), both factors come from shared
+// memory in 16-byte loads at constant offsets, and rows are padded so that the rows of a load lie on different banks.
+// Measured with both quantisers, us back to back: 4.0 / 4.0 / 7.3 / 7.8 / 10.0 / 15.8 at 1 / 8 / 16 / 32 / 64 / 100 tokens. With
+// four warps, rows permuted instead of padded and x fetched row by row it took 4.0 / 8.5 / 9.9 / 10.4 / 10.6 / 18.7; with the chain
+// passed through 16 lanes and the gate in registers 10.8 / 13.2 / 15.9 / 21.7 / 22.6 / 22.9; with K dealt over the lanes and joined
+// by a tree 3.9 / 3.9 / 3.9 / 4.5 / 8.7 / 13.8, but those sums have other last bits, which reach the layer's result.
 #include "common.cuh"
+#include "tc_host.cuh"
 
 namespace b200moe {
 
-constexpr int kRgTokens = 16;             // tokens per CTA
 constexpr int kRgExperts = 16;            // experts per CTA
 constexpr int kRgChunk = 384;             // K elements in shared memory at a time
 constexpr int kRgVecs = kRgChunk / 4;     // 16-byte vectors of a row of them
-constexpr int kRgPerThread = 2;           // tokens (chains) per thread
-constexpr int kRgThreads = kRgTokens * kRgExperts / kRgPerThread;
+constexpr int kRgStride = kRgVecs + 1;    // of a row in shared memory: neighbouring rows start on other banks
+constexpr int kRgThreads = 256;
+constexpr int kRgGroups = kRgThreads / kRgExperts;
+// tokens of a CTA: PT chains per thread
+template <int PT>
+constexpr int rg_smem() { return (kRgExperts + kRgGroups * PT) * kRgStride * 16; }
 
 // What the fused form also writes, row-major: the routed experts' MXFP4 operands and (optionally) the shared expert's
 // MXFP8 operands of the same rows.
@@ -33,9 +41,8 @@ struct QuantOut {
   int atom_shift;
 };
 
-// 16 bytes from an address that need not be aligned (`vec`: it is)
-__device__ __forceinline__ uint4 load_bf16x8(const __nv_bfloat16* p, bool vec) {
-  if (vec) return __ldcg(reinterpret_cast<const uint4*>(p));
+// 16 bytes from an address that is not aligned
+__device__ __forceinline__ uint4 load_bf16x8(const __nv_bfloat16* p) {
   const unsigned short* h = reinterpret_cast<const unsigned short*>(p);
   uint32_t w[4];
 #pragma unroll
@@ -51,23 +58,20 @@ __device__ __forceinline__ void store_bytes(uint8_t* p, T v, bool vec) {
   }
 }
 
-// vector c of row r in shared memory: the eight lanes of a load phase read one c of eight rows, so the vectors of a row are
-// permuted by the row to spread those over the banks
-__device__ __forceinline__ int rg_at(int r, int c) { return r * kRgVecs + (c ^ (r & 7)); }
-
-// grid (ceil(E / 16), S, ceil(T / 16)); thread: one expert (tid % 16), the tokens tid / 16 and tid / 16 + 8 of the CTA's
-template <bool QUANT>
+// grid (ceil(E / 16), S, ceil(T / (16 PT))); thread: one expert (tid % 16), the tokens tid / 16 + 16 j of the CTA's
+template <bool QUANT, int PT>
 __global__ void __launch_bounds__(kRgThreads) router_gemm_kernel(const __nv_bfloat16* __restrict__ x,
                                                                  const float* __restrict__ gate, int64_t tokens,
                                                                  int num_experts, int k_per_split,
                                                                  float* __restrict__ partials, QuantOut q, bool vec) {
-  __shared__ float4 ws[kRgExperts * kRgVecs];
-  __shared__ float4 xs[kRgTokens * kRgVecs];
+  constexpr int kTokens = kRgGroups * PT;
+  extern __shared__ float4 rg_smem_raw[];
+  float4(*ws)[kRgStride] = reinterpret_cast<float4(*)[kRgStride]>(rg_smem_raw);
+  float4(*xs)[kRgStride] = ws + kRgExperts;
   const int tid = threadIdx.x;
   const int e0 = blockIdx.x * kRgExperts, e = tid % kRgExperts, tg = tid / kRgExperts;
-  constexpr int kGroups = kRgThreads / kRgExperts;
-  const int64_t t0 = static_cast<int64_t>(blockIdx.z) * kRgTokens;
-  const int nt = static_cast<int>(min(static_cast<int64_t>(kRgTokens), tokens - t0));
+  const int64_t t0 = static_cast<int64_t>(blockIdx.z) * kTokens;
+  const int nt = static_cast<int>(min(static_cast<int64_t>(kTokens), tokens - t0));
   const int k0 = blockIdx.y * k_per_split;
   // this CTA's slice of the gate: into L2 before the wait, read behind it (the work in front may have written it)
   if (vec && tid < kRgExperts && e0 + tid < num_experts)
@@ -75,11 +79,12 @@ __global__ void __launch_bounds__(kRgThreads) router_gemm_kernel(const __nv_bflo
   pdl_enter(x, gate);
   auto load_gate = [&](int kk) {
     const int vecs = min(kRgChunk, k_per_split - kk) / 4;
-    for (int i = tid; i < kRgExperts * kRgVecs; i += kRgThreads) {
-      const int r = i / kRgVecs, c = i % kRgVecs;
+#pragma unroll
+    for (int it = 0; it < kRgExperts * kRgVecs / kRgThreads; ++it) {
+      const int i = it * kRgThreads + tid, r = i / kRgVecs, c = i % kRgVecs;
       if (c >= vecs || e0 + r >= num_experts) continue;  // never read
       const float* src = gate + static_cast<int64_t>(e0 + r) * kH + k0 + kk + 4 * c;
-      float4* dst = ws + rg_at(r, c);
+      float4* dst = &ws[r][c];
       if (vec)
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
                      "l"(src)
@@ -89,12 +94,12 @@ __global__ void __launch_bounds__(kRgThreads) router_gemm_kernel(const __nv_bflo
     }
   };
   load_gate(0);
-  float acc[kRgPerThread];
-  int row[kRgPerThread];  // (rows beyond the last token: the last one again, not stored)
+  float acc[PT];
+  const float4* row[PT];  // (rows beyond the last token: the last one again, not stored)
 #pragma unroll
-  for (int j = 0; j < kRgPerThread; ++j) {
+  for (int j = 0; j < PT; ++j) {
     acc[j] = 0.0f;
-    row[j] = min(tg + j * kGroups, nt - 1);
+    row[j] = xs[min(tg + j * kRgGroups, nt - 1)];
   }
   for (int kk = 0; kk < k_per_split; kk += kRgChunk) {
     const int chunk = min(kRgChunk, k_per_split - kk), v8s = chunk / 8;  // 16-byte vectors of a bf16 row in this chunk
@@ -102,13 +107,30 @@ __global__ void __launch_bounds__(kRgThreads) router_gemm_kernel(const __nv_bflo
       __syncthreads();
       load_gate(kk);
     }
-    for (int i = tid; i < nt * v8s; i += kRgThreads) {
-      const int r = i / v8s, c = i % v8s;
-      const uint4 raw = load_bf16x8(x + (t0 + r) * kH + k0 + kk + 8 * c, vec);
-      xs[rg_at(r, 2 * c)] = make_float4(__uint_as_float(raw.x << 16), __uint_as_float(raw.x & 0xffff0000u),
-                                        __uint_as_float(raw.y << 16), __uint_as_float(raw.y & 0xffff0000u));
-      xs[rg_at(r, 2 * c + 1)] = make_float4(__uint_as_float(raw.z << 16), __uint_as_float(raw.z & 0xffff0000u),
-                                            __uint_as_float(raw.w << 16), __uint_as_float(raw.w & 0xffff0000u));
+    constexpr int kLoads = kTokens * kRgChunk / 8 / kRgThreads;  // of a thread, all in flight together
+    uint4 raw[kLoads];
+    if (vec) {
+#pragma unroll
+      for (int it = 0; it < kLoads; ++it) {
+        const int i = it * kRgThreads + tid, r = i / (kRgChunk / 8), c = i % (kRgChunk / 8);
+        if (r < nt && c < v8s) raw[it] = __ldcg(reinterpret_cast<const uint4*>(x + (t0 + r) * kH + k0 + kk + 8 * c));
+      }
+    } else {
+#pragma unroll
+      for (int it = 0; it < kLoads; ++it) {
+        const int i = it * kRgThreads + tid, r = i / (kRgChunk / 8), c = i % (kRgChunk / 8);
+        if (r < nt && c < v8s) raw[it] = load_bf16x8(x + (t0 + r) * kH + k0 + kk + 8 * c);
+      }
+    }
+#pragma unroll
+    for (int it = 0; it < kLoads; ++it) {
+      const int i = it * kRgThreads + tid, r = i / (kRgChunk / 8), c = i % (kRgChunk / 8);
+      if (r < nt && c < v8s) {
+        xs[r][2 * c] = make_float4(__uint_as_float(raw[it].x << 16), __uint_as_float(raw[it].x & 0xffff0000u),
+                                   __uint_as_float(raw[it].y << 16), __uint_as_float(raw[it].y & 0xffff0000u));
+        xs[r][2 * c + 1] = make_float4(__uint_as_float(raw[it].z << 16), __uint_as_float(raw[it].z & 0xffff0000u),
+                                       __uint_as_float(raw[it].w << 16), __uint_as_float(raw[it].w & 0xffff0000u));
+      }
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
@@ -118,7 +140,7 @@ __global__ void __launch_bounds__(kRgThreads) router_gemm_kernel(const __nv_bflo
       for (int i = tid; i < ((mine * v8s + 31) & ~31); i += kRgThreads) {  // whole warps stay together for the shuffles
         const bool live = i < mine * v8s;
         const int r = live ? (i / v8s) * groups + static_cast<int>(blockIdx.x) : 0, v8 = live ? i % v8s : 0;
-        const float4 lo = xs[rg_at(r, 2 * v8)], hi = xs[rg_at(r, 2 * v8 + 1)];
+        const float4 lo = xs[r][2 * v8], hi = xs[r][2 * v8 + 1];
         const float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
         float amax = 0.0f;
 #pragma unroll
@@ -152,12 +174,12 @@ __global__ void __launch_bounds__(kRgThreads) router_gemm_kernel(const __nv_bflo
       }
     }
     if (tg < nt) {
-#pragma unroll 8
+#pragma unroll 16
       for (int c = 0; c < chunk / 4; ++c) {
-        const float4 w = ws[rg_at(e, c)];
+        const float4 w = ws[e][c];
 #pragma unroll
-        for (int j = 0; j < kRgPerThread; ++j) {
-          const float4 v = xs[rg_at(row[j], c)];
+        for (int j = 0; j < PT; ++j) {
+          const float4 v = row[j][c];
           acc[j] = fmaf(v.x, w.x, acc[j]);
           acc[j] = fmaf(v.y, w.y, acc[j]);
           acc[j] = fmaf(v.z, w.z, acc[j]);
@@ -168,14 +190,40 @@ __global__ void __launch_bounds__(kRgThreads) router_gemm_kernel(const __nv_bflo
   }
   if (e0 + e >= num_experts) return;
 #pragma unroll
-  for (int j = 0; j < kRgPerThread; ++j)
-    if (tg + j * kGroups < nt)
-      partials[(static_cast<int64_t>(blockIdx.y) * tokens + t0 + tg + j * kGroups) * num_experts + e0 + e] = acc[j];
+  for (int j = 0; j < PT; ++j)
+    if (tg + j * kRgGroups < nt)
+      partials[(static_cast<int64_t>(blockIdx.y) * tokens + t0 + tg + j * kRgGroups) * num_experts + e0 + e] = acc[j];
 }
 
 static bool aligned16(const void* a, const void* b, const void* c, const void* d) {
   return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c) |
            reinterpret_cast<uintptr_t>(d)) & 15) == 0;
+}
+
+template <bool QUANT, int PT>
+static int launch_router(const void* x, const float* gate, int64_t tokens, int num_experts, int splits, float* partials,
+                         const QuantOut& q, bool vec, cudaStream_t stream) {
+  static PerDeviceOnce once;
+  const int rc = once.run([] {
+    return static_cast<int>(cudaFuncSetAttribute(router_gemm_kernel<QUANT, PT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 rg_smem<PT>()));
+  });
+  if (rc) return rc;
+  constexpr int kTokens = kRgGroups * PT;
+  const dim3 grid(static_cast<unsigned>((num_experts + kRgExperts - 1) / kRgExperts), static_cast<unsigned>(splits),
+                  static_cast<unsigned>((tokens + kTokens - 1) / kTokens));
+  B200MOE_LAUNCH((router_gemm_kernel<QUANT, PT>), grid, kRgThreads, rg_smem<PT>(), stream, static_cast<const __nv_bfloat16*>(x),
+                 gate, tokens, num_experts, kH / splits, partials, q, vec);
+  return 0;
+}
+// Up to 32 tokens one chain per thread: the time is a chain's latency (7.8 us at 32 tokens, 9.7 with two). Above, two: half the
+// gate traffic and fewer loads per FMA (10.0 us at 64 tokens and 15.8 at 100, 14.1 and 21.3 with one).
+constexpr int64_t kRgOneChain = 32;
+template <bool QUANT>
+static int launch_router_any(const void* x, const float* gate, int64_t tokens, int num_experts, int splits, float* partials,
+                             const QuantOut& q, bool vec, cudaStream_t stream) {
+  return tokens <= kRgOneChain ? launch_router<QUANT, 1>(x, gate, tokens, num_experts, splits, partials, q, vec, stream)
+                               : launch_router<QUANT, 2>(x, gate, tokens, num_experts, splits, partials, q, vec, stream);
 }
 
 }  // namespace b200moe
@@ -188,12 +236,8 @@ extern "C" int b200moe_router_gemm(const void* x_bf16, const float* gate, int64_
   if (!x_bf16 || !gate || !partials || tokens < 0 || num_experts < 1 || num_experts > kMaxE) return B200MOE_E_ARG;
   if (splits < 1 || kH % splits || (kH / splits) % 32) return B200MOE_E_ARG;
   if (tokens == 0) return 0;
-  const dim3 grid(static_cast<unsigned>((num_experts + kRgExperts - 1) / kRgExperts), static_cast<unsigned>(splits),
-                  static_cast<unsigned>((tokens + kRgTokens - 1) / kRgTokens));
-  B200MOE_LAUNCH(router_gemm_kernel<false>, grid, kRgThreads, 0, static_cast<cudaStream_t>(stream),
-                 static_cast<const __nv_bfloat16*>(x_bf16), gate, tokens, num_experts, kH / splits, partials, QuantOut{},
-                 aligned16(x_bf16, gate, nullptr, nullptr));
-  return 0;
+  return launch_router_any<false>(x_bf16, gate, tokens, num_experts, splits, partials, QuantOut{},
+                                  aligned16(x_bf16, gate, nullptr, nullptr), static_cast<cudaStream_t>(stream));
 }
 
 namespace b200moe {
@@ -208,13 +252,9 @@ int router_gemm_quant(const void* x_bf16, const float* gate, int64_t tokens, int
   if (reinterpret_cast<uintptr_t>(codes8) & 1) return B200MOE_E_ALIGN;
   if (tokens == 0) return 0;
   const int shift = bm8 == 16 ? 4 : bm8 == 32 ? 5 : bm8 == 64 ? 6 : 7;
-  const dim3 grid(static_cast<unsigned>((num_experts + kRgExperts - 1) / kRgExperts), static_cast<unsigned>(splits),
-                  static_cast<unsigned>((tokens + kRgTokens - 1) / kRgTokens));
-  const QuantOut q{codes4, scales4, codes8, scales8, atoms8, shift};
-  B200MOE_LAUNCH(router_gemm_kernel<true>, grid, kRgThreads, 0, static_cast<cudaStream_t>(stream),
-                 static_cast<const __nv_bfloat16*>(x_bf16), gate, tokens, num_experts, kH / splits, partials, q,
-                 aligned16(x_bf16, gate, codes4, codes8));
-  return 0;
+  return launch_router_any<true>(x_bf16, gate, tokens, num_experts, splits, partials,
+                                 QuantOut{codes4, scales4, codes8, scales8, atoms8, shift}, aligned16(x_bf16, gate, codes4, codes8),
+                                 static_cast<cudaStream_t>(stream));
 }
 }  // namespace b200moe
 
