@@ -589,7 +589,7 @@ def _result_flags(sw, slots, shared):
 
 
 # Token count above which the shared expert's GEMMs are launches of their own, on the side stream: below, it is a role of a routed
-# launch (48 against 161 us for the layer at 1 token, 112 against 244 at 32, most of it host time). The side stream's work starts
+# launch (37 against 161 us for the layer at 1 token, 105 against 237 at 32, much of it host time). The side stream's work starts
 # behind the quantisation of x, which serves both experts in one pass, and is joined inside the C call.
 SIDE_STREAM_FROM = 512
 

@@ -279,8 +279,10 @@ def time_steps(torch, fn, steps, warmup, flush):
 
 
 def with_shared_expert(torch, chain, orc, w, layer, flush, args):
-    """The same workload through the package entry with the MXFP8 shared expert (its three launches on the device's side
-    stream, joined before the reduce), as CUDA-graph replays; reported beside the headline, not in it."""
+    """The same workload through the package entry with the MXFP8 shared expert, as CUDA-graph replays; reported beside the
+    headline, not in it. Above 512 tokens both experts' operands come from one quantiser pass and the shared expert's two GEMMs
+    run on the device's side stream, joined before the reduce; below, a quantiser launch of its own and a role of the routed
+    launches."""
     from amd_kernels_b200.moe.mxfp4_h6144_i768_e128_top4 import shared_expert as S
     sw = S.SharedWeights.from_row_major(*(torch.from_numpy(a).cuda() for a in orc.make_shared_weights()))
     w1 = chain.MoeWeights(None, None, w.w13, None, w.w2, None, w.routed_scaling_factor, w.routing_mode, shared_weights=sw)
@@ -303,7 +305,7 @@ def with_shared_expert(torch, chain, orc, w, layer, flush, args):
     t = sum(ms) / len(ms)
     return {"us_per_step": t * 1e3, "tokens_per_s": layer.tokens / (t * 1e-3),
             "shared_expert_alone_us": sum(ms_alone) / len(ms_alone) * 1e3,
-            "launches_per_step": layer.launches_per_step() + 3,
+            "launches_per_step": layer.launches_per_step() + (2 if layer.tokens > 512 else 1),
             "note": "routed layer + MXFP8 shared expert (quantise, GEMM1+SwiGLU+requantise, GEMM2) summed in the reduce"}
 
 
@@ -381,7 +383,7 @@ def gemm1_tensor_roofline(tokens, k, peaks):
 
 
 def entry_with_router(torch, chain, w, flush, args, sizes=(256, 2048, 8192)):
-    """The call a server makes -- mxfp4_moe(x, w) with the router inside (b200moe_forward_x) -- beside the same call fed
+    """The call a server makes -- mxfp4_moe(x, w) with the router inside (b200moe_layer) -- beside the same call fed
     with precomputed logits, as CUDA-graph replays."""
     gate = torch.randn((E, H), device="cuda", generator=torch.Generator(device="cuda").manual_seed(5)) / H ** 0.5
     wg = chain.MoeWeights(gate, None, w.w13, None, w.w2, None, w.routed_scaling_factor, w.routing_mode)

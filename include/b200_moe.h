@@ -389,7 +389,8 @@ typedef struct b200moe_weights {
   int num_experts;
   int route_mode;
   float route_scale;
-  const float* gate;   /* router weight fp32 [num_experts][6144]; needed by b200moe_forward_x only, else may be null */
+  const float* gate;   /* router weight fp32 [num_experts][6144]; needed where the router runs inside the call (b200moe_layer
+                          without logits, b200moe_prepare, b200moe_forward_x), else may be null */
   const void* gate_split; /* b200moe_router_split_gate of `gate` (bf16 [3][128][6144]) or null: the tensor-core router */
 } b200moe_weights;
 size_t b200moe_workspace_bytes(int64_t tokens, int num_experts);
