@@ -56,8 +56,11 @@ int gemm12_beside(const uint8_t* w13t, const uint8_t* w2t, int num_experts, cons
 int gemm1_beside(const uint8_t* w13t, int num_experts, const uint8_t* xq_sorted, const uint8_t* sfx,
                  const int32_t* block_expert, const int32_t* num_valid, int64_t max_rows, int bm, uint8_t* hq, uint8_t* sfh,
                  const uint8_t* prefetch_w2t, int32_t* status, const SharedPlan* sp, void* stream);
-int shared_gemms(const uint8_t* w13t, const uint8_t* w2t, const uint8_t* codes8, int64_t code_rows, const SharedWorkspace& ws,
-                 void* out_bf16, int64_t tokens, int32_t* status, void* stream);
+int shared_gemm1(const uint8_t* w13t, const uint8_t* codes8, int64_t code_rows, const SharedWorkspace& ws, int64_t tokens,
+                 int32_t* status, void* stream);
+bool shared_sums_slots(const SharedWorkspace& ws);
+int shared_gemm2(const uint8_t* w2t, const SharedWorkspace& ws, const void* slots_bf16, void* out_bf16, int64_t tokens,
+                 int32_t* status, void* stream);
 int set_wait_limit_routed(unsigned long long ns);
 int set_wait_limit_shared(unsigned long long ns);
 int set_wait_limit_shared_pair(unsigned long long ns);
@@ -257,6 +260,8 @@ static int run_layer(const LayerCall& c) {
   }
   SharedPlan plan{};
   const SharedPlan* sp = nullptr;
+  // where nobody takes the shared rows, the shared expert's second GEMM sums the slots (shared_pair.cu, MODE 3)
+  const bool sum_in_gemm2 = shared && c.out && !c.shared_out && ws.bm == 128 && shared_sums_slots(ws.sh);
   if (shared) {
     if (ws.bm < 128) {  // decode sizes: a role of the launch that streams the routed experts' W13
       if ((r = shared_plan(&plan, c.shared->w13t, c.shared->w2t, codes8, tokens, ws.sh, shared_out, tokens, ws.done + blocks,
@@ -265,7 +270,9 @@ static int run_layer(const LayerCall& c) {
       sp = &plan;
     } else {  // beside the routing and the sort, whose few short launches leave the SMs to it
       if (c.side && (r = side.fork())) return r;
-      r = shared_gemms(c.shared->w13t, c.shared->w2t, codes8, tokens, ws.sh, shared_out, tokens, c.status, c.side ? c.side : st);
+      void* sst = c.side ? c.side : st;
+      r = shared_gemm1(c.shared->w13t, codes8, tokens, ws.sh, tokens, c.status, sst);
+      if (!r && !sum_in_gemm2) r = shared_gemm2(c.shared->w2t, ws.sh, nullptr, shared_out, tokens, c.status, sst);
       if (r) return r;
     }
   }
@@ -311,6 +318,7 @@ static int run_layer(const LayerCall& c) {
       return r;
   }
   if ((r = side.join())) return r;
+  if (sum_in_gemm2) return shared_gemm2(c.shared->w2t, ws.sh, slots, c.out, tokens, c.status, st);
   if (c.out && (r = b200moe_reduce_slots(slots, shared ? shared_out : nullptr, tokens, c.out, st))) return r;
   return 0;
 }

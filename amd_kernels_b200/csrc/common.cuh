@@ -139,6 +139,16 @@ __device__ __forceinline__ float swiglu_oai(float g, float u) {
   return g * sig * (u + 1.0f);
 }
 
+// acc += eight bf16 values: one step of the slot sum (slots 0..3, then the shared row, fp32)
+__device__ __forceinline__ void add_bf16x8(float (&acc)[8], const uint4 v) {
+  const uint32_t r[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    acc[2 * j] = acc[2 * j] + __uint_as_float(r[j] << 16);
+    acc[2 * j + 1] = acc[2 * j + 1] + __uint_as_float(r[j] & 0xffff0000u);
+  }
+}
+
 // byte offset of scale j (0..3) of row r (0..127) inside a 512-byte scale atom
 __device__ __host__ __forceinline__ int atom_offset(int r, int j) { return (r & 31) * 16 + (r >> 5) * 4 + j; }
 

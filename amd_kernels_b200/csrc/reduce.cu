@@ -3,15 +3,6 @@
 
 namespace b200moe {
 
-__device__ __forceinline__ void add_bf16x8(float (&acc)[8], const uint4 v) {
-  const uint32_t r[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    acc[2 * j] = acc[2 * j] + __uint_as_float(r[j] << 16);
-    acc[2 * j + 1] = acc[2 * j + 1] + __uint_as_float(r[j] & 0xffff0000u);
-  }
-}
-
 // `index` (optional): row of `slots` that holds pair 4*token+slot, for slot rows that sit in another order (rows that came
 // back from other ranks in send order); without it pair q is row q.
 __global__ void __launch_bounds__(256) reduce_slots_kernel(const uint4* __restrict__ slots,

@@ -22,6 +22,13 @@
 // (512 are tensor time), read from the clock in a build made for it: 690, of which the four MMAs and the looks at the next stage's
 // barriers 350, the stage release 74, waiting for scales 190, for codes 55. Before the looks, with two plain waits, two commits
 // per release and the accumulator handed back by a cluster-scope release, it was 750 and the whole 251 us.
+// MODE 3 is MODE 2 for a call that hands out neither the shared rows nor anything but the sum: its epilogue has the shared value
+// of a (token, column) in a register and adds the four slots in front of it, out = bf16((((0 + s0) + s1) + s2) + s3 + bf16(shared)),
+// the slot reduce's sum bit for bit. So the shared rows are never written nor read back, and the slot reduce's traffic (40 KB a
+// token, HBM bound) runs under this GEMM's arithmetic and not behind it. Each epilogue thread keeps 16 to 32 16-byte slot loads in
+// flight, a batch ahead and across units, so the rings give shared memory back (four stages) for the L1 lines those loads need.
+// Measured, second GEMM + slot reduce / MODE 3: 77 + 166 -> 191 us at 16384 tokens (1.05 GB in 191 us; its bytes alone take 160 at
+// the copy rate), I = 1536 41 + 42 -> 56 at 4096.
 // 12 warps start with 168 registers; the issuing warpgroup drops to 72, the epilogue's rise to 216 (4 x 72 + 8 x 216 = 12 x 168:
 // the exchange must balance inside what the CTA was given at launch).
 #include "shared_role.cuh"
@@ -34,7 +41,7 @@ struct SharedPairCfg {
   static constexpr int kTilesM = MODE == 1 ? kW13Tiles : kW2Tiles;
   static constexpr int kTilePairs = kTilesM / 2;
   static constexpr int kTilesK = MODE == 1 ? kS1TilesK : kS2TilesK;
-  static constexpr int kStages = 6;                 // code ring
+  static constexpr int kStages = MODE == 3 ? 4 : 6; // code ring
   static constexpr int kSfStages = 8;               // scale ring = scale sets in tensor memory
   static constexpr int kTokOff = 0;                 // this CTA's 128 token rows x 128 bytes
   static constexpr int kWOff = 128 * 128;           // its 128 weight rows: tile 2 * tp + rank
@@ -44,7 +51,7 @@ struct SharedPairCfg {
   static constexpr int kSfSlotBytes = 3 * kAtomBytes;
   static constexpr int kStripOff = kSfRingOff + kSfStages * kSfSlotBytes;
   static constexpr int kStripRow = 144, kStripBytes = 16 * kStripRow;  // 128 bytes + 16: eight lanes' 16-byte writes hit all banks
-  static constexpr int kSmemBytes = kStripOff + (MODE == 2 ? 8 * kStripBytes : 0) + 1024;
+  static constexpr int kSmemBytes = kStripOff + (MODE >= 2 ? 8 * kStripBytes : 0) + 1024;
   static constexpr int kThreads = 32 * 12;
   static constexpr int kSfCol = 256;                // tensor memory: 256 accumulator columns, then 8 sets of 16
   static constexpr int kTmemCols = 512;
@@ -66,7 +73,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SharedPairCfg<MODE>:
     shared_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_sfx,
                        const __grid_constant__ CUtensorMap map_wc, const __grid_constant__ CUtensorMap map_ws, int n_blocks,
                        int64_t tokens, uint8_t* __restrict__ h8, uint8_t* __restrict__ sfh8,
-                       __nv_bfloat16* __restrict__ out, int32_t* status) {
+                       const __nv_bfloat16* __restrict__ slots, __nv_bfloat16* __restrict__ out, int32_t* status) {
   using C = SharedPairCfg<MODE>;
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t bar_full[C::kStages];     // leader: both CTAs' codes of the stage have landed
@@ -116,6 +123,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SharedPairCfg<MODE>:
   tc_fence_after();
   const uint32_t tmem_base = tmem_base_slot;
   pdl_wait();
+  launder(slots);
 
   const int n_clusters = static_cast<int>(gridDim.x >> 1), cluster = static_cast<int>(blockIdx.x >> 1);
   const int total = (n_blocks + 1) / 2 * C::kTilePairs;
@@ -234,6 +242,20 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SharedPairCfg<MODE>:
     const uint32_t tempty_leader = map_to_cta(smem_u32(&bar_tempty), 0);
     uint8_t* strip = smem_raw + (tiles - smem_u32(smem_raw)) + C::kStripOff + (warp - 4) * C::kStripBytes;
     uint32_t ui = 0;
+    // MODE 3: the slots of batch `part` (0..3: columns 64 * (part / 2), rows 16 * (part % 2)) of unit v, four rows per lane
+    const auto load_slots = [&](int v, int part, uint4 (&s)[4][4]) {
+      const int64_t r0 = static_cast<int64_t>(v / C::kTilePairs * 2 + static_cast<int>(rank)) * 128 + q * 32 + 16 * (part & 1);
+      const __nv_bfloat16* src = slots + (2 * (v % C::kTilePairs) + half) * 128 + (part >> 1) * 64 + (lane & 7) * 8;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int64_t r = r0 + 4 * i + (lane >> 3);
+#pragma unroll
+        for (int k = 0; k < kTopK; ++k)
+          s[i][k] = v < total && r < tokens ? __ldcg(reinterpret_cast<const uint4*>(src + (r * kTopK + k) * kH)) : uint4{};
+      }
+    };
+    uint4 ahead[MODE == 3 ? 2 : 1][4][4];
+    if (MODE == 3) load_slots(cluster, 0, ahead[0]);
     for (int u = cluster; u < total; u += n_clusters, ++ui) {
       const int b = u / C::kTilePairs * 2 + static_cast<int>(rank), tp = u % C::kTilePairs;
       const bool have_rows = b < n_blocks;
@@ -242,18 +264,40 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SharedPairCfg<MODE>:
       if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_tfull), ui & 1u, abort_v, status))) break;
       tc_fence_after();
       const uint32_t t_acc = tmem_base + 128u * half + (static_cast<uint32_t>(q * 32) << 16);
-      uint32_t acc[4][32];
-      if (have_rows) {
+      uint32_t acc[MODE == 1 ? 4 : 2][32];
+      uint4 packed[MODE == 1 ? 1 : 2][8];  // MODE 2, 3: the row's 128 values in bf16
+      if (have_rows && MODE == 1) {
         tc_ld32_nowait(t_acc, acc[0]);
         tc_ld32_nowait(t_acc + 32, acc[1]);
-        tc_ld32_nowait(t_acc + 64, acc[2]);
-        tc_ld32_nowait(t_acc + 96, acc[3]);
+        tc_ld32_nowait(t_acc + 64, acc[MODE == 1 ? 2 : 0]);
+        tc_ld32_nowait(t_acc + 96, acc[MODE == 1 ? 3 : 0]);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      } else if (have_rows) {
+#pragma unroll
+        for (int hh = 0; hh < 2; ++hh) {
+          tc_ld32_nowait(t_acc + 64 * hh, acc[0]);
+          tc_ld32_nowait(t_acc + 64 * hh + 32, acc[1]);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int k = 0; k < 8; ++k) {
+            uint32_t o[4];
+#pragma unroll
+            for (int jj = 0; jj < 4; ++jj) {
+              const int c = 8 * (k & 3) + 2 * jj;
+              const __nv_bfloat162 p2 = __floats2bfloat162_rn(__uint_as_float(acc[k >> 2][c]), __uint_as_float(acc[k >> 2][c + 1]));
+              o[jj] = *reinterpret_cast<const uint32_t*>(&p2);
+            }
+            packed[MODE == 1 ? 0 : hh][k] = make_uint4(o[0], o[1], o[2], o[3]);
+          }
+        }
       }
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(tempty_leader);
-      if (!have_rows) continue;
+      if (!have_rows) {
+        if (MODE == 3) load_slots(u + n_clusters, 0, ahead[0]);
+        continue;
+      }
       if (MODE == 1) {
         // columns of a tile: [gate 32 | up 32 | gate 32 | up 32] of 64 intermediate columns
 #pragma unroll
@@ -262,7 +306,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SharedPairCfg<MODE>:
           float amax = 0.0f;
 #pragma unroll
           for (int k = 0; k < 32; ++k) {
-            h[k] = swiglu_oai(__uint_as_float(acc[2 * g][k]), __uint_as_float(acc[2 * g + 1][k]));
+            h[k] = swiglu_oai(__uint_as_float(acc[MODE == 1 ? 2 * g : 0][k]), __uint_as_float(acc[MODE == 1 ? 2 * g + 1 : 0][k]));
             amax = fmaxf(amax, fabsf(h[k]));
           }
           const int sc = mxfp8_scale(amax);
@@ -284,31 +328,32 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SharedPairCfg<MODE>:
         __nv_bfloat16* dst0 = out + row0 * kH + (2 * tp + half) * 128 + (lane & 7) * 8;
 #pragma unroll
         for (int hh = 0; hh < 2; ++hh) {  // 64 columns = 128 bytes of a row
-          uint4 packed[8];
-#pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            uint32_t o[4];
-#pragma unroll
-            for (int jj = 0; jj < 4; ++jj) {
-              const int c = 8 * (k & 3) + 2 * jj;
-              const __nv_bfloat162 p2 = __floats2bfloat162_rn(__uint_as_float(acc[2 * hh + (k >> 2)][c]),
-                                                              __uint_as_float(acc[2 * hh + (k >> 2)][c + 1]));
-              o[jj] = *reinterpret_cast<const uint32_t*>(&p2);
-            }
-            packed[k] = make_uint4(o[0], o[1], o[2], o[3]);
-          }
 #pragma unroll
           for (int p = 0; p < 2; ++p) {  // 16 rows at a time
+            if (MODE == 3) load_slots(hh + p < 2 ? u : u + n_clusters, (2 * hh + p + 1) & 3, ahead[(p + 1) & (MODE == 3)]);
             if ((lane >> 4) == p) {
 #pragma unroll
               for (int k = 0; k < 8; ++k)
-                *reinterpret_cast<uint4*>(strip + (lane & 15) * C::kStripRow + k * 16) = packed[k];
+                *reinterpret_cast<uint4*>(strip + (lane & 15) * C::kStripRow + k * 16) = packed[MODE == 1 ? 0 : hh][k];
             }
             __syncwarp();
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
               const int r = 4 * i + (lane >> 3);
-              const uint4 val = *reinterpret_cast<const uint4*>(strip + r * C::kStripRow + (lane & 7) * 16);
+              uint4 val = *reinterpret_cast<const uint4*>(strip + r * C::kStripRow + (lane & 7) * 16);
+              if (MODE == 3) {
+                float sum[8] = {};
+#pragma unroll
+                for (int k = 0; k < kTopK; ++k) add_bf16x8(sum, ahead[p & (MODE == 3)][i][k]);
+                add_bf16x8(sum, val);
+                uint32_t o[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                  const __nv_bfloat162 p2 = __floats2bfloat162_rn(sum[2 * k], sum[2 * k + 1]);
+                  o[k] = *reinterpret_cast<const uint32_t*>(&p2);
+                }
+                val = make_uint4(o[0], o[1], o[2], o[3]);
+              }
               if (row0 + 16 * p + r < tokens)
                 *reinterpret_cast<uint4*>(dst0 + static_cast<int64_t>(16 * p + r) * kH + hh * 64) = val;
             }
@@ -342,7 +387,7 @@ static int shared_pairs() {
 
 template <int MODE>
 static int launch_shared_pair(const CUtensorMap& mx, const uint8_t* w_tiles, const uint8_t* sf_x, const SharedWorkspace& ws,
-                              int64_t tokens, void* out_bf16, int32_t* status, cudaStream_t stream) {
+                              int64_t tokens, const void* slots_bf16, void* out_bf16, int32_t* status, cudaStream_t stream) {
   using C = SharedPairCfg<MODE>;
   CUtensorMap msf, mwc, mws;
   const int n_blocks = static_cast<int>(ws.rows / 128);
@@ -353,17 +398,22 @@ static int launch_shared_pair(const CUtensorMap& mx, const uint8_t* w_tiles, con
   if ((r = make_flat_map(&mws, w_tiles, w_rows, 4))) return r;
   const int units = (n_blocks + 1) / 2 * C::kTilePairs, pairs = shared_pairs<MODE>();
   return launch_pairs(shared_pair_kernel<MODE>, units < pairs ? units : pairs, C::kThreads, C::kSmemBytes, stream, mx, msf, mwc,
-                      mws, n_blocks, tokens, ws.h8, ws.sfh8, static_cast<__nv_bfloat16*>(out_bf16), status);
+                      mws, n_blocks, tokens, ws.h8, ws.sfh8, static_cast<const __nv_bfloat16*>(slots_bf16),
+                      static_cast<__nv_bfloat16*>(out_bf16), status);
 }
 
-bool shared_pair_supported() { return shared_pairs<1>() > 0 && shared_pairs<2>() > 0; }
+bool shared_pair_supported() { return shared_pairs<1>() > 0 && shared_pairs<2>() > 0 && shared_pairs<3>() > 0; }
 
-// Both GEMMs on blocks of 128 tokens (ws.bm == 128). `map_x` / `map_h`: the token codes and h as 128-byte swizzled boxes of 128.
-int shared_gemms_pair(const CUtensorMap& map_x, const CUtensorMap& map_h, const uint8_t* w13t, const uint8_t* w2t,
-                      const SharedWorkspace& ws, void* out_bf16, int64_t tokens, int32_t* status, cudaStream_t stream) {
-  const int r = launch_shared_pair<1>(map_x, w13t, ws.sfx8, ws, tokens, out_bf16, status, stream);
-  if (r) return r;
-  return launch_shared_pair<2>(map_h, w2t, ws.sfh8, ws, tokens, out_bf16, status, stream);
+// The GEMMs on blocks of 128 tokens (ws.bm == 128). `map_x` / `map_h`: the token codes and h as 128-byte swizzled boxes of 128.
+int shared_pair_gemm1(const CUtensorMap& map_x, const uint8_t* w13t, const SharedWorkspace& ws, int64_t tokens, int32_t* status,
+                      cudaStream_t stream) {
+  return launch_shared_pair<1>(map_x, w13t, ws.sfx8, ws, tokens, nullptr, nullptr, status, stream);
+}
+// slots_bf16 null: the shared rows; else the sum of the four slots and the shared row
+int shared_pair_gemm2(const CUtensorMap& map_h, const uint8_t* w2t, const SharedWorkspace& ws, const void* slots_bf16,
+                      void* out_bf16, int64_t tokens, int32_t* status, cudaStream_t stream) {
+  return slots_bf16 ? launch_shared_pair<3>(map_h, w2t, ws.sfh8, ws, tokens, slots_bf16, out_bf16, status, stream)
+                    : launch_shared_pair<2>(map_h, w2t, ws.sfh8, ws, tokens, nullptr, out_bf16, status, stream);
 }
 
 int set_wait_limit_shared_pair(unsigned long long ns) { return set_wait_limit_here(ns); }

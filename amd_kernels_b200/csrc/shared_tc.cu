@@ -428,8 +428,10 @@ int shared_plan(SharedPlan* plan, const uint8_t* w13t, const uint8_t* w2t, const
 
 // shared_pair.cu
 bool shared_pair_supported();
-int shared_gemms_pair(const CUtensorMap& map_x, const CUtensorMap& map_h, const uint8_t* w13t, const uint8_t* w2t,
-                      const SharedWorkspace& ws, void* out_bf16, int64_t tokens, int32_t* status, cudaStream_t stream);
+int shared_pair_gemm1(const CUtensorMap& map_x, const uint8_t* w13t, const SharedWorkspace& ws, int64_t tokens, int32_t* status,
+                      cudaStream_t stream);
+int shared_pair_gemm2(const CUtensorMap& map_h, const uint8_t* w2t, const SharedWorkspace& ws, const void* slots_bf16,
+                      void* out_bf16, int64_t tokens, int32_t* status, cudaStream_t stream);
 
 int set_wait_limit_shared(unsigned long long ns) { return set_wait_limit_here(ns); }
 
@@ -488,24 +490,53 @@ namespace b200moe {
 // chain of 48 K-tiles is the time; the one-CTA kernel has four times the units.
 constexpr int kSharedPairBlocks = 12;
 
-int shared_gemms(const uint8_t* w13t, const uint8_t* w2t, const uint8_t* codes8, int64_t code_rows, const SharedWorkspace& ws,
-                 void* out_bf16, int64_t tokens, int32_t* status, void* stream) {
-  const int n_blocks = static_cast<int>(ws.rows / ws.bm);
+static bool on_pairs(const SharedWorkspace& ws) {
+  return ws.bm == 128 && ws.rows / 128 >= kSharedPairBlocks && shared_pair_supported();
+}
+
+int shared_gemm1(const uint8_t* w13t, const uint8_t* codes8, int64_t code_rows, const SharedWorkspace& ws, int64_t tokens,
+                 int32_t* status, void* stream) {
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  CUtensorMap mx, mh;
-  int r;
+  CUtensorMap mx;
   // code_rows may be the unpadded token count: boxes that reach beyond it read zeros
-  if ((r = make_map(&mx, codes8, kH, static_cast<uint64_t>(code_rows), static_cast<uint32_t>(ws.bm)))) return r;
-  if ((r = make_map(&mh, ws.h8, kI, static_cast<uint64_t>(ws.rows), static_cast<uint32_t>(ws.bm)))) return r;
-  if (ws.bm == 128 && n_blocks >= kSharedPairBlocks && shared_pair_supported())
-    return shared_gemms_pair(mx, mh, w13t, w2t, ws, out_bf16, tokens, status, st);
+  const int r = make_map(&mx, codes8, kH, static_cast<uint64_t>(code_rows), static_cast<uint32_t>(ws.bm));
+  if (r) return r;
+  if (on_pairs(ws)) return shared_pair_gemm1(mx, w13t, ws, tokens, status, st);
   SharedEpilogue ep{};
   ep.h8 = ws.h8;
   ep.sfh8 = ws.sfh8;
+  ep.tokens = tokens;
+  return launch_shared_bm<1>(ws.bm, mx, w13t, ws.sfx8, static_cast<int>(ws.rows / ws.bm), ep, status, st);
+}
+
+// From this many blocks of 128 tokens on the second GEMM adds the routed slots itself (shared_pair.cu, MODE 3). Measured, the whole
+// layer with the router inside, slot reduce as a launch of its own behind the side stream / this, us: I = 768 267 / 267 at 1500 tokens,
+// 296 / 300 at 2048, 337 / 329 at 2500, 367 / 354 at 3072, 443 / 413 at 4096, 688 / 671 at 8192, 1289 / 1236 at 16384; I = 1536 477 /
+// 487 at 1500, 535 / 528 at 2048, 637 / 624 at 3072. Below, a unit of 256 x 256 per pair leaves an uneven last round (192 units for
+// 74 pairs at 2048), and the side stream hides the second GEMM.
+constexpr int kSumSlotsBlocks = 18;
+static_assert(kSumSlotsBlocks >= kSharedPairBlocks, "the sum exists on pairs only");
+
+// `slots_bf16` (only where shared_sums_slots says so): out = slots 0..3 + shared row; null: out = the shared rows
+bool shared_sums_slots(const SharedWorkspace& ws) { return on_pairs(ws) && ws.rows / 128 >= kSumSlotsBlocks; }
+int shared_gemm2(const uint8_t* w2t, const SharedWorkspace& ws, const void* slots_bf16, void* out_bf16, int64_t tokens,
+                 int32_t* status, void* stream) {
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  CUtensorMap mh;
+  const int r = make_map(&mh, ws.h8, kI, static_cast<uint64_t>(ws.rows), static_cast<uint32_t>(ws.bm));
+  if (r) return r;
+  if (slots_bf16 && !shared_sums_slots(ws)) return B200MOE_E_ARG;
+  if (on_pairs(ws)) return shared_pair_gemm2(mh, w2t, ws, slots_bf16, out_bf16, tokens, status, st);
+  SharedEpilogue ep{};
   ep.out = static_cast<__nv_bfloat16*>(out_bf16);
   ep.tokens = tokens;
-  if ((r = launch_shared_bm<1>(ws.bm, mx, w13t, ws.sfx8, n_blocks, ep, status, st))) return r;
-  return launch_shared_bm<2>(ws.bm, mh, w2t, ws.sfh8, n_blocks, ep, status, st);
+  return launch_shared_bm<2>(ws.bm, mh, w2t, ws.sfh8, static_cast<int>(ws.rows / ws.bm), ep, status, st);
+}
+
+static int shared_gemms(const uint8_t* w13t, const uint8_t* w2t, const uint8_t* codes8, int64_t code_rows,
+                        const SharedWorkspace& ws, void* out_bf16, int64_t tokens, int32_t* status, void* stream) {
+  const int r = shared_gemm1(w13t, codes8, code_rows, ws, tokens, status, stream);
+  return r ? r : shared_gemm2(w2t, ws, nullptr, out_bf16, tokens, status, stream);
 }
 }  // namespace b200moe
 

@@ -69,6 +69,25 @@ def test_layer_equals_the_separate_calls(C, S, layer, m, router):
     assert C.last_status() == 0
 
 
+@pytest.mark.parametrize("side", [True, False])
+@pytest.mark.parametrize("m", [2176, 2177, 2305, 2432])
+def test_slots_summed_by_the_shared_second_gemm(C, S, layer, m, side):
+    """Around the first size (18 blocks of 128 tokens) at which nobody's shared rows stay in the second GEMM's epilogue: one block
+    below, ragged, an odd count of blocks (a pair's second CTA without rows), full blocks; with and without the side stream. A caller
+    that takes the slots and the shared rows gets them from the other route, with the same bits."""
+    x, lg = inputs(m)
+    slots0, shared0, sum0 = separate_calls(C, S, x, layer, lg)
+    S.set_dbo_query(None if side else lambda: True)
+    try:
+        out = C.mxfp4_moe(x, layer, router_logits=lg)
+        slots, shared = C.mxfp4_moe(x, layer, return_partials=True, router_logits=lg)
+    finally:
+        S.set_dbo_query(None)
+    torch.cuda.synchronize()
+    assert torch.equal(out, sum0) and torch.equal(slots, slots0) and torch.equal(shared, shared0)
+    assert C.last_status() == 0
+
+
 @pytest.mark.parametrize("m", [1, 40, 512, 700, 1600])
 def test_layer_in_a_graph(C, S, layer, m):
     """Capture and replay, the role and (above 512 tokens) the fork to the side stream and its join included: replayed into a
