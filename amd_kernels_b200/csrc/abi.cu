@@ -46,6 +46,9 @@ int prep_small(const float* partials, int64_t stride_t, int64_t stride_s, int sp
 int quant_rows(const void* x_bf16, int64_t tokens, uint8_t* codes, uint8_t* scales, void* stream);
 int quant_rows_both(const void* x_bf16, int64_t tokens, uint8_t* codes, uint8_t* scales, uint8_t* codes8, uint8_t* scales8,
                     uint8_t* atoms8, int bm8, void* stream);
+int router_tc_quant(const void* x_bf16, const void* gate_split_bf16, int64_t tokens, int num_experts, int splits, float* partials,
+                    uint8_t* codes4, uint8_t* scales4, uint8_t* codes8, uint8_t* scales8, uint8_t* atoms8, int bm8, int32_t* status,
+                    void* stream);
 int router_gemm_quant(const void* x_bf16, const float* gate, int64_t tokens, int num_experts, int splits, float* partials,
                       uint8_t* codes4, uint8_t* scales4, uint8_t* codes8, uint8_t* scales8, uint8_t* atoms8, int bm8,
                       void* stream);
@@ -247,9 +250,12 @@ static int run_layer(const LayerCall& c) {
     r = router_gemm_quant(c.x, w->gate, tokens, ne, splits, ws.partials, ws.q4, ws.s4, shared ? ws.sh.x8 : nullptr, nullptr,
                           shared ? ws.sh.sfx8 : nullptr, ws.sh.bm, st);
     if (r) return r;
+  } else if (router) {  // the same from 128 tokens on, the logits on the tensor cores
+    r = router_tc_quant(c.x, w->gate_split, tokens, ne, splits, ws.partials, ws.q4, ws.s4, shared ? ws.sh.x8 : nullptr, nullptr,
+                        shared ? ws.sh.sfx8 : nullptr, ws.sh.bm, c.status, st);
+    if (r) return r;
   } else {
-    if (router && (r = b200moe_router_gemm_tc(c.x, w->gate_split, tokens, ne, splits, ws.partials, c.status, st))) return r;
-    if (router || ws.bm == 128) {
+    if (ws.bm == 128) {
       r = shared ? quant_rows_both(c.x, tokens, ws.q4, ws.s4, ws.sh.x8, nullptr, ws.sh.sfx8, ws.sh.bm, st)
                  : quant_rows(c.x, tokens, ws.q4, ws.s4, st);
     } else {  // decode sizes with logits: the routed rows are quantised by the gather
@@ -352,9 +358,8 @@ extern "C" int b200moe_prepare(const b200moe_weights* w, const void* x_bf16, int
   if (tokens < 128 || !w->gate_split) {
     r = router_gemm_quant(x_bf16, w->gate, tokens, ne, splits, partials, codes4, scales4, codes8, scales8, nullptr, 16, stream);
   } else {
-    if ((r = b200moe_router_gemm_tc(x_bf16, w->gate_split, tokens, ne, splits, partials, status, stream))) return r;
-    r = codes8 ? quant_rows_both(x_bf16, tokens, codes4, scales4, codes8, scales8, nullptr, 16, stream)
-               : quant_rows(x_bf16, tokens, codes4, scales4, stream);
+    r = router_tc_quant(x_bf16, w->gate_split, tokens, ne, splits, partials, codes4, scales4, codes8, scales8, nullptr, 16, status,
+                        stream);
   }
   if (r) return r;
   return b200moe_route_topk(partials, ne, tokens * ne, splits, w->bias, tokens, ne, w->route_mode, w->route_scale, topk_weights,

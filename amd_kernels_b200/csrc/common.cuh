@@ -152,6 +152,22 @@ __device__ __forceinline__ void add_bf16x8(float (&acc)[8], const uint4 v) {
 // byte offset of scale j (0..3) of row r (0..127) inside a 512-byte scale atom
 __device__ __host__ __forceinline__ int atom_offset(int r, int j) { return (r & 31) * 16 + (r >> 5) * 4 + j; }
 
+// Where the MXFP8 operands of quantised rows go (the shared expert's input): codes row-major, the scales row-major or as the scale
+// atoms of 2^atom_shift-row blocks.
+struct QuantRow8 {
+  uint8_t* codes;   // [T][6144]
+  uint8_t* scales;  // [T][192], or null:
+  uint8_t* atoms;   // [ceil(T / 2^atom_shift)][48][512]
+  int atom_shift;
+  // the four scale bytes (blocks 4a .. 4a + 3) of a row
+  __device__ __forceinline__ void store_scales(int64_t row, int a, uint32_t bytes) const {
+    uint8_t* d = scales != nullptr ? scales + row * (kH / 32) + a * 4
+                                   : atoms + ((row >> atom_shift) * (kH / 128) + a) * kAtomBytes +
+                                         atom_offset(static_cast<int>(row & ((1 << atom_shift) - 1)), 0);
+    *reinterpret_cast<uint32_t*>(d) = bytes;
+  }
+};
+
 // 256 threads (t = 0..255, whole warps) quantise one bf16 row of kH values to MXFP4: 3072 code bytes to `dst` and the 192
 // scale bytes into the row's cells of its block's scale atoms (`sdst` = atom 0 + atom_offset(row in block, 0)). The three
 // 16-byte loads of a thread are in flight together. `src` null: a padding row (zero codes, the scale byte of a zero block).

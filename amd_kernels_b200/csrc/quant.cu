@@ -33,15 +33,6 @@ __global__ void __launch_bounds__(256) quant_mxfp4_kernel(const uint4* __restric
   (void)k;
 }
 
-// What the row quantiser also writes when the layer has a shared expert: its MXFP8 operands of the same row, the scales
-// row-major or as the scale atoms of 2^atom_shift-row blocks.
-struct QuantRow8 {
-  uint8_t* codes;   // [T][6144]
-  uint8_t* scales;  // [T][192], or null:
-  uint8_t* atoms;   // [ceil(T / 2^atom_shift)][48][512]
-  int atom_shift;
-};
-
 // Row-major quantisation at prefill sizes: one 256-thread CTA per token row, its three 16-byte loads per thread in flight
 // at once; codes [T][3072] and scales [T][192], the bits of quant_mxfp4_kernel. Used ahead of the gather so that a token is
 // read and quantised once, not once per routed slot -- and (Q8) read once for both quantisers.
@@ -93,13 +84,7 @@ __global__ void __launch_bounds__(256) quant_rows_kernel(const uint4* __restrict
       uint32_t s8 = static_cast<uint32_t>(e8);
       s8 |= __shfl_down_sync(0xffffffffu, s8, 4) << 8;
       s8 |= __shfl_down_sync(0xffffffffu, s8, 8) << 16;
-      if ((lane & 15) == 0) {
-        uint8_t* d8 = q8.scales != nullptr
-                          ? q8.scales + row * (kH / 32) + (idx >> 4) * 4
-                          : q8.atoms + ((row >> q8.atom_shift) * (kH / 128) + (idx >> 4)) * kAtomBytes +
-                                atom_offset(static_cast<int>(row & ((1 << q8.atom_shift) - 1)), 0);
-        *reinterpret_cast<uint32_t*>(d8) = s8;
-      }
+      if ((lane & 15) == 0) q8.store_scales(row, idx >> 4, s8);
     }
   }
 }

@@ -40,6 +40,13 @@ __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
+// True in one lane of a converged warp, the same lane every time. A role that runs its loop with the whole warp and elects a lane
+// around its tcgen05 instructions issues a group of four MMAs, its wait and its commit in 410 to 510 cycles, a loop of one lane in 560.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t one;
+  asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(one));
+  return one != 0;
+}
 __device__ __forceinline__ uint64_t global_timer() {
   uint64_t t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));

@@ -86,6 +86,43 @@ def test_prepared_and_compact_inputs_give_the_entry_bits(P, full_layer, m):
     assert C.last_status() == 0
 
 
+@pytest.mark.parametrize("m", [256, 257, 383, 512, 777, 2049])
+def test_router_gemm_that_quantises_its_tokens(P, full_layer, m):
+    """Around the first size of the one-pass form, ragged and full token blocks, both split counts; rows of zeros, of the largest
+    bf16, of subnormals, with infinities and with NaNs. Bit for bit the separate kernels' operands and routing; into operands that
+    are aligned to 16 bytes only (the separate kernels' route) the same; nothing is written behind the last row."""
+    import ctypes
+    from amd_kernels_b200 import _lib
+    C, S, w = full_layer
+    x = rows(m, 40 + m)
+    x[3] = 0
+    x[5, ::2], x[5, 1::2] = 3.3895313892515355e38, -3.3895313892515355e38
+    x[7] = 1e-39
+    x[9, 17], x[9, 900] = float("inf"), float("-inf")
+    x[11, 40:70] = float("nan")
+    x = x.cuda()
+    q, s = C.mxfp4_quant(x)
+    q8, s8 = S.shared_quant_rows(x)
+    wt, ids = C.route(x, w)
+    for got, want in zip(P.prepare_mxfp4_moe(x, w).tensors(), (q, s, wt, ids, q8, s8)):
+        assert torch.equal(got.view(torch.uint8), want.view(torch.uint8))
+    lib, n4, n8 = _lib.load(), m * H // 2, m * H
+    parts = torch.empty((lib.b200moe_router_splits(m), m, 128), device="cuda")
+    for off in (0, 16):
+        buf4, buf8 = (torch.full((n + 64,), 0xA5, dtype=torch.uint8, device="cuda") for n in (n4, n8))
+        o4, o8 = torch.full((m + 1, H // 32), 0xA5, dtype=torch.uint8, device="cuda"), torch.empty_like(s8)
+        wt1, ids1 = torch.empty_like(wt), torch.empty_like(ids)
+        _lib.check(lib.b200moe_prepare(ctypes.byref(w.abi_now()), x.data_ptr(), m, parts.data_ptr(), buf4.data_ptr() + off,
+                                       o4.data_ptr(), wt1.data_ptr(), ids1.data_ptr(), buf8.data_ptr() + off, o8.data_ptr(),
+                                       C.status_word(x.device).data_ptr(), C._raw_stream(x.device)), "prepare")
+        assert torch.equal(buf4[off:off + n4].view(m, -1), q) and torch.equal(buf8[off:off + n8].view(m, -1), q8)
+        assert torch.equal(o4[:m], s) and torch.equal(o8, s8) and torch.equal(ids1, ids)
+        for guard in (buf4[:off], buf4[off + n4:], buf8[:off], buf8[off + n8:], o4[m]):
+            assert bool((guard == 0xA5).all())
+    torch.cuda.synchronize()
+    assert C.last_status() == 0
+
+
 def test_gather_on_one_rank_and_argument_errors(P, full_layer):
     from tests.test_gpu_moe import _single_rank_group
     C, S, w = full_layer
