@@ -59,6 +59,8 @@ int gemm12_beside(const uint8_t* w13t, const uint8_t* w2t, int num_experts, cons
 int gemm1_beside(const uint8_t* w13t, int num_experts, const uint8_t* xq_sorted, const uint8_t* sfx,
                  const int32_t* block_expert, const int32_t* num_valid, int64_t max_rows, int bm, uint8_t* hq, uint8_t* sfh,
                  const uint8_t* prefetch_w2t, int32_t* status, const SharedPlan* sp, void* stream);
+int sidecar_unpack_atoms(const uint8_t* mask, const uint8_t* s4, const uint8_t* q8, const uint8_t* s8, int64_t tokens, uint8_t* q4,
+                         uint8_t* atoms, int bm, void* stream);
 int shared_gemm1(const uint8_t* w13t, const uint8_t* codes8, int64_t code_rows, const SharedWorkspace& ws, int64_t tokens,
                  int32_t* status, void* stream);
 bool shared_sums_slots(const SharedWorkspace& ws);
@@ -242,10 +244,10 @@ static int run_layer(const LayerCall& c) {
   // the operands: quantised rows and, with the router inside, the logits' split-K partials
   if (c.prep) {
     if (compact) {
-      if ((r = b200moe_sidecar_unpack(c.prep->mask4, s4, codes8, c.prep->scales8, tokens, ws.q4, st))) return r;
+      r = sidecar_unpack_atoms(c.prep->mask4, s4, codes8, c.prep->scales8, tokens, ws.q4, shared ? ws.sh.sfx8 : nullptr, ws.sh.bm, st);
+      if (r) return r;
       q4 = ws.q4;
-    }
-    if (shared && (r = b200moe_scales_to_atoms(c.prep->scales8, tokens, kH / 32, ws.sh.bm, ws.sh.sfx8, st))) return r;
+    } else if (shared && (r = b200moe_scales_to_atoms(c.prep->scales8, tokens, kH / 32, ws.sh.bm, ws.sh.sfx8, st))) return r;
   } else if (router && (tokens < 128 || !w->gate_split)) {  // one pass over x
     r = router_gemm_quant(c.x, w->gate, tokens, ne, splits, ws.partials, ws.q4, ws.s4, shared ? ws.sh.x8 : nullptr, nullptr,
                           shared ? ws.sh.sfx8 : nullptr, ws.sh.bm, st);
