@@ -7,10 +7,15 @@
 //
 //   warp 0    producer: one thread issues the bulk copies of weight tile records and scale atoms and the TMA tile loads of
 //             the token codes
-//   warp 1    MMA: allocates TMEM; one thread issues tcgen05.mma, four per stage
-//   last warp scale copies: one thread moves each stage's scale atoms into TMEM (tcgen05.cp), stages ahead of the MMAs.
-//             Two issuing threads because every tcgen05 / mbarrier instruction costs its thread ~50 cycles whatever the
-//             size of the MMA, and one thread doing both was what bounded the kernel
+//   warp 1    MMA: allocates TMEM, issues tcgen05.mma, four per stage
+//   last warp scale copies: moves each stage's scale atoms into TMEM (tcgen05.cp), stages ahead of the MMAs. Two issuing warps
+//             because every tcgen05 / mbarrier instruction costs its thread ~50 cycles whatever the size of the MMA, and one
+//             doing both was what bounded the kernel
+//             Where a unit's chain of K-tiles bounds the launch (the one-launch kernel, the shared expert's role, 128-row blocks) both
+//             run their loops as whole warps and elect a lane around the instructions, which costs less per K-tile than a loop of
+//             one lane. Measured, layer, one lane / whole warps, us: 109.6 / 107.3 at 32 tokens, 43.7 / 43.4 at 7; I = 1536 238 / 230 at
+//             64, 722 / 657 at 4096; the role alone 37.3 / 36.6 at 1 token. The two decode launches (bm < 128) wait for bytes and keep
+//             the one-lane form: 173.8 / 175.9 at 256 tokens
 //   (the one-launch kernel gemm12_kernel also has warp 6: a second producer for the token-side operand)
 //   warps 2-5 epilogue (bm = 128: a second group, warps 6-9, takes every other unit): tcgen05.ld of the accumulator, then
 //             GEMM1: SwiGLU-OAI (gate and up rows of one tile live in neighbouring lane quarters), MXFP4 requantisation
@@ -153,6 +158,7 @@ __global__ void __launch_bounds__((Cfg<MODE, BM>::kThreads), 1)
                         const __grid_constant__ CUtensorMap map_sh, const SharedArgs sh) {
   using C = Cfg<MODE, BM>;
   constexpr uint32_t kTmemCols = SHARED ? 512 : C::kTmemCols;
+  constexpr bool kWhole = C::kTokensAreM;  // MMA and scale warps in whole-warp form
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t bar_full[C::kStages];
   __shared__ __align__(8) uint64_t bar_unit[SHARED ? kUnitRing : 1];  // the shared expert's units
@@ -286,7 +292,7 @@ __global__ void __launch_bounds__((Cfg<MODE, BM>::kThreads), 1)
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------------- MMA issue
-    if (lane == 0) {
+    if (kWhole || lane == 0) {
       constexpr uint32_t kIdesc = (1u << 7) | (1u << 10) | (static_cast<uint32_t>(BM >> 3) << 17) | (1u << 23) | (8u << 24);
       // The instruction stream of one thread bounds this kernel (every tcgen05 / mbarrier instruction costs it ~50
       // cycles), so the per-stage work is split: the scale-copy thread (last warp) waits for the stage's bytes and copies
@@ -298,28 +304,31 @@ __global__ void __launch_bounds__((Cfg<MODE, BM>::kThreads), 1)
       bool ok = true;
       for (int u = blockIdx.x; u < total_units && ok; u += n_ctas, ++ui) {
         const uint32_t acc = ui & 1u, aph = (ui >> 1) & 1u;
-        if (!mbar_wait(smem_u32(&bar_tempty[acc]), aph ^ 1u, abort_v, status)) break;
+        if (!role_wait<kWhole>(smem_u32(&bar_tempty[acc]), aph ^ 1u, abort_v, status)) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * C::kAccCols;
         for (int kt = 0; kt < C::kTilesK; ++kt) {
-          if (!mbar_wait(full, ph, abort_v, status)) { ok = false; break; }
+          if (!role_wait<kWhole>(full, ph, abort_v, status)) { ok = false; break; }
           tc_fence_after();
           const uint32_t t_sfa = tmem_base + C::kSfaCol + 16u * sfset, t_sfb = t_sfa + 8u;
           // 64 elements = 32 bytes (descriptor + 2) per MMA; scales: atom k/2, bytes {0,1} or {2,3} of each row's cell
           constexpr uint32_t kId0 = kIdesc, kId1 = kIdesc | (2u << 29) | (2u << 4);
           const uint32_t w_lo = lo, x_lo = lo + (C::kBOffset >> 4);
-          if (C::kTokensAreM) {
-            tc_mma_mxf4_lo<2>(d_tmem, x_lo, w_lo, kId0, t_sfb, t_sfa, static_cast<uint32_t>(kt != 0));
-            tc_mma_mxf4_lo<1>(d_tmem, x_lo + 2, w_lo + 2, kId1, t_sfb, t_sfa);
-            tc_mma_mxf4_lo<1>(d_tmem, x_lo + 4, w_lo + 4, kId0, t_sfb + 4, t_sfa + 4);
-            tc_mma_mxf4_lo<1>(d_tmem, x_lo + 6, w_lo + 6, kId1, t_sfb + 4, t_sfa + 4);
-          } else {
-            tc_mma_mxf4_lo<2>(d_tmem, w_lo, x_lo, kId0, t_sfa, t_sfb, static_cast<uint32_t>(kt != 0));
-            tc_mma_mxf4_lo<1>(d_tmem, w_lo + 2, x_lo + 2, kId1, t_sfa, t_sfb);
-            tc_mma_mxf4_lo<1>(d_tmem, w_lo + 4, x_lo + 4, kId0, t_sfa + 4, t_sfb + 4);
-            tc_mma_mxf4_lo<1>(d_tmem, w_lo + 6, x_lo + 6, kId1, t_sfa + 4, t_sfb + 4);
+          if (!kWhole || elect_one()) {
+            if (C::kTokensAreM) {
+              tc_mma_mxf4_lo<2>(d_tmem, x_lo, w_lo, kId0, t_sfb, t_sfa, static_cast<uint32_t>(kt != 0));
+              tc_mma_mxf4_lo<1>(d_tmem, x_lo + 2, w_lo + 2, kId1, t_sfb, t_sfa);
+              tc_mma_mxf4_lo<1>(d_tmem, x_lo + 4, w_lo + 4, kId0, t_sfb + 4, t_sfa + 4);
+              tc_mma_mxf4_lo<1>(d_tmem, x_lo + 6, w_lo + 6, kId1, t_sfb + 4, t_sfa + 4);
+            } else {
+              tc_mma_mxf4_lo<2>(d_tmem, w_lo, x_lo, kId0, t_sfa, t_sfb, static_cast<uint32_t>(kt != 0));
+              tc_mma_mxf4_lo<1>(d_tmem, w_lo + 2, x_lo + 2, kId1, t_sfa, t_sfb);
+              tc_mma_mxf4_lo<1>(d_tmem, w_lo + 4, x_lo + 4, kId0, t_sfa + 4, t_sfb + 4);
+              tc_mma_mxf4_lo<1>(d_tmem, w_lo + 6, x_lo + 6, kId1, t_sfa + 4, t_sfb + 4);
+            }
+            tc_commit(empty);
           }
-          tc_commit(empty);
+          if (kWhole) __syncwarp();
           sfset = (sfset + 1u) & (C::kSfSets - 1);
           if (++slot == C::kStages) {
             slot = 0; ph ^= 1u; lo = tiles >> 4; full = sf0; empty = empty0;
@@ -327,13 +336,13 @@ __global__ void __launch_bounds__((Cfg<MODE, BM>::kThreads), 1)
             lo += C::kStageBytes >> 4; full += 8; empty += 8;
           }
         }
-        if (ok) tc_commit(smem_u32(&bar_tfull[acc]));
+        if (ok && (!kWhole || elect_one())) tc_commit(smem_u32(&bar_tfull[acc]));
       }
-      if (*abort_v) drain_tcgen05(smem_u32(&bar_drain[0]));
+      if (kWhole ? __any_sync(0xffffffffu, *abort_v != 0) && elect_one() : *abort_v != 0) drain_tcgen05(smem_u32(&bar_drain[0]));
     }
   } else if (warp == C::kScaleWarp) {
     // ---------------------------------------------------------------- scale copies: shared memory -> tensor memory
-    if (lane == 0) {
+    if (kWhole || lane == 0) {
       const uint32_t full0 = smem_u32(&bar_full[0]), sf0 = smem_u32(&bar_sf[0]);
       uint32_t slot = 0, ph = 0, sfset = 0;
       uint32_t lo = tiles >> 4, full = full0, sf = sf0;
@@ -342,14 +351,17 @@ __global__ void __launch_bounds__((Cfg<MODE, BM>::kThreads), 1)
         for (int kt = 0; kt < C::kTilesK; ++kt) {
           // full: the stage's bytes have landed, and (through the producer's wait) the MMAs that last read this slot and
           // this scale set, kStages <= kSfSets stages ago, have completed
-          if (!mbar_wait(full, ph, abort_v, status)) { ok = false; break; }
+          if (!role_wait<kWhole>(full, ph, abort_v, status)) { ok = false; break; }
           tc_fence_after();
           const uint32_t t_sfa = tmem_base + C::kSfaCol + 16u * sfset, t_sfb = t_sfa + 8u;
-          tc_cp_scales_lo(t_sfa, lo + (C::kABytes >> 4));
-          tc_cp_scales_lo(t_sfa + 4, lo + ((C::kABytes + kAtomBytes) >> 4));
-          tc_cp_scales_lo(t_sfb, lo + (C::kSfbOffset >> 4));
-          tc_cp_scales_lo(t_sfb + 4, lo + ((C::kSfbOffset + kAtomBytes) >> 4));
-          tc_commit(sf);
+          if (!kWhole || elect_one()) {
+            tc_cp_scales_lo(t_sfa, lo + (C::kABytes >> 4));
+            tc_cp_scales_lo(t_sfa + 4, lo + ((C::kABytes + kAtomBytes) >> 4));
+            tc_cp_scales_lo(t_sfb, lo + (C::kSfbOffset >> 4));
+            tc_cp_scales_lo(t_sfb + 4, lo + ((C::kSfbOffset + kAtomBytes) >> 4));
+            tc_commit(sf);
+          }
+          if (kWhole) __syncwarp();
           sfset = (sfset + 1u) & (C::kSfSets - 1);
           if (++slot == C::kStages) {
             slot = 0; ph ^= 1u; lo = tiles >> 4; full = full0; sf = sf0;
@@ -358,7 +370,7 @@ __global__ void __launch_bounds__((Cfg<MODE, BM>::kThreads), 1)
           }
         }
       }
-      if (*abort_v) drain_tcgen05(smem_u32(&bar_drain[1]));
+      if (kWhole ? __any_sync(0xffffffffu, *abort_v != 0) && elect_one() : *abort_v != 0) drain_tcgen05(smem_u32(&bar_drain[1]));
     }
   } else {
     // ---------------------------------------------------------------- epilogue (groups of 4 warps, TMEM lane quarter = warp % 4)
@@ -775,7 +787,7 @@ __global__ void __launch_bounds__(256, 1)
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------------- MMA issue
-    if (lane == 0) {
+    {
       constexpr uint32_t kIdesc = (1u << 7) | (1u << 10) | (static_cast<uint32_t>(BM >> 3) << 17) | (1u << 23) | (8u << 24);
       constexpr uint32_t kId0 = kIdesc, kId1 = kIdesc | (2u << 29) | (2u << 4);
       // as in grouped_gemm_kernel: warp 7 copies the scales, this thread waits for that and issues the MMAs
@@ -784,23 +796,26 @@ __global__ void __launch_bounds__(256, 1)
       uint32_t lo = tiles >> 4, sf = sf0, empty = empty0;
       bool ok = true;
       for (uint32_t ui = 0; ok; ++ui) {
-        const int u = ring.get(ui, abort_v, status);
+        const int u = __shfl_sync(0xffffffffu, ring.get(ui, abort_v, status), 0);
         if (u >= total_units) break;
         const int tiles_k = u >= units1 ? kK2Tiles : kK1Tiles;
         const uint32_t acc = ui & 1u, aph = (ui >> 1) & 1u;
-        if (!mbar_wait(smem_u32(&bar_tempty[acc]), aph ^ 1u, abort_v, status)) break;
+        if (!warp_wait(smem_u32(&bar_tempty[acc]), aph ^ 1u, abort_v, status)) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * C::kAccCols;
         for (int kt = 0; kt < tiles_k; ++kt) {
-          if (!mbar_wait(sf, ph, abort_v, status)) { ok = false; break; }
+          if (!warp_wait(sf, ph, abort_v, status)) { ok = false; break; }
           tc_fence_after();
           const uint32_t t_sfa = tmem_base + C::kSfaCol + 16u * sfset, t_sfb = t_sfa + 8u;
           const uint32_t w_lo = lo, x_lo = lo + (C::kBOffset >> 4);
-          tc_mma_mxf4_lo<2>(d_tmem, w_lo, x_lo, kId0, t_sfa, t_sfb, static_cast<uint32_t>(kt != 0));
-          tc_mma_mxf4_lo<1>(d_tmem, w_lo + 2, x_lo + 2, kId1, t_sfa, t_sfb);
-          tc_mma_mxf4_lo<1>(d_tmem, w_lo + 4, x_lo + 4, kId0, t_sfa + 4, t_sfb + 4);
-          tc_mma_mxf4_lo<1>(d_tmem, w_lo + 6, x_lo + 6, kId1, t_sfa + 4, t_sfb + 4);
-          tc_commit(empty);
+          if (elect_one()) {
+            tc_mma_mxf4_lo<2>(d_tmem, w_lo, x_lo, kId0, t_sfa, t_sfb, static_cast<uint32_t>(kt != 0));
+            tc_mma_mxf4_lo<1>(d_tmem, w_lo + 2, x_lo + 2, kId1, t_sfa, t_sfb);
+            tc_mma_mxf4_lo<1>(d_tmem, w_lo + 4, x_lo + 4, kId0, t_sfa + 4, t_sfb + 4);
+            tc_mma_mxf4_lo<1>(d_tmem, w_lo + 6, x_lo + 6, kId1, t_sfa + 4, t_sfb + 4);
+            tc_commit(empty);
+          }
+          __syncwarp();
           sfset = (sfset + 1u) & (C::kSfSets - 1);
           if (++slot == CC::kStages) {
             slot = 0; ph ^= 1u; lo = tiles >> 4; sf = sf0; empty = empty0;
@@ -808,30 +823,33 @@ __global__ void __launch_bounds__(256, 1)
             lo += C::kStageBytes >> 4; sf += 8; empty += 8;
           }
         }
-        if (ok) tc_commit(smem_u32(&bar_tfull[acc]));
+        if (ok && elect_one()) tc_commit(smem_u32(&bar_tfull[acc]));
       }
-      if (*abort_v) drain_tcgen05(smem_u32(&bar_drain[0]));
+      if (__any_sync(0xffffffffu, *abort_v != 0) && elect_one()) drain_tcgen05(smem_u32(&bar_drain[0]));
     }
   } else if (warp == 7) {
     // ---------------------------------------------------------------- scale copies: shared memory -> tensor memory
-    if (lane == 0) {
+    {
       const uint32_t full0 = smem_u32(&bar_full[0]), sf0 = smem_u32(&bar_sf[0]);
       uint32_t slot = 0, ph = 0, sfset = 0;
       uint32_t lo = tiles >> 4, full = full0, sf = sf0;
       bool ok = true;
       for (uint32_t ui = 0; ok; ++ui) {
-        const int u = ring.get(ui, abort_v, status);
+        const int u = __shfl_sync(0xffffffffu, ring.get(ui, abort_v, status), 0);
         if (u >= total_units) break;
         const int tiles_k = u >= units1 ? kK2Tiles : kK1Tiles;
         for (int kt = 0; kt < tiles_k; ++kt) {
-          if (!mbar_wait(full, ph, abort_v, status)) { ok = false; break; }
+          if (!warp_wait(full, ph, abort_v, status)) { ok = false; break; }
           tc_fence_after();
           const uint32_t t_sfa = tmem_base + C::kSfaCol + 16u * sfset, t_sfb = t_sfa + 8u;
-          tc_cp_scales_lo(t_sfa, lo + (C::kABytes >> 4));
-          tc_cp_scales_lo(t_sfa + 4, lo + ((C::kABytes + kAtomBytes) >> 4));
-          tc_cp_scales_lo(t_sfb, lo + (C::kSfbOffset >> 4));
-          tc_cp_scales_lo(t_sfb + 4, lo + ((C::kSfbOffset + kAtomBytes) >> 4));
-          tc_commit(sf);
+          if (elect_one()) {
+            tc_cp_scales_lo(t_sfa, lo + (C::kABytes >> 4));
+            tc_cp_scales_lo(t_sfa + 4, lo + ((C::kABytes + kAtomBytes) >> 4));
+            tc_cp_scales_lo(t_sfb, lo + (C::kSfbOffset >> 4));
+            tc_cp_scales_lo(t_sfb + 4, lo + ((C::kSfbOffset + kAtomBytes) >> 4));
+            tc_commit(sf);
+          }
+          __syncwarp();
           sfset = (sfset + 1u) & (C::kSfSets - 1);
           if (++slot == CC::kStages) {
             slot = 0; ph ^= 1u; lo = tiles >> 4; full = full0; sf = sf0;
@@ -840,7 +858,7 @@ __global__ void __launch_bounds__(256, 1)
           }
         }
       }
-      if (*abort_v) drain_tcgen05(smem_u32(&bar_drain[1]));
+      if (__any_sync(0xffffffffu, *abort_v != 0) && elect_one()) drain_tcgen05(smem_u32(&bar_drain[1]));
     }
   } else if (warp < 6) {
     // ---------------------------------------------------------------- epilogue (warps 2..5)

@@ -174,12 +174,12 @@ __global__ void __launch_bounds__(QUANT ? RouterCfg::kQuantThreads : RouterCfg::
     bool ok = true;
     for (int u = blockIdx.x; u < total_units && ok; u += gridDim.x, ++ui) {
       const uint32_t acc = ui & 1u, aph = (ui >> 1) & 1u;
-      if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_tempty[acc]), aph ^ 1u, abort_v, status))) break;
+      if (!warp_wait(smem_u32(&bar_tempty[acc]), aph ^ 1u, abort_v, status)) break;
       tc_fence_after();
       const uint32_t d_tmem = tmem_base + acc * 128u;
       for (int i = 0; i < steps; ++i, ++it) {
         const uint32_t s = it % C::kStages, ph = (it / C::kFullBars) & 1u;
-        if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_full[it % C::kFullBars]), ph, abort_v, status))) { ok = false; break; }
+        if (!warp_wait(smem_u32(&bar_full[it % C::kFullBars]), ph, abort_v, status)) { ok = false; break; }
         tc_fence_after();
         const uint32_t x_lo = (tiles + s * C::kStageBytes) >> 4;
         if (elect_one()) {
@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(QUANT ? RouterCfg::kQuantThreads : RouterCfg::
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           const uint32_t s = (it + h) % C::kStages, ph = ((it + h) / C::kFullBars) & 1u;
-          if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_full[(it + h) % C::kFullBars]), ph, abort_v, status))) {
+          if (!warp_wait(smem_u32(&bar_full[(it + h) % C::kFullBars]), ph, abort_v, status)) {
             ok = false;
             break;
           }

@@ -168,7 +168,7 @@ __device__ __forceinline__ void shared_role(const SharedArgs& a, const CUtensorM
       if (!ok) drain_copies(bar_full, it, stages);
     }
   } else if (warp == 1) {
-    if (lane == 0) {  // ------------------------------------------------ MMA issue
+    {  // ------------------------------------------------ MMA issue
       // E4M3 x E4M3 (format 0), UE8M0 scales, M = 128 weight rows, N = bm tokens; scale byte k of a row's cell for MMA k
       const uint32_t idesc = (static_cast<uint32_t>(bm >> 3) << 17) | (1u << 23) | (8u << 24);
       const uint32_t sf0 = smem_u32(bar_sf), empty0 = smem_u32(bar_empty);
@@ -176,23 +176,26 @@ __device__ __forceinline__ void shared_role(const SharedArgs& a, const CUtensorM
       uint32_t lo = tiles >> 4, sf = sf0, empty = empty0;
       bool ok = true;
       for (uint32_t ui = 0; ok; ++ui) {
-        const int u = ring.get(ui, abort_v, status);
+        const int u = __shfl_sync(0xffffffffu, ring.get(ui, abort_v, status), 0);
         if (u >= total) break;
         const int tiles_k = u >= units1 ? kS2TilesK : kS1TilesK;
         const uint32_t acc = ui & 1u, aph = (ui >> 1) & 1u;
-        if (!mbar_wait(smem_u32(bar_tempty + acc), aph ^ 1u, abort_v, status)) break;
+        if (!warp_wait(smem_u32(bar_tempty + acc), aph ^ 1u, abort_v, status)) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * bm;
         for (int kt = 0; kt < tiles_k; ++kt) {
-          if (!mbar_wait(sf, ph, abort_v, status)) { ok = false; break; }
+          if (!warp_wait(sf, ph, abort_v, status)) { ok = false; break; }
           tc_fence_after();
           const uint32_t t_sfa = tmem_base + sfa_col + 8u * sfset, t_sfb = t_sfa + 4u;
           const uint32_t w_lo = lo, x_lo = lo + (b_off >> 4);
-          tc_mma_mxf8_lo<2>(d_tmem, w_lo, x_lo, idesc, t_sfa, t_sfb, static_cast<uint32_t>(kt != 0));
-          tc_mma_mxf8_lo<1>(d_tmem, w_lo + 2, x_lo + 2, idesc | (1u << 29) | (1u << 4), t_sfa, t_sfb);
-          tc_mma_mxf8_lo<1>(d_tmem, w_lo + 4, x_lo + 4, idesc | (2u << 29) | (2u << 4), t_sfa, t_sfb);
-          tc_mma_mxf8_lo<1>(d_tmem, w_lo + 6, x_lo + 6, idesc | (3u << 29) | (3u << 4), t_sfa, t_sfb);
-          tc_commit(empty);
+          if (elect_one()) {
+            tc_mma_mxf8_lo<2>(d_tmem, w_lo, x_lo, idesc, t_sfa, t_sfb, static_cast<uint32_t>(kt != 0));
+            tc_mma_mxf8_lo<1>(d_tmem, w_lo + 2, x_lo + 2, idesc | (1u << 29) | (1u << 4), t_sfa, t_sfb);
+            tc_mma_mxf8_lo<1>(d_tmem, w_lo + 4, x_lo + 4, idesc | (2u << 29) | (2u << 4), t_sfa, t_sfb);
+            tc_mma_mxf8_lo<1>(d_tmem, w_lo + 6, x_lo + 6, idesc | (3u << 29) | (3u << 4), t_sfa, t_sfb);
+            tc_commit(empty);
+          }
+          __syncwarp();
           sfset = (sfset + 1u) & (kSharedMaxStages - 1);
           if (++slot == stages) {
             slot = 0; ph ^= 1u; lo = tiles >> 4; sf = sf0; empty = empty0;
@@ -200,27 +203,30 @@ __device__ __forceinline__ void shared_role(const SharedArgs& a, const CUtensorM
             lo += stage_bytes >> 4; sf += 8; empty += 8;
           }
         }
-        if (ok) tc_commit(smem_u32(bar_tfull + acc));
+        if (ok && elect_one()) tc_commit(smem_u32(bar_tfull + acc));
       }
-      if (*abort_v) drain_tcgen05(smem_u32(bar_drain));
+      if (__any_sync(0xffffffffu, *abort_v != 0) && elect_one()) drain_tcgen05(smem_u32(bar_drain));
     }
   } else if (warp == 6) {
-    if (lane == 0) {  // ------------------------------------------------ scale copies: shared memory -> tensor memory
+    {  // ------------------------------------------------ scale copies: shared memory -> tensor memory
       const uint32_t full0 = smem_u32(bar_full), sf0 = smem_u32(bar_sf);
       uint32_t slot = 0, ph = 0, sfset = 0;
       uint32_t lo = tiles >> 4, full = full0, sf = sf0;
       bool ok = true;
       for (uint32_t ui = 0; ok; ++ui) {
-        const int u = ring.get(ui, abort_v, status);
+        const int u = __shfl_sync(0xffffffffu, ring.get(ui, abort_v, status), 0);
         if (u >= total) break;
         const int tiles_k = u >= units1 ? kS2TilesK : kS1TilesK;
         for (int kt = 0; kt < tiles_k; ++kt) {
-          if (!mbar_wait(full, ph, abort_v, status)) { ok = false; break; }
+          if (!warp_wait(full, ph, abort_v, status)) { ok = false; break; }
           tc_fence_after();
           const uint32_t t_sfa = tmem_base + sfa_col + 8u * sfset;
-          tc_cp_scales_lo(t_sfa, lo + ((128 * 128) >> 4));
-          tc_cp_scales_lo(t_sfa + 4, lo + (sfb_off >> 4));
-          tc_commit(sf);
+          if (elect_one()) {
+            tc_cp_scales_lo(t_sfa, lo + ((128 * 128) >> 4));
+            tc_cp_scales_lo(t_sfa + 4, lo + (sfb_off >> 4));
+            tc_commit(sf);
+          }
+          __syncwarp();
           sfset = (sfset + 1u) & (kSharedMaxStages - 1);
           if (++slot == stages) {
             slot = 0; ph ^= 1u; lo = tiles >> 4; full = full0; sf = sf0;
@@ -229,7 +235,7 @@ __device__ __forceinline__ void shared_role(const SharedArgs& a, const CUtensorM
           }
         }
       }
-      if (*abort_v) drain_tcgen05(smem_u32(bar_drain + 1));
+      if (__any_sync(0xffffffffu, *abort_v != 0) && elect_one()) drain_tcgen05(smem_u32(bar_drain + 1));
     }
   } else if (warp < 6) {
     // ------------------------------------------------------------------ epilogue (warps 2..5)

@@ -82,6 +82,16 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   }
 }
 
+// The same by a whole warp, whose lanes agree on the answer.
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int32_t* status) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status));
+}
+
+template <bool WHOLE>
+__device__ __forceinline__ bool role_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int32_t* status) {
+  return WHOLE ? warp_wait(bar, parity, abort_flag, status) : mbar_wait(bar, parity, abort_flag, status);
+}
+
 // After an abort: let the copies of the last `stages` pipeline slots land (one overall limit, not one per slot) before
 // the CTA gives up its shared memory. `it` = stages issued so far.
 __device__ __forceinline__ void drain_copies(const uint64_t* bar_full, uint32_t it, uint32_t stages) {
