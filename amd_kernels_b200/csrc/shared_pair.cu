@@ -177,17 +177,20 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SharedPairCfg<MODE>:
       }
     } else if (warp == 1) {
       // ---------------------------------------------------------------- MMA issue (leader only)
-      if (lane == 0 && leader) {
+      if (leader) {
         // E4M3 x E4M3, UE8M0 scales, M = 256, N = 256; scale byte k of a row's cell for MMA k
         constexpr uint32_t kIdesc = (static_cast<uint32_t>(256 >> 3) << 17) | (1u << 23) | (static_cast<uint32_t>(256 >> 4) << 24);
         uint32_t ui = 0, s = 0, ph = 0, j = 0, sph = 0;
         bool ok = true, sf_ready = false, full_ready = false;
         for (int u = cluster; u < total && ok; u += n_clusters, ++ui) {
-          if (!mbar_wait(smem_u32(&bar_tempty), (ui & 1u) ^ 1u, abort_v, status)) break;
+          if (!warp_wait(smem_u32(&bar_tempty), (ui & 1u) ^ 1u, abort_v, status)) break;
           tc_fence_after();
           for (int kt = 0; kt < C::kTilesK; ++kt) {
-            if (!sf_ready && !mbar_wait(smem_u32(&bar_sf[j]), sph, abort_v, status)) { ok = false; break; }
-            if (!full_ready && !mbar_wait(smem_u32(&bar_full[s]), ph, abort_v, status)) { ok = false; break; }
+            if (!__all_sync(0xffffffffu, (sf_ready || mbar_wait(smem_u32(&bar_sf[j]), sph, abort_v, status)) &&
+                                             (full_ready || mbar_wait(smem_u32(&bar_full[s]), ph, abort_v, status)))) {
+              ok = false;
+              break;
+            }
             tc_fence_after();
             const uint32_t s_now = s, j_now = j;
             if (++s == C::kStages) { s = 0; ph ^= 1u; }
@@ -197,26 +200,32 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SharedPairCfg<MODE>:
             const uint32_t lo = (tiles + s_now * C::kStageBytes) >> 4;
             const uint32_t x_lo = lo + (C::kTokOff >> 4), w_lo = lo + (C::kWOff >> 4);
             const uint32_t t_sft = tmem_base + C::kSfCol + 16u * j_now, t_sfw = t_sft + 8u;
-            tc_mma_mxf8_pair(tmem_base, x_lo, w_lo, kIdesc, t_sft, t_sfw, static_cast<uint32_t>(kt != 0));
-            tc_mma_mxf8_pair(tmem_base, x_lo + 2, w_lo + 2, kIdesc | (1u << 29) | (1u << 4), t_sft, t_sfw, 1u);
-            tc_mma_mxf8_pair(tmem_base, x_lo + 4, w_lo + 4, kIdesc | (2u << 29) | (2u << 4), t_sft, t_sfw, 1u);
-            tc_mma_mxf8_pair(tmem_base, x_lo + 6, w_lo + 6, kIdesc | (3u << 29) | (3u << 4), t_sft, t_sfw, 1u);
-            tc_commit_both(smem_u32(&bar_empty[s_now]));  // the stage is free again, in both CTAs
+            if (elect_one()) {
+              tc_mma_mxf8_pair(tmem_base, x_lo, w_lo, kIdesc, t_sft, t_sfw, static_cast<uint32_t>(kt != 0));
+              tc_mma_mxf8_pair(tmem_base, x_lo + 2, w_lo + 2, kIdesc | (1u << 29) | (1u << 4), t_sft, t_sfw, 1u);
+              tc_mma_mxf8_pair(tmem_base, x_lo + 4, w_lo + 4, kIdesc | (2u << 29) | (2u << 4), t_sft, t_sfw, 1u);
+              tc_mma_mxf8_pair(tmem_base, x_lo + 6, w_lo + 6, kIdesc | (3u << 29) | (3u << 4), t_sft, t_sfw, 1u);
+              tc_commit_both(smem_u32(&bar_empty[s_now]));  // the stage is free again, in both CTAs
+            }
+            __syncwarp();
           }
-          if (ok) tc_commit_both(smem_u32(&bar_tfull));
+          if (ok && elect_one()) tc_commit_both(smem_u32(&bar_tfull));
         }
-        if (*abort_v) drain_tcgen05_pair(smem_u32(&bar_drain[0]));
+        if (__any_sync(0xffffffffu, *abort_v != 0) && elect_one()) drain_tcgen05_pair(smem_u32(&bar_drain[0]));
       }
     } else {
       // ---------------------------------------------------------------- scale copies into both CTAs' tensor memory (leader)
-      if (lane == 0 && leader) {
+      if (leader) {
         uint32_t s = 0, ph = 1u, j = 0, sph = 0;
         bool ok = true, landed = false, free_set = false;
         for (int u = cluster; u < total && ok; u += n_clusters) {
           for (int kt = 0; kt < C::kTilesK; ++kt) {
-            if (!landed && !mbar_wait(smem_u32(&bar_sfull[j]), sph, abort_v, status)) { ok = false; break; }
             // set j was last read by the MMAs 8 K-tiles back: complete once those 6 K-tiles back are
-            if (!free_set && !mbar_wait(smem_u32(&bar_empty[s]), ph, abort_v, status)) { ok = false; break; }
+            if (!__all_sync(0xffffffffu, (landed || mbar_wait(smem_u32(&bar_sfull[j]), sph, abort_v, status)) &&
+                                             (free_set || mbar_wait(smem_u32(&bar_empty[s]), ph, abort_v, status)))) {
+              ok = false;
+              break;
+            }
             tc_fence_after();
             const uint32_t lo = (sf_ring + j * C::kSfSlotBytes) >> 4, sf_bar = smem_u32(&bar_sf[j]);
             const uint32_t t_sft = tmem_base + C::kSfCol + 16u * j, t_sfw = t_sft + 8u;
@@ -224,13 +233,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SharedPairCfg<MODE>:
             if (++j == C::kSfStages) { j = 0; sph ^= 1u; }
             landed = mbar_test(smem_u32(&bar_sfull[j]), sph);
             free_set = mbar_test(smem_u32(&bar_empty[s]), ph);
-            tc_cp_scales_pair(t_sft, lo + (C::kSfTokOff >> 4));      // each CTA its own token rows
-            tc_cp_scales_pair(t_sfw, lo + (C::kSfWLoOff >> 4));      // weight rows 0..127 of N
-            tc_cp_scales_pair(t_sfw + 4, lo + (C::kSfWHiOff >> 4));  // 128..255
-            tc_commit_both(sf_bar);
+            if (elect_one()) {
+              tc_cp_scales_pair(t_sft, lo + (C::kSfTokOff >> 4));      // each CTA its own token rows
+              tc_cp_scales_pair(t_sfw, lo + (C::kSfWLoOff >> 4));      // weight rows 0..127 of N
+              tc_cp_scales_pair(t_sfw + 4, lo + (C::kSfWHiOff >> 4));  // 128..255
+              tc_commit_both(sf_bar);
+            }
+            __syncwarp();
           }
         }
-        if (*abort_v) drain_tcgen05_pair(smem_u32(&bar_drain[1]));
+        if (__any_sync(0xffffffffu, *abort_v != 0) && elect_one()) drain_tcgen05_pair(smem_u32(&bar_drain[1]));
       }
     }
   } else {
