@@ -598,7 +598,7 @@ __global__ void __launch_bounds__(WideCfg::kThreads, 1)
     asm volatile("cp.async.wait_all;" ::: "memory");
   } else if (warp == 1) {
     // ---------------------------------------------------------------- MMA issue
-    if (lane == 0) {
+    {
       // E2M1 x E2M1, UE8M0 scales, M = 128 token rows, N = 256 weight rows
       constexpr uint32_t kIdesc = (1u << 7) | (1u << 10) | (static_cast<uint32_t>(256 >> 3) << 17) | (1u << 23) |
                                   (static_cast<uint32_t>(128 >> 4) << 24);
@@ -606,13 +606,16 @@ __global__ void __launch_bounds__(WideCfg::kThreads, 1)
       uint32_t it = 0, ui = 0;
       bool ok = true, sf_ready = false, full_ready = false;
       for (int u = first; u < total && ok; u += stride, ++ui) {
-        if (!mbar_wait(smem_u32(&bar_tempty), (ui & 1u) ^ 1u, abort_v, status)) break;
+        if (!warp_wait(smem_u32(&bar_tempty), (ui & 1u) ^ 1u, abort_v, status)) break;
         tc_fence_after();
         for (int kt = 0; kt < kK1Tiles; ++kt) {
           const uint32_t s = it % C::kStages, ph = (it / C::kStages) & 1u;
           const uint32_t j = it % C::kSfStages, sph = (it / C::kSfStages) & 1u;
-          if (!sf_ready && !mbar_wait(smem_u32(&bar_sf[j]), sph, abort_v, status)) { ok = false; break; }
-          if (!full_ready && !mbar_wait(smem_u32(&bar_full[s]), ph, abort_v, status)) { ok = false; break; }
+          if (!__all_sync(0xffffffffu, (sf_ready || mbar_wait(smem_u32(&bar_sf[j]), sph, abort_v, status)) &&
+                                           (full_ready || mbar_wait(smem_u32(&bar_full[s]), ph, abort_v, status)))) {
+            ok = false;
+            break;
+          }
           tc_fence_after();
           ++it;  // look at the next K-tile's barriers while this one's MMAs are issued (320 -> 308 us at 16384 tokens)
           sf_ready = mbar_test(smem_u32(&bar_sf[it % C::kSfStages]), (it / C::kSfStages) & 1u);
@@ -621,19 +624,22 @@ __global__ void __launch_bounds__(WideCfg::kThreads, 1)
           const uint32_t lo = (tiles + s * C::kStageBytes) >> 4;
           const uint32_t x_lo = lo + (C::kTokOff >> 4), w_lo = lo + (C::kWOff >> 4);
           const uint32_t t_sft = tmem_base + C::kSfCol + 24u * j, t_sfw = t_sft + 8u;
-          tc_mma_mxf4_wide(tmem_base, x_lo, w_lo, kId0, t_sft, t_sfw, static_cast<uint32_t>(kt != 0));
-          tc_mma_mxf4_wide(tmem_base, x_lo + 2, w_lo + 2, kId1, t_sft, t_sfw, 1u);
-          tc_mma_mxf4_wide(tmem_base, x_lo + 4, w_lo + 4, kId0, t_sft + 4, t_sfw + 8, 1u);
-          tc_mma_mxf4_wide(tmem_base, x_lo + 6, w_lo + 6, kId1, t_sft + 4, t_sfw + 8, 1u);
-          tc_commit(smem_u32(&bar_empty[s]));
+          if (elect_one()) {
+            tc_mma_mxf4_wide(tmem_base, x_lo, w_lo, kId0, t_sft, t_sfw, static_cast<uint32_t>(kt != 0));
+            tc_mma_mxf4_wide(tmem_base, x_lo + 2, w_lo + 2, kId1, t_sft, t_sfw, 1u);
+            tc_mma_mxf4_wide(tmem_base, x_lo + 4, w_lo + 4, kId0, t_sft + 4, t_sfw + 8, 1u);
+            tc_mma_mxf4_wide(tmem_base, x_lo + 6, w_lo + 6, kId1, t_sft + 4, t_sfw + 8, 1u);
+            tc_commit(smem_u32(&bar_empty[s]));
+          }
+          __syncwarp();
         }
-        if (ok) tc_commit(smem_u32(&bar_tfull));
+        if (ok && elect_one()) tc_commit(smem_u32(&bar_tfull));
       }
-      if (*abort_v) drain_tcgen05(smem_u32(&bar_drain[0]));
+      if (__any_sync(0xffffffffu, *abort_v != 0) && elect_one()) drain_tcgen05(smem_u32(&bar_drain[0]));
     }
   } else if (warp == 2 || warp == 3) {
     // ---------------------------------------------------------------- scale copies (three of the six atoms each)
-    if (lane == 0) {
+    {
       const bool head = warp == 2;
       uint32_t it = 0;
       bool ok = true, landed = false, free_set = false;
@@ -641,9 +647,12 @@ __global__ void __launch_bounds__(WideCfg::kThreads, 1)
         for (int kt = 0; kt < kK1Tiles; ++kt) {
           const uint32_t s = it % C::kStages, ph = (it / C::kStages) & 1u;
           const uint32_t j = it % C::kSfStages, sph = (it / C::kSfStages) & 1u;
-          if (!landed && !mbar_wait(smem_u32(&bar_sfull[j]), sph, abort_v, status)) { ok = false; break; }
           // scale set j was last read by the MMAs of K-tile it - 8: complete once those of K-tile it - 4 are
-          if (!free_set && !mbar_wait(smem_u32(&bar_empty[s]), ph ^ 1u, abort_v, status)) { ok = false; break; }
+          if (!__all_sync(0xffffffffu, (landed || mbar_wait(smem_u32(&bar_sfull[j]), sph, abort_v, status)) &&
+                                           (free_set || mbar_wait(smem_u32(&bar_empty[s]), ph ^ 1u, abort_v, status)))) {
+            ok = false;
+            break;
+          }
           tc_fence_after();
           ++it;
           landed = mbar_test(smem_u32(&bar_sfull[it % C::kSfStages]), (it / C::kSfStages) & 1u);
@@ -651,19 +660,22 @@ __global__ void __launch_bounds__(WideCfg::kThreads, 1)
           if (GATHER) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
           const uint32_t lo = (sf_ring + j * C::kSfSlotBytes) >> 4;
           const uint32_t t_sft = tmem_base + C::kSfCol + 24u * j, t_sfw = t_sft + 8u;
-          if (head) {
-            tc_cp_scales_lo(t_sft, lo + (C::kSfTokOff >> 4));
-            tc_cp_scales_lo(t_sft + 4, lo + ((C::kSfTokOff + kAtomBytes) >> 4));
-            tc_cp_scales_lo(t_sfw, lo + (C::kSfWLoOff >> 4));
-          } else {
-            tc_cp_scales_lo(t_sfw + 4, lo + (C::kSfWHiOff >> 4));
-            tc_cp_scales_lo(t_sfw + 8, lo + ((C::kSfWLoOff + kAtomBytes) >> 4));
-            tc_cp_scales_lo(t_sfw + 12, lo + ((C::kSfWHiOff + kAtomBytes) >> 4));
+          if (elect_one()) {
+            if (head) {
+              tc_cp_scales_lo(t_sft, lo + (C::kSfTokOff >> 4));
+              tc_cp_scales_lo(t_sft + 4, lo + ((C::kSfTokOff + kAtomBytes) >> 4));
+              tc_cp_scales_lo(t_sfw, lo + (C::kSfWLoOff >> 4));
+            } else {
+              tc_cp_scales_lo(t_sfw + 4, lo + (C::kSfWHiOff >> 4));
+              tc_cp_scales_lo(t_sfw + 8, lo + ((C::kSfWLoOff + kAtomBytes) >> 4));
+              tc_cp_scales_lo(t_sfw + 12, lo + ((C::kSfWHiOff + kAtomBytes) >> 4));
+            }
+            tc_commit(smem_u32(&bar_sf[j]));
           }
-          tc_commit(smem_u32(&bar_sf[j]));
+          __syncwarp();
         }
       }
-      if (*abort_v) drain_tcgen05(smem_u32(&bar_drain[1]));
+      if (__any_sync(0xffffffffu, *abort_v != 0) && elect_one()) drain_tcgen05(smem_u32(&bar_drain[1]));
     }
   }
   } else {

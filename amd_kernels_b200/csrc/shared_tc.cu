@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(224, 1)
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {  // ------------------------------------------------ MMA issue
+    {  // ------------------------------------------------ MMA issue
       // E4M3 x E4M3 (format 0), UE8M0 scales, M = 128, N = BM; scale byte k of each row's 4-byte cell for MMA k
       constexpr uint32_t kIdesc = (static_cast<uint32_t>(BM >> 3) << 17) | (1u << 23) | (8u << 24);
       const uint32_t sf0 = smem_u32(&bar_sf[0]), empty0 = smem_u32(&bar_empty[0]);
@@ -201,20 +201,23 @@ __global__ void __launch_bounds__(224, 1)
       bool ok = true;
       for (int u = blockIdx.x; u < total_units && ok; u += gridDim.x, ++ui) {
         const uint32_t acc = ui & 1u, aph = (ui >> 1) & 1u;
-        if (!mbar_wait(smem_u32(&bar_tempty[acc]), aph ^ 1u, abort_v, status)) break;
+        if (!warp_wait(smem_u32(&bar_tempty[acc]), aph ^ 1u, abort_v, status)) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BM;
         for (int kt = 0; kt < C::kTilesK; ++kt) {
-          if (!mbar_wait(sf, ph, abort_v, status)) { ok = false; break; }
+          if (!warp_wait(sf, ph, abort_v, status)) { ok = false; break; }
           tc_fence_after();
           const uint32_t t_sfa = tmem_base + C::kSfaCol + 8u * sfset, t_sfb = t_sfa + 4u;
           const uint32_t w_lo = lo, x_lo = lo + (C::kBOffset >> 4);
           // 32 elements = 32 bytes (descriptor + 2) per MMA
-          tc_mma_mxf8_lo<2>(d_tmem, w_lo, x_lo, kIdesc, t_sfa, t_sfb, static_cast<uint32_t>(kt != 0));
-          tc_mma_mxf8_lo<1>(d_tmem, w_lo + 2, x_lo + 2, kIdesc | (1u << 29) | (1u << 4), t_sfa, t_sfb);
-          tc_mma_mxf8_lo<1>(d_tmem, w_lo + 4, x_lo + 4, kIdesc | (2u << 29) | (2u << 4), t_sfa, t_sfb);
-          tc_mma_mxf8_lo<1>(d_tmem, w_lo + 6, x_lo + 6, kIdesc | (3u << 29) | (3u << 4), t_sfa, t_sfb);
-          tc_commit(empty);
+          if (elect_one()) {
+            tc_mma_mxf8_lo<2>(d_tmem, w_lo, x_lo, kIdesc, t_sfa, t_sfb, static_cast<uint32_t>(kt != 0));
+            tc_mma_mxf8_lo<1>(d_tmem, w_lo + 2, x_lo + 2, kIdesc | (1u << 29) | (1u << 4), t_sfa, t_sfb);
+            tc_mma_mxf8_lo<1>(d_tmem, w_lo + 4, x_lo + 4, kIdesc | (2u << 29) | (2u << 4), t_sfa, t_sfb);
+            tc_mma_mxf8_lo<1>(d_tmem, w_lo + 6, x_lo + 6, kIdesc | (3u << 29) | (3u << 4), t_sfa, t_sfb);
+            tc_commit(empty);
+          }
+          __syncwarp();
           sfset = (sfset + 1u) & (C::kSfSets - 1);
           if (++slot == C::kStages) {
             slot = 0; ph ^= 1u; lo = tiles >> 4; sf = sf0; empty = empty0;
@@ -222,24 +225,27 @@ __global__ void __launch_bounds__(224, 1)
             lo += C::kStageBytes >> 4; sf += 8; empty += 8;
           }
         }
-        if (ok) tc_commit(smem_u32(&bar_tfull[acc]));
+        if (ok && elect_one()) tc_commit(smem_u32(&bar_tfull[acc]));
       }
-      if (*abort_v) drain_tcgen05(smem_u32(&bar_drain[0]));
+      if (__any_sync(0xffffffffu, *abort_v != 0) && elect_one()) drain_tcgen05(smem_u32(&bar_drain[0]));
     }
   } else if (warp == 6) {
-    if (lane == 0) {  // ------------------------------------------------ scale copies: shared memory -> tensor memory
+    {  // ------------------------------------------------ scale copies: shared memory -> tensor memory
       const uint32_t full0 = smem_u32(&bar_full[0]), sf0 = smem_u32(&bar_sf[0]);
       uint32_t slot = 0, ph = 0, sfset = 0;
       uint32_t lo = tiles >> 4, full = full0, sf = sf0;
       bool ok = true;
       for (int u = blockIdx.x; u < total_units && ok; u += gridDim.x) {
         for (int kt = 0; kt < C::kTilesK; ++kt) {
-          if (!mbar_wait(full, ph, abort_v, status)) { ok = false; break; }
+          if (!warp_wait(full, ph, abort_v, status)) { ok = false; break; }
           tc_fence_after();
           const uint32_t t_sfa = tmem_base + C::kSfaCol + 8u * sfset;
-          tc_cp_scales_lo(t_sfa, lo + ((128 * 128) >> 4));
-          tc_cp_scales_lo(t_sfa + 4, lo + (C::kSfbOffset >> 4));
-          tc_commit(sf);
+          if (elect_one()) {
+            tc_cp_scales_lo(t_sfa, lo + ((128 * 128) >> 4));
+            tc_cp_scales_lo(t_sfa + 4, lo + (C::kSfbOffset >> 4));
+            tc_commit(sf);
+          }
+          __syncwarp();
           sfset = (sfset + 1u) & (C::kSfSets - 1);
           if (++slot == C::kStages) {
             slot = 0; ph ^= 1u; lo = tiles >> 4; full = full0; sf = sf0;
@@ -248,7 +254,7 @@ __global__ void __launch_bounds__(224, 1)
           }
         }
       }
-      if (*abort_v) drain_tcgen05(smem_u32(&bar_drain[1]));
+      if (__any_sync(0xffffffffu, *abort_v != 0) && elect_one()) drain_tcgen05(smem_u32(&bar_drain[1]));
     }
   } else {
     // ------------------------------------------------------------------ epilogue (warps 2..5)
