@@ -43,9 +43,9 @@ int prep_small(const float* partials, int64_t stride_t, int64_t stride_s, int sp
                float* sorted_w, int32_t* block_expert, int32_t* num_valid, const void* x_bf16, const uint8_t* q4,
                const uint8_t* s4, int64_t max_rows, uint8_t* xq_sorted, uint8_t* sfx, int32_t* done, int n_done,
                void* stream);
-int quant_rows(const void* x_bf16, int64_t tokens, uint8_t* codes, uint8_t* scales, void* stream);
-int quant_rows_both(const void* x_bf16, int64_t tokens, uint8_t* codes, uint8_t* scales, uint8_t* codes8, uint8_t* scales8,
-                    uint8_t* atoms8, int bm8, void* stream);
+int route_quant(const float* logits, const float* bias, int64_t tokens, int num_experts, int mode, float scale, const void* x_bf16,
+                float* out_w, int32_t* out_ids, uint8_t* codes4, uint8_t* scales4, uint8_t* codes8, uint8_t* atoms8, int bm8,
+                void* stream);
 int router_tc_quant(const void* x_bf16, const void* gate_split_bf16, int64_t tokens, int num_experts, int splits, float* partials,
                     uint8_t* codes4, uint8_t* scales4, uint8_t* codes8, uint8_t* scales8, uint8_t* atoms8, int bm8, int32_t* status,
                     void* stream);
@@ -100,10 +100,8 @@ static Workspace carve(uint8_t* base, int64_t tokens, int num_experts, int flags
   ws.done = reinterpret_cast<int32_t*>(take((blocks + kSharedDone) * 4));
   if (flags & B200MOE_LAYER_ROUTER)
     ws.partials = reinterpret_cast<float*>(take(static_cast<size_t>(b200moe_router_splits(tokens)) * tokens * num_experts * 4));
-  if ((flags & (B200MOE_LAYER_ROUTER | B200MOE_LAYER_COMPACT)) || ws.bm == 128) {
-    ws.q4 = take(tokens * (kH / 2));
-    ws.s4 = take(tokens * (kH / 32));
-  }
+  ws.q4 = take(tokens * (kH / 2));
+  ws.s4 = take(tokens * (kH / 32));
   if (flags & B200MOE_LAYER_SHARED) {
     ws.sh = carve_shared(nullptr, tokens);
     uint8_t* p = take(ws.sh.bytes);
@@ -238,7 +236,7 @@ static int run_layer(const LayerCall& c) {
   const int64_t stride_s = router ? tokens * ne : 0;
   const uint8_t *q4 = c.prep ? c.prep->codes4 : ws.q4, *s4 = c.prep ? c.prep->scales4 : ws.s4;
   const uint8_t* codes8 = c.prep ? c.prep->codes8 : ws.sh.x8;
-  bool have_q4 = true;
+  bool have_q4 = true, routed = c.prep != nullptr;  // the tokens are quantised / routed
   int r = 0;
   SideStream side(c.stream, c.side);
   // the operands: quantised rows and, with the router inside, the logits' split-K partials
@@ -256,15 +254,14 @@ static int run_layer(const LayerCall& c) {
     r = router_tc_quant(c.x, w->gate_split, tokens, ne, splits, ws.partials, ws.q4, ws.s4, shared ? ws.sh.x8 : nullptr, nullptr,
                         shared ? ws.sh.sfx8 : nullptr, ws.sh.bm, c.status, st);
     if (r) return r;
-  } else {
-    if (ws.bm == 128) {
-      r = shared ? quant_rows_both(c.x, tokens, ws.q4, ws.s4, ws.sh.x8, nullptr, ws.sh.sfx8, ws.sh.bm, st)
-                 : quant_rows(c.x, tokens, ws.q4, ws.s4, st);
-    } else {  // decode sizes with logits: the routed rows are quantised by the gather
-      have_q4 = false;
-      if (shared) r = b200moe_shared_quant(c.x, tokens, ws.sh.bm, ws.sh.x8, ws.sh.sfx8, st);
-    }
+  } else if (tokens > kSmallTokens) {  // logits given: the routing beside the quantisers
+    routed = true;
+    r = route_quant(c.logits, w->bias, tokens, ne, w->route_mode, w->route_scale, c.x, ws.w, ws.ids, ws.q4, ws.s4,
+                    shared ? ws.sh.x8 : nullptr, shared ? ws.sh.sfx8 : nullptr, ws.sh.bm, st);
     if (r) return r;
+  } else {  // a few tokens: the routed rows are quantised by the launch that routes and sorts
+    have_q4 = false;
+    if (shared && (r = b200moe_shared_quant(c.x, tokens, ws.sh.bm, ws.sh.x8, ws.sh.sfx8, st))) return r;
   }
   SharedPlan plan{};
   const SharedPlan* sp = nullptr;
@@ -292,9 +289,9 @@ static int run_layer(const LayerCall& c) {
                    have_q4 ? q4 : nullptr, have_q4 ? s4 : nullptr, ws.rows, ws.xq_sorted, ws.sfx, ws.done, n_done, st);
     if (r) return r;
   } else {
-    if (c.prep)
-      r = b200moe_permute(c.prep->topk_ids, c.prep->topk_weights, tokens, ne, ws.bm, ws.sorted_ids, ws.sorted_w,
-                          ws.block_expert, ws.num_valid, ws.scratch, st);
+    if (routed)
+      r = b200moe_permute(c.prep ? c.prep->topk_ids : ws.ids, c.prep ? c.prep->topk_weights : ws.w, tokens, ne, ws.bm, ws.sorted_ids,
+                          ws.sorted_w, ws.block_expert, ws.num_valid, ws.scratch, st);
     else
       r = b200moe_route_sort_partials(partials, ne, stride_s, splits, w->bias, tokens, ne, w->route_mode, w->route_scale, ws.bm,
                                       ws.w, ws.ids, ws.sorted_ids, ws.sorted_w, ws.block_expert, ws.num_valid, ws.scratch, st);

@@ -224,4 +224,56 @@ __device__ __forceinline__ void copy_row_to_atoms(const uint8_t* codes, const ui
   if (t < kH / 128) *reinterpret_cast<uint32_t*>(sdst + t * kAtomBytes) = __ldcg(reinterpret_cast<const uint32_t*>(scales) + t);
 }
 
+// 256 threads (t = 0..255, whole warps) quantise row `row` of x to row-major MXFP4 and (Q8) MXFP8; a thread's three 16-byte loads are
+// in flight together.
+template <bool Q8>
+__device__ __forceinline__ void quant_row(const uint4* x, int64_t row, int t, uint8_t* codes, uint8_t* scales, const QuantRow8& q8) {
+  constexpr int kIters = kH / 8 / 256;  // 3
+  const int lane = t & 31;
+  const uint4* src = x + row * (kH / 8);
+  uint32_t* dst = reinterpret_cast<uint32_t*>(codes + row * (kH / 2));
+  uint8_t* sdst = scales + row * (kH / 32);
+  uint4 raw[kIters];
+#pragma unroll
+  for (int it = 0; it < kIters; ++it) raw[it] = __ldcs(src + it * 256 + t);
+#pragma unroll
+  for (int it = 0; it < kIters; ++it) {
+    const int idx = it * 256 + t;
+    const uint32_t rr[4] = {raw[it].x, raw[it].y, raw[it].z, raw[it].w};
+    float v[8];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      v[2 * j] = __uint_as_float(rr[j] << 16);
+      v[2 * j + 1] = __uint_as_float(rr[j] & 0xffff0000u);
+    }
+    float amax = 0.0f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(v[j]));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+    const int e = quark_even_e8m0(amax);
+    const float inv = __uint_as_float(static_cast<uint32_t>(254 - e) << 23);  // 2^(127-e), exact
+    uint32_t packed = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) packed |= cvt_e2m1x2(v[2 * j] * inv, v[2 * j + 1] * inv) << (8 * j);
+    dst[idx] = packed;
+    // 4 lanes share a 32-element block; lanes 0 and 16 gather four neighbouring blocks' bytes into one 4-byte store
+    uint32_t sc = static_cast<uint32_t>(e);
+    sc |= __shfl_down_sync(0xffffffffu, sc, 4) << 8;
+    sc |= __shfl_down_sync(0xffffffffu, sc, 8) << 16;
+    if ((lane & 15) == 0) *reinterpret_cast<uint32_t*>(sdst + (idx >> 4) * 4) = sc;
+    if (Q8) {
+      const int e8 = mxfp8_scale(amax);
+      const float inv8 = __uint_as_float(static_cast<uint32_t>(254 - e8) << 23);  // e8 <= 247
+      reinterpret_cast<uint2*>(q8.codes + row * kH)[idx] =
+          make_uint2(cvt_e4m3x2(v[0] * inv8, v[1] * inv8) | (cvt_e4m3x2(v[2] * inv8, v[3] * inv8) << 16),
+                     cvt_e4m3x2(v[4] * inv8, v[5] * inv8) | (cvt_e4m3x2(v[6] * inv8, v[7] * inv8) << 16));
+      uint32_t s8 = static_cast<uint32_t>(e8);
+      s8 |= __shfl_down_sync(0xffffffffu, s8, 4) << 8;
+      s8 |= __shfl_down_sync(0xffffffffu, s8, 8) << 16;
+      if ((lane & 15) == 0) q8.store_scales(row, idx >> 4, s8);
+    }
+  }
+}
+
 }  // namespace b200moe
