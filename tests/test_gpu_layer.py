@@ -98,7 +98,7 @@ def test_routing_beside_the_quantiser(C, S, layer, m, mode):
     x[1], x[2, 5], x[3, 40:70] = 0, float("inf"), float("nan")
     lg[4], lg[5, 1:3] = float("nan"), lg[5, 0]
     bias = torch.linspace(-0.2, 0.2, EXPERTS, device="cuda") if mode == "sigmoid_bias" else None
-    w = replace(layer, shared_weights=None, correction_bias=bias, routing_mode=mode)
+    w = replace(layer, shared_weights=None, correction_bias=bias, routing_mode=mode, _abi=None)
     wt, ids = C.route(x, w, lg)
     want = staged_slots(C, C.mxfp4_quant(x), wt, ids, w)
     slots, shared = C.mxfp4_moe(x, w, return_partials=True, router_logits=lg)
