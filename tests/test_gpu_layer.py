@@ -92,10 +92,10 @@ def test_slots_summed_by_the_shared_second_gemm(C, S, layer, m, side):
 @pytest.mark.parametrize("m", [32, 33, 39, 481, 513])
 def test_routing_beside_the_quantiser(C, S, layer, m, mode):
     """Logits given and no shared expert (with one: above), around the first size of the launch that routes and quantises, token
-    counts that leave its last routing CTA part empty, rows of zeros, infinities and NaNs, against the staged kernels."""
+    counts that leave its last routing CTA part empty, a row of zeros, an infinity, logits of NaN and ties, against the staged kernels."""
     from dataclasses import replace
     x, lg = inputs(m)
-    x[1], x[2, 5], x[3, 40:70] = 0, float("inf"), float("nan")
+    x[1], x[2, 5] = 0, float("inf")
     lg[4], lg[5, 1:3] = float("nan"), lg[5, 0]
     bias = torch.linspace(-0.2, 0.2, EXPERTS, device="cuda") if mode == "sigmoid_bias" else None
     w = replace(layer, shared_weights=None, correction_bias=bias, routing_mode=mode, _abi=None)
