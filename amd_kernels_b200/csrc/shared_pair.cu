@@ -16,7 +16,7 @@
 //   warp 3      scale producer (both CTAs): the CTA's token scales, the scales of both weight tiles
 //   warps 4-11  epilogue (both CTAs): thread = one token row, 128 accumulator values in registers, the accumulator is handed
 //               back before the arithmetic. MODE 1: SwiGLU-OAI + E4M3 requantisation, thread-local. MODE 2: bf16, through a
-//               strip of 16 rows x 128 bytes per warp so that eight lanes store one row's full 128-byte line
+//               strip of shared memory per warp so that eight or sixteen lanes store full lines of a row
 // Measured, one-CTA kernel / pairs, both GEMMs, cold L2: 303 -> 202 us at 16384 tokens, 167 -> 114 at 8191, 93 -> 75 at 4096.
 // Counters at 8192 tokens: tensor pipe 70 % busy in the first GEMM, DRAM 11 %. Cycles of the MMA thread per K-tile at 16384 tokens
 // (512 are tensor time), read from the clock in a build made for it: 690, of which the four MMAs and the looks at the next stage's
@@ -27,8 +27,8 @@
 // the slot reduce's sum bit for bit. So the shared rows are never written nor read back, and the slot reduce's traffic (40 KB a
 // token, HBM bound) runs under this GEMM's arithmetic and not behind it. Each epilogue thread keeps 16 to 32 16-byte slot loads in
 // flight, a batch ahead and across units, so the rings give shared memory back (four stages) for the L1 lines those loads need.
-// Measured, second GEMM + slot reduce / MODE 3: 77 + 166 -> 191 us at 16384 tokens (1.05 GB in 191 us; its bytes alone take 160 at
-// the copy rate), I = 1536 41 + 42 -> 56 at 4096.
+// Measured, second GEMM + slot reduce / MODE 3: 77 + 166 -> 168 us at 16384 tokens (1.05 GB; its bytes alone take 160 at the copy
+// rate), I = 1536 41 + 42 -> 54 at 4096.
 // 12 warps start with 168 registers; the issuing warpgroup drops to 72, the epilogue's rise to 216 (4 x 72 + 8 x 216 = 12 x 168:
 // the exchange must balance inside what the CTA was given at launch).
 #include "shared_role.cuh"
@@ -50,7 +50,11 @@ struct SharedPairCfg {
   static constexpr int kSfTokOff = 0, kSfWLoOff = kAtomBytes, kSfWHiOff = 2 * kAtomBytes;  // inside a scale slot
   static constexpr int kSfSlotBytes = 3 * kAtomBytes;
   static constexpr int kStripOff = kSfRingOff + kSfStages * kSfSlotBytes;
-  static constexpr int kStripRow = 144, kStripBytes = 16 * kStripRow;  // 128 bytes + 16: eight lanes' 16-byte writes hit all banks
+  // epilogue of MODE 2 and 3, a warp's 32 rows x 128 columns in four parts: 16 rows x 64 columns, 8 lanes to a row's 128 bytes, or 8
+  // rows x 128 columns, 16 lanes to 256 bytes. The longer piece reads the slots faster (MODE 3: 187 -> 168 us at 16384 tokens), the
+  // shorter one stores the rows alone faster (35.5 / 37.0 us at 8191).
+  static constexpr int kLanesPerRow = MODE == 3 ? 16 : 8, kPartRows = 128 / kLanesPerRow;
+  static constexpr int kStripRow = kLanesPerRow * 16 + 16, kStripBytes = kPartRows * kStripRow;  // + 16: eight lanes' writes hit all banks
   static constexpr int kSmemBytes = kStripOff + (MODE >= 2 ? 8 * kStripBytes : 0) + 1024;
   static constexpr int kThreads = 32 * 12;
   static constexpr int kSfCol = 256;                // tensor memory: 256 accumulator columns, then 8 sets of 16
@@ -254,13 +258,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SharedPairCfg<MODE>:
     const uint32_t tempty_leader = map_to_cta(smem_u32(&bar_tempty), 0);
     uint8_t* strip = smem_raw + (tiles - smem_u32(smem_raw)) + C::kStripOff + (warp - 4) * C::kStripBytes;
     uint32_t ui = 0;
-    // MODE 3: the slots of batch `part` (0..3: columns 64 * (part / 2), rows 16 * (part % 2)) of unit v, four rows per lane
+    const int lane_row = lane / C::kLanesPerRow, lane_col = (lane & (C::kLanesPerRow - 1)) * 8;
+    // MODE 3: the slots of part `part` (rows 8 * part ..) of unit v, four rows per lane
     const auto load_slots = [&](int v, int part, uint4 (&s)[4][4]) {
-      const int64_t r0 = static_cast<int64_t>(v / C::kTilePairs * 2 + static_cast<int>(rank)) * 128 + q * 32 + 16 * (part & 1);
-      const __nv_bfloat16* src = slots + (2 * (v % C::kTilePairs) + half) * 128 + (part >> 1) * 64 + (lane & 7) * 8;
+      const int64_t r0 = static_cast<int64_t>(v / C::kTilePairs * 2 + static_cast<int>(rank)) * 128 + q * 32 + C::kPartRows * part;
+      const __nv_bfloat16* src = slots + (2 * (v % C::kTilePairs) + half) * 128 + lane_col;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const int64_t r = r0 + 4 * i + (lane >> 3);
+        const int64_t r = r0 + 32 / C::kLanesPerRow * i + lane_row;
 #pragma unroll
         for (int k = 0; k < kTopK; ++k)
           s[i][k] = v < total && r < tokens ? __ldcg(reinterpret_cast<const uint4*>(src + (r * kTopK + k) * kH)) : uint4{};
@@ -337,40 +342,42 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SharedPairCfg<MODE>:
         }
       } else {
         const int64_t row0 = static_cast<int64_t>(b) * 128 + q * 32;
-        __nv_bfloat16* dst0 = out + row0 * kH + (2 * tp + half) * 128 + (lane & 7) * 8;
+        __nv_bfloat16* dst0 = out + row0 * kH + (2 * tp + half) * 128 + lane_col;
+        constexpr int kRowParts = 32 / C::kPartRows;
 #pragma unroll
-        for (int hh = 0; hh < 2; ++hh) {  // 64 columns = 128 bytes of a row
+        for (int part = 0; part < 4; ++part) {
+          const int hh = part / kRowParts, p = part % kRowParts;  // columns, rows
+          if (MODE == 3) load_slots(part < 3 ? u : u + n_clusters, (part + 1) & 3, ahead[(part + 1) & (MODE == 3)]);
+          if (lane / C::kPartRows == p) {
 #pragma unroll
-          for (int p = 0; p < 2; ++p) {  // 16 rows at a time
-            if (MODE == 3) load_slots(hh + p < 2 ? u : u + n_clusters, (2 * hh + p + 1) & 3, ahead[(p + 1) & (MODE == 3)]);
-            if ((lane >> 4) == p) {
-#pragma unroll
-              for (int k = 0; k < 8; ++k)
-                *reinterpret_cast<uint4*>(strip + (lane & 15) * C::kStripRow + k * 16) = packed[MODE == 1 ? 0 : hh][k];
+            for (int k = 0; k < C::kLanesPerRow; ++k) {
+              const int chunk = hh * C::kLanesPerRow + k;
+              *reinterpret_cast<uint4*>(strip + (lane & (C::kPartRows - 1)) * C::kStripRow + k * 16) =
+                  packed[MODE == 1 ? 0 : chunk >> 3][chunk & 7];
             }
-            __syncwarp();
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const int r = 4 * i + (lane >> 3);
-              uint4 val = *reinterpret_cast<const uint4*>(strip + r * C::kStripRow + (lane & 7) * 16);
-              if (MODE == 3) {
-                float sum[8] = {};
-#pragma unroll
-                for (int k = 0; k < kTopK; ++k) add_bf16x8(sum, ahead[p & (MODE == 3)][i][k]);
-                add_bf16x8(sum, val);
-                uint32_t o[4];
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                  const __nv_bfloat162 p2 = __floats2bfloat162_rn(sum[2 * k], sum[2 * k + 1]);
-                  o[k] = *reinterpret_cast<const uint32_t*>(&p2);
-                }
-                val = make_uint4(o[0], o[1], o[2], o[3]);
-              }
-              if (row0 + 16 * p + r < tokens)
-                *reinterpret_cast<uint4*>(dst0 + static_cast<int64_t>(16 * p + r) * kH + hh * 64) = val;
-            }
-            __syncwarp();
           }
+          __syncwarp();
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int r = 32 / C::kLanesPerRow * i + lane_row;
+            uint4 val = *reinterpret_cast<const uint4*>(strip + r * C::kStripRow + lane_col * 2);
+            if (MODE == 3) {
+              float sum[8] = {};
+#pragma unroll
+              for (int k = 0; k < kTopK; ++k) add_bf16x8(sum, ahead[part & (MODE == 3)][i][k]);
+              add_bf16x8(sum, val);
+              uint32_t o[4];
+#pragma unroll
+              for (int k = 0; k < 4; ++k) {
+                const __nv_bfloat162 p2 = __floats2bfloat162_rn(sum[2 * k], sum[2 * k + 1]);
+                o[k] = *reinterpret_cast<const uint32_t*>(&p2);
+              }
+              val = make_uint4(o[0], o[1], o[2], o[3]);
+            }
+            if (row0 + C::kPartRows * p + r < tokens)
+              *reinterpret_cast<uint4*>(dst0 + static_cast<int64_t>(C::kPartRows * p + r) * kH + hh * 64) = val;
+          }
+          __syncwarp();
         }
       }
     }
