@@ -36,8 +36,6 @@ struct Workspace {
 int dispatch_rows_done(const uint8_t* codes, const uint8_t* scales, const int32_t* sorted_ids, const int32_t* num_valid,
                        int64_t tokens, int bm, int by_pair, int64_t max_rows, uint8_t* xq_sorted, uint8_t* sfx,
                        int32_t* done, int n_done, void* stream);
-int quant_dispatch_done(const void* x_bf16, const int32_t* sorted_ids, const int32_t* num_valid, int64_t tokens, int bm,
-                        int64_t max_rows, uint8_t* xq_sorted, uint8_t* sfx, int32_t* done, int n_done, void* stream);
 int prep_small(const float* partials, int64_t stride_t, int64_t stride_s, int splits, const float* bias, int64_t tokens,
                int num_experts, int mode, float scale, int bm, float* out_w, int32_t* out_ids, int32_t* sorted_ids,
                float* sorted_w, int32_t* block_expert, int32_t* num_valid, const void* x_bf16, const uint8_t* q4,
@@ -297,10 +295,7 @@ static int run_layer(const LayerCall& c) {
                                       ws.w, ws.ids, ws.sorted_ids, ws.sorted_w, ws.block_expert, ws.num_valid, ws.scratch, st);
     if (r) return r;
     if (ws.bm < 128) {
-      r = have_q4 ? dispatch_rows_done(q4, s4, ws.sorted_ids, ws.num_valid, tokens, ws.bm, 0, ws.rows, ws.xq_sorted, ws.sfx,
-                                       ws.done, n_done, st)
-                  : quant_dispatch_done(c.x, ws.sorted_ids, ws.num_valid, tokens, ws.bm, ws.rows, ws.xq_sorted, ws.sfx, ws.done,
-                                        n_done, st);
+      r = dispatch_rows_done(q4, s4, ws.sorted_ids, ws.num_valid, tokens, ws.bm, 0, ws.rows, ws.xq_sorted, ws.sfx, ws.done, n_done, st);
       if (r) return r;
     }
   }

@@ -295,10 +295,10 @@ extern "C" int b200moe_dispatch_rows(const uint8_t* codes, const uint8_t* scales
                                      nullptr, 0, stream);
 }
 
-namespace b200moe {
-// b200moe_quant_dispatch zeroing `n_done` counts (the grid has 256 threads per sorted row, more than counts)
-int quant_dispatch_done(const void* x_bf16, const int32_t* sorted_ids, const int32_t* num_valid, int64_t tokens, int bm,
-                        int64_t max_rows, uint8_t* xq_sorted, uint8_t* sfx, int32_t* done, int n_done, void* stream) {
+extern "C" int b200moe_quant_dispatch(const void* x_bf16, const int32_t* sorted_ids, const int32_t* num_valid,
+                                      int64_t tokens, int bm, int64_t max_rows, uint8_t* xq_sorted, uint8_t* sfx,
+                                      int32_t* done, void* stream) {
+  using namespace b200moe;
   if (!x_bf16 || !sorted_ids || !num_valid || !xq_sorted || !sfx || tokens < 0 || max_rows < 0) return B200MOE_E_ARG;
   const int shift = bm == 16 ? 4 : bm == 32 ? 5 : bm == 64 ? 6 : bm == 128 ? 7 : -1;
   if (shift < 0) return B200MOE_E_ARG;
@@ -307,14 +307,7 @@ int quant_dispatch_done(const void* x_bf16, const int32_t* sorted_ids, const int
     return B200MOE_E_ALIGN;
   if (max_rows == 0) return 0;
   B200MOE_LAUNCH(quant_dispatch_kernel, static_cast<unsigned>(max_rows), 256, 0, static_cast<cudaStream_t>(stream),
-                 static_cast<const uint4*>(x_bf16), sorted_ids, num_valid, tokens, shift, xq_sorted, sfx, done, n_done);
+                 static_cast<const uint4*>(x_bf16), sorted_ids, num_valid, tokens, shift, xq_sorted, sfx, done,
+                 static_cast<int>(max_rows / bm));
   return 0;
-}
-}  // namespace b200moe
-
-extern "C" int b200moe_quant_dispatch(const void* x_bf16, const int32_t* sorted_ids, const int32_t* num_valid,
-                                      int64_t tokens, int bm, int64_t max_rows, uint8_t* xq_sorted, uint8_t* sfx,
-                                      int32_t* done, void* stream) {
-  return b200moe::quant_dispatch_done(x_bf16, sorted_ids, num_valid, tokens, bm, max_rows, xq_sorted, sfx, done,
-                                      bm > 0 ? static_cast<int>(max_rows / bm) : 0, stream);
 }
