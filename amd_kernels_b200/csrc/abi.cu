@@ -215,6 +215,10 @@ static int run_layer(const LayerCall& c) {
   // (the rebuild of a compact input checks its own operands: 8 bytes for the FP8 codes)
   if (c.prep && ((reinterpret_cast<uintptr_t>(c.prep->codes4) | (shared ? reinterpret_cast<uintptr_t>(c.prep->codes8) : 0)) & 15))
     return B200MOE_E_ALIGN;
+  // the last launch reads the slots and writes `out` 16 bytes at a time, whichever kernel it is (the slot reduce or the shared expert's
+  // second GEMM); GEMM2 writes the slots in pieces of 16 bytes from blocks of 128 rows, of 8 bytes from smaller ones
+  const uintptr_t slot_bytes = c.out || b200moe_block_rows(c.tokens) == 128 ? 16 : 8;
+  if ((reinterpret_cast<uintptr_t>(c.out) & 15) || (reinterpret_cast<uintptr_t>(c.slots) & (slot_bytes - 1))) return B200MOE_E_ALIGN;
   const int ne = w->num_experts;
   const int64_t tokens = c.tokens;
   void* st = c.stream;

@@ -210,6 +210,32 @@ def test_c_abi_refuses_shared_weights_of_another_intermediate_size(inter):
                                           one, None, None) == want
 
 
+@pytest.mark.parametrize("tokens", [1, 512, 513, 2176, 2177, 16384])
+def test_c_abi_refuses_misaligned_results_at_every_size(tokens):
+    """Whichever kernel ends the call: the same answer on both sides of 18 blocks of 128 tokens, and before anything is launched.
+    (A workspace of 0 bytes ends the accepted calls there.)"""
+    lib = _lib.load()
+    at = ctypes.c_void_p
+    w = _lib.Weights(256, 256, None, 128, _lib.ROUTE_SOFTMAX, 1.0, None, None)
+    sw = _lib.SharedWeights(256, 256, 768)
+    prep = _lib.Prepared(256, 256, 256, 256, 256, 256, None)
+
+    def calls(slots, shared_out, out, shared=True):
+        s = ctypes.byref(sw) if shared else None
+        p = [None if a is None else at(a) for a in (slots, shared_out, out)]
+        yield lib.b200moe_layer(ctypes.byref(w), s, at(256), at(256), tokens, at(256), 0, *p, at(256), None, None)
+        yield lib.b200moe_layer_prepared(ctypes.byref(w), s, ctypes.byref(prep), tokens, at(256), 0, *p, at(256), None, None)
+
+    for off in (2, 4, 8):
+        for refused in ((None, None, 256 + off), (256, None, 256 + off), (256 + off, None, 256), (256, 256, 256 + off)):
+            assert all(r == _lib.E_ALIGN for r in calls(*refused)), refused
+            assert all(r == _lib.E_ALIGN for r in calls(refused[0], None, refused[2], shared=False)), refused
+        # slots alone: 8 bytes are enough in blocks of up to 32 rows
+        want = _lib.E_ARG if off == 8 and tokens <= 512 else _lib.E_ALIGN
+        assert all(r == want for r in calls(256 + off, 256, None))
+    assert all(r == _lib.E_ARG for r in calls(256, 256, 256))
+
+
 class _Recorder(_NoLaunch):
     """The library handle's stand-in that accepts the whole-layer calls and keeps the weights struct they were given."""
     def __init__(self, real):
