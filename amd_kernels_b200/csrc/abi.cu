@@ -209,6 +209,8 @@ static int run_layer(const LayerCall& c) {
                  ((shared || compact) && (!c.prep->codes8 || !c.prep->scales8))))
     return B200MOE_E_ARG;
   if (reinterpret_cast<uintptr_t>(c.workspace) & 255) return B200MOE_E_ALIGN;
+  // (with the router inside, its GEMM takes any row address below 128 tokens and says what it needs above)
+  if (c.x && c.logits && (reinterpret_cast<uintptr_t>(c.x) & 15)) return B200MOE_E_ALIGN;
   if (shared && ((reinterpret_cast<uintptr_t>(c.shared->w13t) | reinterpret_cast<uintptr_t>(c.shared->w2t) |
                   reinterpret_cast<uintptr_t>(c.shared_out)) & 15))
     return B200MOE_E_ALIGN;

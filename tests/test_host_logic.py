@@ -236,6 +236,19 @@ def test_c_abi_refuses_misaligned_results_at_every_size(tokens):
     assert all(r == _lib.E_ARG for r in calls(256, 256, 256))
 
 
+@pytest.mark.parametrize("shared", [False, True])
+@pytest.mark.parametrize("tokens", [1, 32, 33, 513])
+def test_c_abi_refuses_misaligned_rows_with_logits(tokens, shared):
+    """The quantisers read 16 bytes at a time in every form; up to 32 tokens without a shared expert nobody looked."""
+    lib = _lib.load()
+    at = ctypes.c_void_p
+    w = _lib.Weights(256, 256, None, 128, _lib.ROUTE_SOFTMAX, 1.0, None, None)
+    sw = ctypes.byref(_lib.SharedWeights(256, 256, 768)) if shared else None
+    for off, want in ((2, _lib.E_ALIGN), (8, _lib.E_ALIGN), (16, _lib.E_ARG)):  # (0 bytes of workspace end the accepted call)
+        assert lib.b200moe_layer(ctypes.byref(w), sw, at(256 + off), at(256), tokens, at(256), 0, at(256), at(256), at(256), at(256),
+                                 None, None) == want
+
+
 class _Recorder(_NoLaunch):
     """The library handle's stand-in that accepts the whole-layer calls and keeps the weights struct they were given."""
     def __init__(self, real):
