@@ -19,14 +19,14 @@ struct Workspace {
   uint8_t* hq;            // [R][384]
   uint8_t* sfh;           // [R/bm][6][512]
   int32_t* done;          // [R/bm] GEMM1 tiles finished per row block, then [kSharedDone]: the shared expert's
-  // only with the router inside the call:
-  float* partials;        // [S][T][E] split-K logit partials
-  uint8_t* q4;            // [T][3072] row-major MXFP4 codes of x (also rebuilt from a compact prepared input)
-  uint8_t* s4;            // [T][192] their scales
+  float* partials;        // [S][T][E] split-K logit partials; only with the router inside the call
+  uint8_t* q4;            // [T][3072] row-major MXFP4 codes of x or rebuilt from a compact input; not where up to 32 tokens with
+  uint8_t* s4;            // [T][192] their scales                        logits are quantised on the way into sorted order
   // only with the shared expert:
   SharedWorkspace sh;
+  bool sum_in_gemm2;          // nobody takes the shared rows: the shared expert's second GEMM sums the slots (shared_pair.cu, MODE 3)
   // results the caller does not take:
-  __nv_bfloat16* shared_out;  // [T][6144]
+  __nv_bfloat16* shared_out;  // [T][6144]; not with sum_in_gemm2
   __nv_bfloat16* slots;       // [T][4][6144]
   size_t bytes;
   int bm;
@@ -71,6 +71,8 @@ int set_wait_limit_pair(unsigned long long ns);
 int set_wait_limit_router(unsigned long long ns);
 int set_wait_limit_ep_sync(unsigned long long ns);
 
+constexpr int64_t kSmallTokens = 32;  // up to here routing, sort and gather are one launch
+
 static Workspace carve(uint8_t* base, int64_t tokens, int num_experts, int flags) {
   Workspace ws{};
   ws.bm = b200moe_block_rows(tokens);
@@ -98,13 +100,18 @@ static Workspace carve(uint8_t* base, int64_t tokens, int num_experts, int flags
   ws.done = reinterpret_cast<int32_t*>(take((blocks + kSharedDone) * 4));
   if (flags & B200MOE_LAYER_ROUTER)
     ws.partials = reinterpret_cast<float*>(take(static_cast<size_t>(b200moe_router_splits(tokens)) * tokens * num_experts * 4));
-  ws.q4 = take(tokens * (kH / 2));
-  ws.s4 = take(tokens * (kH / 32));
+  if ((flags & (B200MOE_LAYER_ROUTER | B200MOE_LAYER_COMPACT)) || tokens > kSmallTokens) {
+    ws.q4 = take(tokens * (kH / 2));
+    ws.s4 = take(tokens * (kH / 32));
+  }
   if (flags & B200MOE_LAYER_SHARED) {
     ws.sh = carve_shared(nullptr, tokens);
     uint8_t* p = take(ws.sh.bytes);
     if (p) ws.sh = carve_shared(p, tokens);
-    if (flags & B200MOE_LAYER_OWN_SHARED_OUT) ws.shared_out = reinterpret_cast<__nv_bfloat16*>(take(tokens * kH * 2));
+    if (flags & B200MOE_LAYER_OWN_SHARED_OUT) {
+      ws.sum_in_gemm2 = ws.bm == 128 && shared_sums_slots(ws.sh);
+      if (!ws.sum_in_gemm2) ws.shared_out = reinterpret_cast<__nv_bfloat16*>(take(tokens * kH * 2));
+    }
   }
   if (flags & B200MOE_LAYER_OWN_SLOTS) ws.slots = reinterpret_cast<__nv_bfloat16*>(take(tokens * kTopK * kH * 2));
   ws.bytes = off;
@@ -141,7 +148,6 @@ extern "C" int b200moe_set_wait_limit_ns(uint64_t ns) {
 }
 
 namespace b200moe {
-constexpr int64_t kSmallTokens = 32;  // up to here routing, sort and gather are one launch
 // Both grouped GEMMs in one persistent launch: up to 32 tokens, and with I = 1536 wherever the row blocks have 16 rows (up to 480).
 // Measured, whole layer, two launches / one, us: I = 1536 287 / 255 at 64 tokens, 330 / 294 at 128, 355 / 318 at 400 (router and
 // shared expert inside: 318 / 298, 342 / 321, 385 / 367): 24 W13 tiles of an expert leave more of an unfinished last round, and
@@ -269,8 +275,6 @@ static int run_layer(const LayerCall& c) {
   }
   SharedPlan plan{};
   const SharedPlan* sp = nullptr;
-  // where nobody takes the shared rows, the shared expert's second GEMM sums the slots (shared_pair.cu, MODE 3)
-  const bool sum_in_gemm2 = shared && c.out && !c.shared_out && ws.bm == 128 && shared_sums_slots(ws.sh);
   if (shared) {
     if (ws.bm < 128) {  // decode sizes: a role of the launch that streams the routed experts' W13
       if ((r = shared_plan(&plan, c.shared->w13t, c.shared->w2t, codes8, tokens, ws.sh, shared_out, tokens, ws.done + blocks,
@@ -281,7 +285,7 @@ static int run_layer(const LayerCall& c) {
       if (c.side && (r = side.fork())) return r;
       void* sst = c.side ? c.side : st;
       r = shared_gemm1(c.shared->w13t, codes8, tokens, ws.sh, tokens, c.status, sst);
-      if (!r && !sum_in_gemm2) r = shared_gemm2(c.shared->w2t, ws.sh, nullptr, shared_out, tokens, c.status, sst);
+      if (!r && !ws.sum_in_gemm2) r = shared_gemm2(c.shared->w2t, ws.sh, nullptr, shared_out, tokens, c.status, sst);
       if (r) return r;
     }
   }
@@ -324,7 +328,7 @@ static int run_layer(const LayerCall& c) {
       return r;
   }
   if ((r = side.join())) return r;
-  if (sum_in_gemm2) return shared_gemm2(c.shared->w2t, ws.sh, slots, c.out, tokens, c.status, st);
+  if (ws.sum_in_gemm2) return shared_gemm2(c.shared->w2t, ws.sh, slots, c.out, tokens, c.status, st);
   if (c.out && (r = b200moe_reduce_slots(slots, shared ? shared_out : nullptr, tokens, c.out, st))) return r;
   return 0;
 }

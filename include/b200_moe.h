@@ -414,8 +414,8 @@ int b200moe_forward_x(const b200moe_weights* w, const void* x_bf16, int64_t toke
  * runs inside the call (w->gate). shared may be null.
  * slots [T][4][6144], shared_out [T][6144] and out [T][6144] are bf16; a null slots (shared_out) means that the caller does
  * not want it: it then lives in the workspace, and out must be given. Same bits as the separate calls.
- * workspace: b200moe_layer_workspace_bytes(T, num_experts, flags) bytes, 256-byte aligned; flags: the sum of those below that
- * hold for the call. */
+ * workspace: b200moe_layer_workspace_bytes(T, num_experts, flags) bytes, 256-byte aligned, asked for on the device of the call;
+ * flags: the sum of those below that hold for the call. */
 typedef struct b200moe_shared_weights {
   const uint8_t* w13t; /* b200moe_preshuffle_shared */
   const uint8_t* w2t;

@@ -145,3 +145,11 @@ def test_layer_inside_a_dual_batch_microbatch(C, S, layer, m):
         S.set_dbo_query(None)
     torch.cuda.synchronize()
     assert C.last_status() == 0
+
+
+def test_workspace_has_no_shared_rows_where_the_slots_are_summed_in_the_second_gemm(layer):
+    from amd_kernels_b200 import _lib
+    lib = layer.lib()
+    for m in (513, 2176, 2177, 16384):
+        kept, own = (lib.b200moe_layer_workspace_bytes(m, EXPERTS, _lib.LAYER_SHARED | f) for f in (0, _lib.LAYER_OWN_SHARED_OUT))
+        assert own - kept == (0 if m > 2176 else -(-m * 2 * H // 1024) * 1024)

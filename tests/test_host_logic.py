@@ -50,6 +50,18 @@ def test_sizes_match_oracle_and_reference_bounds():
     assert lib.b200moe_permute_scratch_bytes(256, 128) == 0 and lib.b200moe_permute_scratch_bytes(257, 128) == 2 * 128 * 4
 
 
+def test_workspace_holds_the_quantised_rows_where_something_writes_them():
+    """(The rest of the layout is that of the call without the flag.) Up to 32 tokens with logits the rows are quantised on their
+    way into sorted order; a compact input is expanded into the workspace at every size."""
+    lib = _lib.load()
+    for tokens in (1, 32, 33, 512, 513):
+        full, compact = (lib.b200moe_layer_workspace_bytes(tokens, 128, f) for f in (0, _lib.LAYER_COMPACT))
+        if tokens <= 32:
+            assert tokens * 3264 <= compact - full <= tokens * 3264 + 2048
+        else:
+            assert compact == full
+
+
 def test_dispatch_range():
     # the reference's variant_for: 1..87381, ValueError outside (tests/moe/.../test_entry.py:107-114)
     for m in (1, 8, 512, 513, 4097, 87381):
