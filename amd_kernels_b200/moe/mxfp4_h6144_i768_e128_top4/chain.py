@@ -680,7 +680,9 @@ def set_wait_limit_ns(ns: int) -> None:
             _lib.check(_lib.load(inter).b200moe_set_wait_limit_ns(int(ns)), "set_wait_limit_ns")
 
 
-WARM_UP_TOKENS = (1, 64, 481, 513, 5000)  # one-launch GEMMs, one size per block height the entry uses
+# The one-launch GEMMs, one size per block height of the entry, the router GEMM that does not quantise (128 to 256 tokens), the shared
+# expert's CTA pairs without and with the slot sum (1409, 2177 tokens on).
+WARM_UP_TOKENS = (1, 64, 200, 481, 513, 1600, 5000)
 
 
 def warm_up_mxfp4_moe(w, *, partials=False, workers=None):

@@ -153,3 +153,32 @@ def test_workspace_has_no_shared_rows_where_the_slots_are_summed_in_the_second_g
     for m in (513, 2176, 2177, 16384):
         kept, own = (lib.b200moe_layer_workspace_bytes(m, EXPERTS, _lib.LAYER_SHARED | f) for f in (0, _lib.LAYER_OWN_SHARED_OUT))
         assert own - kept == (0 if m > 2176 else -(-m * 2 * H // 1024) * 1024)
+
+
+def launched(calls):
+    """The kernels of the library that ``calls`` launches, by name and template arguments."""
+    from torch.profiler import ProfilerActivity, profile
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        calls()
+        torch.cuda.synchronize()
+    return {e.key for e in prof.key_averages() if "b200moe" in e.key}
+
+
+@pytest.mark.parametrize("partials", [False, True])
+def test_warm_up_runs_every_kernel_of_the_served_calls(C, layer, partials):
+    """Every rule that chooses a kernel by the token count, on both sides of its line: what a call launches, warm-up has launched."""
+    sizes = [1, 16, 17, 32, 33, 64, 65, 127, 128, 200, 256, 257, 480, 481, 512, 513, 777, 1024, 1025, 1408, 1409, 2048, 2049, 2176, 2177,
+             3000, 4500, 6000, 9000]
+
+    def calls():
+        for m in sizes:
+            x, lg = inputs(m)
+            for logits in (lg, None):
+                C.mxfp4_moe(x, layer, router_logits=logits)
+                if partials:
+                    C.mxfp4_moe(x, layer, router_logits=logits, return_partials=True)
+    warm = launched(lambda: C.warm_up_mxfp4_moe(layer, partials=partials))
+    if not warm:
+        pytest.skip("no kernel trace here: another program holds the profiling interface")
+    assert len(warm) > 10 and launched(calls) <= warm
