@@ -92,24 +92,26 @@ def test_slots_summed_by_the_shared_second_gemm(C, S, layer, m, side):
 @pytest.mark.parametrize("m", [32, 33, 39, 481, 513])
 def test_routing_beside_the_quantiser(C, S, layer, m, mode):
     """Logits given and no shared expert (with one: above), around the first size of the launch that routes and quantises, token
-    counts that leave its last routing CTA part empty, a row of zeros, an infinity, logits of NaN and ties, against the staged kernels."""
+    counts that leave its last routing CTA part empty, a row of zeros, an infinity, a NaN, logits of NaN and ties, against the staged
+    kernels. (The staged quantiser gives a NaN another code below 64 rows, so it gets 64.)"""
     from dataclasses import replace
     x, lg = inputs(m)
-    x[1], x[2, 5] = 0, float("inf")
+    x[1], x[2, 5], x[3, 40:70] = 0, float("inf"), float("nan")
     lg[4], lg[5, 1:3] = float("nan"), lg[5, 0]
     bias = torch.linspace(-0.2, 0.2, EXPERTS, device="cuda") if mode == "sigmoid_bias" else None
     w = replace(layer, shared_weights=None, correction_bias=bias, routing_mode=mode, _abi=None)
     wt, ids = C.route(x, w, lg)
-    want = staged_slots(C, C.mxfp4_quant(x), wt, ids, w)
+    padded = torch.cat([x, torch.zeros((max(0, 64 - m), H), dtype=x.dtype, device="cuda")])
+    want = staged_slots(C, tuple(t[:m].contiguous() for t in C.mxfp4_quant(padded)), wt, ids, w)
     slots, shared = C.mxfp4_moe(x, w, return_partials=True, router_logits=lg)
     torch.cuda.synchronize()
     assert shared is None and torch.equal(slots.view(torch.int16), want.view(torch.int16)) and C.last_status() == 0
 
 
-@pytest.mark.parametrize("m", [1, 40, 512, 700, 1600])
+@pytest.mark.parametrize("m", [1, 40, 512, 700, 1600, 2305])
 def test_layer_in_a_graph(C, S, layer, m):
-    """Capture and replay, the role and (above 512 tokens) the fork to the side stream and its join included: replayed into a
-    poisoned result, and again with other tokens in the same buffers."""
+    """Capture and replay, the role and (above 512 tokens) the fork to the side stream and its join included, at 2305 in front of the
+    second shared GEMM that sums the slots: replayed into a poisoned result, and again with other tokens in the same buffers."""
     x, lg = inputs(m)
     C.mxfp4_moe(x, layer, router_logits=lg)
     torch.cuda.synchronize()

@@ -64,7 +64,7 @@ def test_sidecar_kernels_match_golden_and_oracle(P):
     assert torch.equal(compact.expand().routed_codes, q4)
 
 
-@pytest.mark.parametrize("m", [1, 5, 48, 300, 1600])
+@pytest.mark.parametrize("m", [1, 5, 48, 300, 1600, 2305])
 def test_prepared_and_compact_inputs_give_the_entry_bits(P, full_layer, m):
     C, S, w = full_layer
     x = rows(m, 20 + m).cuda()
