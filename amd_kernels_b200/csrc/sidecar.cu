@@ -36,9 +36,14 @@ __device__ __forceinline__ float inverse_ratio(const uint8_t* s4, const uint8_t*
   return __uint_as_float(static_cast<uint32_t>(min(max(d, -126), 127) + 127) << 23);  // 2^(s8 - s4), exact
 }
 
-// One thread = one 32-value block = one mask word: 32 FP8 codes, 16 bytes of FP4 codes, both scale bytes, read once per block. (One
-// thread per 8 values, a byte of mask each: 9.4 and 13.7 us at 2048 tokens; 32 values: 6.3 and, with the scale atoms that were a launch of 3.4 us of their own, 11.4.) A block's FP8 codes are read as two or four
-// vectors, so that operands aligned to 8 bytes only are taken as before (`wide` false).
+// One thread = one 32-value block = one mask word: 32 FP8 codes, 16 bytes of FP4 codes, both scale bytes, read once per block. One
+// thread per 8 values, with a byte of mask each, took 9.4 and 13.7 us at 2048 tokens; 32 values take 6.3 and 11.4, in which the scale
+// atoms, once a launch of 3.4 us of their own, are included. A block's FP8 codes are read as two or four vectors, so that operands
+// aligned to 8 bytes only are taken as before (`wide` false).
+// Neither kernel launches its successor early: with 32 values to a thread their CTAs are all resident up to about 1500 tokens, the
+// launches behind them followed at once, and at decode sizes GEMM1's first requests for weights ran beside the unpack and the gather,
+// whose loads queue behind them (unpack 7.3 us at 400 tokens instead of 4.0). The prepared call, launch early / behind, us: 192.9 / 188.0
+// at 257 tokens, 223.8 / 217.2 at 400, 253.1 / 246.6 at 480, 214.3 / 209.2 at 512, 231.9 / 226.6 at 777, 293.0 / 290.0 at 2048.
 __device__ __forceinline__ void load_codes8(const uint8_t* q8, uint32_t block, bool wide, uint2 (&v)[4]) {
   if (wide) {
     const uint4* p = reinterpret_cast<const uint4*>(q8) + 2 * static_cast<int64_t>(block);
@@ -56,7 +61,8 @@ __device__ __forceinline__ void load_codes8(const uint8_t* q8, uint32_t block, b
 __global__ void __launch_bounds__(256) sidecar_pack_kernel(const uint8_t* __restrict__ q4, const uint8_t* __restrict__ s4,
                                                            const uint8_t* __restrict__ q8, const uint8_t* __restrict__ s8,
                                                            uint32_t n_blocks, bool wide, uint32_t* __restrict__ mask) {
-  pdl_enter(q4, s4, q8, s8);
+  pdl_wait();
+  launder(q4), launder(s4), launder(q8), launder(s8);
   const uint32_t i = blockIdx.x * 256 + threadIdx.x;
   if (i >= n_blocks) return;
   uint2 v8[4];
@@ -87,7 +93,8 @@ __global__ void __launch_bounds__(256) sidecar_unpack_kernel(const uint32_t* __r
                                                              const uint8_t* __restrict__ q8, const uint8_t* __restrict__ s8,
                                                              uint32_t n_blocks, bool wide, uint2* __restrict__ q4,
                                                              uint8_t* __restrict__ atoms, int atom_shift) {
-  pdl_enter(mask, s4, q8, s8);
+  pdl_wait();
+  launder(mask), launder(s4), launder(q8), launder(s8);
   const uint32_t i = blockIdx.x * 256 + threadIdx.x;
   if (i >= n_blocks) return;
   if (atoms != nullptr && (i & 3u) == 0u) {
