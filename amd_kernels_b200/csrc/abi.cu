@@ -41,6 +41,8 @@ int prep_small(const float* partials, int64_t stride_t, int64_t stride_s, int sp
                float* sorted_w, int32_t* block_expert, int32_t* num_valid, const void* x_bf16, const uint8_t* q4,
                const uint8_t* s4, int64_t max_rows, uint8_t* xq_sorted, uint8_t* sfx, int32_t* done, int n_done,
                void* stream);
+int quant_rows_both(const void* x_bf16, int64_t tokens, uint8_t* codes, uint8_t* scales, uint8_t* codes8, uint8_t* scales8,
+                    uint8_t* atoms8, int bm8, void* stream);
 int route_quant(const float* logits, const float* bias, int64_t tokens, int num_experts, int mode, float scale, const void* x_bf16,
                 float* out_w, int32_t* out_ids, uint8_t* codes4, uint8_t* scales4, uint8_t* codes8, uint8_t* atoms8, int bm8,
                 void* stream);
@@ -203,6 +205,24 @@ class SideStream {
   bool forked_ = false;
 };
 
+// Logits given and a shared expert on the side stream: where the routing stays a launch of its own behind the quantisers. The
+// side stream starts when x is quantised, and its first GEMM takes every SM, as GEMM1 does: whichever is there first, the other
+// waits. With a routing launch in front of the sort the shared GEMM is first and hides the routing and the sort; without
+// (route_quant) the early launches of the chain put GEMM1 first, and the shared GEMMs run against its tail and GEMM2's. That is
+// the better order again where GEMM2 and the shared rows are stored side by side, from 18 blocks of 128 tokens on, and where the
+// slots are summed from 44 on. Measured, the layer with logits, one launch / two, us: I = 768 reduced 231 / 236 at 1152 tokens,
+// 233 / 235 at 1153, 246 / 236 at 1183, 248 / 243 at 1408, 260 / 252 at 1800, 274 / 265 at 2176, (the exception:) 269 / 277 at
+// 2200, 278 / 267 at 2304, 279 / 263 at 2560, 292 / 288 at 3072, 437 / 427 at 5120, 461 / 456 at 5632, 477 / 487 at 5900, 826 /
+// 855 at 12288, 1075 / 1095 at 16384; slots handed out 237 / 240 at 1152, 252 / 242 at 1183, 273 / 261 at 1800, 303 / 286 at
+// 2240, 299 / 278 at 2280, 304 / 302 at 2299, 321 / 326 at 3072, 383 / 403 at 4096, 1174 / 1242 at 16384. I = 1536 reduced 414 /
+// 400 at 1280, 453 / 437 at 2176, 486 / 476 at 3072; slots handed out 435 / 410 at 1280, 500 / 483 at 2240, 494 / 501 at 2299,
+// 574 / 594 at 3328.
+constexpr int64_t kRouteBehindFrom = 9 * 128 + 1, kRouteBehindToStored = 18 * 128, kRouteBehindToSummed = 44 * 128;
+static bool routes_behind_quant(const LayerCall& c, const Workspace& ws) {
+  return c.x && c.logits && c.shared && c.side && c.tokens >= kRouteBehindFrom &&
+         c.tokens <= (ws.sum_in_gemm2 ? kRouteBehindToSummed : kRouteBehindToStored);
+}
+
 static int run_layer(const LayerCall& c) {
   const b200moe_weights* w = c.w;
   if (!w || !c.workspace || !c.status || (!c.x == !c.prep) || (!c.slots && !c.out)) return B200MOE_E_ARG;
@@ -263,6 +283,9 @@ static int run_layer(const LayerCall& c) {
   } else if (router) {  // the same from 128 tokens on, the logits on the tensor cores
     r = router_tc_quant(c.x, w->gate_split, tokens, ne, splits, ws.partials, ws.q4, ws.s4, shared ? ws.sh.x8 : nullptr, nullptr,
                         shared ? ws.sh.sfx8 : nullptr, ws.sh.bm, c.status, st);
+    if (r) return r;
+  } else if (routes_behind_quant(c, ws)) {
+    r = quant_rows_both(c.x, tokens, ws.q4, ws.s4, ws.sh.x8, nullptr, ws.sh.sfx8, ws.sh.bm, st);
     if (r) return r;
   } else if (tokens > kSmallTokens) {  // logits given: the routing beside the quantisers
     routed = true;

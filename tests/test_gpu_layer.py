@@ -108,6 +108,21 @@ def test_routing_beside_the_quantiser(C, S, layer, m, mode):
     assert shared is None and torch.equal(slots.view(torch.int16), want.view(torch.int16)) and C.last_status() == 0
 
 
+@pytest.mark.parametrize("m", [1152, 1153, 2304, 2305, 5632, 5633])
+def test_routing_behind_or_beside_the_quantisers_with_a_shared_expert(C, S, layer, m):
+    """Around the sizes between which the routing is a launch of its own; without a side stream it never is."""
+    x, lg = inputs(m)
+    results = []
+    for dbo in (None, lambda: True):
+        S.set_dbo_query(dbo)
+        try:
+            results.append((C.mxfp4_moe(x, layer, router_logits=lg), *C.mxfp4_moe(x, layer, router_logits=lg, return_partials=True)))
+        finally:
+            S.set_dbo_query(None)
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(*results)) and C.last_status() == 0
+
+
 @pytest.mark.parametrize("m", [1, 40, 512, 700, 1600, 2305])
 def test_layer_in_a_graph(C, S, layer, m):
     """Capture and replay, the role and (above 512 tokens) the fork to the side stream and its join included, at 2305 in front of the
