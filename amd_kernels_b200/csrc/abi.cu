@@ -169,7 +169,8 @@ struct LayerCall {
   void *slots, *shared_out, *out;
   int32_t* status;
   void* stream;
-  void* side;  // may be null: another stream of the device, for the shared expert's two GEMMs above 512 tokens
+  void* side;  // may be null: another stream of the device, for the shared expert's GEMMs above 512 tokens (the first only, where
+               // the second sums the slots behind GEMM2)
 };
 
 // The side stream's part of a call: starts behind what the main stream holds at fork() and is joined by join(), at the latest when

@@ -125,7 +125,8 @@ __device__ __forceinline__ uint32_t cvt_e4m3x2(float lo, float hi) {
 }
 
 // two E2M1 codes in one byte: `lo` in the low nibble, `hi` in the high nibble; round to nearest even, saturating.
-// Same codes as e2m1_code on a value already divided by the block scale (ties go to the even code, -0 keeps its sign).
+// Same codes as e2m1_code on a value already divided by the block scale (ties go to the even code, -0 keeps its sign), except that a
+// NaN becomes +6, the largest, where e2m1_code gives it a signed zero.
 __device__ __forceinline__ uint32_t cvt_e2m1x2(float lo, float hi) {
   uint16_t out;
   asm("{\n.reg .b8 t;\ncvt.rn.satfinite.e2m1x2.f32 t, %1, %2;\ncvt.u16.u8 %0, t;\n}\n" : "=h"(out) : "f"(hi), "f"(lo));

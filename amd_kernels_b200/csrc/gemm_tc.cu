@@ -13,9 +13,9 @@
 //             doing both was what bounded the kernel
 //             Where a unit's chain of K-tiles bounds the launch (the one-launch kernel, the shared expert's role, 128-row blocks) both
 //             run their loops as whole warps and elect a lane around the instructions, which costs less per K-tile than a loop of
-//             one lane. Measured, layer, one lane / whole warps, us: 109.6 / 107.3 at 32 tokens, 43.7 / 43.4 at 7; I = 1536 238 / 230 at
-//             64, 722 / 657 at 4096; the role alone 37.3 / 36.6 at 1 token. The two decode launches (bm < 128) wait for bytes and keep
-//             the one-lane form: 173.8 / 175.9 at 256 tokens
+//             one lane. Measured, layer, one lane / whole warps, us: 109.8 / 107.7 at 32 tokens, 78.9 / 76.9 at 16, 35.4 / 34.7 at 1, 44.3
+//             / 43.9 at 7 without the shared expert; I = 1536 226 / 216 at 64, 326 / 305 at 200, 752 / 641 at 4096 (spread 5 %). The
+//             two decode launches (bm < 128) wait for bytes and keep the one-lane form: 173.8 / 175.9 at 256 tokens
 //   (the one-launch kernel gemm12_kernel also has warp 6: a second producer for the token-side operand)
 //   warps 2-5 epilogue (bm = 128: a second group, warps 6-9, takes every other unit): tcgen05.ld of the accumulator, then
 //             GEMM1: SwiGLU-OAI (gate and up rows of one tile live in neighbouring lane quarters), MXFP4 requantisation

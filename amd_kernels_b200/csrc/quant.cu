@@ -34,8 +34,8 @@ __global__ void __launch_bounds__(256) quant_mxfp4_kernel(const uint4* __restric
 }
 
 // Row-major quantisation at prefill sizes: one 256-thread CTA per token row, its three 16-byte loads per thread in flight
-// at once; codes [T][3072] and scales [T][192], the bits of quant_mxfp4_kernel. Used ahead of the gather so that a token is
-// read and quantised once, not once per routed slot -- and (Q8) read once for both quantisers.
+// at once; codes [T][3072] and scales [T][192], the bits of quant_mxfp4_kernel but for NaNs (cvt_e2m1x2). Used ahead of the gather so
+// that a token is read and quantised once, not once per routed slot -- and (Q8) read once for both quantisers.
 template <bool Q8>
 __global__ void __launch_bounds__(256) quant_rows_kernel(const uint4* __restrict__ x, uint8_t* __restrict__ codes,
                                                          uint8_t* __restrict__ scales, QuantRow8 q8) {

@@ -147,8 +147,9 @@ __global__ void __launch_bounds__(256) route_topk_kernel(const float* __restrict
 // latencies on ceil(tokens / 8) CTAs) costs nothing beside the quantiser. The first `route_ctas` CTAs route, the others quantise a
 // row each (Q8: for the shared expert too). Above 32 tokens, in 16- and 32-row blocks, this also takes the quantiser out of the gather
 // behind the sort, which then copies a token's codes once per slot instead of quantising its row once per slot.
-// Measured, the routed layer before / after, us: 115.9 / 114.0 at 33 tokens, 154.2 / 150.7 at 64, 172.0 / 168.9 at 128, 176.5 / 174.1 at
-// 256, 205 / 201 at 700, 235 / 230 at 2048, 323 / 320 at 4096; with the shared expert 113.7 / 108.7 at 40, 212.5 / 205.9 at 500.
+// Measured, the routed layer before / after, us: 118.2 / 116.1 at 33 tokens, 143.0 / 140.8 at 64, 170.4 / 168.3 at 128, 176.8 / 173.2 at
+// 256, 202.6 / 199.2 at 700, 233.7 / 230.6 at 2048, within the spread (3 %) at 4096; with the shared expert 113.6 / 108.3 at 40, 210 /
+// 201 at 500. (Where a shared expert on the side stream makes it the slower form: routes_behind_quant in abi.cu.)
 template <int MODE, bool Q8>
 __global__ void __launch_bounds__(256) route_quant_kernel(const float* __restrict__ logits, const float* __restrict__ bias,
                                                           int64_t tokens, int num_experts, float scale, int route_ctas,

@@ -358,8 +358,8 @@ int router_tc_quant(const void* x_bf16, const void* gate_split_bf16, int64_t tok
                     uint8_t* codes4, uint8_t* scales4, uint8_t* codes8, uint8_t* scales8, uint8_t* atoms8, int bm8, int32_t* status,
                     void* stream) {
   if (!codes4 || !scales4 || (codes8 && !scales8 && !atoms8)) return B200MOE_E_ARG;
-  const bool one_pass = tokens >= kOnePassFrom && splits >= 1 && RouterCfg::kKSteps % (2 * splits) == 0 && !misaligned(codes4, 32) && !misaligned(codes8, 32) &&
-                        !misaligned(scales4, 4) && !misaligned(scales8, 4) && !misaligned(atoms8, 16);
+  const bool one_pass = tokens >= kOnePassFrom && splits >= 1 && RouterCfg::kKSteps % (2 * splits) == 0 && !misaligned(codes4, 32) &&
+                        !misaligned(codes8, 32) && !misaligned(scales4, 4) && !misaligned(scales8, 4) && !misaligned(atoms8, 16);
   if (one_pass) {
     const int shift = bm8 == 16 ? 4 : bm8 == 32 ? 5 : bm8 == 64 ? 6 : 7;
     return launch_router_tc<true>(x_bf16, gate_split_bf16, tokens, num_experts, splits, partials,

@@ -7,21 +7,23 @@
 // stages its own 128 token rows and half of the weight rows, 33.5 KB for 512 cycles. The dense blocks leave no odd half inside
 // the work (only the last block of an odd count runs with an idle partner).
 //
-// Unit = (pair of token blocks) x (pair of weight tiles). Two rings, as in gemm1_wide_kernel: 6 stages of codes, and 8 slots of
-// scales that travel ahead of them, so that the MMA thread waits for codes only.
+// Unit = (pair of token blocks) x (pair of weight tiles). Two rings, as in gemm1_wide_kernel: 6 stages of codes (MODE 3: 4), and 8
+// slots of scales that travel ahead of them, so that the MMA warp waits for codes only.
 //
 //   warp 0      code producer (both CTAs): TMA of the CTA's 128 token rows and of its weight tile, counted on the leader's barrier
-//   warp 1      tensor memory (both CTAs); in the leader one thread issues the MMAs for both
-//   warp 2      leader: one thread copies the scales into tensor memory in both CTAs
+//   warp 1      tensor memory (both CTAs); in the leader it issues the MMAs for both, the whole warp around one elected lane
+//   warp 2      leader: copies the scales into tensor memory in both CTAs, in the same way
 //   warp 3      scale producer (both CTAs): the CTA's token scales, the scales of both weight tiles
-//   warps 4-11  epilogue (both CTAs): thread = one token row, 128 accumulator values in registers, the accumulator is handed
-//               back before the arithmetic. MODE 1: SwiGLU-OAI + E4M3 requantisation, thread-local. MODE 2: bf16, through a
-//               strip of shared memory per warp so that eight or sixteen lanes store full lines of a row
-// Measured, one-CTA kernel / pairs, both GEMMs, cold L2: 303 -> 202 us at 16384 tokens, 167 -> 114 at 8191, 93 -> 75 at 4096.
-// Counters at 8192 tokens: tensor pipe 70 % busy in the first GEMM, DRAM 11 %. Cycles of the MMA thread per K-tile at 16384 tokens
-// (512 are tensor time), read from the clock in a build made for it: 690, of which the four MMAs and the looks at the next stage's
-// barriers 350, the stage release 74, waiting for scales 190, for codes 55. Before the looks, with two plain waits, two commits
-// per release and the accumulator handed back by a cluster-scope release, it was 750 and the whole 251 us.
+//   warps 4-11  epilogue (both CTAs): thread = one token row. MODE 1: 128 accumulator values into registers, the accumulator is
+//               handed back, then SwiGLU-OAI + E4M3 requantisation, thread-local. MODE 2 and 3: the values are read in two halves
+//               and rounded to bf16, 64 registers a row, before it is handed back; then through a strip of shared memory per
+//               warp so that eight or sixteen lanes store full lines of a row
+// Measured, one-CTA kernel / pairs, both GEMMs and the scale layout, cold L2: 348 / 192 us at 16384 tokens, 173 / 99 at 8191, 93 / 67
+// at 4096. Counters at 8192 tokens, before the issuing warps elected a lane: tensor pipe 70 % busy in the first GEMM, DRAM 11 %.
+// Cycles of the MMA thread per K-tile at 16384 tokens (512 are tensor time), read from the clock in a build of that form: 690, of
+// which the four MMAs and the looks at the next stage's barriers 350, the stage release 74, waiting for scales 190, for codes 55.
+// Before the looks, with two plain waits, two commits per release and the accumulator handed back by a cluster-scope release, it was
+// 750 and the whole 251 us.
 // MODE 3 is MODE 2 for a call that hands out neither the shared rows nor anything but the sum: its epilogue has the shared value
 // of a (token, column) in a register and adds the four slots in front of it, out = bf16((((0 + s0) + s1) + s2) + s3 + bf16(shared)),
 // the slot reduce's sum bit for bit. So the shared rows are never written nor read back, and the slot reduce's traffic (40 KB a
@@ -30,7 +32,8 @@
 // Measured, second GEMM + slot reduce / MODE 3: 77 + 166 -> 168 us at 16384 tokens (1.05 GB; its bytes alone take 160 at the copy
 // rate), I = 1536 41 + 42 -> 54 at 4096.
 // 12 warps start with 168 registers; the issuing warpgroup drops to 72, the epilogue's rise to 216 (4 x 72 + 8 x 216 = 12 x 168:
-// the exchange must balance inside what the CTA was given at launch).
+// the exchange must balance inside what the CTA was given at launch). MODE 3 spills 24 bytes a thread (stores; 60 bytes of loads),
+// MODE 1 and 2 nothing.
 #include "shared_role.cuh"
 #include "tc_pair.cuh"
 
@@ -60,8 +63,14 @@ struct SharedPairCfg {
   static constexpr int kSfCol = 256;                // tensor memory: 256 accumulator columns, then 8 sets of 16
   static constexpr int kTmemCols = 512;
 };
-static_assert(SharedPairCfg<2>::kSmemBytes <= 227 * 1024, "shared memory");
-static_assert(SharedPairCfg<1>::kSfStages >= SharedPairCfg<1>::kStages, "a scale set is free once the code stage is");
+template <int MODE>
+constexpr bool shared_pair_fits() {
+  using C = SharedPairCfg<MODE>;
+  static_assert(C::kSmemBytes <= 227 * 1024, "shared memory");
+  static_assert(C::kSfStages >= C::kStages, "a scale set is free once the code stage is");
+  return true;
+}
+static_assert(shared_pair_fits<1>() && shared_pair_fits<2>() && shared_pair_fits<3>());
 
 __device__ __forceinline__ void tc_mma_mxf8_pair(uint32_t d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t sfa,
                                                  uint32_t sfb, uint32_t accumulate) {
@@ -224,7 +233,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SharedPairCfg<MODE>:
         bool ok = true, landed = false, free_set = false;
         for (int u = cluster; u < total && ok; u += n_clusters) {
           for (int kt = 0; kt < C::kTilesK; ++kt) {
-            // set j was last read by the MMAs 8 K-tiles back: complete once those 6 K-tiles back are
+            // set j was last read by the MMAs 8 K-tiles back: complete once those that read stage s, kStages back, are
             if (!__all_sync(0xffffffffu, (landed || mbar_wait(smem_u32(&bar_sfull[j]), sph, abort_v, status)) &&
                                              (free_set || mbar_wait(smem_u32(&bar_empty[s]), ph, abort_v, status)))) {
               ok = false;

@@ -490,10 +490,12 @@ extern "C" int b200moe_shared_quant_rows(const void* x_bf16, int64_t tokens, uin
 }
 
 namespace b200moe {
-// From this many blocks of 128 tokens on both GEMMs run on CTA pairs (shared_pair.cu). Measured, both GEMMs and the scale layout,
-// one-CTA kernel / pairs, us: 38 / 42 at 777 tokens, 40 / 42 at 1024, 44 / 44 at 1400, 60 / 46 at 1800, 93 / 75 at 4096, 167 / 114
-// at 8191, 303 / 202 at 16384. Below, a GEMM1 unit per pair leaves most SMs idle (24 pairs busy at 1024 tokens) and one unit's
-// chain of 48 K-tiles is the time; the one-CTA kernel has four times the units.
+// From this many blocks of 128 tokens on both GEMMs run on CTA pairs (shared_pair.cu). Measured, both GEMMs and the scale layout alone,
+// one-CTA kernel / pairs, us: I = 768 38 / 38 at 777 tokens, 40 / 38 at 1024, 42 / 40 at 1400, 44 / 40 at 1536, 58 / 42 at 1664, 62 / 42
+// at 2048, 93 / 67 at 4096, 173 / 99 at 8191, 348 / 192 at 16384; I = 1536 54 / 44 at 777, 60 / 46 at 1400, 77 / 63 at 1664, 148 / 99 at
+// 4096. (The line is where the two met before the issuing warps elected a lane, 44 / 44 at 1400; it has not been drawn again since, so
+// alone pairs are ahead from about 1000 tokens on.) At few blocks a GEMM1 unit per pair leaves most SMs idle (24 pairs busy at 1024
+// tokens) and one unit's chain of 48 K-tiles is the time; the one-CTA kernel has four times the units.
 constexpr int kSharedPairBlocks = 12;
 
 static bool on_pairs(const SharedWorkspace& ws) {
@@ -516,10 +518,11 @@ int shared_gemm1(const uint8_t* w13t, const uint8_t* codes8, int64_t code_rows, 
 }
 
 // From this many blocks of 128 tokens on the second GEMM adds the routed slots itself (shared_pair.cu, MODE 3). Measured, the whole
-// layer with the router inside, slot reduce as a launch of its own behind the side stream / this, us: I = 768 267 / 267 at 1500 tokens,
-// 296 / 300 at 2048, 337 / 329 at 2500, 367 / 354 at 3072, 443 / 413 at 4096, 688 / 671 at 8192, 1289 / 1236 at 16384; I = 1536 477 /
-// 487 at 1500, 535 / 528 at 2048, 637 / 624 at 3072. Below, a unit of 256 x 256 per pair leaves an uneven last round (192 units for
-// 74 pairs at 2048), and the side stream hides the second GEMM.
+// layer with the router inside, slot reduce as a launch of its own behind the side stream / this, us: I = 768 270 / 276 at 13 blocks,
+// 281 / 287 at 14, 291 / 294 at 16, 301 / 298 at 17, 315 / 289 at 18, 334 / 312 at 20, 364 / 339 at 24, 438 / 403 at 32, 705 / 652 at
+// 64, 1290 / 1186 at 128; I = 1536 457 / 459 at 13, 486 / 490 at 16, 499 / 497 at 17, 526 / 506 at 18, 555 / 529 at 20, 598 / 564 at 24,
+// 701 / 672 at 32. Below 18 the side stream hides the second GEMM and the pairs' last round is uneven (192 units for 74 pairs at 16
+// blocks); from 18 on the round trip of the shared rows and the reduce behind both costs more than an uneven round does.
 constexpr int kSumSlotsBlocks = 18;
 static_assert(kSumSlotsBlocks >= kSharedPairBlocks, "the sum exists on pairs only");
 

@@ -517,7 +517,8 @@ def router_gemm_quant(x: torch.Tensor, gate: torch.Tensor, shared: bool = False,
     """The split-K logit partials of ``router_gemm_partials``, the row-major MXFP4 operands of ``mxfp4_quant`` and, with
     ``shared``, the row-major MXFP8 operands of ``shared_quant_rows`` (else None), all with those kernels' bits (reference
     router_mxfp4_mxfp8_quant_row_scales.py). Below 128 tokens (or without ``split``) ONE kernel makes one pass over x; from
-    128 tokens on the router runs on the tensor cores (``split`` = ``split_gate(gate)``) with the quantisers beside it."""
+    128 tokens on the router runs on the tensor cores (``split`` = ``split_gate(gate)``) and the quantisers are launches of their own.
+    (The layer call and ``prepare_mxfp4_moe`` have a tensor-core kernel from 257 tokens on that quantises as well.)"""
     if x.ndim != 2 or x.shape[1] != H or x.dtype != torch.bfloat16 or not x.is_contiguous():
         raise ValueError("expected contiguous BF16 [M,6144]")
     if gate.dtype != torch.float32 or gate.ndim != 2 or gate.shape[1] != H or not gate.is_contiguous():
@@ -590,7 +591,8 @@ def _result_flags(sw, slots, shared):
 
 # Token count above which the shared expert's GEMMs are launches of their own, on the side stream: below, it is a role of a routed
 # launch (37 against 161 us for the layer at 1 token, 105 against 237 at 32, much of it host time). The side stream's work starts
-# behind the quantisation of x, which serves both experts in one pass, and is joined inside the C call.
+# behind the quantisation of x, which serves both experts in one pass, and is joined inside the C call (in reduced mode from 2177
+# tokens on it is the first GEMM only).
 SIDE_STREAM_FROM = 512
 
 
@@ -627,7 +629,9 @@ def mxfp4_moe(x, w, *, return_partials=False, router_logits=None):
     returns (slots BF16 [M, 4, H], shared BF16 [M, H]); without ``w.shared_weights`` the shared term is absent (None).
     ``router_logits`` fp32 [M, E] skips the router GEMM. The whole layer is one C-ABI call (``b200moe_layer``) on the current
     stream: up to 512 tokens the shared expert runs on SMs of its own inside the routed experts' launches; above, its GEMMs run
-    on the device's side stream, which the current stream joins before the reduce. Scratch and outputs come from ``torch.empty``."""
+    on the device's side stream, which the current stream joins before the reduce. In reduced mode from 2177 tokens on only the
+    first does; the second follows GEMM2 on the current stream and adds the slots, so that no reduce is left. Scratch and outputs
+    come from ``torch.empty``."""
     if not isinstance(x, torch.Tensor):
         from .prepared_input import MoeInput, MoeInputCompact, mxfp4_moe_prepared
         if not isinstance(x, (MoeInput, MoeInputCompact)):

@@ -89,7 +89,8 @@ int b200moe_router_gemm_tc(const void* x_bf16, const void* gate_split_bf16, int6
  * the routed experts' MXFP4 operands (codes4 [T][3072], scales4 [T][192], the bits of b200moe_quant_mxfp4) and, when
  * codes8 / scales8 are given, the shared expert's MXFP8 operands ([T][6144], [T][192], the bits of
  * b200moe_shared_quant_rows) (MOE/router_mxfp4_quant_line_layout.py:48-400,
- * MOE/router_mxfp4_mxfp8_quant_row_scales.py router_mxfp4_mxfp8_quant_row_scales). */
+ * MOE/router_mxfp4_mxfp8_quant_row_scales.py router_mxfp4_mxfp8_quant_row_scales). This is the CUDA-core form at every size; inside
+ * b200moe_layer and b200moe_prepare it serves fewer than 128 tokens, and more where gate_split is null. */
 int b200moe_router_gemm_quant(const void* x_bf16, const float* gate, int64_t tokens, int num_experts, int splits,
                               float* partials, uint8_t* codes4, uint8_t* scales4, uint8_t* codes8, uint8_t* scales8,
                               void* stream);
@@ -104,7 +105,9 @@ int b200moe_route_topk(const float* partials, int64_t stride_t, int64_t stride_s
                        void* stream);
 
 /* Activation quantisation bf16 [T][K] -> codes [T][K/2], scales [T][K/32], row-major, bit-exact "Quark even" rule
- * (MOE/quant.py:32-106 mxfp4_quant; oracle MOE/reference.py:32-46). K is a multiple of 256. */
+ * (MOE/quant.py:32-106 mxfp4_quant; oracle MOE/reference.py:32-46). K is a multiple of 256. A NaN does not count in its block's
+ * maximum; its code is 0 with the NaN's sign up to 63 rows or with K other than 6144, and 7, the largest, from 64 rows of 6144 on and
+ * in every layer call. */
 int b200moe_quant_mxfp4(const void* x_bf16, int64_t tokens, int k, uint8_t* codes, uint8_t* scales, void* stream);
 
 /* Routing sort (MOE/common/sort.py:19-65 SortBuffers; MOE/sort_a16w4.py:217-242 moe_sort_a16w4;
@@ -410,7 +413,8 @@ int b200moe_forward_x(const b200moe_weights* w, const void* x_bf16, int64_t toke
 /* The whole layer in one call, with or without the shared expert (MOE/chain.py:127-197 mxfp4_moe; the shared expert runs
  * beside the routed experts inside the same launches up to 512 tokens; above, its two GEMMs are launches of their own, on
  * side_stream when one is given: they start behind the input's quantisation and are joined before the reduce, or before the call
- * returns. side_stream, another stream of the same device, may be null). logits fp32 [T][num_experts], or null: the router
+ * returns. Where shared_out is null, from 2177 tokens on, only the first is there: the second runs on stream behind GEMM2, joined
+ * to the first, and adds the slots itself. side_stream, another stream of the same device, may be null). logits fp32 [T][num_experts], or null: the router
  * runs inside the call (w->gate). shared may be null.
  * slots [T][4][6144], shared_out [T][6144] and out [T][6144] are bf16; a null slots (shared_out) means that the caller does
  * not want it: it then lives in the workspace, and out must be given. Same bits as the separate calls.
